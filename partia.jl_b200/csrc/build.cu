@@ -324,7 +324,8 @@ __global__ void k_span_roots(int64_t n, const int32_t* parent, const int32_t* rl
 template <class T>
 __global__ void k_pack_leaves(int64_t n, const T* x, const T* y, const T* z, const T* h, const T* m, const T* rho,
                               const int32_t* sfirst, float4* leaf4, float* mrho, float* mf, float4* leafK,
-                              float2* spanb, float sig) {
+                              float2* spanb, double2* d0, double2* d1, double2* d2, double sigd) {
+    const float sig = (float)sigd;
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     double ax = 0, ay = 0, az = 0;
@@ -340,9 +341,15 @@ __global__ void k_pack_leaves(int64_t n, const T* x, const T* y, const T* z, con
         r = make_float4((float)x[i], (float)y[i], (float)z[i], (float)h[i]);
     }
     leaf4[i] = r;
-    const float mr = (float)((double)m[i] / (double)rho[i]);
+    const double mrd = (double)m[i] / (double)rho[i];
+    const float mr = (float)mrd;
     mrho[i] = mr;
     mf[i] = (float)m[i];
+    // the same factors for the double pair sums
+    const double ihd = 1.0 / (double)h[i];
+    d0[i] = make_double2((double)x[i], (double)y[i]);
+    d1[i] = make_double2((double)z[i], ihd);
+    d2[i] = make_double2(sigd * ihd * ihd * ihd, mrd);
     // kernel-weight factors of the float pair bodies
     const float ih = 1.f / r.w;
     const float s3 = sig * ih * ih * ih;  // sig = the kernel's 3D norm
@@ -382,14 +389,17 @@ static int pack_columns(psb_ctx* c, cudaStream_t s) {
     return PSB_OK;
 }
 
-// The mass-dependent parts of the leaf records (m/rho, m and leafK.w), with
+// The mass-dependent parts of the leaf records (m/rho, m, leafK.w and leafD[2].y), with
 // k_pack_leaves' arithmetic: a values-only update leaves them as a full
 // build over the same particles would.
 template <class T>
-__global__ void k_pack_values(int64_t n, const T* m, const T* rho, float* mrho, float* mf, float4* leafK) {
+__global__ void k_pack_values(int64_t n, const T* m, const T* rho, float* mrho, float* mf, float4* leafK,
+                              double2* d2) {
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    const float mr = (float)((double)m[i] / (double)rho[i]);
+    const double mrd = (double)m[i] / (double)rho[i];
+    const float mr = (float)mrd;
+    d2[i].y = mrd;
     mrho[i] = mr;
     mf[i] = (float)m[i];
     reinterpret_cast<float*>(leafK + i)[3] = mr;
@@ -502,6 +512,7 @@ static int build_typed(psb_ctx* c) {
     PSB_CUDA_TRY(c, dgrow_t(c, &c->mf, sizeof(float) * n), "cudaMalloc mf");
     PSB_CUDA_TRY(c, dgrow_t(c, &c->leafK, sizeof(float4) * n), "cudaMalloc leafK");
     PSB_CUDA_TRY(c, dgrow_t(c, &c->spanb, sizeof(float2) * n), "cudaMalloc span bounds");
+    for (double2*& d : c->leafD) PSB_CUDA_TRY(c, dgrow_t(c, &d, sizeof(double2) * n), "cudaMalloc double leaf records");
     PSB_CUDA_TRY(c, cudaMemsetAsync(c->spanb, 0, sizeof(float2) * n, s), "memset span bounds");
     if (nint > 0)
         k_pack_nodes<T><<<grid_for(nint), BT, 0, s>>>(nint, (const T*)c->nmin[0], (const T*)c->nmin[1],
@@ -512,7 +523,8 @@ static int build_typed(psb_ctx* c) {
     k_span_roots<<<grid_for(n), BT, 0, s>>>(n, c->parent, c->range_lo, c->range_hi, sfirst);
     k_pack_leaves<T><<<grid_for(n), BT, 0, s>>>(n, (const T*)c->x, (const T*)c->y, (const T*)c->z, (const T*)c->h,
                                                 (const T*)c->m, (const T*)c->rho, sfirst, c->leaf4, c->mrho, c->mf,
-                                                c->leafK, c->spanb, (float)kern_norm3(c->kern));
+                                                c->leafK, c->spanb, c->leafD[0], c->leafD[1], c->leafD[2],
+                                                kern_norm3(c->kern));
     if (sizeof(T) == 8 && c->ncol > 0) {
         const int rc = pack_columns(c, s);
         if (rc != PSB_OK) return rc;
@@ -520,8 +532,9 @@ static int build_typed(psb_ctx* c) {
     PSB_CUDA_TRY(c, cudaGetLastError(), "pack kernels");
 
     // bbox to host (used for sample ordering and float error bounds)
-    T hb[6];
+    T hb[6], hmax = T(0);
     PSB_CUDA_TRY(c, cudaMemcpyAsync(hb, bb, es * 6, cudaMemcpyDeviceToHost, s), "bbox copy");
+    PSB_CUDA_TRY(c, cudaMemcpyAsync(&hmax, nint > 0 ? c->nscale : c->h, es, cudaMemcpyDeviceToHost, s), "largest h copy");
     unsigned herr = 0;
     PSB_CUDA_TRY(c, cudaMemcpyAsync(&herr, c->d_err, sizeof(unsigned), cudaMemcpyDeviceToHost, s), "error word copy");
     PSB_CUDA_TRY(c, cudaStreamSynchronize(s), "build synchronize");
@@ -539,6 +552,13 @@ static int build_typed(psb_ctx* c) {
         c->bbox[k] = (double)hb[k];
         maxabs = std::max(maxabs, std::fabs((double)hb[k]));
     }
+    // The float band tests carry absolute floors of 1e-18 (lengths) and 1e-36
+    // (squares), so they are exact supersets as long as squares of extents and
+    // radii neither overflow a float nor all lie below those floors; outside
+    // this range the single kernel interpolates.
+    double ext = 0;
+    for (int d = 0; d < 3; ++d) ext = std::max(ext, (double)hb[3 + d] - (double)hb[d]);
+    c->band_ok = maxabs <= 1e15 && ext >= 1e-12 && (double)hmax <= 1e15;
     // |float(v) - v| <= 2^-24 |v|; the node tests allow twice that
     c->coord_err = (float)(maxabs * 1.1920928955078125e-07);
     c->built = true;
@@ -549,7 +569,8 @@ template <class T>
 static int repack_values_typed(psb_ctx* c) {
     const int64_t n = c->n;
     cudaStream_t s = c->stream;
-    k_pack_values<T><<<grid_for(n), BT, 0, s>>>(n, (const T*)c->m, (const T*)c->rho, c->mrho, c->mf, c->leafK);
+    k_pack_values<T><<<grid_for(n), BT, 0, s>>>(n, (const T*)c->m, (const T*)c->rho, c->mrho, c->mf, c->leafK,
+                                              c->leafD[2]);
     if (sizeof(T) == 8 && c->ncol > 0) {
         const int rc = pack_columns(c, s);
         if (rc != PSB_OK) return rc;

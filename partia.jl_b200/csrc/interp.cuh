@@ -253,12 +253,61 @@ __device__ __forceinline__ void f32c_pair_weights(int kern, float Kf, float qe, 
     csum = __fmul_rn(csum, invr);
 }
 
-template <class C> __device__ __forceinline__ C m4_f(C q) {
-    C a = C(2) - q, b = C(1) - q;
-    C fo = C(0.25) * a * a * a;
-    C fi = fo - b * b * b;
-    return (q < C(1)) ? fi : ((q < C(2)) ? fo : C(0));
+// The FP64 weights of one pair (both pair-sum kernels, double and float
+// particles): d the separation, ia, sa3 the sample's 1/h and sigma/h^3, ib,
+// sb3 the particle's.  Returns W and the gradient factor c (grad W = c d).
+// One rsqrt gives 1/r and r, and the particle's 1/h, sigma/h^3 and m/rho come
+// from its records (leafD), so a pair does no division.
+template <int ST, int KF>
+__device__ __forceinline__ void f64_pair_weights(int kern, double dx, double dy, double dz, double ia, double sa3,
+                                                 double ib, double sb3, double& W, double& c) {
+    const double d2 = __fma_rn(dz, dz, __fma_rn(dy, dy, __dmul_rn(dx, dx)));
+    const double ir = d2 > 0.0 ? rsqrt(d2) : 0.0;
+    const double r = __dmul_rn(d2, ir);
+    auto one = [&](double ih, double s3, double& w, double& g) {
+        double f, dr;
+        if constexpr (KF == 0) m4_fdr_f64(__dmul_rn(r, ih), ih, ir, f, dr);
+        else kern_fdr_f64(kern, __dmul_rn(r, ih), ih, ir, f, dr);
+        w = __dmul_rn(s3, f);
+        g = __dmul_rn(__dmul_rn(s3, ih), dr);
+    };
+    if (ST == ST_GATHER) {
+        one(ia, sa3, W, c);
+    } else if (ST == ST_SCATTER) {
+        one(ib, sb3, W, c);
+    } else {
+        double wa, ga, wb, gb;
+        one(ia, sa3, wa, ga);
+        one(ib, sb3, wb, gb);
+        W = __dmul_rn(0.5, __dadd_rn(wa, wb));
+        c = __dmul_rn(0.5, __dadd_rn(ga, gb));
+    }
 }
+
+// The same in float for float particles (FP32C): d2 the squared separation,
+// sa4 = sigma/h^4 of the sample, ib and sb3 from the particle's record (leafK).
+template <int ST, int KF>
+__device__ __forceinline__ void f32_pair_weights(int kern, float d2, float ia, float sa3, float sa4, float ib,
+                                                 float sb3, float& W, float& c) {
+    const float r = sqrtf(d2);
+    const float ir = (d2 > 0.f) ? 1.f / r : 0.f;
+    W = 0.f;
+    c = 0.f;
+    if (ST != ST_SCATTER) {
+        float f, df;
+        kfdf<KF, float>(kern, __fmul_rn(r, ia), f, df);
+        W = __fmul_rn(sa3, f);
+        c = __fmul_rn(__fmul_rn(sa4, df), ir);
+    }
+    if (ST != ST_GATHER) {
+        float f, df;
+        kfdf<KF, float>(kern, __fmul_rn(r, ib), f, df);
+        const float Wb = __fmul_rn(sb3, f), cb = __fmul_rn(__fmul_rn(__fmul_rn(sb3, ib), df), ir);
+        if (ST == ST_SCATTER) { W = Wb; c = cb; }
+        else { W = __fmul_rn(0.5f, __fadd_rn(W, Wb)); c = __fmul_rn(0.5f, __fadd_rn(c, cb)); }
+    }
+}
+
 template <class C> __device__ __forceinline__ C inv_pi();
 template <> __device__ __forceinline__ double inv_pi<double>() { return 0.31830988618379067154; }
 template <> __device__ __forceinline__ float inv_pi<float>() { return 0.318309886183790671538f; }
@@ -294,9 +343,15 @@ __device__ __forceinline__ float span_shift(const T* col, int64_t lo, int64_t fi
 struct PlainD {
     double s;
     __device__ __forceinline__ void zero() { s = 0.0; }
-    __device__ __forceinline__ void add(double v) { s += v; }
+    __device__ __forceinline__ void add(double v) { s = __dadd_rn(s, v); }
     __device__ __forceinline__ double get() const { return s; }
 };
+// products and accumulated products of the pair sums, with their roundings
+// spelled out (one fused step in double, a rounded product in float)
+__device__ __forceinline__ double acc_mul(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ float acc_mul(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ void acc_mac(PlainD& A, double a, double b) { A.s = __fma_rn(a, b, A.s); }
+__device__ __forceinline__ void acc_mac(KahanF& A, float a, float b) { A.add(__fmul_rn(a, b)); }
 
 // ---------------------------------------------------------------------------
 // Warp-cooperative stackless DFS over left + escape links

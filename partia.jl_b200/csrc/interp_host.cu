@@ -12,6 +12,7 @@ template <class T> TreeView<T> tree_view(psb_ctx* c) {
     v.n = c->n;
     v.root = c->root;
     v.left = c->left;
+    v.right = c->right;
     v.escape = c->escape;
     v.range_lo = c->range_lo;
     v.range_hi = c->range_hi;
@@ -30,6 +31,7 @@ template <class T> TreeView<T> tree_view(psb_ctx* c) {
     v.ncol = c->ncol;
     v.node_lo = c->node_lo; v.node_hi = c->node_hi; v.leaf4 = c->leaf4;
     v.mrho = c->mrho; v.mf = c->mf; v.leafK = c->leafK; v.spanb = c->spanb;
+    for (int d = 0; d < 3; ++d) v.leafD[d] = c->leafD[d];
     v.coord_err = c->coord_err;
     v.kern = (int)c->kern;
     v.Kd = kern_support(v.kern);
@@ -106,9 +108,11 @@ static float ms_between(cudaEvent_t a, cudaEvent_t b) {
 }
 
 // Two-kernel point path over batches of tiles: k_collect writes the pair
-// lists of a batch, k_bodies sums them, and k_points takes the tiles whose
-// lists overflowed.  A batch holds at most SPLIT_BATCH tiles, which bounds the
-// list memory at SPLIT_BATCH * RCAP * 32 * 20 bytes (640 MiB) per stream.
+// lists of a batch, k_bodies sums them, k_fold adds up the samples of several
+// parts, and k_points takes the tiles that found the chunk pool exhausted.  A
+// batch holds at most SPLIT_BATCH tiles, which bounds the lists' memory at
+// SPLIT_BATCH * RCAP * 32 * 20 bytes (640 MiB) per stream, and the pool's at
+// about the same (M5, M6) or a quarter of it.
 //
 // A direct call (multi_stream) of at least two batches' worth of tiles
 // spreads its batches over up to SPLIT_STREAMS streams (the context stream and
@@ -120,8 +124,8 @@ static float ms_between(cudaEvent_t a, cudaEvent_t b) {
 constexpr int64_t SPLIT_BATCH = 32768;
 constexpr int SPLIT_STREAMS = 4;
 template <class T>
-static int run_split(psb_ctx* c, Args<T>& A, int prec, int st, int* launches, int slot_off = 0,
-                     bool multi_stream = true) {
+static int run_split(psb_ctx* c, Args<T>& A, int prec, int st, int* launches, int what = WHAT_INTERP,
+                     int slot_off = 0, bool multi_stream = true) {
     cudaStream_t s = c->stream;
     const int64_t nt = A.src.ntiles;
     int nsets = 1;
@@ -144,56 +148,89 @@ static int run_split(psb_ctx* c, Args<T>& A, int prec, int st, int* launches, in
         }
     }
     struct Lists {
-        float4* ent4; uint32_t* emask; float* eshift; uint8_t* cnt; void* hab; unsigned* ovf_count; int32_t* ovf_tiles;
+        float4* ent4; uint32_t* emask; float* eshift; uint8_t* cnt; void* hab; int32_t* head; unsigned* ctr;
+        int32_t* ovf_tiles; uint32_t* own; int32_t* next; uint8_t* ccnt; double* part; uint32_t* hlist; uint32_t* mlist;
     };
     // FP32C sums of double inputs take per-entry column shifts for the kernels
     // other than M4 (span_shift; slots 80-86)
-    const bool shifts = sizeof(T) == 8 && prec == PREC_FP32C && A.rec.kc > 0 && c->kern != PSB_KERNEL_M4;
+    const int kc = A.rec.kc;
+    const bool shifts = sizeof(T) == 8 && prec == PREC_FP32C && kc > 0 && c->kern != PSB_KERNEL_M4;
+    const int kcl = kc <= 1 ? 1 : (kc <= 2 ? 2 : (kc <= 4 ? 4 : 8));
+    const int nf = what == WHAT_DENSITY ? 1 : 8 + 4 * kcl;
+    const bool seq = sizeof(T) == 8 && prec == PREC_FP32C;  // samples of several parts go to k_seq
+    // The chunk pool: a quarter of a chunk per sample for the kernels of support 2 h
+    // (neighbourhoods of more than RCAP spans are rare there), one per
+    // sample for M5 and M6, whose ordinary samples often take two parts.
+    const int64_t lanes = 32 * B;
+    // At least 65536 for calls with a few large neighbourhoods, but no more than
+    // the samples of a small call can fill (a chunk holds RCAP spans of the tree).
+    const int64_t most = std::min<int64_t>(lanes, A.src.ns) * (c->n / 256 + 2);
+    const unsigned ncap = (unsigned)std::min<int64_t>(std::max<int64_t>(65536, A.tv.Kd > 2.0 ? lanes : lanes / 4), most);
+    constexpr unsigned HCAP = 4096;  // samples of a batch for k_heavy (the rest stay in their tiles' walks)
     Lists ls[SPLIT_STREAMS];
     for (int k = 0; k < nsets; ++k) {
         // scratch slots 16-20 (+ slot_off), 48-52, 37-41 and 42-46 (clear of the
-        // build, sort, sample-order and adjoint slots)
+        // build, sort, sample-order and adjoint slots), and 80-86 and 96-102
         static const int set_off[SPLIT_STREAMS] = {0, 32, 21, 26};
         const int so = slot_off + set_off[k];
-        ls[k].ent4 = (float4*)scratch(c, 16 + so, sizeof(float4) * (size_t)RCAP * 32 * B);
-        ls[k].emask = (uint32_t*)scratch(c, 20 + so, sizeof(uint32_t) * (size_t)RCAP * 32 * B);
+        const int es_slot = slot_off == 0 ? k : (slot_off == 32 ? 4 : (slot_off == 14 ? 5 : 6));
+        const size_t nent = (size_t)RCAP * 32 * B + (size_t)RCAP * ncap;
+        ls[k].ent4 = (float4*)scratch(c, 16 + so, sizeof(float4) * nent);
+        ls[k].emask = (uint32_t*)scratch(c, 20 + so, sizeof(uint32_t) * nent);
         ls[k].eshift = nullptr;
         if (shifts) {
-            const int es_slot = 80 + (slot_off == 0 ? k : (slot_off == 32 ? 4 : (slot_off == 14 ? 5 : 6)));
-            ls[k].eshift = (float*)scratch(c, es_slot, sizeof(float) * (size_t)RCAP * 32 * B * A.rec.kc);
+            ls[k].eshift = (float*)scratch(c, 80 + es_slot, sizeof(float) * nent * kc);
             if (!ls[k].eshift) return fail(c, PSB_ENOMEM, "scratch allocation failed (pair-list shifts)");
         }
-        ls[k].cnt = (uint8_t*)scratch(c, 17 + so, (size_t)32 * B);
+        char* cnt = (char*)scratch(c, 17 + so, (size_t)(1 + sizeof(int32_t)) * lanes);
         ls[k].hab = scratch(c, 18 + so, sizeof(double) * 32 * (size_t)B);
-        char* ovf = (char*)scratch(c, 19 + so, 256 + sizeof(int32_t) * (size_t)B);
-        if (!ls[k].ent4 || !ls[k].emask || !ls[k].cnt || !ls[k].hab || !ovf)
+        char* ovf = (char*)scratch(c, 19 + so, 256 + sizeof(int32_t) * ((size_t)B * 33 + HCAP));
+        char* pool = (char*)scratch(c, 96 + es_slot, (size_t)ncap * ((seq ? sizeof(uint32_t) : sizeof(double) * 2 * nf) + 2 * sizeof(int32_t) + 1));
+        if (!ls[k].ent4 || !ls[k].emask || !cnt || !ls[k].hab || !ovf || !pool)
             return fail(c, PSB_ENOMEM, "scratch allocation failed (pair lists)");
-        ls[k].ovf_count = (unsigned*)ovf;
-        ls[k].ovf_tiles = (int32_t*)(ovf + 256);
+        ls[k].head = (int32_t*)cnt;
+        ls[k].cnt = (uint8_t*)(cnt + sizeof(int32_t) * lanes);
+        ls[k].ctr = (unsigned*)ovf;
+        ls[k].hlist = (uint32_t*)(ovf + 256);
+        ls[k].ovf_tiles = (int32_t*)(ls[k].hlist + HCAP);
+        ls[k].part = seq ? nullptr : (double*)pool;
+        ls[k].mlist = seq ? (uint32_t*)pool : nullptr;
+        ls[k].own = (uint32_t*)(pool + (seq ? sizeof(uint32_t) : sizeof(double) * 2 * nf) * (size_t)ncap);
+        ls[k].next = (int32_t*)(ls[k].own + ncap);
+        ls[k].ccnt = (uint8_t*)(ls[k].next + ncap);
     }
-    // The adjoint's cotangent pass (double particles) collects its pair lists
-    // with the FP32C walk: float tests with the exact double test for every
-    // undecided pair give the same pairs in the same order as the double
-    // walk, at about half its cost; the sums stay in double.
-    const int cprec = (sizeof(T) == 8 && A.lam) ? PREC_FP32C : prec;
+    A.sp.ncap = ncap;
+    A.sp.ebase = (uint32_t)((int64_t)RCAP * 32 * B);
+    A.sp.fp64 = prec == PREC_FP64 ? 1 : 0;
+    // A warp walks for 32 samples where that leaves enough warps to fill the
+    // GPU (4096 of its 7104), for fewer in smaller calls: a call of some
+    // probe points is as long as its longest walk.
+    A.sp.lspt = 5;
+    while (A.sp.lspt > 0 && (nt << (5 - A.sp.lspt)) < 4096) --A.sp.lspt;
     int64_t bi = 0;
     for (int64_t t0 = 0; t0 < nt; t0 += B, ++bi) {
         const int k = (int)(bi % nsets);
         const cudaStream_t sk = ss[k];
         const int64_t nb = std::min<int64_t>(B, nt - t0);
-        PSB_CUDA_TRY(c, cudaMemsetAsync(ls[k].ovf_count, 0, sizeof(unsigned), sk), "memset overflow count");
+        PSB_CUDA_TRY(c, cudaMemsetAsync(ls[k].ctr, 0, 4 * sizeof(unsigned), sk), "memset list counters");
         A.sp.ent4 = ls[k].ent4; A.sp.emask = ls[k].emask; A.sp.cnt = ls[k].cnt; A.sp.ha = ls[k].hab;
-        A.sp.eshift = ls[k].eshift;
-        A.sp.ovf_tiles = ls[k].ovf_tiles; A.sp.ovf_count = ls[k].ovf_count;
+        A.sp.eshift = ls[k].eshift; A.sp.head = ls[k].head;
+        A.sp.ovf_tiles = ls[k].ovf_tiles; A.sp.ovf_count = ls[k].ctr; A.sp.top = ls[k].ctr + 1;
+        A.sp.own = ls[k].own; A.sp.next = ls[k].next; A.sp.ccnt = ls[k].ccnt; A.sp.part = ls[k].part;
+        A.sp.hcount = ls[k].ctr + 2; A.sp.hlist = ls[k].hlist; A.sp.hcap = HCAP;
+        A.sp.mcount = ls[k].ctr + 3; A.sp.mlist = ls[k].mlist;
         A.sp.tile0 = t0; A.sp.ntiles = nb;
-        PSB_CUDA_TRY(c, launch_split(A, cprec, st, A.rec.kc, false, sk), "pair-list kernel launch");
-        PSB_CUDA_TRY(c, launch_split(A, prec, st, A.rec.kc, true, sk), "pair-sum kernel launch");
+        const bool dens = what == WHAT_DENSITY;
+        PSB_CUDA_TRY(c, launch_split(A, prec, st, kc, SPLIT_WALK, sk), "pair-list kernel launch");
+        PSB_CUDA_TRY(c, launch_split(A, prec, st, kc, SPLIT_HEAVY, sk), "heavy-sample kernel launch");
+        PSB_CUDA_TRY(c, launch_split(A, prec, st, kc, dens ? SPLIT_DENSITY : SPLIT_FIELDS, sk), "pair-sum kernel launch");
+        PSB_CUDA_TRY(c, launch_split(A, prec, st, kc, dens ? SPLIT_FOLD_DENSITY : SPLIT_FOLD, sk), "fold kernel launch");
         Args<T> F = A;
         F.tile_list = ls[k].ovf_tiles;
-        F.tile_count = ls[k].ovf_count;
+        F.tile_count = ls[k].ctr;
         F.src.ntiles = nb;  // grid of the list pass: at most nb tiles
-        PSB_CUDA_TRY(c, launch_points<T>(F, prec, st, A.rec.kc, WHAT_INTERP, sk), "overflow pass launch");
-        *launches += 3;
+        PSB_CUDA_TRY(c, launch_points<T>(F, prec, st, A.rec.kc, what, sk), "overflow pass launch");
+        *launches += 5;
     }
     for (int k = 1; k < nsets; ++k) {  // the call's later work on s follows every stream
         PSB_CUDA_TRY(c, cudaEventRecord(c->sev[k], ss[k]), "event");
@@ -396,9 +433,9 @@ static int run_typed(psb_ctx* c, const SampleReq& rq, int hmode, const void* hs,
 
     // ---- launch ----
     if (ns > 0) {
-        const bool split = what == WHAT_INTERP && !rq.line && !(flags & PSB_FLAG_SINGLE_KERNEL);
+        const bool split = what != WHAT_DIGEST && !rq.line && c->band_ok && !(flags & PSB_FLAG_SINGLE_KERNEL);
         if (split) {
-            int rc = run_split(c, A, prec, st, &launches);
+            int rc = run_split(c, A, prec, st, &launches, what);
             if (rc) return rc;
         } else {
             if (rq.line && A.src.kind == SRC_BEAM && A.src.ntiles >= 4096) {  // heavy tiles first
@@ -613,9 +650,9 @@ static int run_points_pipelined(psb_ctx* c, const SampleReq& rq, int hmode, cons
             PSB_CUDA_TRY(c, radix_sort_pairs(codes[b], idx[b], cn, c, sort_slot[b], &launches, false, SAMPLE_KEY_BITS), "sample sort");
             S.order = idx[b];
         }
-        const bool split = !(flags & PSB_FLAG_SINGLE_KERNEL);
+        const bool split = c->band_ok && !(flags & PSB_FLAG_SINGLE_KERNEL);
         if (split) {
-            rc = run_split(c, A, prec, st, &launches, list_off[b], false);  // chunks already overlap
+            rc = run_split(c, A, prec, st, &launches, WHAT_INTERP, list_off[b], false);  // chunks already overlap
             if (rc) return rc;
         } else {
             PSB_CUDA_TRY(c, launch_points<T>(A, prec, st, A.rec.kc, WHAT_INTERP, sc_), "interpolation kernel launch");

@@ -29,23 +29,59 @@ namespace psb {
 // kernel writes, for every sample, its accepted leaves as one entry per span
 // (the span's first leaf, a mask over its <= 32 leaves, and the sample's
 // position relative to that first leaf, rounded to float from double), and
-// its smoothing length; the body kernel reads them.  A tile with a sample of
-// more than RCAP entries is marked (cnt = 0xFF for all its lanes) and listed
-// in ovf_tiles; the single-kernel path computes those tiles instead.
+// its smoothing length; the body kernel reads them.
+//
+// A sample's first RCAP entries lie in its tile's list, lane by lane.  Further
+// entries go to chunks of RCAP entries of the sample's own, taken from the
+// batch's pool and chained in order.  Each list part is summed on its own, and
+// the parts' sums are added in order (k_fold): the same sum whatever tile the
+// sample is in, and a sample of thousands of entries is summed by as many
+// lanes as it has chunks.  k_points sums in the same parts.  (FP32C with
+// double particles: a compensated sum's bits depend on its order to a float
+// rounding of its terms, so there the sums run on through the parts, a warp
+// per sample: k_seq.)  A tile of which
+// a sample finds the pool exhausted is marked (cnt = 0xFF for all its lanes)
+// and listed in ovf_tiles; the single-kernel path computes those tiles.
 constexpr int RCAP = 32;
 struct SplitBufs {
-    float4* ent4;        // [tile][RCAP][32]: (rx, ry, rz, first leaf as int bits)
-    uint32_t* emask;     // [tile][RCAP][32]
-    float* eshift;       // FP32C sums of double inputs, kernels other than M4, else null:
-                         // [tile][RCAP][kc][32], the column shifts A[first leaf] - A0 of each entry
-                         // (span_shift)
-    uint8_t* cnt;        // [tile][32]
+    // entries: [tile][RCAP][32] lists, then [chunk][RCAP]
+    float4* ent4;        // (rx, ry, rz, first leaf as int bits)
+    uint32_t* emask;
+    float* eshift;       // FP32C sums of double inputs, kernels other than M4, else null: the column shifts
+                         // A[first leaf] - A0 of each entry (span_shift), [tile][RCAP][kc][32], then [chunk][RCAP][kc]
+    uint8_t* cnt;        // [tile][32]: entries in the tile's list
     void* ha;            // [tile][32], element type T
+    int32_t* head;       // [tile][32]: the sample's first chunk, or -1
     int32_t* ovf_tiles;  // absolute tile ids
     unsigned* ovf_count;
     int64_t tile0;       // first tile of the batch
     int64_t ntiles;      // tiles in the batch
+    int fp64;            // the pair sums run in double: entries need no relative positions
+    int lspt;            // k_collect: log2 of the samples a warp walks for (5 but in calls of few samples)
+    // the chunk pool
+    unsigned* top;       // chunks taken
+    unsigned ncap;       // chunks in the pool
+    uint32_t ebase;      // index of the first chunk's first entry: tiles of the lists * RCAP * 32
+    uint32_t* own;       // [chunk]: its sample (tile in the batch * 32 + lane) and OWN_* flags, or OWN_NONE
+    int32_t* next;       // [chunk]: the sample's next chunk, or -1
+    uint8_t* ccnt;       // [chunk]: entries
+    double* part;        // [field][2][chunk]: sums of the chunk, and (first chunks) of the sample's list
+    // samples handed to k_heavy (cnt = CNT_HEAVY): all their entries are in consecutive chunks of the pool
+    unsigned* hcount;
+    uint32_t* hlist;     // tile in the batch * 32 + lane
+    unsigned hcap;
+    // FP32C of double particles: the samples of several parts, for k_seq (null otherwise)
+    unsigned* mcount;
+    uint32_t* mlist;     // first chunk of each
 };
+constexpr uint8_t CNT_DEAD = 0xFF;   // the tile is the single-kernel pass's
+constexpr uint8_t CNT_HEAVY = 0xFE;  // the sample's entries are k_heavy's
+constexpr uint32_t OWN_LATER = 0x80000000u;  // not the sample's first chunk
+constexpr uint32_t OWN_HEAVY = 0x40000000u;  // a chunk of k_heavy
+constexpr uint32_t OWN_IDX = 0x3fffffffu;
+constexpr uint32_t OWN_NONE = 0xffffffffu;
+// A sample leaves its tile's walk for k_heavy when it starts its fifth part.
+constexpr int HEAVY_PARTS = 4;
 
 template <class T> struct Args {
     TreeView<T> tv;

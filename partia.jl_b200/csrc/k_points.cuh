@@ -19,14 +19,16 @@
 namespace psb {
 
 // Per-warp shared memory: the span's leaves and the tile's samples.
-template <class T, bool BAND, int KC> struct PStage {
+template <class T, int PREC, int KC> struct PStage {
+    using CT = typename std::conditional<PREC == PREC_FP64, double, float>::type;
     // leaves
-    T x[SPAN], y[SPAN], z[SPAN], h[SPAN], m[SPAN], rho[SPAN];
+    T x[SPAN], y[SPAN], z[SPAN], h[SPAN], m[SPAN];
+    CT ib[SPAN], s3[SPAN], mr[SPAN];  // 1/h, sigma/h^3, m/rho
     T col[KC][SPAN];
     // samples
     T px[SPAN], py[SPAN], pz[SPAN], ra2[SPAN], best[SPAN];
 };
-template <class T, int KC> struct PStage<T, true, KC> {
+template <int KC> struct PStage<double, PREC_FP32C, KC> {
     static constexpr int NB = 1;            // spans batched before the pair bodies run
     static constexpr int SB = NB * SPAN;
     // leaves of up to NB spans (slot b*32 + j = leaf j of batched span b)
@@ -36,7 +38,6 @@ template <class T, int KC> struct PStage<T, true, KC> {
     float mf[SB];       // m
     float col[KC][SB];
     int64_t lo[NB];     // first leaf of each batched span
-    float eq[SPAN];     // nearest search: error bound of Q
     // samples: position relative to the warp anchor + its error, radius bounds
     float4 P[SPAN];
     float2 R[SPAN];
@@ -181,39 +182,43 @@ __device__ __forceinline__ void write_interp_outputs(const Args<T>& A, int64_t k
 // in DFS order with the minimum distance.  stage_span(lo, cnt, false) stages
 // the positions of leaves [lo, lo+cnt) in st (Q and eq for float tests, x y z
 // otherwise); st.P / st.px.. hold the samples.
-constexpr int64_t NEAREST_SEED = 8;
+constexpr int32_t NEAREST_SEED = 8;
+
+// The seed: the (up to) 2 NEAREST_SEED particles around the sample's place in
+// Morton order.  A closer seed prunes more of the walk.
+template <class T>
+__device__ __forceinline__ void nearest_seed(const TreeView<T>& tv, const T p[3], double& best, int32_t& bidx) {
+    uint64_t q[3];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        double f = ((double)p[d] - tv.qlo[d]) * tv.qscale[d];
+        f = f < 0.0 ? 0.0 : (f > 2097151.0 ? 2097151.0 : f);
+        q[d] = (uint64_t)f;
+    }
+    const uint64_t code = (spread3(q[0]) << 2) | (spread3(q[1]) << 1) | spread3(q[2]);
+    int32_t lo = 0, hi = (int32_t)tv.n;  // first index with codes[i] >= code
+    while (lo < hi) {
+        const int32_t mid = lo + ((hi - lo) >> 1);
+        if (__ldg(&tv.codes[mid]) < code) lo = mid + 1;
+        else hi = mid;
+    }
+    // in increasing index: the first strict minimum keeps the smallest index
+    const int32_t c0 = lo >= NEAREST_SEED ? lo - NEAREST_SEED : 0;
+    const int32_t c1 = (lo + NEAREST_SEED <= (int32_t)tv.n) ? lo + NEAREST_SEED : (int32_t)tv.n;
+#pragma unroll 4
+    for (int32_t ci = c0; ci < c1; ++ci) {
+        const double dc = (double)ex_d2_pp<T>(p, __ldg(&tv.x[ci]), __ldg(&tv.y[ci]), __ldg(&tv.z[ci]));
+        if (dc < best) { best = dc; bidx = ci; }
+    }
+}
 
 template <class T, bool BAND, class Stage, class StageSpan>
 __device__ __forceinline__ T nearest_h_pass(const TreeView<T>& tv, Stage& st, StageSpan& stage_span, int lane,
                                             bool valid, const T p[3], const float pf[3], float pem, int32_t start,
                                             int64_t& steps, bool& ok) {
     double best = INFINITY;
-    int64_t bidx = -1;
-    if (valid) {
-        uint64_t q[3];
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-            double f = ((double)p[d] - tv.qlo[d]) * tv.qscale[d];
-            f = f < 0.0 ? 0.0 : (f > 2097151.0 ? 2097151.0 : f);
-            q[d] = (uint64_t)f;
-        }
-        const uint64_t code = (spread3(q[0]) << 2) | (spread3(q[1]) << 1) | spread3(q[2]);
-        int64_t lo = 0, hi = tv.n;  // first index with codes[i] >= code
-        while (lo < hi) {
-            int64_t mid = (lo + hi) >> 1;
-            if (__ldg(&tv.codes[mid]) < code) lo = mid + 1;
-            else hi = mid;
-        }
-        // the (up to) 2 NEAREST_SEED particles around that position in Morton
-        // order, in increasing index: the first strict minimum keeps the
-        // smallest index.  A closer seed prunes more of the walk.
-        const int64_t c0 = lo >= NEAREST_SEED ? lo - NEAREST_SEED : 0;
-        const int64_t c1 = (lo + NEAREST_SEED <= tv.n) ? lo + NEAREST_SEED : tv.n;
-        for (int64_t ci = c0; ci < c1; ++ci) {
-            const double dc = (double)ex_d2_pp<T>(p, tv.x[ci], tv.y[ci], tv.z[ci]);
-            if (dc < best) { best = dc; bidx = ci; }
-        }
-    }
+    int32_t bidx = -1;
+    if (valid) nearest_seed<T>(tv, p, best, bidx);
     auto better = [&](double d2, int64_t li) { return d2 < best || (d2 == best && li < bidx); };
     // the node test compares in float against best rounded up (lb > bestf
     // implies lb > best): one conversion per improvement, not per step
@@ -268,7 +273,7 @@ __device__ __forceinline__ T nearest_h_pass(const TreeView<T>& tv, Stage& st, St
             for (; cand; cand &= cand - 1) {
                 const int64_t li = lo + __ffs(cand) - 1;
                 double d2 = (double)ex_d2_pp<T>(p, tv.x[li], tv.y[li], tv.z[li]);
-                if (better(d2, li)) { best = d2; bidx = li; bestf = __double2float_ru(best); }
+                if (better(d2, li)) { best = d2; bidx = (int32_t)li; bestf = __double2float_ru(best); }
             }
         } else {
             st.best[lane] = (T)best;
@@ -285,12 +290,18 @@ __device__ __forceinline__ T nearest_h_pass(const TreeView<T>& tv, Stage& st, St
             for (; cand; cand &= cand - 1) {
                 const int jj = __ffs(cand) - 1;
                 double d2 = (double)ex_d2_pp<T>(p, st.x[jj], st.y[jj], st.z[jj]);
-                if (better(d2, lo + jj)) { best = d2; bidx = lo + jj; }
+                if (better(d2, lo + jj)) { best = d2; bidx = (int32_t)(lo + jj); }
             }
         }
     };
     ok = warp_traverse_spans(start, tv.n, tv.links, tv.escape, valid, node_fn, span_fn, steps) && ok;
     return valid ? ((bidx >= 0) ? tv.h[bidx] : qnan<T>()) : T(0);
+}
+
+// Sums of one list part added to the sample's total.  A call of its own, so
+// that the totals stay in local memory: few samples have a second part.
+static __device__ __noinline__ void fold_part(double* tot, const double* part, int n, bool first) {
+    for (int q = 0; q < n; ++q) tot[q] = first ? part[q] : __dadd_rn(tot[q], part[q]);
 }
 
 template <class T, int PREC, int ST, int KC, int WHAT, int KF>
@@ -300,7 +311,7 @@ __global__ void __launch_bounds__(128) k_points(const Args<T> A) {
     constexpr bool BAND = (PREC == PREC_FP32C) && (sizeof(T) == 8);
     constexpr bool SHIFT = (PREC == PREC_FP32C);  // accumulate A - A0 (cancellation-free gradients)
     constexpr bool EXS = BAND && KF == 1;         // A - A0 from span-relative columns (span_shift)
-    __shared__ PStage<T, BAND, KC> stage_all[4];
+    __shared__ PStage<T, PREC, KC> stage_all[4];
     const TreeView<T>& tv = A.tv;
     const int lane = threadIdx.x & 31;
     const int wib = threadIdx.x >> 5;
@@ -364,7 +375,14 @@ __global__ void __launch_bounds__(128) k_points(const Args<T> A) {
                 st.x[lane] = __ldg(&tv.x[li]); st.y[lane] = __ldg(&tv.y[li]); st.z[lane] = __ldg(&tv.z[li]);
                 st.h[lane] = __ldg(&tv.h[li]);
                 if (with_cols) {
-                    st.m[lane] = __ldg(&tv.m[li]); st.rho[lane] = __ldg(&tv.rho[li]);
+                    st.m[lane] = __ldg(&tv.m[li]);
+                    if constexpr (PREC == PREC_FP64) {
+                        const double2 s = __ldg(&tv.leafD[2][li]);
+                        st.ib[lane] = __ldg(&tv.leafD[1][li]).y; st.s3[lane] = s.x; st.mr[lane] = s.y;
+                    } else {
+                        const float4 K = __ldg(&tv.leafK[li]);
+                        st.ib[lane] = K.x; st.s3[lane] = K.y; st.mr[lane] = K.w;
+                    }
 #pragma unroll
                     for (int c = 0; c < KC; ++c)
                         if (c < kc) st.col[c][lane] = __ldg(&A.colT[c][li]);
@@ -416,7 +434,6 @@ __global__ void __launch_bounds__(128) k_points(const Args<T> A) {
 
     // ---- accumulators ----
     Acc S1, G[3], Sw[KC], Sg[KC][3], Dm, Dg[3];
-    CT dens = CT(0);
     CT a0[KC];
     bool have0 = false;
     int64_t first0 = -1;  // EXS: the first accepted leaf (its column values are A0)
@@ -433,68 +450,104 @@ __global__ void __launch_bounds__(128) k_points(const Args<T> A) {
     uint64_t hsum = 0;
     int64_t hcount = 0;
 
-    // kernel weights and accumulation of one accepted pair (leaf j of the stage)
-    auto body = [&](int64_t li, int j, CT dx, CT dy, CT dz, CT d2, CT hb) {
+    // The sums run in parts of RCAP entries (spans with accepted leaves), added
+    // up in order, as the two-kernel path adds its list parts (SplitBufs); the
+    // compensated sums of double particles run on through the parts there and here.
+    constexpr int NF = (WHAT == WHAT_DENSITY) ? 1 : 8 + 4 * KC;
+    double tot[NF];
+    int nent = 0;
+    bool folded = false;
+    auto get_part = [&](double* v) {
+        if (WHAT == WHAT_DENSITY) {
+            v[0] = Dm.get();
+            return;
+        }
+        v[0] = S1.get();
+        v[4] = Dm.get();
+#pragma unroll
+        for (int d = 0; d < 3; ++d) { v[1 + d] = G[d].get(); v[5 + d] = Dg[d].get(); }
+#pragma unroll
+        for (int c = 0; c < KC; ++c) {
+            v[8 + c] = Sw[c].get();
+#pragma unroll
+            for (int d = 0; d < 3; ++d) v[8 + KC + 3 * c + d] = Sg[c][d].get();
+        }
+    };
+    auto count_entry = [&]() {
+        if (WHAT == WHAT_DIGEST || BAND) return;
+        if (nent == RCAP) {
+            double v[NF];
+            get_part(v);
+            fold_part(tot, v, NF, !folded);
+            folded = true;
+            nent = 0;
+            S1.zero(); Dm.zero();
+#pragma unroll
+            for (int d = 0; d < 3; ++d) { G[d].zero(); Dg[d].zero(); }
+#pragma unroll
+            for (int c = 0; c < KC; ++c) {
+                Sw[c].zero();
+#pragma unroll
+                for (int d = 0; d < 3; ++d) Sg[c][d].zero();
+            }
+        }
+        ++nent;
+    };
+
+    // kernel weights and accumulation of one accepted pair (leaf j of the
+    // stage, exact geometry): the arithmetic of k_bodies
+    auto body = [&](int64_t li, int j) {
         ++n_pairs;
         if (WHAT == WHAT_DIGEST) {
             ++hcount;
             hsum += mix64((uint64_t)(li + 1));
             return;
         }
-        const CT r = sqrt(d2);
-        const CT invr = (d2 > CT(0)) ? CT(1) / r : CT(0);
-        CT Wsum = CT(0), csum = CT(0);  // kernel value and gradient coefficient (grad W = c * delta)
-        if (ST != ST_SCATTER) {
-            CT f, df;
-            kfdf<KF, CT>(tv.kern, r * ia, f, df);
-            Wsum = sa3 * f;
-            csum = sa4 * df * invr;
-        }
-        if (ST != ST_GATHER) {
-            CT ib = CT(1) / hb;
-            CT sb3 = sig * ib * ib * ib;
-            CT f, df;
-            kfdf<KF, CT>(tv.kern, r * ib, f, df);
-            CT Wb = sb3 * f, cb = sb3 * ib * df * invr;
-            if (ST == ST_SCATTER) { Wsum = Wb; csum = cb; }
-            else { Wsum = CT(0.5) * (Wsum + Wb); csum = CT(0.5) * (csum + cb); }
-        }
-        CT mb, mr;
-        if constexpr (BAND) {
-            mr = (CT)st.K[j].w;
-            mb = (CT)st.mf[j];
-        } else {
-            mb = (CT)st.m[j];
-            mr = (CT)((double)st.m[j] / (double)st.rho[j]);
-        }
-        if (WHAT == WHAT_DENSITY) {
-            dens += (A.unit_mass ? CT(1) : mb) * Wsum;
-            return;
-        }
-        const CT w = mr * Wsum;
-        const CT gc = mr * csum;
-        const CT gx = gc * dx, gy = gc * dy, gz = gc * dz;
-        S1.add(w);
-        G[0].add(gx); G[1].add(gy); G[2].add(gz);
-        if (SHIFT && !have0) {
-            have0 = true;
-#pragma unroll
-            for (int c = 0; c < KC; ++c)
-                if (c < kc) a0[c] = (CT)st.col[c][j];
-        }
-#pragma unroll
-        for (int c = 0; c < KC; ++c) {
-            if (c < kc) {
-                CT a = (CT)st.col[c][j];
-                if (SHIFT) a -= a0[c];
-                Sw[c].add(a * w);
-                Sg[c][0].add(a * gx); Sg[c][1].add(a * gy); Sg[c][2].add(a * gz);
+        if constexpr (!BAND) {
+            const T xb = st.x[j], yb = st.y[j], zb = st.z[j];
+            CT dx, dy, dz, Wsum, csum;
+            if constexpr (PREC == PREC_FP64) {
+                dx = __dsub_rn((double)p[0], (double)xb);
+                dy = __dsub_rn((double)p[1], (double)yb);
+                dz = __dsub_rn((double)p[2], (double)zb);
+                f64_pair_weights<ST, KF>(tv.kern, dx, dy, dz, ia, sa3, st.ib[j], st.s3[j], Wsum, csum);
+            } else {
+                dx = __fsub_rn(p[0], xb);
+                dy = __fsub_rn(p[1], yb);
+                dz = __fsub_rn(p[2], zb);
+                f32_pair_weights<ST, KF>(tv.kern, ex_d2_pp<T>(p, xb, yb, zb), ia, sa3, sa4, st.ib[j], st.s3[j], Wsum,
+                                         csum);
             }
-        }
-        if (need_dg) {
-            Dm.add(mb * Wsum);
-            CT mc = mb * csum;
-            Dg[0].add(mc * dx); Dg[1].add(mc * dy); Dg[2].add(mc * dz);
+            const CT mb = (CT)st.m[j], mr = st.mr[j];
+            if (WHAT == WHAT_DENSITY) {
+                acc_mac(Dm, A.unit_mass ? CT(1) : mb, Wsum);
+                return;
+            }
+            const CT w = acc_mul(mr, Wsum);
+            const CT gc = acc_mul(mr, csum);
+            const CT gx = acc_mul(gc, dx), gy = acc_mul(gc, dy), gz = acc_mul(gc, dz);
+            S1.add(w);
+            G[0].add(gx); G[1].add(gy); G[2].add(gz);
+            if (SHIFT && !have0) {
+                have0 = true;
+#pragma unroll
+                for (int c = 0; c < KC; ++c)
+                    if (c < kc) a0[c] = (CT)st.col[c][j];
+            }
+#pragma unroll
+            for (int c = 0; c < KC; ++c) {
+                if (c < kc) {
+                    CT a = (CT)st.col[c][j];
+                    if constexpr (SHIFT) a = __fsub_rn(a, a0[c]);
+                    acc_mac(Sw[c], a, w);
+                    acc_mac(Sg[c][0], a, gx); acc_mac(Sg[c][1], a, gy); acc_mac(Sg[c][2], a, gz);
+                }
+            }
+            if (need_dg) {
+                acc_mac(Dm, mb, Wsum);
+                const CT mc = acc_mul(mb, csum);
+                acc_mac(Dg[0], mc, dx); acc_mac(Dg[1], mc, dy); acc_mac(Dg[2], mc, dz);
+            }
         }
     };
 
@@ -708,7 +761,6 @@ __global__ void __launch_bounds__(128) k_points(const Args<T> A) {
         };
         ok = warp_traverse_spans(start, tv.n, tv.links, tv.escape, valid, node_fn, span_fn, steps) && ok;
         if (nb > 0) flush();
-        if (WHAT == WHAT_DENSITY) dens = (CT)Dm.get();
     } else {
         const bool with_cols = (WHAT != WHAT_DIGEST);
         auto span_fn = [&](int64_t lo, int cnt, bool part) {
@@ -717,65 +769,25 @@ __global__ void __launch_bounds__(128) k_points(const Args<T> A) {
             if (!parts) return;
             ++n_spans;
             n_parts += __popc(parts);
-            unsigned acc = 0, unc = 0;
+            unsigned acc = 0;
             const int j = lane < cnt ? lane : 0;
-            if constexpr (BAND) {
-                const float4 Q = st.Q[j];
-                const float eq = st.eq[j];
-                const float rblo = tv.Kf * Q.w * (1.f - 3.f * U1), rbhi = tv.Kf * Q.w * (1.f + 3.f * U1);
-                for (unsigned pp = parts; pp; pp &= pp - 1) {
-                    const int s = __ffs(pp) - 1;
-                    const float4 P = st.P[s];
-                    const float2 R = st.R[s];
-                    float dx = P.x - Q.x, dy = P.y - Q.y, dz = P.z - Q.z;
-                    float d2 = dx * dx + dy * dy + dz * dz;
-                    float rlo, rhi;
-                    if (ST == ST_GATHER) { rlo = R.x; rhi = R.y; }
-                    else if (ST == ST_SCATTER) { rlo = rblo; rhi = rbhi; }
-                    else { rlo = fmaxf(R.x, rblo); rhi = fmaxf(R.y, rbhi); }
-                    float e = 1.7320508f * (P.w + eq) + 4.f * U1 * rhi + 1e-30f;
-                    float il = (rlo - e) * (1.f - 4.f * U1), ih = (rhi + e) * (1.f + 4.f * U1);
-                    bool in = (lane < cnt) && il > 0.f && d2 < il * il;
-                    bool un = (lane < cnt) && !in && !(d2 > ih * ih);
-                    unsigned bi = __ballot_sync(PSB_FULL, in), bu = __ballot_sync(PSB_FULL, un);
-                    if (lane == s) { acc = bi; unc = bu; }
-                }
-                // undecided pairs: the reference's double test
-                for (unsigned u = unc; u; u &= u - 1) {
-                    const int jj = __ffs(u) - 1;
-                    const int64_t li = lo + jj;
-                    ++n_retest;
-                    T e2 = ex_d2_pp<T>(p, tv.x[li], tv.y[li], tv.z[li]);
-                    if (e2 <= ex_r2<ST, T>(ra2, tv.h[li], Kt)) acc |= 1u << jj;
-                }
-                const float sr0 = st.P[lane].x, sr1 = st.P[lane].y, sr2 = st.P[lane].z;
-                n_bodyit += __reduce_max_sync(PSB_FULL, (unsigned)__popc(acc));
-                for (; acc; acc &= acc - 1) {
-                    const int jj = __ffs(acc) - 1;
-                    const float4 Qj = st.Q[jj];
-                    float fx = sr0 - Qj.x, fy = sr1 - Qj.y, fz = sr2 - Qj.z;
-                    body(lo + jj, jj, (CT)fx, (CT)fy, (CT)fz, (CT)(fx * fx + fy * fy + fz * fz), (CT)Qj.w);
-                }
-            } else {
-                const T xj = st.x[j], yj = st.y[j], zj = st.z[j], hj = st.h[j];
-                const T r2b = ex_r2<ST_SCATTER, T>(T(0), hj, Kt);  // (K hb)^2
-                for (unsigned pp = parts; pp; pp &= pp - 1) {
-                    const int s = __ffs(pp) - 1;
-                    const T ps[3] = {st.px[s], st.py[s], st.pz[s]};
-                    const T ra2s = st.ra2[s];
-                    T e2 = ex_d2_pp<T>(ps, xj, yj, zj);
-                    T r2 = (ST == ST_GATHER) ? ra2s : ((ST == ST_SCATTER) ? r2b : jmax(ra2s, r2b));
-                    bool in = (lane < cnt) && (e2 <= r2);
-                    unsigned bi = __ballot_sync(PSB_FULL, in);
-                    if (lane == s) acc = bi;
-                }
-                n_bodyit += __reduce_max_sync(PSB_FULL, (unsigned)__popc(acc));
-                for (; acc; acc &= acc - 1) {
-                    const int jj = __ffs(acc) - 1;
-                    const T xb = st.x[jj], yb = st.y[jj], zb = st.z[jj];
-                    const T e2 = ex_d2_pp<T>(p, xb, yb, zb);
-                    body(lo + jj, jj, (CT)(p[0] - xb), (CT)(p[1] - yb), (CT)(p[2] - zb), (CT)e2, (CT)st.h[jj]);
-                }
+            const T xj = st.x[j], yj = st.y[j], zj = st.z[j], hj = st.h[j];
+            const T r2b = ex_r2<ST_SCATTER, T>(T(0), hj, Kt);  // (K hb)^2
+            for (unsigned pp = parts; pp; pp &= pp - 1) {
+                const int s = __ffs(pp) - 1;
+                const T ps[3] = {st.px[s], st.py[s], st.pz[s]};
+                const T ra2s = st.ra2[s];
+                T e2 = ex_d2_pp<T>(ps, xj, yj, zj);
+                T r2 = (ST == ST_GATHER) ? ra2s : ((ST == ST_SCATTER) ? r2b : jmax(ra2s, r2b));
+                bool in = (lane < cnt) && (e2 <= r2);
+                unsigned bi = __ballot_sync(PSB_FULL, in);
+                if (lane == s) acc = bi;
+            }
+            n_bodyit += __reduce_max_sync(PSB_FULL, (unsigned)__popc(acc));
+            if (acc) count_entry();
+            for (; acc; acc &= acc - 1) {
+                const int jj = __ffs(acc) - 1;
+                body(lo + jj, jj);
             }
         };
 
@@ -790,13 +802,35 @@ __global__ void __launch_bounds__(128) k_points(const Args<T> A) {
             A.dig_hash[k] = hsum;
             if (A.ha_out) A.ha_out[k] = ha;
         } else if (WHAT == WHAT_DENSITY) {
-            A.out[0][k] = (T)dens;
+            double v[NF];
+            get_part(v);
+            if (folded) fold_part(tot, v, NF, false);
+            const double t = folded ? tot[0] : v[0];
+            A.out[0][k] = (PREC == PREC_FP64) ? (T)t : (T)(CT)t;
         } else {
             double a0o[KC];
 #pragma unroll
             for (int c = 0; c < KC; ++c)
                 a0o[c] = EXS ? ((c < kc && first0 >= 0) ? (double)A.colT[c][first0] : 0.0) : (double)a0[c];
-            write_interp_outputs<T, Acc, CT, KC>(A, k, S1, G, Sw, Sg, Dm, Dg, a0o);
+            if (folded) {
+                double v[NF];
+                get_part(v);
+                fold_part(tot, v, NF, false);
+                PlainD s1, g[3], dm, dg[3], sw[KC], sg[KC][3];
+                s1.s = tot[0];
+                dm.s = tot[4];
+#pragma unroll
+                for (int d = 0; d < 3; ++d) { g[d].s = tot[1 + d]; dg[d].s = tot[5 + d]; }
+#pragma unroll
+                for (int c = 0; c < KC; ++c) {
+                    sw[c].s = tot[8 + c];
+#pragma unroll
+                    for (int d = 0; d < 3; ++d) sg[c][d].s = tot[8 + KC + 3 * c + d];
+                }
+                write_interp_outputs<T, PlainD, CT, KC>(A, k, s1, g, sw, sg, dm, dg, a0o);
+            } else {
+                write_interp_outputs<T, Acc, CT, KC>(A, k, S1, G, Sw, Sg, Dm, Dg, a0o);
+            }
         }
     }
     // ---- statistics and errors ----

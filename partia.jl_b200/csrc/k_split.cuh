@@ -1,101 +1,346 @@
-// k_split.cuh -- the two-kernel point path.
+// k_split.cuh -- the point path over pair lists: walk, then sums.
 //
 // k_collect walks the LBVH for a tile of 32 samples (one warp, the same walk,
 // spans and inclusion decisions as k_points) and records, per sample, the
 // accepted leaves as one entry per span (first leaf, 32-bit mask, the sample's
 // offset from the first leaf) plus the sample's smoothing length.  It keeps no accumulators, so it runs with few registers.
 // k_bodies then evaluates the kernel weights and sums of every recorded pair:
-// each lane runs through its own sample's list in one flattened loop, so a
-// warp iteration does 32 pair bodies until the shortest lists run out, instead
-// of idling lanes once per span.  Pairs are visited in the same order as in
-// k_points (span order, then leaf order), with the same arithmetic.
+// each lane runs through a list part (a sample's list in its tile, or one of
+// its chunks) in one flattened loop, so a warp iteration does 32 pair bodies
+// until the shortest parts run out, instead of idling lanes once per span.
+// Pairs are visited in the same order as in k_points (span order, then leaf
+// order), with the same arithmetic.
 #pragma once
 
 #include "k_points.cuh"
 
 namespace psb {
 
-template <class T, bool BAND> struct CStage {
-    T x[SPAN], y[SPAN], z[SPAN], h[SPAN];
-    T px[SPAN], py[SPAN], pz[SPAN], ra2[SPAN], best[SPAN];
+// Per-warp shared memory of the walk.
+constexpr int WQ = 192;  // stack of the walk
+template <class T> struct CStage {
+    float4 Q[SPAN];   // leaves: position relative to the warp anchor and h (double inputs), or as they
+                      // are and the squared radius (float inputs)
+    float4 P[SPAN];   // samples: position relative to the warp anchor and its error bound, or as they are
+    float2 AB[SPAN];  // double inputs: per-span squared thresholds of each leaf
+    float2 SAB[SPAN]; // per-span squared thresholds of each sample; float inputs: (squared radius, -)
+    float4 W[SPAN];   // samples: float position and squared radius bound, for node tests one by one
+    int32_t q[WQ];
 };
-template <class T> struct CStage<T, true> {
-    float4 Q[SPAN];   // leaf position relative to the warp anchor, h (nearest search)
-    float4 P[SPAN];   // sample position relative to the warp anchor, error bound
-    float2 R[SPAN];   // sample radius bounds
-    float2 AB[SPAN];  // per-span squared thresholds of each leaf
-    float2 SAB[SPAN]; // per-span squared thresholds of each sample
-    float thr[SPAN];  // nearest search: candidate threshold
-};
+// found spans that reached none of the warp's samples, after which its node
+// tests go sample by sample
+constexpr int WALK_MISSES = 12;
 
-// 12 CTAs (48 warps) per SM, 40 registers: the walk is bound by issue and
-// by its node loads, and more resident warps beat the few spills this costs
-// (C2: FP32C step 5.52 -> 5.42 ms, FP64 7.95 -> 7.37 ms; 16 CTAs at 32
-// registers spill too much: 5.67 / 8.18 ms).
-template <class T, int PREC, int ST>
-__global__ void __launch_bounds__(128, 12) k_collect(const Args<T> A) {
-    constexpr bool BAND = (PREC == PREC_FP32C) && (sizeof(T) == 8);
-    __shared__ CStage<T, BAND> stage_all[4];
+// A sample's list part is full: start its next one.  Takes a chunk of the
+// pool, or after HEAVY_PARTS parts hands the sample to k_heavy, as long as its
+// list has room.  Returns the sample's current chunk and its parts: parts = 0
+// if it is k_heavy's, unchanged if the pool has run out.
+static __device__ __noinline__ int2 next_part(const SplitBufs& sp, uint32_t idx, int32_t chunk, int nparts) {
+    if (nparts == HEAVY_PARTS) {
+        const unsigned slot = atomicAdd(sp.hcount, 1u);
+        if (slot < sp.hcap) {
+            sp.hlist[slot] = idx;
+            return make_int2(chunk, 0);
+        }
+    }
+    const unsigned c = atomicAdd(sp.top, 1u);
+    if (c >= sp.ncap) return make_int2(chunk, nparts);
+    if (chunk >= 0) {
+        sp.next[chunk] = (int32_t)c;
+        sp.ccnt[chunk] = (uint8_t)RCAP;
+    } else {
+        sp.head[idx] = (int32_t)c;
+    }
+    sp.own[c] = idx | (chunk >= 0 ? OWN_LATER : 0u);
+    if (chunk < 0 && sp.mlist) sp.mlist[atomicAdd(sp.mcount, 1u)] = c;
+    return make_int2((int32_t)c, nparts + 1);
+}
+
+// The walk of one warp: the nodes that reach the warp's samples, found 32 at a
+// time.  The stack holds nodes (id) and found spans (-id) with the leftmost
+// item on top.  A step takes the top items of the stack, one per lane, tests
+// the nodes against the box around the samples, and puts the survivors'
+// children back where the nodes were (a subtree of at most SPAN leaves as a
+// found span), so the spans come off the top in leaf order.  The union walk
+// of 32 samples that tested one node a step took as many dependent loads as
+// it visited nodes; here a step's loads are independent and a walk takes a
+// few more steps than the tree has levels.  ORDERED = false hands out the spans as
+// they come (the nearest search, whose bound they tighten).
+// node_ok(ni): whether internal node ni may hold something; span_fn(id) is
+// called by all lanes.  Corrupt links end the walk with an error: the links
+// are those the escape-link walks use, so a tree whose root has an escape (it
+// has none) is refused, and steps and stack are bounded.
+template <bool ORDERED, class T, class NodeOk, class SpanFn>
+__device__ __forceinline__ bool window_walk(const TreeView<T>& tv, int32_t* q, NodeOk node_ok, SpanFn span_fn,
+                                            uint32_t& steps) {
+    const int lane = threadIdx.x & 31;
+    const unsigned below = (1u << lane) - 1u;
+    const int32_t n = (int32_t)tv.n;
+    if (tv.root == 0) {  // a single particle
+        span_fn(n);
+        return true;
+    }
+    if (__ldg(&tv.links[tv.root - 1]).y != 0) return false;
+    __syncwarp();
+    if (lane == 0) q[0] = tv.root;
+    __syncwarp();
+    int top = 1;
+    const uint32_t bound = (uint32_t)(4 * tv.n + 8 < 0xFFFFFFFFll ? 4 * tv.n + 8 : 0xFFFFFFFFll);
+    uint32_t k = 0;
+    while (top > 0) {
+        if (++k >= bound) return false;
+        // near the stack's end the window narrows to one node: depth first, one item a level
+        const int w = min(32, min(top, max(1, WQ - 64 - top)));
+        const int32_t id = lane < w ? q[top - 1 - lane] : 0;
+        const unsigned spans = __ballot_sync(PSB_FULL, id < 0);
+        if (ORDERED) {
+            const int lead = __ffs(~spans) - 1;  // spans on top (-1: all 32)
+            if (spans & 1u) {
+                const int m = lead < 0 ? 32 : lead;
+                top -= m;
+                for (int c = 0; c < m; ++c) span_fn(-__shfl_sync(PSB_FULL, id, c));
+                continue;
+            }
+        }
+        int out = 0;
+        int32_t c0 = 0, c1 = 0;
+        if (id < 0) {
+            out = ORDERED ? 1 : 0;
+            c0 = id;
+        } else if (id >= n) {  // a leaf reached directly: a span of one
+            out = 1;
+            c0 = -id;
+        } else if (id > 0) {
+            const int4 lk = __ldg(&tv.links[id - 1]);
+            if (node_ok(id - 1)) {
+                if (lk.w - lk.z < SPAN) {
+                    out = 1;
+                    c0 = -id;
+                } else {
+                    out = 2;
+                    c0 = lk.x;
+                    c1 = __ldg(&tv.right[id - 1]);
+                }
+            }
+        }
+        const unsigned b1 = __ballot_sync(PSB_FULL, out == 1), b2 = __ballot_sync(PSB_FULL, out == 2);
+        top += __popc(b1) + 2 * __popc(b2) - w;
+        if (top > WQ) return false;
+        const int at = top - 1 - __popc(b1 & below) - 2 * __popc(b2 & below);
+        __syncwarp();
+        if (out) q[at] = c0;
+        if (out == 2) q[at - 1] = c1;
+        __syncwarp();
+        if (!ORDERED)
+            for (unsigned m = spans; m; m &= m - 1) span_fn(-__shfl_sync(PSB_FULL, id, __ffs(m) - 1));
+    }
+    steps += k;
+    return true;
+}
+
+// The pair lists of a tile's samples (or, in a call of few samples, of
+// 2^lspt of them, so that the call has enough warps): the nearest particle's
+// h where it is asked for, then every leaf within the support radii.
+// Node tests are conservative in float (records rounded outwards) against the
+// box around the samples; a span is then tested against each sample, and its
+// leaves decided as k_points decides them.
+//
+// Bound by issue (compare and vote work of the span tests) on full grids, by
+// the longest walk in small calls.  10 CTAs (40 warps) per SM: 8 / 10 / 12 CTAs
+// take 4.75 / 4.68 / 4.78 ms on the 2M-particle 128^3 grid (FP32C, 8 fields)
+// and 2.79 / 2.72 / 2.82 ms on 700k unordered points.  Before, with one node a
+// step: 5.45 and 2.97 ms; FP64 on 500k particles and a 101 x 67 x 53 grid,
+// which walked in double, 4.05 -> 1.66 ms; 37 points 4.7 -> 0.37 ms.
+template <class T, int ST>
+__global__ void __launch_bounds__(128, 10) k_collect(const __grid_constant__ Args<T> A) {
+    constexpr bool BAND = sizeof(T) == 8;
+    __shared__ CStage<T> stage_all[4];
     const TreeView<T>& tv = A.tv;
     const int lane = threadIdx.x & 31;
     const int wib = threadIdx.x >> 5;
     auto& st = stage_all[wib];
-    const int64_t bt = (int64_t)blockIdx.x * (blockDim.x >> 5) + wib;
+    const int lspt = A.sp.lspt;
+    const int64_t wid = (int64_t)blockIdx.x * (blockDim.x >> 5) + wib;
+    const int64_t bt = wid >> (5 - lspt);
     if (bt >= A.sp.ntiles) return;  // warp-uniform
     const int64_t tile = A.sp.tile0 + bt;
+    // this warp's samples: lanes 0 .. 2^lspt - 1 take the tile's samples slot
+    const int s0 = ((int)wid & ((32 >> lspt) - 1)) << lspt;
+    const bool mine = lane < (1 << lspt);
+    const uint32_t slot = (uint32_t)(bt * 32) + (uint32_t)(s0 + (mine ? lane : 0));
 
-    const int64_t k = sample_of(A.src, tile, lane);
+    const int64_t k = mine ? sample_of(A.src, tile, s0 + lane) : -1;
     const bool valid = k >= 0;
     T p[3] = {T(0), T(0), T(0)}, dd[3];
     if (valid) sample_coords(A.src, k, p, dd);
-    const float pf[3] = {(float)p[0], (float)p[1], (float)p[2]};
-    const float pem = U1 * fmaxf(fmaxf(fabsf(pf[0]), fabsf(pf[1])), fabsf(pf[2])) + 1e-30f;
-    const int32_t start = (tv.root == 0) ? (int32_t)tv.n : tv.root;
+    // A sample whose position or h is not finite, or beyond the range of the
+    // float tests, sends its tile to the single kernel.
+    {
+        bool wild = valid && !(fabs((double)p[0]) <= 1e18 && fabs((double)p[1]) <= 1e18 && fabs((double)p[2]) <= 1e18);
+        if (ST != ST_SCATTER && A.hmode != PSB_H_NEAREST && valid)
+            wild = wild || !(fabs((double)((A.hmode == PSB_H_PER_SAMPLE) ? A.hs[k] : A.hs[0])) <= 1e18);
+        const bool any_wild = __any_sync(PSB_FULL, wild);
+        if (any_wild || !__any_sync(PSB_FULL, valid)) {
+            if (mine) {
+                A.sp.cnt[slot] = any_wild ? CNT_DEAD : 0;
+                A.sp.head[slot] = -1;
+            }
+            if (any_wild && lane == 0) A.sp.ovf_tiles[atomicAdd(A.sp.ovf_count, 1u)] = (int32_t)tile;
+            return;
+        }
+    }
     uint32_t n_pairs = 0, n_retest = 0, n_spans = 0, n_parts = 0;  // per lane / warp, widened below
-    int64_t steps = 0;
+    uint32_t steps = 0;
     bool ok = true;
 
-    const unsigned vmask = __ballot_sync(PSB_FULL, valid);
-    const int first = vmask ? __ffs(vmask) - 1 : 0;
+    // the box around the warp's samples (float, rounded outwards)
+    float blo[3], bhi[3];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        float a = valid ? __double2float_rd((double)p[d]) : INFINITY, b = valid ? __double2float_ru((double)p[d]) : -INFINITY;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            a = fminf(a, __shfl_xor_sync(PSB_FULL, a, o));
+            b = fmaxf(b, __shfl_xor_sync(PSB_FULL, b, o));
+        }
+        blo[d] = a;
+        bhi[d] = b;
+    }
+    // lower bound of the squared distance between that box and a node's
+    auto box_d2 = [&](const float4& lo, const float4& hi) -> float {
+        const float tx = fmaxf(fmaxf(lo.x - bhi[0], blo[0] - hi.x), 0.f);
+        const float ty = fmaxf(fmaxf(lo.y - bhi[1], blo[1] - hi.y), 0.f);
+        const float tz = fmaxf(fmaxf(lo.z - bhi[2], blo[2] - hi.z), 0.f);
+        return (tx * tx + ty * ty + tz * tz) * (1.f - RELM);
+    };
+    const float pf[3] = {(float)p[0], (float)p[1], (float)p[2]};
+    const float pem = U1 * fmaxf(fmaxf(fabsf(pf[0]), fabsf(pf[1])), fabsf(pf[2])) + 1e-30f;
+    // The box test serves samples close to one another.  Where they are not (a
+    // tile across a jump of the Morton curve, one sample of a far larger
+    // radius), the box reaches nodes that no sample does: after WALK_MISSES
+    // such spans a node must also reach one of the samples themselves.
+    int misses = 0;  // warp-uniform
+    const float pemx = __uint_as_float(__reduce_max_sync(PSB_FULL, valid ? __float_as_uint(pem) : 0u));
+    auto set_sample = [&](float r2) { st.W[lane] = make_float4(valid ? pf[0] : 1e30f, pf[1], pf[2], r2); };
+    auto any_sample = [&](const float4& lo, const float4& hi, float r2n) -> bool {
+        for (int s = 0; s < (1 << lspt); ++s) {
+            const float4 w = st.W[s];
+            const float q[3] = {w.x, w.y, w.z};
+            if (!(lb_d2_pbox(q, pemx, lo, hi) > fmaxf(w.w, r2n))) return true;
+        }
+        return false;
+    };
+
+    // the warp anchor (its first sample) and the samples relative to it
+    const int first = __ffs(__ballot_sync(PSB_FULL, valid)) - 1;
     const double cw[3] = {__shfl_sync(PSB_FULL, (double)p[0], first), __shfl_sync(PSB_FULL, (double)p[1], first),
                           __shfl_sync(PSB_FULL, (double)p[2], first)};
+    float esmax = 0.f;  // largest error of a relative sample position
     if constexpr (BAND) {
-        float sr[3] = {(float)((double)p[0] - cw[0]), (float)((double)p[1] - cw[1]), (float)((double)p[2] - cw[2])};
-        float es = U1 * (fabsf(sr[0]) + fabsf(sr[1]) + fabsf(sr[2])) + 1e-30f;
-        st.P[lane] = make_float4(sr[0], sr[1], sr[2], es);
+        const float sr[3] = {(float)((double)p[0] - cw[0]), (float)((double)p[1] - cw[1]), (float)((double)p[2] - cw[2])};
+        st.P[lane] = make_float4(sr[0], sr[1], sr[2], 0.f);
+        if (valid) esmax = U1 * (fabsf(sr[0]) + fabsf(sr[1]) + fabsf(sr[2])) + 1e-30f;
+        esmax = __uint_as_float(__reduce_max_sync(PSB_FULL, __float_as_uint(esmax)));
     } else {
-        st.px[lane] = p[0]; st.py[lane] = p[1]; st.pz[lane] = p[2];
+        st.P[lane] = make_float4(pf[0], pf[1], pf[2], 0.f);
     }
-
-    // positions of leaves [lo, lo+cnt): lane j takes leaf lo+j (all lanes call)
-    // (the span's float error bound is the same for every leaf; see k_points)
-    auto stage_span = [&](int64_t lo, int cnt, bool) -> float {
-        __syncwarp();
-        float eqmax = 0.f;
-        if constexpr (BAND) {
-            // the span's leaves are stored relative to its first leaf
-            const float o0 = (float)((double)__ldg(&tv.x[lo]) - cw[0]);
-            const float o1 = (float)((double)__ldg(&tv.y[lo]) - cw[1]);
-            const float o2 = (float)((double)__ldg(&tv.z[lo]) - cw[2]);
-            const float lm = __ldg(&tv.spanb[lo]).x;
-            eqmax = U1 * (2.f * lm + 2.f * (fabsf(o0) + fabsf(o1) + fabsf(o2))) * (1.f + 4.f * U1);
-            if (lane < cnt) {
-                const float4 L = __ldg(&tv.leaf4[lo + lane]);
-                st.Q[lane] = make_float4(L.x + o0, L.y + o1, L.z + o2, L.w);
-            }
-        } else if (lane < cnt) {
-            const int64_t li = lo + lane;
-            st.x[lane] = __ldg(&tv.x[li]); st.y[lane] = __ldg(&tv.y[li]); st.z[lane] = __ldg(&tv.z[li]);
-            st.h[lane] = __ldg(&tv.h[li]);
+    // the span of node id: first leaf and leaf count
+    auto span_of = [&](int32_t id, int64_t& lo, int& cnt) {
+        if (id >= (int32_t)tv.n) {
+            lo = (int64_t)id - tv.n;
+            cnt = 1;
+        } else {
+            const int4 lk = __ldg(&tv.links[id - 1]);
+            lo = (int64_t)lk.z - 1;
+            cnt = lk.w - lk.z + 1;
         }
-        __syncwarp();
-        return eqmax;
+    };
+    // the span's anchor (first leaf) relative to the warp anchor, and the
+    // error bound of its leaves' relative positions (the same for every leaf)
+    auto anchor = [&](int64_t lo, float o[3], float lmax) -> float {
+        o[0] = (float)((double)__ldg(&tv.x[lo]) - cw[0]);
+        o[1] = (float)((double)__ldg(&tv.y[lo]) - cw[1]);
+        o[2] = (float)((double)__ldg(&tv.z[lo]) - cw[2]);
+        return U1 * (2.f * lmax + 2.f * (fabsf(o[0]) + fabsf(o[1]) + fabsf(o[2]))) * (1.f + 4.f * U1);
     };
 
     T ha = T(0);
     if (ST != ST_SCATTER) {
         if (A.hmode == PSB_H_NEAREST) {
-            ha = nearest_h_pass<T, BAND>(tv, st, stage_span, lane, valid, p, pf, pem, start, steps, ok);
+            // LBVH_find_nearest_h (LinearBVHQueries.jl:118-140), see nearest_h_pass
+            double best = INFINITY;
+            int32_t bidx = -1;
+            if (valid) nearest_seed<T>(tv, p, best, bidx);
+            float bestf = __double2float_ru(best);
+            set_sample(bestf);
+            float bmax = __uint_as_float(__reduce_max_sync(PSB_FULL, valid ? __float_as_uint(bestf) : 0u));
+            auto node_ok = [&](int ni) -> bool {
+                const float4 lo = __ldg(&tv.node_lo[ni]), hi = __ldg(&tv.node_hi[ni]);
+                return !(box_d2(lo, hi) > bmax) && (misses < WALK_MISSES || any_sample(lo, hi, 0.f));
+            };
+            auto span_fn = [&](int32_t id) {
+                bool part = valid;
+                if (id < (int32_t)tv.n)
+                    part = part && !(lb_d2_pbox(pf, pem, __ldg(&tv.node_lo[id - 1]), __ldg(&tv.node_hi[id - 1])) > bestf);
+                const unsigned parts = __ballot_sync(PSB_FULL, part);
+                if (!parts) {
+                    ++misses;
+                    return;
+                }
+                int64_t lo;
+                int cnt;
+                span_of(id, lo, cnt);
+                // candidates: float d2 not above (sqrt(best) + error)^2, or exactly not above best
+                float thr;
+                __syncwarp();
+                if constexpr (BAND) {
+                    float o[3];
+                    const float eqm = anchor(lo, o, __ldg(&tv.spanb[lo]).x);
+                    const float bs = (float)sqrt(best);
+                    const float e = 1.7320508f * (esmax + eqm) + 4.f * U1 * bs + 1e-18f;
+                    const float t = (bs + e) * (1.f + 4.f * U1);
+                    thr = isinf(best) ? INFINITY : t * t;
+                    if (lane < cnt) {
+                        const float4 L = __ldg(&tv.leaf4[lo + lane]);
+                        st.Q[lane] = make_float4(L.x + o[0], L.y + o[1], L.z + o[2], L.w);
+                    }
+                } else {
+                    thr = (float)best;  // a float distance: exact
+                    if (lane < cnt) st.Q[lane] = __ldg(&tv.leaf4[lo + lane]);
+                }
+                const bool by_sample = 3 * __popc(parts) >= 2 * cnt;
+                if (!by_sample) st.SAB[lane].x = thr;
+                __syncwarp();
+                auto d2_of = [&](const float4& P, const float4& Q) -> float {
+                    const float dx = P.x - Q.x, dy = P.y - Q.y, dz = P.z - Q.z;
+                    if constexpr (BAND) return dx * dx + dy * dy + dz * dz;
+                    return __fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz));
+                };
+                unsigned cand = 0;
+                if (by_sample) {  // each taking lane tests its sample against every leaf
+                    if (part) {
+                        const float4 P = st.P[lane];
+#pragma unroll 4
+                        for (int j = 0; j < cnt; ++j) cand |= (unsigned)(d2_of(P, st.Q[j]) <= thr) << j;
+                    }
+                } else {  // lane j tests leaf j against each taking sample
+                    const float4 Q = st.Q[lane < cnt ? lane : 0];
+                    for (unsigned pp = parts; pp; pp &= pp - 1) {
+                        const int s = __ffs(pp) - 1;
+                        const unsigned b = __ballot_sync(PSB_FULL, lane < cnt && d2_of(st.P[s], Q) <= st.SAB[s].x);
+                        if (lane == s) cand = b;
+                    }
+                }
+                for (; cand; cand &= cand - 1) {
+                    const int64_t li = lo + __ffs(cand) - 1;
+                    const double d2 = (double)ex_d2_pp<T>(p, tv.x[li], tv.y[li], tv.z[li]);
+                    if (d2 < best || (d2 == best && li < bidx)) { best = d2; bidx = (int32_t)li; bestf = __double2float_ru(best); }
+                }
+                st.W[lane].w = bestf;
+                bmax = __uint_as_float(__reduce_max_sync(PSB_FULL, valid ? __float_as_uint(bestf) : 0u));
+            };
+            ok = window_walk<false>(tv, st.q, node_ok, span_fn, steps);
+            ha = valid ? ((bidx >= 0) ? tv.h[bidx] : qnan<T>()) : T(0);
         } else if (valid) {
             ha = (A.hmode == PSB_H_PER_SAMPLE) ? A.hs[k] : A.hs[0];
         }
@@ -103,97 +348,109 @@ __global__ void __launch_bounds__(128, 12) k_collect(const Args<T> A) {
     const T Kt = (T)tv.Kd;
     const T ra = X<T>::mul(Kt, ha);
     const T ra2 = X<T>::mul(ra, ra);
-    float ra2_hi = 0.f;
-    if constexpr (BAND) {
-        float ralo = 0.f, rahi = 0.f;
-        if (ST != ST_SCATTER) {
-            ralo = __double2float_rd((double)ra) * (1.f - 2.f * U1);
-            rahi = __double2float_ru((double)ra) * (1.f + 2.f * U1);
-            ra2_hi = __double2float_ru((double)ra2) * (1.f + RELM);
-        }
-        st.R[lane] = make_float2(ralo, rahi);
-    } else {
-        st.ra2[lane] = ra2;
+    float ra2_hi = 0.f, ralo = 0.f, rahi = 0.f;
+    if (ST != ST_SCATTER) {
+        ralo = __double2float_rd(fabs((double)ra)) * (1.f - 2.f * U1);
+        rahi = __double2float_ru(fabs((double)ra)) * (1.f + 2.f * U1);
+        ra2_hi = valid ? __double2float_ru((double)ra2) * (1.f + RELM) + 1e-36f : 0.f;
     }
+    // tile-wide maxima (a NaN h, of a set without particles nearby, reaches nothing)
+    auto warp_max = [&](float v) { return __uint_as_float(__reduce_max_sync(PSB_FULL, v > 0.f ? __float_as_uint(v) : 0u)); };
+    const float rahimax = warp_max(rahi);
+    float ra2max = warp_max(ra2_hi);
+    misses = 0;
+    __syncwarp();
+    set_sample(ra2_hi);
 
-    // this lane's pair list
-    float4* ent4 = A.sp.ent4 + (size_t)bt * RCAP * 32 + lane;
-    uint32_t* emask = A.sp.emask + (size_t)bt * RCAP * 32 + lane;
-    int nent = 0;
-    bool ovf = false;
+    // this lane's pair list: the next entry goes to index epos
+    uint32_t epos = (uint32_t)bt * (RCAP * 32) + (slot & 31);
+    int nent = 0;         // entries in the current part
+    int32_t chunk = -1;   // the current chunk (-1: the tile's list)
+    int nparts = 1;       // parts so far; 0: the sample is k_heavy's
+    bool dead = false;    // warp-uniform: the pool ran out, the tile is k_points'
     auto emit = [&](int64_t lo, unsigned acc) {
-        if (!acc) return;
-        n_pairs += __popc(acc);
-        if (nent < RCAP) {
-            // the sample relative to the span's first leaf, in double then
-            // rounded: the pair separation R - L carries only the rounding of
-            // two small vectors
-            float r0 = 0.f, r1 = 0.f, r2 = 0.f;
-            if (BAND) {
-                r0 = (float)((double)p[0] - (double)__ldg(&tv.x[lo]));
-                r1 = (float)((double)p[1] - (double)__ldg(&tv.y[lo]));
-                r2 = (float)((double)p[2] - (double)__ldg(&tv.z[lo]));
+        if (__any_sync(PSB_FULL, acc && nent == RCAP)) {
+            if (acc && nent == RCAP) {
+                const int2 q = next_part(A.sp, slot, chunk, nparts);
+                if (q.y > nparts) {
+                    chunk = q.x;
+                    epos = A.sp.ebase + (uint32_t)chunk * RCAP;
+                    nent = 0;
+                }
+                nparts = q.y;
             }
-            ent4[(size_t)nent * 32] = make_float4(r0, r1, r2, __int_as_float((int)lo));
-            emask[(size_t)nent * 32] = acc;
-            ++nent;
-        } else {
-            ovf = true;
+            if (nparts == 0) {
+                acc = 0;
+                ra2_hi = 0.f;
+                st.W[lane].x = 1e30f;
+            }
+            dead = __any_sync(PSB_FULL, acc && nent == RCAP);
+            if (ST == ST_GATHER) ra2max = warp_max(ra2_hi);  // (the other strategies reach nodes by h_b too)
         }
+        if (!acc || dead) return;
+        n_pairs += __popc(acc);
+        // the sample relative to the span's first leaf, in double then
+        // rounded: the pair separation R - L carries only the rounding of
+        // two small vectors
+        float r0 = 0.f, r1 = 0.f, r2 = 0.f;
+        if (BAND && !A.sp.fp64) {
+            r0 = (float)((double)p[0] - (double)__ldg(&tv.x[lo]));
+            r1 = (float)((double)p[1] - (double)__ldg(&tv.y[lo]));
+            r2 = (float)((double)p[2] - (double)__ldg(&tv.z[lo]));
+        }
+        A.sp.ent4[epos] = make_float4(r0, r1, r2, __int_as_float((int)lo));
+        A.sp.emask[epos] = acc;
+        epos += chunk >= 0 ? 1 : 32;
+        ++nent;
     };
 
-    auto node_fn = [&](int ni) -> bool {
+    auto node_ok = [&](int ni) -> bool {
+        if (dead) return false;
+        const float4 lo = __ldg(&tv.node_lo[ni]), hi = __ldg(&tv.node_hi[ni]);
+        if (box_d2(lo, hi) > hi_r2_node<ST>(ra2max, lo.w, tv.Kf)) return false;
+        return misses < WALK_MISSES || any_sample(lo, hi, ST == ST_GATHER ? 0.f : hi_r2_node<ST_SCATTER>(0.f, lo.w, tv.Kf));
+    };
+    auto span_fn = [&](int32_t id) {
+        bool part = valid && nparts > 0 && !dead;
+        if (id < (int32_t)tv.n) {
+            const float4 lo = __ldg(&tv.node_lo[id - 1]), hi = __ldg(&tv.node_hi[id - 1]);
+            part = part && !(lb_d2_pbox(pf, pem, lo, hi) > hi_r2_node<ST>(ra2_hi, lo.w, tv.Kf));
+        }
+        const unsigned parts = __ballot_sync(PSB_FULL, part);
+        if (!parts) {
+            ++misses;
+            return;
+        }
+        int64_t lo;
+        int cnt;
+        span_of(id, lo, cnt);
+        // few samples take part: lane j tests leaf j against each of them;
+        // otherwise each taking lane tests its sample against every leaf
+        const bool by_sample = 3 * __popc(parts) >= 2 * cnt;  // warp-uniform
+        unsigned myacc = 0;
+        __syncwarp();
         if constexpr (BAND) {
-            float4 lo = __ldg(&tv.node_lo[ni]), hi = __ldg(&tv.node_hi[ni]);
-            float lb = lb_d2_pbox(pf, pem, lo, hi);
-            return !(lb > hi_r2_node<ST>(ra2_hi, lo.w, tv.Kf));
-        } else {
-            T d2n = ex_d2_pbox<T>(p, tv, ni);
-            T r2 = (ST == ST_GATHER) ? ra2 : ex_r2<ST, T>(ra2, __ldg(&tv.nscale[ni]), Kt);
-            return !(d2n > r2);
-        }
-    };
-
-    if constexpr (BAND) {
-        const float4 Pme = st.P[lane];
-        const float2 Rme = st.R[lane];
-        float esmax = Pme.w, rahimax = Rme.y;  // tile-wide maxima (sample error, sample radius)
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            esmax = fmaxf(esmax, __shfl_xor_sync(PSB_FULL, esmax, o));
-            rahimax = fmaxf(rahimax, __shfl_xor_sync(PSB_FULL, rahimax, o));
-        }
-        auto span_fn = [&](int64_t lo, int cnt, bool part) {
-            const unsigned parts = __ballot_sync(PSB_FULL, part);
-            if (!parts) return;
-            // the span's anchor (first leaf) relative to the warp anchor and its
-            // bounds: one error bound E for every float distance of the span
-            const float o0 = (float)((double)__ldg(&tv.x[lo]) - cw[0]);
-            const float o1 = (float)((double)__ldg(&tv.y[lo]) - cw[1]);
-            const float o2 = (float)((double)__ldg(&tv.z[lo]) - cw[2]);
+            // one error bound E for every float distance of the span
+            float o[3];
             const float2 sb = __ldg(&tv.spanb[lo]);
-            const float eqm = U1 * (2.f * sb.x + 2.f * (fabsf(o0) + fabsf(o1) + fabsf(o2))) * (1.f + 4.f * U1);
+            const float eqm = anchor(lo, o, sb.x);
             // the rounding of r itself enters through 4 U1 r (r <= the larger radius)
             float rmax = rahimax;
             if (ST != ST_GATHER) rmax = fmaxf(rmax, tv.Kf * sb.y * (1.f + 3.f * U1));
-            const float E = 1.7320508f * (esmax + eqm) + 4.f * U1 * rmax + 1e-30f;
+            const float E = 1.7320508f * (esmax + eqm) + 4.f * U1 * rmax + 1e-18f;
             // this lane's sample thresholds
             float As = 0.f, Bs = 0.f;
             if (ST != ST_SCATTER) {
-                const float il = fmaxf((Rme.x - E) * (1.f - 4.f * U1), 0.f), ih2 = (Rme.y + E) * (1.f + 4.f * U1);
+                const float il = fmaxf((ralo - E) * (1.f - 4.f * U1), 0.f), ih2 = (rahi + E) * (1.f + 4.f * U1);
                 As = il * il;
                 Bs = ih2 * ih2;
             }
-            // few samples take part: lane j tests leaf j against each of them;
-            // otherwise each taking lane tests its sample against every leaf
-            const bool by_sample = 3 * __popc(parts) >= 2 * cnt;  // warp-uniform
             // the span's leaves (and their radius thresholds) in shared memory
-            __syncwarp();
             float4 Qme = make_float4(0.f, 0.f, 0.f, 0.f);
             float Aj = 0.f, Bj = 0.f;
             if (lane < cnt) {
                 const float4 L = __ldg(&tv.leaf4[lo + lane]);
-                Qme = make_float4(L.x + o0, L.y + o1, L.z + o2, L.w);
+                Qme = make_float4(L.x + o[0], L.y + o[1], L.z + o[2], L.w);
                 st.Q[lane] = Qme;
                 if (ST != ST_GATHER) {
                     const float rbhi = tv.Kf * L.w * (1.f + 3.f * U1), rblo = tv.Kf * L.w * (1.f - 3.f * U1);
@@ -206,7 +463,7 @@ __global__ void __launch_bounds__(128, 12) k_collect(const Args<T> A) {
             if (!by_sample) st.SAB[lane] = make_float2(As, Bs);
             __syncwarp();
             // surely in: d2 < A; maybe in: d2 <= B (undecided = maybe and not surely)
-            unsigned myacc = 0, mymaybe = 0;
+            unsigned mymaybe = 0;
             if (!by_sample) {
                 for (unsigned pp = parts; pp; pp &= pp - 1) {
                     const int s = __ffs(pp) - 1;
@@ -221,6 +478,7 @@ __global__ void __launch_bounds__(128, 12) k_collect(const Args<T> A) {
                     if (lane == s) { myacc = bi; mymaybe = bm; }
                 }
             } else if (part) {
+                const float4 Pme = st.P[lane];
 #pragma unroll 4
                 for (int j = 0; j < cnt; ++j) {
                     const float4 Q = st.Q[j];
@@ -236,70 +494,85 @@ __global__ void __launch_bounds__(128, 12) k_collect(const Args<T> A) {
                     mymaybe |= (unsigned)(d2 <= Bt) << j;
                 }
             }
-            const unsigned myunc = mymaybe & ~myacc;
             // undecided pairs: the reference's double test
-            for (unsigned u = myunc; u; u &= u - 1) {
+            for (unsigned u = mymaybe & ~myacc; u; u &= u - 1) {
                 const int jj = __ffs(u) - 1;
                 const int64_t li = lo + jj;
                 ++n_retest;
                 T e2 = ex_d2_pp<T>(p, tv.x[li], tv.y[li], tv.z[li]);
                 if (e2 <= ex_r2<ST, T>(ra2, tv.h[li], Kt)) myacc |= 1u << jj;
             }
-            emit(lo, myacc);
-            ++n_spans;
-            n_parts += __popc(parts);
-        };
-        ok = warp_traverse_spans(start, tv.n, tv.links, tv.escape, valid, node_fn, span_fn, steps) && ok;
-    } else {
-        auto span_fn = [&](int64_t lo, int cnt, bool part) {
-            stage_span(lo, cnt, false);
-            const unsigned parts = __ballot_sync(PSB_FULL, part);
-            if (!parts) return;
-            ++n_spans;
-            n_parts += __popc(parts);
-            unsigned acc = 0;
-            const int j = lane < cnt ? lane : 0;
-            const T xj = st.x[j], yj = st.y[j], zj = st.z[j], hj = st.h[j];
-            const T r2b = ex_r2<ST_SCATTER, T>(T(0), hj, Kt);  // (K hb)^2
-            for (unsigned pp = parts; pp; pp &= pp - 1) {
-                const int s = __ffs(pp) - 1;
-                const T ps[3] = {st.px[s], st.py[s], st.pz[s]};
-                const T ra2s = st.ra2[s];
-                T e2 = ex_d2_pp<T>(ps, xj, yj, zj);
-                T r2 = (ST == ST_GATHER) ? ra2s : ((ST == ST_SCATTER) ? r2b : jmax(ra2s, r2b));
-                bool in = (lane < cnt) && (e2 <= r2);
-                unsigned bi = __ballot_sync(PSB_FULL, in);
-                if (lane == s) acc = bi;
+        } else {
+            // float inputs: the reference's float arithmetic on the leaf records
+            float4 Qme = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (lane < cnt) {
+                Qme = __ldg(&tv.leaf4[lo + lane]);
+                if (ST != ST_GATHER) Qme.w = ex_r2<ST_SCATTER, float>(0.f, Qme.w, (float)Kt);  // (K hb)^2
+                st.Q[lane] = Qme;
             }
-            emit(lo, acc);
-        };
-        ok = warp_traverse_spans(start, tv.n, tv.links, tv.escape, valid, node_fn, span_fn, steps) && ok;
-    }
+            if (!by_sample) st.SAB[lane].x = (float)ra2;
+            __syncwarp();
+            auto inside = [&](const float4& P, const float4& Q, float r2a) -> bool {
+                const float dx = __fsub_rn(P.x, Q.x), dy = __fsub_rn(P.y, Q.y), dz = __fsub_rn(P.z, Q.z);
+                const float e2 = __fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz));
+                return e2 <= ((ST == ST_GATHER) ? r2a : ((ST == ST_SCATTER) ? Q.w : jmax(r2a, Q.w)));
+            };
+            if (!by_sample) {
+                for (unsigned pp = parts; pp; pp &= pp - 1) {
+                    const int s = __ffs(pp) - 1;
+                    const unsigned b = __ballot_sync(PSB_FULL, lane < cnt && inside(st.P[s], Qme, st.SAB[s].x));
+                    if (lane == s) myacc = b;
+                }
+            } else if (part) {
+                const float4 Pme = st.P[lane];
+#pragma unroll 4
+                for (int j = 0; j < cnt; ++j) myacc |= (unsigned)inside(Pme, st.Q[j], (float)ra2) << j;
+            }
+        }
+        emit(lo, myacc);
+        ++n_spans;
+        n_parts += __popc(parts);
+    };
+    ok = window_walk<true>(tv, st.q, node_ok, span_fn, steps) && ok;
 
-    const bool tovf = __any_sync(PSB_FULL, ovf);
-    if (BAND && A.sp.eshift && !tovf && nent > 0) {
+    const int n0 = chunk >= 0 ? RCAP : nent;  // entries in the tile's list
+    if (mine) {
+        if (chunk >= 0) {
+            A.sp.ccnt[chunk] = (uint8_t)nent;
+            A.sp.next[chunk] = -1;
+        } else {
+            A.sp.head[slot] = -1;
+        }
+        A.sp.cnt[slot] = dead ? CNT_DEAD : (nparts == 0 ? CNT_HEAVY : (uint8_t)n0);
+        ((T*)A.sp.ha)[slot] = ha;
+    }
+    if (BAND && A.sp.eshift && !dead && nparts > 0 && n0 > 0) {
         // the column shifts of this lane's entries, A[lo] - A0 (span_shift),
         // after the walk: here the entries' loads are independent and overlap,
         // where inside the walk each would stall it.  A0 are the column values
         // of the first accepted leaf.
         const int kc = A.rec.kc;
-        float* esh = A.sp.eshift + (size_t)bt * RCAP * kc * 32 + lane;
-        const int32_t fl = __float_as_int(ent4[0].w) + __ffs(emask[0]) - 1;
+        const size_t q0 = (size_t)bt * RCAP * 32 + (slot & 31);
+        const float4* ent4 = A.sp.ent4 + q0;
+        float* esh = A.sp.eshift + (size_t)bt * RCAP * kc * 32 + (slot & 31);
+        const int32_t fl = __float_as_int(ent4[0].w) + __ffs(A.sp.emask[q0]) - 1;
         for (int c = 0; c < kc; ++c) {
 #pragma unroll 4
-            for (int e = 0; e < nent; ++e)
+            for (int e = 0; e < n0; ++e)
                 esh[((size_t)e * kc + c) * 32] = span_shift(A.colT[c], (int64_t)__float_as_int(ent4[(size_t)e * 32].w), fl);
+        }
+        for (int32_t q = chunk >= 0 ? A.sp.head[slot] : -1; q >= 0; q = A.sp.next[q]) {
+            const size_t e0 = (size_t)A.sp.ebase + (size_t)q * RCAP;
+            const int n = A.sp.ccnt[q];
+            for (int c = 0; c < kc; ++c)
+                for (int e = 0; e < n; ++e)
+                    A.sp.eshift[(e0 + e) * kc + c] = span_shift(A.colT[c], (int64_t)__float_as_int(A.sp.ent4[e0 + e].w), fl);
         }
     }
     if (valid && A.ha_out) A.ha_out[k] = ha;
-    A.sp.cnt[bt * 32 + lane] = tovf ? (uint8_t)0xFF : (uint8_t)nent;
-    ((T*)A.sp.ha)[bt * 32 + lane] = ha;
-    if (tovf && lane == 0) {
-        const unsigned slot = atomicAdd(A.sp.ovf_count, 1u);
-        A.sp.ovf_tiles[slot] = (int32_t)tile;
-    }
-    // the single-kernel pass counts the pairs of an overflowed tile
-    unsigned long long t_pairs = tovf ? 0ull : n_pairs, t_retest = n_retest;
+    if (dead && lane == 0) A.sp.ovf_tiles[atomicAdd(A.sp.ovf_count, 1u)] = (int32_t)tile;
+    // the single-kernel pass counts the pairs of a dead tile, k_heavy those of its samples
+    unsigned long long t_pairs = (dead || nparts == 0) ? 0ull : n_pairs, t_retest = n_retest;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         t_pairs += __shfl_xor_sync(PSB_FULL, t_pairs, o);
@@ -315,20 +588,223 @@ __global__ void __launch_bounds__(128, 12) k_collect(const Args<T> A) {
     if (!ok && lane == 0) atomicOr(A.err, PSB_DERR_TRAVERSAL);
 }
 
-// The data of one pair for k_bodies: float records for the FP32C path of
-// double inputs, the exact particle values otherwise.
-template <class T, bool BAND, int KC> struct PairData {
-    T x, y, z, h, m, rho;
+// The pair lists of the samples whose neighbourhoods outgrew their tile's walk
+// (HEAVY_PARTS parts): one CTA per sample.  The walk is a frontier of tree
+// nodes in shared memory, expanded level by level in depth-first order (a
+// block scan places each node's children where the node was), so that its
+// spans end up in leaf order without a serial chain over thousands of nodes;
+// then a warp per span tests the leaves with the exact arithmetic, and a scan
+// of the non-empty spans gives each entry its place in consecutive chunks.
+// The entries are those of the tile's walk, in the same order.  One warp
+// walking such a sample alone ran for milliseconds after every other warp had
+// finished (150k clump particles, M5, 50k points: 8.0 of 13.5 ms).
+constexpr int HEAVY_THREADS = 512;
+constexpr int HEAVY_CAP = 12288;  // frontier nodes (a sample of more goes to k_points)
+constexpr size_t HEAVY_SMEM = 2 * HEAVY_CAP * sizeof(int32_t);
+constexpr int HEAVY_IPT = HEAVY_CAP / HEAVY_THREADS;  // items of a thread
+static_assert(HEAVY_IPT <= 32, "two bits per item in a 64-bit word");
+
+// exclusive scan of one value per thread; *total = the sum (all threads call)
+static __device__ __forceinline__ int heavy_scan(int v, int* wt, int* total) {
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    int s = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int t = __shfl_up_sync(PSB_FULL, s, o);
+        if (lane >= o) s += t;
+    }
+    __syncthreads();  // the last scan's totals are read
+    if (lane == 31) wt[w] = s;
+    __syncthreads();
+    int before = 0, all = 0;
+#pragma unroll
+    for (int q = 0; q < HEAVY_THREADS / 32; ++q) {
+        const int t = wt[q];
+        if (q < w) before += t;
+        all += t;
+    }
+    *total = all;
+    return before + s - v;
+}
+
+template <class T, int ST>
+__global__ void __launch_bounds__(HEAVY_THREADS, 2) k_heavy(const Args<T> A) {
+    extern __shared__ __align__(16) int32_t hbuf[];
+    __shared__ int wt[HEAVY_THREADS / 32];
+    __shared__ unsigned s_base;
+    const TreeView<T>& tv = A.tv;
+    const SplitBufs& sp = A.sp;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const unsigned nh = min(*sp.hcount, sp.hcap);
+    for (unsigned i = blockIdx.x; i < nh; i += gridDim.x) {
+        const uint32_t idx = sp.hlist[i];
+        const int64_t k = sample_of(A.src, sp.tile0 + (idx >> 5), idx & 31);
+        T p[3], dd[3];
+        sample_coords(A.src, k, p, dd);
+        const T ha = ((const T*)sp.ha)[idx];
+        const float pf[3] = {(float)p[0], (float)p[1], (float)p[2]};
+        const float pem = U1 * fmaxf(fmaxf(fabsf(pf[0]), fabsf(pf[1])), fabsf(pf[2])) + 1e-30f;
+        const T Kt = (T)tv.Kd;
+        const T ra = X<T>::mul(Kt, ha);
+        const T ra2 = X<T>::mul(ra, ra);
+        const float ra2_hi = (ST == ST_SCATTER) ? 0.f : __double2float_ru((double)ra2) * (1.f + RELM) + 1e-36f;
+        int32_t* cur = hbuf;
+        int32_t* nxt = hbuf + HEAVY_CAP;
+        // items: a node still to be tested (id > 0) or a span (-id); the root
+        // has more than SPAN leaves (its sample has more than one span)
+        __syncthreads();
+        if (tid == 0) cur[0] = tv.root;
+        __syncthreads();
+        int f = 1;
+        bool fits = true;
+        for (int level = 0;; ++level) {
+            const int ipt = (f + HEAVY_THREADS - 1) / HEAVY_THREADS;
+            const int a = min(f, tid * ipt), b = min(f, a + ipt);
+            unsigned long long res = 0;  // per item: 0 none, 1 a span, 2 its two children
+            int out = 0;
+            bool open = false;
+            for (int q = a; q < b; ++q) {
+                const int32_t id = cur[q];
+                unsigned r = 1;
+                if (id > 0 && id < tv.n) {
+                    const int4 lk = __ldg(&tv.links[id - 1]);
+                    const float4 lo = __ldg(&tv.node_lo[id - 1]), hi = __ldg(&tv.node_hi[id - 1]);
+                    if (lb_d2_pbox(pf, pem, lo, hi) > hi_r2_node<ST>(ra2_hi, lo.w, tv.Kf)) r = 0;
+                    else if (lk.w - lk.z + 1 > SPAN) { r = 2; open = true; }
+                }
+                res |= (unsigned long long)r << (2 * (q - a));
+                out += (int)r;
+            }
+            int nf;
+            int w = heavy_scan(out, wt, &nf);
+            if (nf > HEAVY_CAP || level > 4 * 64) { fits = false; break; }  // (a corrupt tree never closes)
+            for (int q = a; q < b; ++q) {
+                const int32_t id = cur[q];
+                const unsigned r = (unsigned)(res >> (2 * (q - a))) & 3u;
+                if (r == 1) {
+                    nxt[w++] = id > 0 ? -id : id;
+                } else if (r == 2) {
+                    nxt[w++] = __ldg(&tv.left[id - 1]);
+                    nxt[w++] = __ldg(&tv.right[id - 1]);
+                }
+            }
+            open = __syncthreads_or(open);
+            int32_t* t = cur; cur = nxt; nxt = t;
+            f = nf;
+            if (!open) break;
+        }
+        if (fits) {
+            // accept masks of the spans (nxt), a warp per span
+            uint32_t* msk = (uint32_t*)nxt;
+            unsigned n_pairs = 0;
+#pragma unroll 2
+            for (int q = warp; q < f; q += HEAVY_THREADS / 32) {
+                const int32_t id = -cur[q];
+                int64_t lo;
+                int cnt;
+                if (id >= tv.n) {
+                    lo = (int64_t)id - tv.n;
+                    cnt = 1;
+                } else {
+                    const int4 lk = __ldg(&tv.links[id - 1]);
+                    lo = (int64_t)lk.z - 1;
+                    cnt = lk.w - lk.z + 1;
+                }
+                bool in = false;
+                if (lane < cnt) {
+                    const int64_t li = lo + lane;
+                    const T e2 = ex_d2_pp<T>(p, __ldg(&tv.x[li]), __ldg(&tv.y[li]), __ldg(&tv.z[li]));
+                    in = e2 <= ex_r2<ST, T>(ra2, __ldg(&tv.h[li]), Kt);
+                }
+                const unsigned m = __ballot_sync(PSB_FULL, in);
+                __syncwarp();
+                if (lane == 0) {
+                    cur[q] = (int32_t)lo;  // the entry's first leaf
+                    msk[q] = m;
+                }
+                n_pairs += __popc(m);
+            }
+            __syncthreads();
+            const int ipt = (f + HEAVY_THREADS - 1) / HEAVY_THREADS;
+            const int a = min(f, tid * ipt), b = min(f, a + ipt);
+            int out = 0;
+            for (int q = a; q < b; ++q) out += msk[q] != 0;
+            int ne;
+            int w = heavy_scan(out, wt, &ne);
+            const unsigned nch = (unsigned)((ne + RCAP - 1) / RCAP);
+            if (tid == 0) s_base = atomicAdd(sp.top, nch);
+            __syncthreads();
+            const unsigned base = s_base;
+            fits = base < sp.ncap && nch <= sp.ncap - base;
+            for (unsigned c = tid; c < nch; c += HEAVY_THREADS) {
+                if (base + c >= sp.ncap) break;
+                sp.own[base + c] = fits ? (idx | OWN_HEAVY | (c ? OWN_LATER : 0u)) : OWN_NONE;
+                sp.next[base + c] = c + 1 < nch ? (int32_t)(base + c + 1) : -1;
+                sp.ccnt[base + c] = (uint8_t)min(RCAP, ne - (int)c * RCAP);
+            }
+            if (fits) {
+                const size_t e0 = (size_t)sp.ebase + (size_t)base * RCAP;
+                const size_t q0 = (size_t)(idx >> 5) * RCAP * 32 + (idx & 31);
+                // A0 of the column shifts: the sample's first accepted leaf (its list's first pair)
+                const int32_t fl = __float_as_int(sp.ent4[q0].w) + __ffs(sp.emask[q0]) - 1;
+                for (int q = a; q < b; ++q) {
+                    if (!msk[q]) continue;
+                    const int64_t lo = cur[q];
+                    float r0 = 0.f, r1 = 0.f, r2 = 0.f;
+                    if (sizeof(T) == 8 && !sp.fp64) {
+                        r0 = (float)((double)p[0] - (double)__ldg(&tv.x[lo]));
+                        r1 = (float)((double)p[1] - (double)__ldg(&tv.y[lo]));
+                        r2 = (float)((double)p[2] - (double)__ldg(&tv.z[lo]));
+                    }
+                    sp.ent4[e0 + w] = make_float4(r0, r1, r2, __int_as_float((int)lo));
+                    sp.emask[e0 + w] = msk[q];
+                    if (sp.eshift)
+                        for (int c = 0; c < A.rec.kc; ++c)
+                            sp.eshift[(e0 + w) * A.rec.kc + c] = span_shift(A.colT[c], lo, fl);
+                    ++w;
+                }
+                if (A.stats && lane == 0) atomicAdd(&A.stats[0], (unsigned long long)n_pairs);
+                if (sp.mlist && tid == 0) sp.mlist[atomicAdd(sp.mcount, 1u)] = base;
+            }
+        }
+        if (!fits && tid == 0) {  // k_points takes the tile (once)
+            const uint32_t t0 = idx & ~31u;
+            for (int q = 0; q < 32; ++q) sp.cnt[t0 + q] = CNT_DEAD;
+            if (atomicExch(&sp.head[t0], -2) != -2)
+                sp.ovf_tiles[atomicAdd(sp.ovf_count, 1u)] = (int32_t)(sp.tile0 + (idx >> 5));
+        }
+    }
+}
+
+// The data of one pair for k_bodies: the double records for the FP64 sums, the
+// float records for FP32C (with double inputs relative to the span's first leaf).
+template <class T, int PREC, int KC> struct PairData {  // PREC_FP64
+    double2 a, b, s;  // (x, y), (z, 1/h), (sigma/h^3, m/rho)
+    T mb;             // mass (density gradient only)
     T col[KC];
-    __device__ __forceinline__ void load(const TreeView<T>& tv, const Args<T>& A, int64_t li, int kc, bool,
+    __device__ __forceinline__ void load(const TreeView<T>& tv, const Args<T>& A, int64_t li, int kc, bool need_dg,
                                          const float*, const float* const*) {
-        x = __ldg(&tv.x[li]); y = __ldg(&tv.y[li]); z = __ldg(&tv.z[li]);
-        h = __ldg(&tv.h[li]); m = __ldg(&tv.m[li]); rho = __ldg(&tv.rho[li]);
+        a = __ldg(&tv.leafD[0][li]); b = __ldg(&tv.leafD[1][li]); s = __ldg(&tv.leafD[2][li]);
+        mb = need_dg ? __ldg(&tv.m[li]) : T(0);
 #pragma unroll
         for (int c = 0; c < KC; ++c) col[c] = (c < kc) ? __ldg(&A.colT[c][li]) : T(0);
     }
 };
-template <class T, int KC> struct PairData<T, true, KC> {
+template <int KC> struct PairData<float, PREC_FP32C, KC> {
+    float4 L, K;  // leaf4 (the exact position and h) and leafK
+    float mb;
+    float col[KC];
+    __device__ __forceinline__ void load(const TreeView<float>& tv, const Args<float>& A, int64_t li, int kc,
+                                         bool need_dg, const float*, const float* const*) {
+        L = __ldg(&tv.leaf4[li]);
+        K = __ldg(&tv.leafK[li]);
+        mb = need_dg ? __ldg(&tv.m[li]) : 0.f;
+#pragma unroll
+        for (int c = 0; c < KC; ++c) col[c] = (c < kc) ? __ldg(&A.colT[c][li]) : 0.f;
+    }
+};
+template <int KC> struct PairData<double, PREC_FP32C, KC> {
+    using T = double;
     float4 L, K;      // leaf4 and leafK of the particle
     float col[KC];    // the column in float, or for EXS span-relative (A - A0 once the entry's shift is added)
     float mb;         // mass (density gradient only)
@@ -348,22 +824,76 @@ template <class T, int KC> struct PairData<T, true, KC> {
     }
 };
 
+// The list part of a thread of the pair-sum kernels.  Blocks below `nlist` take
+// four tiles' lists (one lane per sample), the blocks after them 128 chunks of
+// the pool each.
+struct ListPart {
+    int64_t bt;      // the sample's tile in the batch
+    int lane;        // and its lane there
+    int n;           // entries (0: nothing to do)
+    uint32_t e0;     // index of the first entry
+    int step;        // distance of consecutive entries
+    int32_t chunk;   // the chunk, or -1 for a list
+    int32_t dst;     // chunk whose partial sums this part writes, or -1: the sample's only part
+};
+__device__ __forceinline__ ListPart list_part(const SplitBufs& sp, unsigned nlist) {
+    ListPart q;
+    q.n = 0;
+    q.dst = -1;
+    q.lane = threadIdx.x & 31;
+    if (blockIdx.x < nlist) {
+        q.bt = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+        q.chunk = -1;
+        q.e0 = (uint32_t)q.bt * (RCAP * 32) + q.lane;
+        q.step = 32;
+        if (q.bt < sp.ntiles) {
+            const int n = sp.cnt[q.bt * 32 + q.lane];
+            q.n = n >= CNT_HEAVY ? -1 : n;  // -1: the single-kernel pass's tile, or k_heavy's sample
+            q.dst = n == RCAP ? sp.head[q.bt * 32 + q.lane] : -1;
+            if (sp.mlist && q.dst >= 0) q.n = -1;  // k_seq's
+        } else {
+            q.n = -1;
+        }
+        return q;
+    }
+    const unsigned c = (blockIdx.x - nlist) * blockDim.x + threadIdx.x;
+    const unsigned used = min(*sp.top, sp.ncap);
+    q.bt = 0;
+    q.chunk = (int32_t)c;
+    q.e0 = sp.ebase + c * RCAP;
+    q.step = 1;
+    q.n = -1;
+    if (c < used) {
+        const uint32_t w = sp.own[c], o = w & OWN_IDX;
+        if (w != OWN_NONE) {
+            q.bt = o >> 5;
+            q.lane = (int)(o & 31);
+            const int n = sp.cnt[o];
+            // a sample handed to k_heavy leaves the chunks of its tile's walk behind
+            if (n != CNT_DEAD && (n == CNT_HEAVY) == ((w & OWN_HEAVY) != 0)) {
+                q.n = sp.ccnt[c];
+                q.dst = (int32_t)c;
+            }
+        }
+    }
+    return q;
+}
+
 template <class T, int PREC, int ST, int KC, int KF, bool DG>
-__global__ void __launch_bounds__(128, (KC <= 4) ? 4 : 2) k_bodies(const Args<T> A) {
+__global__ void __launch_bounds__(128, (KC <= 4) ? 4 : 2) k_bodies(const Args<T> A, unsigned nlist) {
     using CT = typename std::conditional<PREC == PREC_FP64, double, float>::type;
     using Acc = typename std::conditional<PREC == PREC_FP64, PlainD, KahanF>::type;
     constexpr bool BAND = (PREC == PREC_FP32C) && (sizeof(T) == 8);
     constexpr bool SHIFT = (PREC == PREC_FP32C);
     constexpr bool EXS = BAND && KF == 1;  // column shifts formed in double (span_shift), from k_collect
     const TreeView<T>& tv = A.tv;
-    const int lane = threadIdx.x & 31;
-    const int wib = threadIdx.x >> 5;
-    const int64_t bt = (int64_t)blockIdx.x * (blockDim.x >> 5) + wib;
-    if (bt >= A.sp.ntiles) return;  // warp-uniform
-    const int n = A.sp.cnt[bt * 32 + lane];
-    if (n == 0xFF) return;  // overflowed tile (every lane): the single-kernel pass owns it
+    const ListPart Q = list_part(A.sp, nlist);
+    if (!__any_sync(PSB_FULL, Q.n >= 0)) return;
+    const int n = max(Q.n, 0);
+    const int64_t bt = Q.bt;
+    const int lane = Q.lane;  // the sample's lane in its tile
     const int64_t tile = A.sp.tile0 + bt;
-    const int64_t k = sample_of(A.src, tile, lane);
+    const int64_t k = Q.n >= 0 ? sample_of(A.src, tile, lane) : -1;
     const bool valid = k >= 0;
     T p[3] = {T(0), T(0), T(0)}, dd[3];
     if (valid) sample_coords(A.src, k, p, dd);
@@ -383,8 +913,14 @@ __global__ void __launch_bounds__(128, (KC <= 4) ? 4 : 2) k_bodies(const Args<T>
     const double ika = (KF == 1 && ST != ST_SCATTER) ? 0.5 / (double)ha : 0.0;  // Wendland pair terms
     const float qe = (KF == 0) ? 1.f : tv.qedge;
     Acc S1, G[3], Sw[KC], Sg[KC][3], Dm, Dg[3];
+    // FP32C sums are of A - A0, A0 the column values of the sample's first
+    // accepted leaf (the first pair of its list)
     CT a0[KC];
-    bool have0 = false;
+    int64_t first = -1;
+    if (SHIFT && n > 0) {
+        const size_t q0 = (size_t)bt * RCAP * 32 + lane;
+        first = (int64_t)__float_as_int(A.sp.ent4[q0].w) + __ffs(A.sp.emask[q0]) - 1;
+    }
     S1.zero(); Dm.zero();
 #pragma unroll
     for (int d = 0; d < 3; ++d) { G[d].zero(); Dg[d].zero(); }
@@ -392,53 +928,43 @@ __global__ void __launch_bounds__(128, (KC <= 4) ? 4 : 2) k_bodies(const Args<T>
     for (int c = 0; c < KC; ++c) {
         Sw[c].zero();
         a0[c] = CT(0);
+        if (SHIFT && !EXS && first >= 0 && c < kc) a0[c] = (CT)__ldg(&A.colF[c][first]);
 #pragma unroll
         for (int d = 0; d < 3; ++d) Sg[c][d].zero();
     }
 
-    // Kernel weights and sums of one pair; weights as in k_points.
-    // (FP32C: every product rounded on its own, as in k_points; FP64 as written)
-    auto mul = [](CT a, CT b) -> CT {
-        if constexpr (std::is_same<CT, float>::value) return __fmul_rn(a, b);
-        else return a * b;
-    };
-    auto sub = [](CT a, CT b) -> CT {
-        if constexpr (std::is_same<CT, float>::value) return __fsub_rn(a, b);
-        else return a - b;
-    };
+    // Kernel weights and sums of one pair; weights as in k_points, every
+    // rounding spelled out (acc_mul, acc_mac).
     auto accumulate = [&](const auto& col, CT dx, CT dy, CT dz, CT Wsum, CT csum, CT mr, CT mb) {
-        const CT w = mul(mr, Wsum);
-        const CT gc = mul(mr, csum);
-        const CT gx = mul(gc, dx), gy = mul(gc, dy), gz = mul(gc, dz);
+        const CT w = acc_mul(mr, Wsum);
+        const CT gc = acc_mul(mr, csum);
+        const CT gx = acc_mul(gc, dx), gy = acc_mul(gc, dy), gz = acc_mul(gc, dz);
         S1.add(w);
         G[0].add(gx); G[1].add(gy); G[2].add(gz);
-        if (SHIFT && !EXS && !have0) {
-            have0 = true;
-#pragma unroll
-            for (int c = 0; c < KC; ++c)
-                if (c < kc) a0[c] = (CT)col[c];
-        }
 #pragma unroll
         for (int c = 0; c < KC; ++c) {
             if (c < kc) {
                 CT a = (CT)col[c];  // EXS: already A - A0
-                if constexpr (SHIFT && !EXS) a = sub(a, a0[c]);
-                Sw[c].add(mul(a, w));
-                Sg[c][0].add(mul(a, gx)); Sg[c][1].add(mul(a, gy)); Sg[c][2].add(mul(a, gz));
+                if constexpr (SHIFT && !EXS) a = __fsub_rn(a, a0[c]);
+                acc_mac(Sw[c], a, w);
+                acc_mac(Sg[c][0], a, gx); acc_mac(Sg[c][1], a, gy); acc_mac(Sg[c][2], a, gz);
             }
         }
         if (need_dg) {
-            Dm.add(mul(mb, Wsum));
-            const CT mc = mul(mb, csum);
-            Dg[0].add(mul(mc, dx)); Dg[1].add(mul(mc, dy)); Dg[2].add(mul(mc, dz));
+            acc_mac(Dm, mb, Wsum);
+            const CT mc = acc_mul(mb, csum);
+            acc_mac(Dg[0], mc, dx); acc_mac(Dg[1], mc, dy); acc_mac(Dg[2], mc, dz);
         }
     };
 
     // The pairs of this lane's list, one ahead: the loads of the next pair are
     // in flight while the current pair is summed.
-    const float4* ent4 = A.sp.ent4 + (size_t)bt * RCAP * 32 + lane;
-    const uint32_t* emask = A.sp.emask + (size_t)bt * RCAP * 32 + lane;
-    const float* esh = EXS ? A.sp.eshift + (size_t)bt * RCAP * kc * 32 + lane : nullptr;
+    const float4* ent4 = A.sp.ent4 + Q.e0;
+    const uint32_t* emask = A.sp.emask + Q.e0;
+    const float* esh = !EXS ? nullptr
+                       : Q.chunk < 0 ? A.sp.eshift + (size_t)bt * RCAP * kc * 32 + lane
+                                     : A.sp.eshift + (size_t)Q.e0 * kc;
+    const int est = Q.step;
     int e = 0;
     unsigned m = 0;
     int64_t lo = 0;
@@ -446,18 +972,18 @@ __global__ void __launch_bounds__(128, (KC <= 4) ? 4 : 2) k_bodies(const Args<T>
     float sh[KC];          // EXS: the entry's column shifts A[lo] - A0 (written by k_collect)
 #pragma unroll
     for (int c = 0; c < KC; ++c) sh[c] = 0.f;
-    PairData<T, BAND, KC> nx;
+    PairData<T, PREC, KC> nx;
     bool hn = false;
     auto fetch = [&]() {
         if (m == 0 && e < n) {
-            const float4 q = ent4[(size_t)e * 32];
-            m = emask[(size_t)e * 32];  // never 0: k_collect writes entries with accepted leaves only
+            const float4 q = ent4[e * est];
+            m = emask[e * est];  // never 0: k_collect writes entries with accepted leaves only
             ++e;
             lo = (int64_t)__float_as_int(q.w);
             Rs[0] = q.x; Rs[1] = q.y; Rs[2] = q.z;
             if constexpr (EXS) {
 #pragma unroll
-                for (int c = 0; c < KC; ++c) sh[c] = (c < kc) ? esh[((size_t)(e - 1) * kc + c) * 32] : 0.f;
+                for (int c = 0; c < KC; ++c) sh[c] = (c < kc) ? esh[((e - 1) * kc + c) * est] : 0.f;
             }
         }
         hn = m != 0;
@@ -471,7 +997,7 @@ __global__ void __launch_bounds__(128, (KC <= 4) ? 4 : 2) k_bodies(const Args<T>
     fetch();
     while (__any_sync(PSB_FULL, hn)) {
         const bool hc = hn;
-        PairData<T, BAND, KC> cur = nx;
+        PairData<T, PREC, KC> cur = nx;
         if constexpr (EXS) {
             // A - A0: the shifts of cur's entry (fetch may start the next one);
             // added here, an iteration after the loads, not as they return
@@ -496,49 +1022,350 @@ __global__ void __launch_bounds__(128, (KC <= 4) ? 4 : 2) k_bodies(const Args<T>
                 },
                 [&]() { return __dmul_rn(tv.Kd, cur.hd); }, Wsum, csum);
             accumulate(cur.col, dx, dy, dz, Wsum, csum, cur.K.w, cur.mb);
-        } else {
-            const T e2 = ex_d2_pp<T>(p, cur.x, cur.y, cur.z);
-            const CT d2 = (CT)e2;
-            const CT r = sqrt(d2);
-            const CT invr = (d2 > CT(0)) ? CT(1) / r : CT(0);
-            CT Wsum = CT(0), csum = CT(0);
-            if (ST != ST_SCATTER) {
-                CT f, df;
-                kfdf<KF, CT>(tv.kern, r * ia, f, df);
-                Wsum = sa3 * f;
-                csum = sa4 * df * invr;
-            }
-            if (ST != ST_GATHER) {
-                const CT hb = (CT)cur.h;
-                CT ib = CT(1) / hb;
-                CT sb3 = sig * ib * ib * ib;
-                CT f, df;
-                kfdf<KF, CT>(tv.kern, r * ib, f, df);
-                CT Wb = sb3 * f, cb = sb3 * ib * df * invr;
-                if (ST == ST_SCATTER) { Wsum = Wb; csum = cb; }
-                else { Wsum = CT(0.5) * (Wsum + Wb); csum = CT(0.5) * (csum + cb); }
-            }
-            const CT mb = (CT)cur.m;
-            const CT mr = (CT)((double)cur.m / (double)cur.rho);
+        } else if constexpr (PREC == PREC_FP64) {
+            const double dx = __dsub_rn((double)p[0], cur.a.x), dy = __dsub_rn((double)p[1], cur.a.y),
+                         dz = __dsub_rn((double)p[2], cur.b.x);
+            double W, cg;
+            f64_pair_weights<ST, KF>(tv.kern, dx, dy, dz, ia, sa3, cur.b.y, cur.s.x, W, cg);
             CT cc[KC];
 #pragma unroll
             for (int c = 0; c < KC; ++c) cc[c] = (CT)cur.col[c];
-            accumulate(cc, (CT)(p[0] - cur.x), (CT)(p[1] - cur.y), (CT)(p[2] - cur.z), Wsum, csum, mr, mb);
+            accumulate(cc, dx, dy, dz, W, cg, cur.s.y, (CT)cur.mb);
+        } else {
+            float W, cg;
+            const float dx = __fsub_rn(p[0], cur.L.x), dy = __fsub_rn(p[1], cur.L.y), dz = __fsub_rn(p[2], cur.L.z);
+            f32_pair_weights<ST, KF>(tv.kern, ex_d2_pp<T>(p, cur.L.x, cur.L.y, cur.L.z), ia, sa3, sa4, cur.K.x,
+                                     cur.K.y, W, cg);
+            accumulate(cur.col, dx, dy, dz, W, cg, cur.K.w, cur.mb);
         }
     }
 
-    if (valid) {
-        // EXS: A0 are the column values of the first accepted leaf (the first
-        // pair of the first entry)
-        int64_t first = -1;
-        if (EXS && n > 0) first = (int64_t)__float_as_int(ent4[0].w) + __ffs(emask[0]) - 1;
+    if (valid && Q.dst >= 0) {
+        // one of several parts: its sums, folded by k_fold
+        double* o = A.sp.part + (Q.chunk < 0 ? A.sp.ncap : 0) + Q.dst;
+        const size_t fs = 2 * (size_t)A.sp.ncap;  // distance of fields
+        o[0] = S1.get();
+#pragma unroll
+        for (int d = 0; d < 3; ++d) o[(1 + d) * fs] = G[d].get();
+        if (DG) {
+            o[4 * fs] = Dm.get();
+#pragma unroll
+            for (int d = 0; d < 3; ++d) o[(5 + d) * fs] = Dg[d].get();
+        }
+#pragma unroll
+        for (int c = 0; c < KC; ++c) {
+            o[(8 + c) * fs] = Sw[c].get();
+#pragma unroll
+            for (int d = 0; d < 3; ++d) o[(8 + KC + 3 * c + d) * fs] = Sg[c][d].get();
+        }
+    } else if (valid) {
         double a0o[KC];
 #pragma unroll
         for (int c = 0; c < KC; ++c)
             a0o[c] = EXS ? ((c < kc && first >= 0) ? (double)A.colT[c][first] : 0.0) : (double)a0[c];
         write_interp_outputs<T, Acc, CT, KC>(A, k, S1, G, Sw, Sg, Dm, Dg, a0o);
     }
-    if (lane == 0 && A.stats) atomicAdd(&A.stats[5], n_bodyit);
+    if ((threadIdx.x & 31) == 0 && A.stats) atomicAdd(&A.stats[5], n_bodyit);
+}
+
+// The density sums over the pair lists (psb_density: sum m W, or sum W with
+// unit masses), one lane per sample as in k_bodies, with the arithmetic and
+// order of k_points' density.  One sum and no gradient fit 64 registers, so
+// the pair loads are hidden by 8 CTAs per SM; the single kernel summed span
+// by span behind its walk with a third of its lanes busy
+// (1M clump particles, gather at the particles: 10.4 ms in k_points; now the
+// walk, k_heavy and this kernel take 3.5 ms).
+template <class T, int PREC, int ST, int KF>
+__global__ void __launch_bounds__(128, 8) k_density(const Args<T> A, unsigned nlist) {
+    using CT = typename std::conditional<PREC == PREC_FP64, double, float>::type;
+    using Acc = typename std::conditional<PREC == PREC_FP64, PlainD, KahanF>::type;
+    constexpr bool BAND = (PREC == PREC_FP32C) && (sizeof(T) == 8);
+    const TreeView<T>& tv = A.tv;
+    const ListPart Q = list_part(A.sp, nlist);
+    if (Q.n < 0) return;
+    const int n = Q.n;
+    const int64_t k = sample_of(A.src, A.sp.tile0 + Q.bt, Q.lane);
+    if (k < 0) return;
+    T p[3], dd[3];
+    sample_coords(A.src, k, p, dd);
+    const T ha = ((const T*)A.sp.ha)[Q.bt * 32 + Q.lane];
+    const CT sig = (KF == 0) ? inv_pi<CT>() : (CT)tv.sig;
+    CT ia = CT(0), sa3 = CT(0), sa4 = CT(0);
+    if (ST != ST_SCATTER) {
+        ia = CT(1) / (CT)ha;
+        sa3 = sig * ia * ia * ia;
+        sa4 = sa3 * ia;
+    }
+    const double kha = tv.Kd * (double)ha;
+    const double fa2 = kha * kha;
+    const double ika = (KF == 1 && ST != ST_SCATTER) ? 0.5 / (double)ha : 0.0;
+    const float qe = (KF == 0) ? 1.f : tv.qedge;
+    const bool unit = A.unit_mass != 0;
+    Acc D;
+    D.zero();
+    const float4* ent4 = A.sp.ent4 + Q.e0;
+    const uint32_t* emask = A.sp.emask + Q.e0;
+    const int est = Q.step;
+    PairData<T, PREC, 1> nx;
+    float Rs[3] = {0.f, 0.f, 0.f};
+    int e = 0;
+    unsigned m = 0;
+    int64_t lo = 0;
+    auto fetch = [&]() -> bool {
+        if (m == 0) {
+            if (e >= n) return false;
+            const float4 q = ent4[e * est];
+            m = emask[e * est];
+            ++e;
+            lo = (int64_t)__float_as_int(q.w);
+            Rs[0] = q.x; Rs[1] = q.y; Rs[2] = q.z;
+        }
+        const int j = __ffs(m) - 1;
+        m &= m - 1;
+        nx.load(tv, A, lo + j, 0, !unit, Rs, nullptr);
+        return true;
+    };
+    bool has = fetch();
+    while (has) {
+        const PairData<T, PREC, 1> cur = nx;
+        has = fetch();
+        CT W, c;
+        if constexpr (BAND) {
+            f32c_pair_weights<ST, KF>(
+                tv.kern, tv.Kf, qe, __fsub_rn(cur.r[0], cur.L.x), __fsub_rn(cur.r[1], cur.L.y),
+                __fsub_rn(cur.r[2], cur.L.z), (float)ia, (float)sa3, (float)sa4, fa2, ika, (float)ha, cur.K, cur.L.w,
+                [&]() {
+                    const double ex = __dsub_rn((double)p[0], cur.xd);
+                    const double ey = __dsub_rn((double)p[1], cur.yd);
+                    const double ez = __dsub_rn((double)p[2], cur.zd);
+                    return __fma_rn(ex, ex, __fma_rn(ey, ey, __dmul_rn(ez, ez)));
+                },
+                [&]() { return __dmul_rn(tv.Kd, cur.hd); }, W, c);
+        } else if constexpr (PREC == PREC_FP64) {
+            f64_pair_weights<ST, KF>(tv.kern, __dsub_rn((double)p[0], cur.a.x), __dsub_rn((double)p[1], cur.a.y),
+                                     __dsub_rn((double)p[2], cur.b.x), ia, sa3, cur.b.y, cur.s.x, W, c);
+        } else {
+            f32_pair_weights<ST, KF>(tv.kern, ex_d2_pp<T>(p, cur.L.x, cur.L.y, cur.L.z), ia, sa3, sa4, cur.K.x,
+                                     cur.K.y, W, c);
+        }
+        acc_mac(D, unit ? CT(1) : (CT)cur.mb, W);
+    }
+    if (Q.dst >= 0) A.sp.part[(Q.chunk < 0 ? A.sp.ncap : 0) + Q.dst] = D.get();
+    else A.out[0][k] = (PREC == PREC_FP64) ? (T)D.get() : (T)(CT)D.get();
+}
+
+// The samples of several list parts: the list's sums, then the chunks' in the
+// chain's order, added up; then the outputs (all but FP32C of double
+// particles, see k_seq).  One thread per chunk of the pool; a sample's first
+// chunk does the work.  WHAT is k_points'.
+template <class T, int PREC, int KC, int WHAT>
+__global__ void __launch_bounds__(128) k_fold(const Args<T> A) {
+    using CT = typename std::conditional<PREC == PREC_FP64, double, float>::type;
+    const unsigned c0 = blockIdx.x * blockDim.x + threadIdx.x;
+    if (c0 >= min(*A.sp.top, A.sp.ncap)) return;
+    const uint32_t w = A.sp.own[c0], own = w & OWN_IDX;
+    if (w & OWN_LATER) return;  // a later chunk, or none
+    const int cn = A.sp.cnt[own];
+    const bool heavy = (w & OWN_HEAVY) != 0;
+    if (cn == CNT_DEAD || (cn == CNT_HEAVY) != heavy) return;
+    const int64_t k = sample_of(A.src, A.sp.tile0 + (own >> 5), own & 31);
+    if (k < 0) return;
+    // the first part: the tile's list, or a heavy sample's first chunk
+    const size_t f0 = heavy ? c0 : A.sp.ncap + c0;
+    const int32_t c1 = heavy ? A.sp.next[c0] : (int32_t)c0;
+    const size_t fs = 2 * (size_t)A.sp.ncap;
+    if (WHAT == WHAT_DENSITY) {
+        double t = A.sp.part[f0];
+        for (int32_t c = c1; c >= 0; c = A.sp.next[c]) t = __dadd_rn(t, A.sp.part[c]);
+        A.out[0][k] = (PREC == PREC_FP64) ? (T)t : (T)(CT)t;
+        return;
+    }
+    constexpr int NF = 8 + 4 * KC;
+    double t[NF];
+    const bool dg = A.rec.need_dg != 0;
+#pragma unroll
+    for (int q = 0; q < NF; ++q) t[q] = (q >= 4 && q < 8 && !dg) ? 0.0 : A.sp.part[q * fs + f0];
+    for (int32_t c = c1; c >= 0; c = A.sp.next[c]) {
+#pragma unroll
+        for (int q = 0; q < NF; ++q)
+            if (!(q >= 4 && q < 8) || dg) t[q] = __dadd_rn(t[q], A.sp.part[q * fs + c]);
+    }
+    PlainD S1, G[3], Dm, Dg[3], Sw[KC], Sg[KC][3];
+    S1.s = t[0];
+    Dm.s = t[4];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) { G[d].s = t[1 + d]; Dg[d].s = t[5 + d]; }
+    double a0[KC];
+    const size_t q0 = (size_t)(own >> 5) * RCAP * 32 + (own & 31);
+    const int64_t first = (int64_t)__float_as_int(A.sp.ent4[q0].w) + __ffs(A.sp.emask[q0]) - 1;
+#pragma unroll
+    for (int c = 0; c < KC; ++c) {
+        Sw[c].s = t[8 + c];
+#pragma unroll
+        for (int d = 0; d < 3; ++d) Sg[c][d].s = t[8 + KC + 3 * c + d];
+        a0[c] = (PREC == PREC_FP64 || c >= A.rec.kc) ? 0.0
+                : (double)A.colF[c][first];
+    }
+    write_interp_outputs<T, PlainD, CT, KC>(A, k, S1, G, Sw, Sg, Dm, Dg, a0);
+}
+
+// The FP32C sums of double particles' samples of several list parts: one warp
+// per sample, the parts in order.  Lane j of an entry evaluates the weights of
+// the entry's leaf j, with k_bodies' arithmetic; then each compensated sum runs
+// through the entry's pairs in leaf order in a lane of its own (4 + 4 kc sums,
+// 4 more with a density gradient, two to a lane past 32).  The sums have the
+// bits of one lane adding pair after pair, without its other 31 lanes idle.
+constexpr int SEQ_COMP = 8;              // weights of a pair: w, w d (3); with a density gradient m W, m W' d (3)
+constexpr int SEQ_ROWS = SEQ_COMP + MAX_KC;
+template <int ST, int KF, int WHAT>
+__global__ void __launch_bounds__(128) k_seq(const __grid_constant__ Args<double> A) {
+    constexpr bool EXS = KF == 1;
+    __shared__ float rows_all[4][SEQ_ROWS][33];  // [component or column][leaf]
+    __shared__ double sums_all[4][8 + 4 * MAX_KC];
+    const TreeView<double>& tv = A.tv;
+    const SplitBufs& sp = A.sp;
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    auto& rows = rows_all[wib];
+    auto& sums = sums_all[wib];
+    const int kc = (WHAT == WHAT_DENSITY) ? 0 : A.rec.kc;
+    const bool dg = WHAT == WHAT_INTERP && A.rec.need_dg != 0;
+    const bool unit = WHAT == WHAT_DENSITY && A.unit_mass != 0;
+    // the sums of this lane: component ra of a pair times column rb (-1: none), to field fo of the outputs
+    const int nsum = (WHAT == WHAT_DENSITY) ? 1 : 4 + 4 * kc + (dg ? 4 : 0);
+    int ra[2], rb[2], fo[2];
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+        const int q = lane + 32 * u;
+        ra[u] = 0; rb[u] = -1; fo[u] = -1;
+        if (q >= nsum) continue;
+        if (q < 4) { ra[u] = q; fo[u] = q; }
+        else if (q < 4 + 4 * kc) {
+            const int c = (q - 4) >> 2, d = (q - 4) & 3;
+            ra[u] = d; rb[u] = SEQ_COMP + c;
+            fo[u] = d == 0 ? 8 + c : 8 + MAX_KC + 3 * c + d - 1;
+        } else { ra[u] = 4 + (q - 4 - 4 * kc); fo[u] = 4 + (q - 4 - 4 * kc); }
+    }
+    const bool two = nsum > 32;
+    const unsigned nm = min(*sp.mcount, sp.ncap);
+    const unsigned nw = gridDim.x * (blockDim.x >> 5);
+    for (unsigned i = blockIdx.x * (blockDim.x >> 5) + wib; i < nm; i += nw) {
+        const uint32_t c0 = sp.mlist[i];
+        const uint32_t w0 = sp.own[c0], own = w0 & OWN_IDX;
+        const int cn = sp.cnt[own];
+        const bool heavy = (w0 & OWN_HEAVY) != 0;
+        if (cn == CNT_DEAD || (cn == CNT_HEAVY) != heavy) continue;  // warp-uniform
+        const int64_t k = sample_of(A.src, sp.tile0 + (own >> 5), own & 31);
+        if (k < 0) continue;
+        double p[3], dd[3];
+        sample_coords(A.src, k, p, dd);
+        const double ha = ((const double*)sp.ha)[own];
+        const float sig = (KF == 0) ? inv_pi<float>() : (float)tv.sig;
+        float ia = 0.f, sa3 = 0.f, sa4 = 0.f;
+        if (ST != ST_SCATTER) {
+            ia = 1.f / (float)ha;
+            sa3 = sig * ia * ia * ia;
+            sa4 = sa3 * ia;
+        }
+        const double kha = tv.Kd * ha;
+        const double fa2 = kha * kha;
+        const double ika = (KF == 1 && ST != ST_SCATTER) ? 0.5 / ha : 0.0;
+        const float qe = (KF == 0) ? 1.f : tv.qedge;
+        const size_t q0 = (size_t)(own >> 5) * RCAP * 32 + (own & 31);
+        const int64_t first = (int64_t)__float_as_int(sp.ent4[q0].w) + __ffs(sp.emask[q0]) - 1;
+        KahanF S[2];
+        S[0].zero();
+        S[1].zero();
+        // parts: the tile's list (not a heavy sample's), then the chunks
+        int32_t chunk = heavy ? (int32_t)c0 : -1;
+        while (true) {
+            const int n = chunk < 0 ? RCAP : sp.ccnt[chunk];
+            const size_t e0 = chunk < 0 ? q0 : (size_t)sp.ebase + (size_t)chunk * RCAP;
+            const int est = chunk < 0 ? 32 : 1;
+            const float* esh = !EXS || kc == 0 ? nullptr
+                               : chunk < 0 ? sp.eshift + (size_t)(own >> 5) * RCAP * kc * 32 + (own & 31)
+                                           : sp.eshift + e0 * kc;
+            for (int e = 0; e < n; ++e) {
+                const float4 q = sp.ent4[e0 + (size_t)e * est];
+                const unsigned m = sp.emask[e0 + (size_t)e * est];
+                const int64_t lo = (int64_t)__float_as_int(q.w);
+                __syncwarp();
+                if ((m >> lane) & 1u) {
+                    const int64_t li = lo + lane;
+                    const float4 L = __ldg(&tv.leaf4[li]), K = __ldg(&tv.leafK[li]);
+                    const float dx = __fsub_rn(q.x, L.x), dy = __fsub_rn(q.y, L.y), dz = __fsub_rn(q.z, L.z);
+                    float W, c;
+                    f32c_pair_weights<ST, KF>(
+                        tv.kern, tv.Kf, qe, dx, dy, dz, ia, sa3, sa4, fa2, ika, (float)ha, K, L.w,
+                        [&]() {
+                            const double ex = __dsub_rn(p[0], __ldg(&tv.x[li]));
+                            const double ey = __dsub_rn(p[1], __ldg(&tv.y[li]));
+                            const double ez = __dsub_rn(p[2], __ldg(&tv.z[li]));
+                            return __fma_rn(ex, ex, __fma_rn(ey, ey, __dmul_rn(ez, ez)));
+                        },
+                        [&]() { return __dmul_rn(tv.Kd, __ldg(&tv.h[li])); }, W, c);
+                    if (WHAT == WHAT_DENSITY) {
+                        rows[0][lane] = __fmul_rn(unit ? 1.f : __ldg(&tv.mf[li]), W);
+                    } else {
+                        const float gc = __fmul_rn(K.w, c);
+                        rows[0][lane] = __fmul_rn(K.w, W);
+                        rows[1][lane] = __fmul_rn(gc, dx);
+                        rows[2][lane] = __fmul_rn(gc, dy);
+                        rows[3][lane] = __fmul_rn(gc, dz);
+                        if (dg) {
+                            const float mb = __ldg(&tv.mf[li]), mc = __fmul_rn(mb, c);
+                            rows[4][lane] = __fmul_rn(mb, W);
+                            rows[5][lane] = __fmul_rn(mc, dx);
+                            rows[6][lane] = __fmul_rn(mc, dy);
+                            rows[7][lane] = __fmul_rn(mc, dz);
+                        }
+                        for (int s = 0; s < kc; ++s)
+                            rows[SEQ_COMP + s][lane] =
+                                EXS ? __fadd_rn(__ldg(&A.colR[s][li]), esh[(e * kc + s) * est])
+                                    : __fsub_rn(__ldg(&A.colF[s][li]), __ldg(&A.colF[s][first]));
+                    }
+                }
+                __syncwarp();
+#pragma unroll 4
+                for (unsigned b = m; b; b &= b - 1) {
+                    const int j = __ffs(b) - 1;
+                    const float v = rows[ra[0]][j];
+                    S[0].add(rb[0] < 0 ? v : __fmul_rn(rows[rb[0]][j], v));
+                    if (two) {
+                        const float v1 = rows[ra[1]][j];
+                        S[1].add(rb[1] < 0 ? v1 : __fmul_rn(rows[rb[1]][j], v1));
+                    }
+                }
+            }
+            chunk = chunk < 0 ? (int32_t)c0 : sp.next[chunk];
+            if (chunk < 0) break;
+        }
+#pragma unroll
+        for (int u = 0; u < 2; ++u)
+            if (fo[u] >= 0) sums[fo[u]] = S[u].get();
+        __syncwarp();
+        if (lane == 0) {
+            if (WHAT == WHAT_DENSITY) {
+                A.out[0][k] = (double)(float)sums[0];
+            } else {
+                PlainD S1, G[3], Dm, Dg[3], Sw[MAX_KC], Sg[MAX_KC][3];
+                double a0[MAX_KC];
+                S1.s = sums[0];
+                Dm.s = dg ? sums[4] : 0.0;
+                for (int d = 0; d < 3; ++d) {
+                    G[d].s = sums[1 + d];
+                    Dg[d].s = dg ? sums[5 + d] : 0.0;
+                }
+                for (int c = 0; c < MAX_KC; ++c) {
+                    const bool on = c < kc;
+                    Sw[c].s = on ? sums[8 + c] : 0.0;
+                    for (int d = 0; d < 3; ++d) Sg[c][d].s = on ? sums[8 + MAX_KC + 3 * c + d] : 0.0;
+                    a0[c] = !on ? 0.0 : (EXS ? A.colT[c][first] : (double)A.colF[c][first]);
+                }
+                write_interp_outputs<double, PlainD, float, MAX_KC>(A, k, S1, G, Sw, Sg, Dm, Dg, a0);
+            }
+        }
+        __syncwarp();
+    }
 }
 
 }  // namespace psb

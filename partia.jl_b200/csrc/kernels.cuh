@@ -178,6 +178,67 @@ __device__ __forceinline__ void wendland_fdf_f32(int k, float q, float a, float&
     }
 }
 
+// f(q) and f'(q)/r of the FP64 pair sums, K - q and the like in double.  The
+// gradient factor comes as f'/r, so that pieces whose f' carries a factor q
+// need no 1/r (q/r = 1/h = ih); ir = 1/r (0 at r = 0, where the separation it
+// multiplies is 0 too).  Every rounding is spelled out, as in the float pair
+// terms: the pair-sum kernel and the single kernel give a pair the same bits
+// whatever code they are inlined into.
+__device__ __forceinline__ void m4_fdr_f64(double q, double ih, double ir, double& f, double& dr) {
+    if (q < 1.0) {
+        f = __fma_rn(__dmul_rn(q, q), __fma_rn(0.75, q, -1.5), 1.0);
+        dr = __dmul_rn(ih, __fma_rn(2.25, q, -3.0));
+    } else {
+        const double a = fmax(__dsub_rn(2.0, q), 0.0), a2 = __dmul_rn(a, a);
+        f = __dmul_rn(__dmul_rn(0.25, a2), a);
+        dr = __dmul_rn(__dmul_rn(-0.75, a2), ir);
+    }
+}
+__device__ __forceinline__ void kern_fdr_f64(int k, double q, double ih, double ir, double& f, double& dr) {
+    f = 0.0;
+    dr = 0.0;
+    if (k == KERN_M5) {
+        const double a = fmax(__dsub_rn(2.5, q), 0.0), b = fmax(__dsub_rn(1.5, q), 0.0);
+        if (q < 0.5) {  // 14.375 - 15 q^2 + 6 q^4
+            const double q2 = __dmul_rn(q, q);
+            f = __fma_rn(q2, __fma_rn(6.0, q2, -15.0), 14.375);
+            dr = __dmul_rn(ih, __fma_rn(24.0, q2, -30.0));
+        } else {
+            const double a3 = __dmul_rn(__dmul_rn(a, a), a), b3 = __dmul_rn(__dmul_rn(b, b), b);
+            f = __fma_rn(-5.0, __dmul_rn(b3, b), __dmul_rn(a3, a));
+            dr = __dmul_rn(__fma_rn(20.0, b3, __dmul_rn(-4.0, a3)), ir);
+        }
+    } else if (k == KERN_M6) {
+        const double a = fmax(__dsub_rn(3.0, q), 0.0), b = fmax(__dsub_rn(2.0, q), 0.0);
+        if (q < 1.0) {  // 66 - 60 q^2 + 30 q^4 - 10 q^5
+            const double q2 = __dmul_rn(q, q);
+            f = __fma_rn(q2, __fma_rn(q2, __fma_rn(-10.0, q, 30.0), -60.0), 66.0);
+            dr = __dmul_rn(ih, __fma_rn(q2, __fma_rn(-50.0, q, 120.0), -120.0));
+        } else {
+            const double a2 = __dmul_rn(a, a), b2 = __dmul_rn(b, b);
+            const double a4 = __dmul_rn(a2, a2), b4 = __dmul_rn(b2, b2);
+            f = __fma_rn(-6.0, __dmul_rn(b4, b), __dmul_rn(a4, a));
+            dr = __dmul_rn(__fma_rn(30.0, b4, __dmul_rn(-5.0, a4)), ir);
+        }
+    } else {  // Wendland: f' = q P(q) a^n, so f'/r = P(q) a^n / h
+        const double a = fmax(__fma_rn(-0.5, q, 1.0), 0.0), a2 = __dmul_rn(a, a);
+        if (k == KERN_C2) {
+            const double a3 = __dmul_rn(a2, a);
+            f = __dmul_rn(__dmul_rn(a3, a), __fma_rn(2.0, q, 1.0));
+            dr = __dmul_rn(__dmul_rn(-5.0, ih), a3);
+        } else if (k == KERN_C4) {
+            const double a5 = __dmul_rn(__dmul_rn(a2, a2), a);
+            f = __dmul_rn(__dmul_rn(a5, a), __fma_rn(__fma_rn(35.0 / 12.0, q, 3.0), q, 1.0));
+            dr = __dmul_rn(__dmul_rn(__dmul_rn(-14.0 / 3.0, ih), __fma_rn(2.5, q, 1.0)), a5);
+        } else {
+            const double a7 = __dmul_rn(__dmul_rn(__dmul_rn(a2, a2), a2), a);
+            const double pf = __fma_rn(__fma_rn(__fma_rn(4.0, q, 6.25), q, 4.0), q, 1.0);
+            f = __dmul_rn(__dmul_rn(a7, a), pf);
+            dr = __dmul_rn(__dmul_rn(__dmul_rn(-5.5, ih), __fma_rn(__fma_rn(4.0, q, 3.5), q, 1.0)), a7);
+        }
+    }
+}
+
 // g1 = f'(q)/q and g2 = d g1/dq for k != M4 (the adjoint's gradient and
 // Hessian factors): g2 = (f'' - g1)/q on the pieces away from q = 0; the
 // pieces that contain q = 0 are written without the division (M5 on q < 1/2

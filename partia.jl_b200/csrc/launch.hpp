@@ -2,6 +2,8 @@
 // instantiations are split over inst_*.cu so that they compile in parallel.
 #pragma once
 
+#include <algorithm>
+
 #include "k_split.cuh"
 
 namespace psb {
@@ -70,55 +72,104 @@ static cudaError_t dispatch_lines_p(const Args<T>& a, int st, int kc, int what, 
     return cudaGetLastError();
 }
 
-// two-kernel point path: k_collect (bodies = false) or k_bodies (bodies = true)
-// over the batch a.sp
+// two-kernel point path over the batch a.sp: the walk (k_collect, then k_heavy for its largest samples), the sums
+// over its lists (k_bodies, k_density; first the tiles' blocks,
+// then the chunks'), and the fold of the samples with chunks (k_fold)
+enum { SPLIT_WALK = 0, SPLIT_FIELDS = 1, SPLIT_DENSITY = 2, SPLIT_FOLD = 3, SPLIT_FOLD_DENSITY = 4, SPLIT_HEAVY = 5 };
 template <class T, int P, int S, int KF, bool DG>
-static void dispatch_bodies_kfd(const Args<T>& a, int kc, unsigned g, cudaStream_t s) {
-    if (kc <= 1) k_bodies<T, P, S, 1, KF, DG><<<g, 128, 0, s>>>(a);
-    else if (kc <= 2) k_bodies<T, P, S, 2, KF, DG><<<g, 128, 0, s>>>(a);
-    else if (kc <= 4) k_bodies<T, P, S, 4, KF, DG><<<g, 128, 0, s>>>(a);
-    else k_bodies<T, P, S, 8, KF, DG><<<g, 128, 0, s>>>(a);
+static void dispatch_bodies_kfd(const Args<T>& a, int kc, unsigned g, unsigned gc, cudaStream_t s) {
+    if (kc <= 1) k_bodies<T, P, S, 1, KF, DG><<<g + gc, 128, 0, s>>>(a, g);
+    else if (kc <= 2) k_bodies<T, P, S, 2, KF, DG><<<g + gc, 128, 0, s>>>(a, g);
+    else if (kc <= 4) k_bodies<T, P, S, 4, KF, DG><<<g + gc, 128, 0, s>>>(a, g);
+    else k_bodies<T, P, S, 8, KF, DG><<<g + gc, 128, 0, s>>>(a, g);
 }
 // DG: the catalog has a density gradient (its sums and the masses in
 // registers only where they are used)
 template <class T, int P, int S, int KF>
-static void dispatch_bodies_kf(const Args<T>& a, int kc, unsigned g, cudaStream_t s) {
-    if (a.rec.need_dg) dispatch_bodies_kfd<T, P, S, KF, true>(a, kc, g, s);
-    else dispatch_bodies_kfd<T, P, S, KF, false>(a, kc, g, s);
+static void dispatch_bodies_kf(const Args<T>& a, int kc, unsigned g, unsigned gc, cudaStream_t s) {
+    if (a.rec.need_dg) dispatch_bodies_kfd<T, P, S, KF, true>(a, kc, g, gc, s);
+    else dispatch_bodies_kfd<T, P, S, KF, false>(a, kc, g, gc, s);
 }
 template <class T, int P, int S>
-static void dispatch_bodies_k(const Args<T>& a, int kc, unsigned g, cudaStream_t s) {
-    if (a.tv.kern == KERN_M4) dispatch_bodies_kf<T, P, S, 0>(a, kc, g, s);
-    else dispatch_bodies_kf<T, P, S, 1>(a, kc, g, s);
+static void dispatch_bodies_k(const Args<T>& a, int kc, unsigned g, unsigned gc, cudaStream_t s) {
+    if (a.tv.kern == KERN_M4) dispatch_bodies_kf<T, P, S, 0>(a, kc, g, gc, s);
+    else dispatch_bodies_kf<T, P, S, 1>(a, kc, g, gc, s);
+}
+
+template <class T, int P, int S>
+static void dispatch_density_k(const Args<T>& a, unsigned g, unsigned gc, cudaStream_t s) {
+    if (a.tv.kern == KERN_M4) k_density<T, P, S, 0><<<g + gc, 128, 0, s>>>(a, g);
+    else k_density<T, P, S, 1><<<g + gc, 128, 0, s>>>(a, g);
+}
+
+// k_seq: enough warps to fill the GPU, each takes samples until none is left
+template <int S>
+static void dispatch_seq_s(const Args<double>& a, bool density, cudaStream_t s) {
+    const unsigned g = std::min(148u * 8u, (a.sp.ncap + 3) / 4);
+    const bool m4 = a.tv.kern == KERN_M4;
+    if (density) {
+        if (m4) k_seq<S, 0, WHAT_DENSITY><<<g, 128, 0, s>>>(a);
+        else k_seq<S, 1, WHAT_DENSITY><<<g, 128, 0, s>>>(a);
+    } else {
+        if (m4) k_seq<S, 0, WHAT_INTERP><<<g, 128, 0, s>>>(a);
+        else k_seq<S, 1, WHAT_INTERP><<<g, 128, 0, s>>>(a);
+    }
+}
+static inline void dispatch_seq(const Args<double>& a, int st, bool density, cudaStream_t s) {
+    if (st == ST_GATHER) dispatch_seq_s<ST_GATHER>(a, density, s);
+    else if (st == ST_SCATTER) dispatch_seq_s<ST_SCATTER>(a, density, s);
+    else dispatch_seq_s<ST_SYMMETRIC>(a, density, s);
 }
 
 template <class T, int P>
-static cudaError_t dispatch_split_p(const Args<T>& a, int st, int kc, bool bodies, cudaStream_t s) {
-    unsigned g = (unsigned)((a.sp.ntiles + 3) / 4);
+static cudaError_t dispatch_split_p(const Args<T>& a, int st, int kc, int pass, cudaStream_t s) {
+    // blocks of the tiles' lists and of the chunk pool
+    constexpr bool SEQ = sizeof(T) == 8 && P == PREC_FP32C;
+    const unsigned g = (unsigned)((a.sp.ntiles + 3) / 4), gc = SEQ ? 0 : (a.sp.ncap + 127) / 128;
     if (g == 0) return cudaSuccess;
-    if (!bodies) {
-        if (st == ST_GATHER) k_collect<T, P, ST_GATHER><<<g, 128, 0, s>>>(a);
-        else if (st == ST_SCATTER) k_collect<T, P, ST_SCATTER><<<g, 128, 0, s>>>(a);
-        else k_collect<T, P, ST_SYMMETRIC><<<g, 128, 0, s>>>(a);
+    if (pass == SPLIT_FOLD || pass == SPLIT_FOLD_DENSITY) {
+        if constexpr (SEQ) {
+            dispatch_seq(a, st, pass == SPLIT_FOLD_DENSITY, s);
+        } else {
+            if (pass == SPLIT_FOLD_DENSITY) k_fold<T, P, 1, WHAT_DENSITY><<<gc, 128, 0, s>>>(a);
+            else if (kc <= 1) k_fold<T, P, 1, WHAT_INTERP><<<gc, 128, 0, s>>>(a);
+            else if (kc <= 2) k_fold<T, P, 2, WHAT_INTERP><<<gc, 128, 0, s>>>(a);
+            else if (kc <= 4) k_fold<T, P, 4, WHAT_INTERP><<<gc, 128, 0, s>>>(a);
+            else k_fold<T, P, 8, WHAT_INTERP><<<gc, 128, 0, s>>>(a);
+        }
+    } else if (pass == SPLIT_HEAVY) {
+        auto kern = st == ST_GATHER ? k_heavy<T, ST_GATHER> : (st == ST_SCATTER ? k_heavy<T, ST_SCATTER> : k_heavy<T, ST_SYMMETRIC>);
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)HEAVY_SMEM);
+        if (e != cudaSuccess) return e;
+        kern<<<std::min(2 * 148u, a.sp.hcap), HEAVY_THREADS, HEAVY_SMEM, s>>>(a);
+    } else if (pass == SPLIT_WALK) {
+        const unsigned gw = (unsigned)(((a.sp.ntiles << (5 - a.sp.lspt)) + 3) / 4);
+        if (st == ST_GATHER) k_collect<T, ST_GATHER><<<gw, 128, 0, s>>>(a);
+        else if (st == ST_SCATTER) k_collect<T, ST_SCATTER><<<gw, 128, 0, s>>>(a);
+        else k_collect<T, ST_SYMMETRIC><<<gw, 128, 0, s>>>(a);
+    } else if (pass == SPLIT_DENSITY) {
+        if (st == ST_GATHER) dispatch_density_k<T, P, ST_GATHER>(a, g, gc, s);
+        else if (st == ST_SCATTER) dispatch_density_k<T, P, ST_SCATTER>(a, g, gc, s);
+        else dispatch_density_k<T, P, ST_SYMMETRIC>(a, g, gc, s);
     } else {
-        if (st == ST_GATHER) dispatch_bodies_k<T, P, ST_GATHER>(a, kc, g, s);
-        else if (st == ST_SCATTER) dispatch_bodies_k<T, P, ST_SCATTER>(a, kc, g, s);
-        else dispatch_bodies_k<T, P, ST_SYMMETRIC>(a, kc, g, s);
+        if (st == ST_GATHER) dispatch_bodies_k<T, P, ST_GATHER>(a, kc, g, gc, s);
+        else if (st == ST_SCATTER) dispatch_bodies_k<T, P, ST_SCATTER>(a, kc, g, gc, s);
+        else dispatch_bodies_k<T, P, ST_SYMMETRIC>(a, kc, g, gc, s);
     }
     return cudaGetLastError();
 }
 
 // defined in inst_*.cu
 template <class T> cudaError_t launch_points(const Args<T>& a, int prec, int st, int kc, int what, cudaStream_t s);
-cudaError_t launch_split_d0(const Args<double>& a, int st, int kc, bool bodies, cudaStream_t s);
-cudaError_t launch_split_d1(const Args<double>& a, int st, int kc, bool bodies, cudaStream_t s);
-cudaError_t launch_split_f0(const Args<float>& a, int st, int kc, bool bodies, cudaStream_t s);
-cudaError_t launch_split_f1(const Args<float>& a, int st, int kc, bool bodies, cudaStream_t s);
-inline cudaError_t launch_split(const Args<double>& a, int prec, int st, int kc, bool bodies, cudaStream_t s) {
-    return prec == PREC_FP64 ? launch_split_d0(a, st, kc, bodies, s) : launch_split_d1(a, st, kc, bodies, s);
+cudaError_t launch_split_d0(const Args<double>& a, int st, int kc, int pass, cudaStream_t s);
+cudaError_t launch_split_d1(const Args<double>& a, int st, int kc, int pass, cudaStream_t s);
+cudaError_t launch_split_f0(const Args<float>& a, int st, int kc, int pass, cudaStream_t s);
+cudaError_t launch_split_f1(const Args<float>& a, int st, int kc, int pass, cudaStream_t s);
+inline cudaError_t launch_split(const Args<double>& a, int prec, int st, int kc, int pass, cudaStream_t s) {
+    return prec == PREC_FP64 ? launch_split_d0(a, st, kc, pass, s) : launch_split_d1(a, st, kc, pass, s);
 }
-inline cudaError_t launch_split(const Args<float>& a, int prec, int st, int kc, bool bodies, cudaStream_t s) {
-    return prec == PREC_FP64 ? launch_split_f0(a, st, kc, bodies, s) : launch_split_f1(a, st, kc, bodies, s);
+inline cudaError_t launch_split(const Args<float>& a, int prec, int st, int kc, int pass, cudaStream_t s) {
+    return prec == PREC_FP64 ? launch_split_f0(a, st, kc, pass, s) : launch_split_f1(a, st, kc, pass, s);
 }
 template <class T> cudaError_t launch_lines(const Args<T>& a, int prec, int st, int kc, int what, cudaStream_t s);
 

@@ -90,6 +90,7 @@ template <class T> struct TreeView {
     int64_t n;
     int32_t root;
     const int32_t* left;     // 2n-1
+    const int32_t* right;    // 2n-1
     const int32_t* escape;   // 2n-1
     const int4* links;       // n-1: (left, escape, range_lo, range_hi) of internal nodes
     const uint64_t* codes;   // n sorted, de-duplicated Morton codes
@@ -113,6 +114,8 @@ template <class T> struct TreeView {
     const float* mrho;       // m / rho (float)
     const float* mf;         // m (float)
     const float4* leafK;     // (1/h, sigma/h^3, sigma/h^4, m/rho) in float
+    // FP64 pair sums: (x, y), (z, 1/h) and (sigma/h^3, m/rho) in double
+    const double2* leafD[3];
     // at the first leaf of every span: (max over the span of |leaf4.x| +
     // |leaf4.y| + |leaf4.z|, max h), both rounded up (float error bounds)
     const float2* spanb;

@@ -44,6 +44,11 @@ struct psb_ctx {
     float4* node_lo = nullptr; float4* node_hi = nullptr; float4* leaf4 = nullptr;
     float* mrho = nullptr; float* mf = nullptr;
     float4* leafK = nullptr;  // per leaf (1/h, sigma/h^3, sigma/h^4, m/rho), float
+    // FP64 pair sums, per leaf in double: (x, y), (z, 1/h), (sigma/h^3, m/rho)
+    double2* leafD[3] = {nullptr, nullptr, nullptr};
+    // coordinates and h lie in the range where the float tests of the walk are
+    // proven (build_typed); other sets are interpolated by the single kernel
+    bool band_ok = false;
     float2* spanb = nullptr;  // at a span's first leaf: (max |leaf4.xyz|_1, max h) over the span, rounded up
     float* colsf = nullptr;  // float copies of the columns (double inputs), ncol x n
     int32_t* sfirst = nullptr;  // first leaf of each leaf's span (double inputs)
@@ -59,7 +64,7 @@ struct psb_ctx {
 
     // reusable scratch (grown on demand, freed with the context)
     struct Slot { void* p = nullptr; size_t bytes = 0; };
-    Slot scratch[96];
+    Slot scratch[104];
     // sizes of the particle and tree buffers above, keyed by the address of
     // the pointer member: they are kept across set_particles and builds and
     // reallocated only to grow, so repeated builds of the same size (the
