@@ -20,4 +20,13 @@ template <> cudaError_t launch_lines<float>(const Args<float>& a, int prec, int 
     return prec == PREC_FP64 ? dispatch_lines_p<float, PREC_FP64>(a, st, kc, what, s)
                              : dispatch_lines_p<float, PREC_FP32C>(a, st, kc, what, s);
 }
+// defined in inst_line_tile_*.cu
+cudaError_t launch_line_tile_d0(const Args<double>&, int, int, bool, cudaStream_t);
+cudaError_t launch_line_tile_d1(const Args<double>&, int, int, bool, cudaStream_t);
+cudaError_t launch_line_tile(const Args<double>& a, int prec, int st, int kc, bool wide, cudaStream_t s) {
+    return prec == PREC_FP64 ? launch_line_tile_d0(a, st, kc, wide, s) : launch_line_tile_d1(a, st, kc, wide, s);
+}
+cudaError_t launch_line_warp(const Args<double>& a, int prec, int st, cudaStream_t s) {
+    return prec == PREC_FP64 ? dispatch_line_warp<PREC_FP64>(a, st, s) : dispatch_line_warp<PREC_FP32C>(a, st, s);
+}
 }  // namespace psb

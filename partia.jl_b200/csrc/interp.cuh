@@ -348,6 +348,8 @@ struct PlainD {
 };
 // products and accumulated products of the pair sums, with their roundings
 // spelled out (one fused step in double, a rounded product in float)
+__device__ __forceinline__ double rn_add(double a, double b) { return __dadd_rn(a, b); }
+__device__ __forceinline__ float rn_add(float a, float b) { return __fadd_rn(a, b); }
 __device__ __forceinline__ double acc_mul(double a, double b) { return __dmul_rn(a, b); }
 __device__ __forceinline__ float acc_mul(float a, float b) { return __fmul_rn(a, b); }
 __device__ __forceinline__ void acc_mac(PlainD& A, double a, double b) { A.s = __fma_rn(a, b, A.s); }

@@ -239,40 +239,109 @@ static int run_split(psb_ctx* c, Args<T>& A, int prec, int st, int* launches, in
     return PSB_OK;
 }
 
-// Heavy tiles first for parallel beams.  A line's work is the particles
-// whose support it crosses, and lines through dense clumps take many times
-// the mean: in index order the heaviest tiles can start last and leave the
-// SMs idle at the end (on the 8M-particle clump beam, a list-scheduling
-// estimate from the per-tile pair counts puts the last CTA at 1.19x the
-// ideal finish, 1.01x with the heaviest first).  The cost of a tile is
-// estimated from the particles projected onto the frame plane: each adds
-// the lines its support can cross, pi (K h / dx) (K h / dy) + 1, to the
-// tile of its centre pixel.  Only the order of the tiles changes, never a
-// result.
-template <class T>
-__global__ void k_beam_tile_cost(const TreeView<T> tv, const SampleSrc<T> s, int64_t nbx, float* cost) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= tv.n) return;
-    const double v0 = (double)tv.x[i] - (double)s.frame[0], v1 = (double)tv.y[i] - (double)s.frame[1],
-                 v2 = (double)tv.z[i] - (double)s.frame[2];
-    const double xi = v0 * (double)s.frame[3] + v1 * (double)s.frame[4] + v2 * (double)s.frame[5];
-    const double eta = v0 * (double)s.frame[6] + v1 * (double)s.frame[7] + v2 * (double)s.frame[8];
-    const double dx = ((double)s.params[1] - (double)s.params[0]) / (double)(s.nx - 1);
-    const double dy = ((double)s.params[3] - (double)s.params[2]) / (double)(s.ny - 1);
-    const double u = (xi - (double)s.params[0]) / dx, w = (eta - (double)s.params[2]) / dy;
-    const double r = tv.Kd * (double)tv.h[i];
-    const double ru = fabs(r / dx), rw = fabs(r / dy);
-    if (!(u > -ru - 1.0 && u < (double)s.nx + ru && w > -rw - 1.0 && w < (double)s.ny + rw)) return;
-    const int64_t ic = (int64_t)fmin(fmax(rint(u), 0.0), (double)(s.nx - 1));
-    const int64_t jc = (int64_t)fmin(fmax(rint(w), 0.0), (double)(s.ny - 1));
-    atomicAdd(&cost[(jc >> 2) * nbx + (ic >> 3)], (float)(3.141592653589793 * ru * rw + 1.0));
+// Line calls of fewer tiles than LINE_WARP_TILES take a warp per line
+// (k_line_warp), those of fewer than LINE_WIDE_TILES eight lanes per line
+// (k_line_tile's G): a warp per tile would not fill the GPU (4736 warps at a time).
+constexpr int64_t LINE_WARP_TILES = 512, LINE_WIDE_TILES = 4096;
+
+// Tile costs of parallel beams.  A line's work is the particles whose support
+// it crosses and the spans that hold them, and the lines through dense clumps
+// have many times the mean's: a tile of them can run on alone long after every
+// other one has finished.  Two forms share the tiles: a warp for a tile's 32
+// lines (k_line_tile, fewest instructions where supports span several pixels;
+// in calls of few tiles its G = 8), and a warp per line (k_line_warp, where a
+// line visits only its own spans; a 32nd of the time for one tile at two to
+// eight times the instructions).  The cost of a tile in either form is
+// estimated in instructions from a sample of the particles projected onto the
+// frame plane (a support of more than COST_SPAN tiles either way goes to a
+// term common to all tiles).  A tile takes the cheaper form, but a warp per
+// line also if it alone would take more than half of the beam's share of a
+// warp (4736 run at a time); the tiles run heaviest first.  Only the order
+// and the kernel change, never a result.
+//
+// 8M clump particles, 1024^2 beam: the tile through the densest clump (72,499
+// particles tested, 9 times the mean tile's instructions) ran for 65M cycles
+// of which the others took 34M.  The beam takes 32.1 -> 18.3 ms (FP32C), 2M on
+// 512^2 13.0 -> 7.9 ms, 1M on 512^2 in FP64 30.5 -> 6.1 ms.
+constexpr int COST_SPAN = 8;
+constexpr int64_t COST_SAMPLE = int64_t(1) << 18;  // particles looked at, at most twice as many
+struct TileCost { float tile, line; };
+// a particle's instructions in one tile it reaches: n lines of it inside the support
+__device__ __forceinline__ TileCost tile_cost(float n) {
+    return {33.f + 3.6f * n, 7.5f * fminf(1.f + 3.8f * n, 32.f) + 15.f * n};
 }
-// keys for an ascending sort that puts the largest cost first
-__global__ void k_cost_keys(const float* cost, int64_t n, uint64_t* keys, uint32_t* vals) {
-    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= n) return;
-    keys[t] = 0xFFFFFFFFull - (uint64_t)__float_as_uint(cost[t]);
-    vals[t] = (uint32_t)t;
+template <class T>
+__global__ void k_beam_tile_cost(const TreeView<T> tv, const SampleSrc<T> s, int64_t stride, int64_t nbx, int64_t nby,
+                                 TileCost* cost) {
+    const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * stride;
+    TileCost wide = {0.f, 0.f};  // this particle's part of the common term
+    if (i < tv.n) {
+        const double v0 = (double)tv.x[i] - (double)s.frame[0], v1 = (double)tv.y[i] - (double)s.frame[1],
+                     v2 = (double)tv.z[i] - (double)s.frame[2];
+        const double xi = v0 * (double)s.frame[3] + v1 * (double)s.frame[4] + v2 * (double)s.frame[5];
+        const double eta = v0 * (double)s.frame[6] + v1 * (double)s.frame[7] + v2 * (double)s.frame[8];
+        const double dx = ((double)s.params[1] - (double)s.params[0]) / (double)(s.nx - 1);
+        const double dy = ((double)s.params[3] - (double)s.params[2]) / (double)(s.ny - 1);
+        const double u = (xi - (double)s.params[0]) / dx, w = (eta - (double)s.params[2]) / dy;
+        const double r = tv.Kd * (double)tv.h[i];
+        const double ru = fabs(r / dx), rw = fabs(r / dy);
+        if (u > -ru - 1.0 && u < (double)s.nx + ru && w > -rw - 1.0 && w < (double)s.ny + rw) {
+            const double i0 = fmax(floor((u - ru) / 8.0), 0.0), i1 = fmin(floor((u + ru) / 8.0), (double)(nbx - 1));
+            const double j0 = fmax(floor((w - rw) / 4.0), 0.0), j1 = fmin(floor((w + rw) / 4.0), (double)(nby - 1));
+            const float nt = (float)((i1 - i0 + 1.0) * (j1 - j0 + 1.0));
+            const TileCost c = tile_cost((float)fmin(3.141592653589793 * ru * rw / nt, 32.0));
+            if (i1 - i0 < COST_SPAN && j1 - j0 < COST_SPAN) {
+                for (int64_t b = (int64_t)j0; b <= (int64_t)j1; ++b)
+                    for (int64_t a = (int64_t)i0; a <= (int64_t)i1; ++a) {
+                        atomicAdd(&cost[b * nbx + a].tile, c.tile);
+                        atomicAdd(&cost[b * nbx + a].line, c.line);
+                    }
+            } else {
+                wide.tile = nt * c.tile;
+                wide.line = nt * c.line;
+            }
+        }
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+        wide.tile += __shfl_xor_sync(PSB_FULL, wide.tile, o);
+        wide.line += __shfl_xor_sync(PSB_FULL, wide.line, o);
+    }
+    if ((threadIdx.x & 31) == 0 && wide.tile > 0.f) {
+        atomicAdd(&cost[nbx * nby].tile, wide.tile);
+        atomicAdd(&cost[nbx * nby].line, wide.line);
+    }
+}
+// cost[n] holds the sum of the common terms; cost[n + 1].tile becomes the sum
+// of the tile costs, that included
+__global__ void k_cost_total(TileCost* cost, int64_t n) {
+    __shared__ double part[32];
+    double t = 0.0;
+    for (int64_t i = threadIdx.x; i < n; i += blockDim.x) t += (double)cost[i].tile;
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(PSB_FULL, t, o);
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = t;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (unsigned w = 1; w < blockDim.x / 32; ++w) t += part[w];
+        cost[n + 1].tile = (float)(t + (double)cost[n].tile);
+    }
+}
+// The form of each tile, and keys for an ascending sort that puts the largest
+// cost first.  wide: the tile kernel is its G = 8.  list, count: the tiles
+// handed to k_line_warp (null: none); their cost is marked negative.
+__global__ void k_cost_keys(TileCost* cost, int64_t n, bool wide, uint64_t* keys, uint32_t* vals, unsigned* count,
+                            int32_t* list) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const float t = cost[i].tile + cost[n].tile / (float)n, l = cost[i].line + cost[n].line / (float)n;
+    keys[i] = 0xFFFFFFFFull - (uint64_t)__float_as_uint(t);
+    vals[i] = (uint32_t)i;
+    const float share = cost[n + 1].tile * fmaxf(0.5f / 4736.f, 1.5f / (float)n);
+    // G = 8: about 1.6 times the instructions, half the time
+    const bool by_line = l < (wide ? 1.6f : 1.f) * t || ((wide ? 0.5f : 1.f) * t > share && l < 10.f * t);
+    if (list && by_line) {
+        list[atomicAdd(count, 1u)] = (int32_t)i;
+        cost[i].tile = -1.f;
+    }
 }
 
 template <class T>
@@ -434,29 +503,104 @@ static int run_typed(psb_ctx* c, const SampleReq& rq, int hmode, const void* hs,
     // ---- launch ----
     if (ns > 0) {
         const bool split = what != WHAT_DIGEST && !rq.line && c->band_ok && !(flags & PSB_FLAG_SINGLE_KERNEL);
+        // line integrals of double particles in the float tests' range (a
+        // beam's direction must be a unit vector for them)
+        bool line_warp = rq.line && what == WHAT_INTERP && sizeof(T) == 8 && c->band_ok;
+        if (line_warp) {
+            A.line_extent = 0.0;
+            for (int d = 0; d < 3; ++d) {
+                A.line_centre[d] = 0.5 * (c->bbox[d] + c->bbox[3 + d]);
+                A.line_extent = std::max(A.line_extent, c->bbox[3 + d] - c->bbox[d]);
+            }
+            A.line_tube = LINE_TUBE * A.line_extent / std::cbrt((double)std::max<int64_t>(c->n, 1));
+        }
+        if (line_warp && A.src.kind == SRC_BEAM) {
+            double mm = 0.0, ox = 0.0;
+            for (int d = 0; d < 3; ++d) {
+                mm += (double)A.src.frame[9 + d] * (double)A.src.frame[9 + d];
+                ox = std::max(ox, std::fabs((double)A.src.frame[d]));
+            }
+            for (int q = 0; q < 4; ++q) ox = std::max(ox, std::fabs((double)A.src.params[q]));
+            line_warp = std::fabs(mm - 1.0) <= 1e-12 && ox <= 1e15;
+        }
         if (split) {
             int rc = run_split(c, A, prec, st, &launches, what);
             if (rc) return rc;
+        } else if (line_warp && A.src.ntiles < LINE_WARP_TILES) {
+            if constexpr (sizeof(T) == 8) PSB_CUDA_TRY(c, launch_line_warp(A, prec, st, s), "line kernel launch");
+            ++launches;
         } else {
-            if (rq.line && A.src.kind == SRC_BEAM && A.src.ntiles >= 4096) {  // heavy tiles first
-                const int64_t nt = A.src.ntiles, nbx = (A.src.nx + 7) >> 3;
-                float* cost = (float*)scratch(c, 93, sizeof(float) * nt);
+            const bool wide = line_warp && A.src.ntiles < LINE_WIDE_TILES;
+            const bool costs = rq.line && what == WHAT_INTERP && A.src.kind == SRC_BEAM && (line_warp || A.src.ntiles >= 4096);
+            if (costs) {
+                const int64_t nt = A.src.ntiles, nbx = (A.src.nx + 7) >> 3, nby = (A.src.ny + 3) >> 2;
+                TileCost* cost = (TileCost*)scratch(c, 93, sizeof(TileCost) * (nt + 2));
                 uint64_t* keys = (uint64_t*)scratch(c, 94, sizeof(uint64_t) * nt);
                 uint32_t* vals = (uint32_t*)scratch(c, 95, sizeof(uint32_t) * nt);
-                if (!cost || !keys || !vals) return fail(c, PSB_ENOMEM, "scratch allocation failed (tile order)");
-                PSB_CUDA_TRY(c, cudaMemsetAsync(cost, 0, sizeof(float) * nt, s), "memset tile costs");
-                if (c->n > 0)
-                    k_beam_tile_cost<T><<<(unsigned)((c->n + 255) / 256), 256, 0, s>>>(A.tv, A.src, nbx, cost);
-                k_cost_keys<<<(unsigned)((nt + 255) / 256), 256, 0, s>>>(cost, nt, keys, vals);
+                char* hv = (char*)scratch(c, 19, 256 + sizeof(int32_t) * (size_t)nt);
+                if (!cost || !keys || !vals || !hv) return fail(c, PSB_ENOMEM, "scratch allocation failed (tile order)");
+                unsigned* count = (unsigned*)hv;
+                int32_t* list = (int32_t*)(hv + 256);
+                PSB_CUDA_TRY(c, cudaMemsetAsync(cost, 0, sizeof(TileCost) * (nt + 2), s), "memset tile costs");
+                PSB_CUDA_TRY(c, cudaMemsetAsync(count, 0, sizeof(unsigned), s), "memset tile list");
+                const int64_t stride = std::max<int64_t>(1, c->n / COST_SAMPLE);
+                k_beam_tile_cost<T><<<(unsigned)((c->n / stride + 256) / 256), 256, 0, s>>>(A.tv, A.src, stride, nbx, nby, cost);
+                k_cost_total<<<1, 1024, 0, s>>>(cost, nt);
+                k_cost_keys<<<(unsigned)((nt + 255) / 256), 256, 0, s>>>(cost, nt, wide, keys, vals, count,
+                                                                         line_warp ? list : nullptr);
                 PSB_CUDA_TRY(c, cudaGetLastError(), "tile cost kernels");
                 PSB_CUDA_TRY(c, radix_sort_pairs(keys, vals, nt, c, 6, &launches, false, 32), "tile order sort");
+                launches += 3;
+                if (line_warp) {
+                    // the tiles handed over run beside the others, on a stream of the context's own
+                    A.tile_cost = (const float*)cost;
+                    for (int e = 0; e < 2; ++e)
+                        if (!c->sev[e]) PSB_CUDA_TRY(c, cudaEventCreateWithFlags(&c->sev[e], cudaEventDisableTiming), "event");
+                    cudaStream_t& sq = c->sstream[0];
+                    if (!sq) PSB_CUDA_TRY(c, cudaStreamCreateWithFlags(&sq, cudaStreamNonBlocking), "stream");
+                    PSB_CUDA_TRY(c, cudaEventRecord(c->sev[0], s), "event");
+                    PSB_CUDA_TRY(c, cudaStreamWaitEvent(sq, c->sev[0], 0), "stream wait");
+                    if constexpr (sizeof(T) == 8) {
+                        Args<T> H = A;
+                        H.tile_list = list;
+                        H.tile_count = count;
+                        H.tile_lines = 32;
+                        PSB_CUDA_TRY(c, launch_line_warp(H, prec, st, sq), "line kernel launch");
+                    }
+                    ++launches;
+                    PSB_CUDA_TRY(c, cudaEventRecord(c->sev[1], sq), "event");
+                }
                 A.tile_list = (const int32_t*)vals;
-                launches += 2;
             }
-            cudaError_t e = rq.line ? launch_lines<T>(A, prec, st, A.rec.kc, what, s)
-                                    : launch_points<T>(A, prec, st, A.rec.kc, what, s);
-            PSB_CUDA_TRY(c, e, "interpolation kernel launch");
-            ++launches;
+            if (line_warp) {
+                // tiles of lines together; those of an explicit call that do not
+                // run together come back in a list, one warp per line
+                const bool listed = A.src.kind == SRC_ARRAYS;
+                if (listed) {
+                    char* ovf = (char*)scratch(c, 19, 256 + sizeof(int32_t) * (size_t)A.src.ntiles * 8);
+                    if (!ovf) return fail(c, PSB_ENOMEM, "scratch allocation failed (line tiles)");
+                    PSB_CUDA_TRY(c, cudaMemsetAsync(ovf, 0, sizeof(unsigned), s), "memset line tiles");
+                    A.sp.ovf_count = (unsigned*)ovf;
+                    A.sp.ovf_tiles = (int32_t*)(ovf + 256);
+                }
+                if constexpr (sizeof(T) == 8) {
+                    PSB_CUDA_TRY(c, launch_line_tile(A, prec, st, A.rec.kc, wide, s), "line kernel launch");
+                    if (listed) {
+                        A.tile_list = A.sp.ovf_tiles;
+                        A.tile_count = A.sp.ovf_count;
+                        A.tile_lines = wide ? 4 : 32;
+                        PSB_CUDA_TRY(c, launch_line_warp(A, prec, st, s), "line kernel launch");
+                    }
+                }
+                launches += listed ? 2 : 1;
+                if (costs) PSB_CUDA_TRY(c, cudaStreamWaitEvent(s, c->sev[1], 0), "stream wait");
+            } else if (rq.line) {
+                PSB_CUDA_TRY(c, launch_lines<T>(A, prec, st, A.rec.kc, what, s), "line kernel launch");
+                ++launches;
+            } else {
+                PSB_CUDA_TRY(c, launch_points<T>(A, prec, st, A.rec.kc, what, s), "interpolation kernel launch");
+                ++launches;
+            }
         }
     }
     PSB_CUDA_TRY(c, cudaEventRecord(c->ev[3], s), "event");

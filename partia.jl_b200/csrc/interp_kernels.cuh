@@ -112,6 +112,13 @@ template <class T> struct Args {
     // single-kernel path over a device list of tiles (nullptr: every tile)
     const int32_t* tile_list;
     const unsigned* tile_count;
+    // line calls: the particles' box (centre, largest extent) and the distance
+    // within which a tile's lines run together (k_lines)
+    double line_centre[3];
+    double line_extent;
+    double line_tube;
+    const float* tile_cost;  // or null: two floats per tile, the first negative if the tile is handed over
+    int tile_lines;          // k_line_warp: lines of an entry of tile_list
     // WHAT_DENSITY: every particle mass taken as 1, the number density
     // sum W of _number_density_kernel (scalar_interpolation.jl:86-166)
     int unit_mass;
@@ -233,67 +240,157 @@ template <int ST> __device__ __forceinline__ float hi_r2_node(float ra2_hi, floa
     return fmaxf(ra2_hi, r2);
 }
 
-// lower bound of the squared distance between a line and a node box.
+// Lower bound of the squared distance between a line and a node box: the line
+// runs in the plane through it that faces the box's centre, w its offset from
+// there and n = w / |w| the plane's normal, and no point of the box is nearer
+// to that plane than |w| - sum |n_d| (half side d).  (The box's bounding sphere
+// in its place let through twice the spans.)
 // o, m: float line; el: absolute error allowance of the float line near the
-// box (origin and direction rounding).
-__device__ __forceinline__ float lb_d2_line_box(const float o[3], const float m[3], float el, float4 lo, float4 hi) {
-    float a[3] = {lo.x, lo.y, lo.z}, b[3] = {hi.x, hi.y, hi.z};
-    // centre / half-diagonal of the outward-rounded box
-    float c[3], r2 = 0.f;
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-        c[d] = 0.5f * (a[d] + b[d]);
-        float hh = 0.5f * (b[d] - a[d]);
-        r2 += hh * hh;
-    }
-    float rb = sqrtf(r2) * (1.f + 4.f * U1);
+// box (origin and direction rounding); tube: for lines within that distance
+// of this one.
+__device__ __forceinline__ float lb_d2_line_box(const float o[3], const float m[3], float el, float4 lo, float4 hi,
+                                                float tube = 0.f) {
+    const float a[3] = {lo.x, lo.y, lo.z}, b[3] = {hi.x, hi.y, hi.z};
     float v[3], vm = 0.f, vv = 0.f;
 #pragma unroll
-    for (int d = 0; d < 3; ++d) { v[d] = c[d] - o[d]; vm += v[d] * m[d]; }
-    float pp = 0.f;
+    for (int d = 0; d < 3; ++d) { v[d] = 0.5f * (a[d] + b[d]) - o[d]; vm += v[d] * m[d]; vv += v[d] * v[d]; }
+    float pp = 0.f, side = 0.f;
 #pragma unroll
-    for (int d = 0; d < 3; ++d) { float w = v[d] - vm * m[d]; pp += w * w; vv += v[d] * v[d]; }
-    float dc = sqrtf(pp);
-    float err = el + 8.f * U1 * sqrtf(vv);
-    float g = dc - rb - err;
-    if (g <= 0.f) return 0.f;
+    for (int d = 0; d < 3; ++d) {
+        const float w = v[d] - vm * m[d];
+        pp += w * w;
+        side += fabsf(w) * (0.5f * (b[d] - a[d]));
+    }
+    // |w| - side / |w|, less the roundings of w and n (a few 2^-23 |v| each)
+    const float g = (pp * (1.f - 8.f * U1) - side * (1.f + 8.f * U1)) * rsqrtf(fmaxf(pp, 1e-36f)) * (1.f - 4.f * U1) -
+                    (el + 24.f * U1 * sqrtf(vv) + tube);
+    if (!(g > 0.f)) return 0.f;
     return g * g * (1.f - RELM);
 }
 
 // ---------------------------------------------------------------------------
 // Line kernel (line-integrated scalars, LUT kernel)
 // ---------------------------------------------------------------------------
+// Rounding-exact pieces of a line's pair terms: the tile kernel and the
+// warp-per-line kernel give a pair the same bits.
+__device__ __forceinline__ float rn_fma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ double rn_fma(double a, double b, double c) { return __fma_rn(a, b, c); }
+__device__ __forceinline__ float rn_sub(float a, float b) { return __fsub_rn(a, b); }
+__device__ __forceinline__ double rn_sub(double a, double b) { return __dsub_rn(a, b); }
+
 // _lin_lut, kernel_function/line_integrated_kernel.jl:13-19, with the
 // q >= q_max cut (:90-94) and the 1/h factor (:132-137).
-// n = entries of the table, dq its spacing (idq = 1/dq: the float path
-// multiplies, FP64 divides as the reference does), K the kernel's support.
-template <class C> __device__ __forceinline__ C line_W(C r, C h, C invh, const C* lut, C dq, C idq, int n, C K) {
-    C q = r * invh;
+// n = entries of the table, idq = 1/dq of its spacing, K the kernel's support.
+template <class C, class Lut> __device__ __forceinline__ C line_W(C r, C invh, const Lut& lut, C idq, int n, C K) {
+    const C q = acc_mul(r, invh);
     if (q >= K) return C(0);
-    C idxf = (sizeof(C) == 4 ? q * idq : q / dq) + C(1);
+    const C idxf = rn_fma(q, idq, C(1));
     int i = (int)idxf;  // q >= 0
     i = i < 1 ? 1 : (i > n - 1 ? n - 1 : i);
-    C t = idxf - C(i);
-    C v = lut[i - 1] * (C(1) - t) + lut[i] * t;
-    return invh * v;
+    const C t = rn_sub(idxf, C(i));
+    const C v = rn_fma(lut(i - 1), rn_sub(C(1), t), acc_mul(lut(i), t));
+    return acc_mul(invh, v);
 }
 
-// Per-warp shared-memory stage of a span of leaves (FP32C line path).
-template <int KC> struct LStage {
+// W of one pair for the strategy: r the distance, (ia, ib) = 1/h of the line and of the particle
+template <int ST, class C, class Lut>
+__device__ __forceinline__ C line_pair_W(C r, C ia, C ib, const Lut& lut, C idq, int n, C K) {
+    if (ST == ST_GATHER) return line_W<C>(r, ia, lut, idq, n, K);
+    const C Wb = line_W<C>(r, ib, lut, idq, n, K);
+    if (ST == ST_SCATTER) return Wb;
+    const C Wa = line_W<C>(r, ia, lut, idq, n, K);
+    return acc_mul(C(0.5), rn_add(Wa, Wb));
+}
+
+// Perpendicular offset of (x, y, z) from a line, formed in double and rounded;
+// returns the absolute error allowance of the double steps.
+__device__ __forceinline__ float line_perp(const double o[3], const double m[3], double x, double y, double z,
+                                           float c[3]) {
+    const double q0 = __dsub_rn(x, o[0]), q1 = __dsub_rn(y, o[1]), q2 = __dsub_rn(z, o[2]);
+    const double t = __fma_rn(q2, m[2], __fma_rn(q0, m[0], __dmul_rn(q1, m[1])));
+    c[0] = __double2float_rn(__fma_rn(-t, m[0], q0));
+    c[1] = __double2float_rn(__fma_rn(-t, m[1], q1));
+    c[2] = __double2float_rn(__fma_rn(-t, m[2], q2));
+    return 1e-15f * (float)(fabs(q0) + fabs(q1) + fabs(q2) + 1.0);
+}
+// Squared float distance of a leaf from the line: L its offset from its span's
+// first leaf, c that leaf's perpendicular offset (line_perp).
+__device__ __forceinline__ float line_fs_f32(const float4& L, const float c[3], const float m[3]) {
+    const float v0 = __fadd_rn(L.x, c[0]), v1 = __fadd_rn(L.y, c[1]), v2 = __fadd_rn(L.z, c[2]);
+    const float vm = __fmaf_rn(v2, m[2], __fmaf_rn(v0, m[0], __fmul_rn(v1, m[1])));
+    const float w0 = __fmaf_rn(-vm, m[0], v0), w1 = __fmaf_rn(-vm, m[1], v1), w2 = __fmaf_rn(-vm, m[2], v2);
+    return __fmaf_rn(w2, w2, __fmaf_rn(w0, w0, __fmul_rn(w1, w1)));
+}
+
+__device__ __forceinline__ float line_r_f32(const float4& L, const float c[3], const float m[3]) {
+    return sqrtf(line_fs_f32(L, c, m));
+}
+// The distance of the FP64 sums, from the exact squared one (which can round below 0 on the line)
+__device__ __forceinline__ double line_r_f64(double e2) { return e2 > 0.0 ? __dmul_rn(e2, rsqrt(e2)) : 0.0; }
+
+// Outputs of one line from its sums, or (adjoint) the cotangents of the sums.
+template <class T, class Acc, int KC>
+__device__ __forceinline__ void write_line_outputs(const Args<T>& A, int64_t k, const Acc& S1, const Acc (&Sw)[KC]) {
+    const int kc = A.rec.kc;
+    const double s1 = S1.get();
+    if (A.lam) {
+        // cotangents of S1 (q = 0) and Sw_c (q = 1 + c), zero where S1 = 0
+        double l[1 + MAX_KC];
+        for (int q = 0; q <= kc; ++q) l[q] = 0.0;
+        if (s1 != 0.0) {
+            const double inv = 1.0 / s1;
+            for (int q = 0; q < A.rec.L; ++q) {
+                const double go = A.gout[q][k];
+                const int c = A.rec.a0[q];
+                l[1 + c] += A.rec.a1[q] ? go * inv : go;
+            }
+            // Shepard terms: d(Sw_c/S1)/dS1 = -Sw_c/S1^2
+            for (int q = 0; q < A.rec.L; ++q) {
+                if (!A.rec.a1[q]) continue;
+                const int c = A.rec.a0[q];
+                double swc = 0.0;
+#pragma unroll
+                for (int cc = 0; cc < KC; ++cc)
+                    if (cc == c) swc = Sw[cc].get();
+                l[0] -= A.gout[q][k] * swc * inv * inv;
+            }
+        }
+        for (int q = 0; q <= kc; ++q) A.lam[q * A.lam_stride + k] = l[q];
+        return;
+    }
+    const int L = A.rec.L;
+    if (s1 == 0.0) {
+        for (int q = 0; q < L; ++q) A.out[q][k] = qnan<T>();
+    } else {
+        double sw[MAX_KC];
+#pragma unroll
+        for (int c = 0; c < KC; ++c) sw[c] = Sw[c].get();
+        const double inv = 1.0 / s1;
+        for (int q = 0; q < L; ++q) {
+            const int a0 = A.rec.a0[q];
+            A.out[q][k] = (T)(A.rec.a1[q] ? sw[a0] * inv : sw[a0]);
+        }
+    }
+}
+
+// Per-warp shared-memory stage of a span of leaves (tile kernel, double inputs).
+template <class CT, int KC> struct LStage {
     float4 L[SPAN];
-    float ih[SPAN];  // 1/h (float)
-    float mr[SPAN];
-    float col[KC][SPAN];
+    CT ih[SPAN];  // 1/h
+    CT mr[SPAN];  // m/rho
+    CT col[KC][SPAN];
 };
 
+// The general line kernel: float inputs, digests, and sets or frames outside
+// the float tests' range (the others take k_line_tile and k_line_warp).
+// FP32C with double inputs: float tests with a double fallback, leaf spans.
+// Otherwise the reference's own arithmetic node by node, so that the pruning
+// decisions (including the rounding of the line-box lower bound) are the
+// reference's.
 template <class T, int PREC, int ST, int KC, int WHAT>
 __global__ void __launch_bounds__(128) k_lines(const Args<T> A) {
     using CT = typename std::conditional<PREC == PREC_FP64, double, float>::type;
     using Acc = typename std::conditional<PREC == PREC_FP64, PlainD, KahanF>::type;
-    // FP32C with double inputs: float tests with a double fallback, leaf
-    // spans.  Otherwise the reference's own arithmetic node by node, so that
-    // the pruning decisions (including the rounding of the line-box lower
-    // bound) are the reference's.
     constexpr bool BAND = (PREC == PREC_FP32C) && (sizeof(T) == 8);
     // The line table is read from global memory: one copy (16 or 32 KB) in
     // each SM's L1 serves every CTA there, where a copy per CTA in shared
@@ -301,7 +398,7 @@ __global__ void __launch_bounds__(128) k_lines(const Args<T> A) {
     // (C3: FP32C 35.7 -> 35.0 ms, FP64 145.9 -> 130.8 ms).  Only the FP64 sums
     // over the short float table convert it into shared memory.
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ LStage<KC> lstage_all[4];
+    __shared__ LStage<CT, BAND ? KC : 1> lstage_all[4];
     const int nlut = A.lut_n;
     const bool short_lut = nlut == LUT_SHORT_N;
     const CT* lut;
@@ -314,14 +411,14 @@ __global__ void __launch_bounds__(128) k_lines(const Args<T> A) {
         lut = short_lut ? (const CT*)A.lut_fs : ((PREC == PREC_FP64) ? (const CT*)A.lut_d : (const CT*)A.lut_f);
     }
     // dq = Q[2] - Q[1] of the n-point table over [0, K] = K/(n-1) rounded to CT
-    const CT dq = (CT)(A.tv.Kd / (double)(nlut - 1));
     const CT Kc = (CT)A.tv.Kd;
-    const CT idq = CT(1) / dq;
+    const CT idq = CT(1) / (CT)(A.tv.Kd / (double)(nlut - 1));
+    auto lutv = [&](int i) -> CT { return lut[i]; };
 
     const TreeView<T>& tv = A.tv;
     const int lane = threadIdx.x & 31;
     const int wib = threadIdx.x >> 5;
-    LStage<KC>& st = lstage_all[wib];
+    auto& st = lstage_all[wib];
     int64_t tile = (int64_t)blockIdx.x * (blockDim.x >> 5) + wib;
     if (tile >= A.src.ntiles) return;
     if (A.tile_list) tile = A.tile_list[tile];  // a permutation of the tiles (heavy first)
@@ -360,26 +457,20 @@ __global__ void __launch_bounds__(128) k_lines(const Args<T> A) {
     int64_t hcount = 0;
     const int kc = A.rec.kc;
 
-    // line-integrated weight of one accepted pair (s = squared distance)
-    // dr = the line's distance from the particle, ib = 1/hb
-    auto body = [&](int64_t li, CT dr, CT hb, CT ib, CT mr, const CT* cols) {
+    // line-integrated weight of one accepted pair: dr = the line's distance
+    // from the particle, ib = 1/hb
+    auto body = [&](int64_t li, CT dr, CT ib, CT mr, const CT* cols) {
         ++n_pairs;
         if (WHAT == WHAT_DIGEST) {
             ++hcount;
             hsum += mix64((uint64_t)(li + 1));
             return;
         }
-        CT W;
-        if (ST == ST_GATHER) W = line_W<CT>(dr, (CT)ha, ia, lut, dq, idq, nlut, Kc);
-        else {
-            CT Wb = line_W<CT>(dr, hb, ib, lut, dq, idq, nlut, Kc);
-            W = (ST == ST_SCATTER) ? Wb : CT(0.5) * (line_W<CT>(dr, (CT)ha, ia, lut, dq, idq, nlut, Kc) + Wb);
-        }
-        const CT w = mr * W;
+        const CT w = acc_mul(mr, line_pair_W<ST, CT>(dr, ia, ib, lutv, idq, nlut, Kc));
         S1.add(w);
 #pragma unroll
         for (int c = 0; c < KC; ++c)
-            if (c < kc) Sw[c].add(cols[c] * w);
+            if (c < kc) acc_mac(Sw[c], cols[c], w);
     };
 
     bool ok;
@@ -389,18 +480,7 @@ __global__ void __launch_bounds__(128) k_lines(const Args<T> A) {
             float lb = lb_d2_line_box(of, mf3, el, lo, hi);
             return !(lb > hi_r2_node<ST>(ra2_hi, lo.w, tv.Kf));
         };
-        // perpendicular offset of a span's anchor (its first leaf) from the
-        // line, in double
-        auto perp_anchor = [&](int64_t a, float c[3], float& cerr) {
-            double q0 = (double)__ldg(&tv.x[a]) - (double)o[0];
-            double q1 = (double)__ldg(&tv.y[a]) - (double)o[1];
-            double q2 = (double)__ldg(&tv.z[a]) - (double)o[2];
-            double t0 = q0 * (double)m[0] + q1 * (double)m[1] + q2 * (double)m[2];
-            c[0] = (float)(q0 - t0 * (double)m[0]);
-            c[1] = (float)(q1 - t0 * (double)m[1]);
-            c[2] = (float)(q2 - t0 * (double)m[2]);
-            cerr = 1e-15f * (float)(fabs(q0) + fabs(q1) + fabs(q2) + 1.0);
-        };
+        const double od[3] = {(double)o[0], (double)o[1], (double)o[2]}, md[3] = {(double)m[0], (double)m[1], (double)m[2]};
         auto span_fn = [&](int64_t lo, int cnt, bool part) {
             __syncwarp();
             if (lane < cnt) {
@@ -416,8 +496,9 @@ __global__ void __launch_bounds__(128) k_lines(const Args<T> A) {
             }
             __syncwarp();
             if (!part) return;
-            float cf[3], cerr;
-            perp_anchor(lo, cf, cerr);
+            // perpendicular offset of the span's anchor (its first leaf) from the line
+            float cf[3];
+            const float cerr = line_perp(od, md, __ldg(&tv.x[lo]), __ldg(&tv.y[lo]), __ldg(&tv.z[lo]), cf);
             // one error bound for every leaf of the span: |v|_1 <= |L|_1 + |cf|_1
             // with |L|_1 <= spanb.x (the span's largest, rounded up)
             const float sbx = __ldg(&tv.spanb[lo]).x;
@@ -425,11 +506,7 @@ __global__ void __launch_bounds__(128) k_lines(const Args<T> A) {
                              cerr + 1e-30f;
             for (int j = 0; j < cnt; ++j) {
                 const float4 L = st.L[j];
-                float v0 = L.x + cf[0], v1 = L.y + cf[1], v2 = L.z + cf[2];
-                float vm = v0 * mf3[0] + v1 * mf3[1] + v2 * mf3[2];
-                float w0 = v0 - vm * mf3[0], w1 = v1 - vm * mf3[1], w2 = v2 - vm * mf3[2];
-                float fs = w0 * w0 + w1 * w1 + w2 * w2;
-                float r = sqrtf(fs);
+                const float r = line_r_f32(L, cf, mf3);
                 float up = r + ev, dn = fmaxf(r - ev, 0.f);
                 const float kb = tv.Kf * L.w;
                 float rb2 = kb * kb;
@@ -452,8 +529,8 @@ __global__ void __launch_bounds__(128) k_lines(const Args<T> A) {
                 if (!acc) continue;
                 CT cols[KC];
 #pragma unroll
-                for (int c = 0; c < KC; ++c) cols[c] = (c < kc) ? (CT)st.col[c][j] : CT(0);
-                body(lo + j, (CT)r, (CT)L.w, (CT)st.ih[j], (CT)st.mr[j], cols);
+                for (int c = 0; c < KC; ++c) cols[c] = (c < kc && WHAT != WHAT_DIGEST) ? st.col[c][j] : CT(0);
+                body(lo + j, (CT)r, st.ih[j], st.mr[j], cols);
             }
         };
         ok = warp_traverse_spans(start, tv.n, tv.links, tv.escape, valid, node_fn, span_fn, steps);
@@ -473,7 +550,7 @@ __global__ void __launch_bounds__(128) k_lines(const Args<T> A) {
             for (int c = 0; c < KC; ++c) cols[c] = (c < kc) ? (CT)__ldg(&A.colT[c][li]) : CT(0);
             CT mr = (WHAT == WHAT_DIGEST) ? CT(0) : (CT)((double)tv.m[li] / (double)tv.rho[li]);
             const CT s2 = (CT)e2;
-            body(li, sqrt(s2 < CT(0) ? CT(0) : s2), (CT)hb, CT(1) / (CT)hb, mr, cols);
+            body(li, sqrt(s2 < CT(0) ? CT(0) : s2), CT(1) / (CT)hb, mr, cols);
         };
         ok = warp_traverse(start, tv.n, tv.left, tv.escape, valid, node_fn, leaf_fn);
     }
@@ -483,45 +560,8 @@ __global__ void __launch_bounds__(128) k_lines(const Args<T> A) {
             A.dig_count[k] = hcount;
             A.dig_hash[k] = hsum;
             if (A.ha_out) A.ha_out[k] = ha;
-        } else if (A.lam) {
-            // adjoint: cotangents of S1 (q = 0) and Sw_c (q = 1 + c), zero where S1 = 0
-            const double s1 = S1.get();
-            double l[1 + MAX_KC];
-            for (int q = 0; q <= kc; ++q) l[q] = 0.0;
-            if (s1 != 0.0) {
-                const double inv = 1.0 / s1;
-                for (int q = 0; q < A.rec.L; ++q) {
-                    const double go = A.gout[q][k];
-                    const int c = A.rec.a0[q];
-                    l[1 + c] += A.rec.a1[q] ? go * inv : go;
-                }
-                // Shepard terms: d(Sw_c/S1)/dS1 = -Sw_c/S1^2
-                for (int q = 0; q < A.rec.L; ++q) {
-                    if (!A.rec.a1[q]) continue;
-                    const int c = A.rec.a0[q];
-                    double swc = 0.0;
-#pragma unroll
-                    for (int cc = 0; cc < KC; ++cc)
-                        if (cc == c) swc = Sw[cc].get();
-                    l[0] -= A.gout[q][k] * swc * inv * inv;
-                }
-            }
-            for (int q = 0; q <= kc; ++q) A.lam[q * A.lam_stride + k] = l[q];
         } else {
-            const double s1 = S1.get();
-            const int L = A.rec.L;
-            if (s1 == 0.0) {
-                for (int q = 0; q < L; ++q) A.out[q][k] = qnan<T>();
-            } else {
-                double sw[MAX_KC];
-#pragma unroll
-                for (int c = 0; c < KC; ++c) sw[c] = Sw[c].get();
-                const double inv = 1.0 / s1;
-                for (int q = 0; q < L; ++q) {
-                    const int a0 = A.rec.a0[q];
-                    A.out[q][k] = (T)(A.rec.a1[q] ? sw[a0] * inv : sw[a0]);
-                }
-            }
+            write_line_outputs<T, Acc, KC>(A, k, S1, Sw);
         }
     }
 #pragma unroll

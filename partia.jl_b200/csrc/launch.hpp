@@ -4,7 +4,7 @@
 
 #include <algorithm>
 
-#include "k_split.cuh"
+#include "k_line_warp.cuh"
 
 namespace psb {
 
@@ -50,7 +50,8 @@ static void dispatch_lines_k(const Args<T>& a, int kc, unsigned g, size_t smem, 
         k_lines<T, P, S, 1, W><<<g, 128, smem, s>>>(a);
     } else {
         if (kc <= 1) k_lines<T, P, S, 1, W><<<g, 128, smem, s>>>(a);
-        else k_lines<T, P, S, 4, W><<<g, 128, smem, s>>>(a);
+        else if (kc <= 4) k_lines<T, P, S, 4, W><<<g, 128, smem, s>>>(a);
+        else k_lines<T, P, S, 8, W><<<g, 128, smem, s>>>(a);
     }
 }
 
@@ -69,6 +70,39 @@ static cudaError_t dispatch_lines_p(const Args<T>& a, int st, int kc, int what, 
     size_t smem = (P == PREC_FP64 && a.lut_n == LUT_SHORT_N) ? (size_t)LUT_SHORT_N * sizeof(double) : 0;
     if (what == WHAT_INTERP) dispatch_lines_s<T, P, WHAT_INTERP>(a, st, kc, g, smem, s);
     else dispatch_lines_s<T, P, WHAT_DIGEST>(a, st, kc, g, smem, s);
+    return cudaGetLastError();
+}
+
+// tiles of lines that run together; wide: eight lanes per line (k_line_tile's G)
+template <int P, int S, int G>
+static void dispatch_line_tile_s(const Args<double>& a, int kc, cudaStream_t s) {
+    const unsigned g = (unsigned)((a.src.ntiles * G + 3) / 4);
+    if (kc <= 1) k_line_tile<P, S, 1, G><<<g, 128, 0, s>>>(a);
+    else if (kc <= 4) k_line_tile<P, S, 4, G><<<g, 128, 0, s>>>(a);
+    else k_line_tile<P, S, 8, G><<<g, 128, 0, s>>>(a);
+}
+template <int P, int G>
+static void dispatch_line_tile_g(const Args<double>& a, int st, int kc, cudaStream_t s) {
+    if (st == ST_GATHER) dispatch_line_tile_s<P, ST_GATHER, G>(a, kc, s);
+    else if (st == ST_SCATTER) dispatch_line_tile_s<P, ST_SCATTER, G>(a, kc, s);
+    else dispatch_line_tile_s<P, ST_SYMMETRIC, G>(a, kc, s);
+}
+template <int P>
+static cudaError_t dispatch_line_tile(const Args<double>& a, int st, int kc, bool wide, cudaStream_t s) {
+    if (a.src.ntiles == 0) return cudaSuccess;
+    if (wide) dispatch_line_tile_g<P, 8>(a, st, kc, s);
+    else dispatch_line_tile_g<P, 1>(a, st, kc, s);
+    return cudaGetLastError();
+}
+
+// one warp per line: every line, or those of the listed groups
+template <int P>
+static cudaError_t dispatch_line_warp(const Args<double>& a, int st, cudaStream_t s) {
+    const unsigned g = (unsigned)(a.src.ntiles * 8);
+    if (g == 0) return cudaSuccess;
+    if (st == ST_GATHER) k_line_warp<P, ST_GATHER><<<g, 128, 0, s>>>(a);
+    else if (st == ST_SCATTER) k_line_warp<P, ST_SCATTER><<<g, 128, 0, s>>>(a);
+    else k_line_warp<P, ST_SYMMETRIC><<<g, 128, 0, s>>>(a);
     return cudaGetLastError();
 }
 
@@ -172,5 +206,7 @@ inline cudaError_t launch_split(const Args<float>& a, int prec, int st, int kc, 
     return prec == PREC_FP64 ? launch_split_f0(a, st, kc, pass, s) : launch_split_f1(a, st, kc, pass, s);
 }
 template <class T> cudaError_t launch_lines(const Args<T>& a, int prec, int st, int kc, int what, cudaStream_t s);
+cudaError_t launch_line_tile(const Args<double>& a, int prec, int st, int kc, bool wide, cudaStream_t s);
+cudaError_t launch_line_warp(const Args<double>& a, int prec, int st, cudaStream_t s);
 
 }  // namespace psb

@@ -162,3 +162,57 @@ def test_particle_sets_of_any_scale(scale):
     # a Shepard mean of 64-bit coordinates rounded at another scale: 1e-16 of
     # the separations, amplified at the support edge by less than 1e3
     assert rel_err(got[0], ref[0]) <= 1e-12
+
+
+@pytest.mark.parametrize("prec", [L.PSB_PREC_FP64, L.PSB_PREC_FP32C])
+@pytest.mark.parametrize("nl", [1, 33, 1000, 40_000])
+def test_lines_alone_and_in_tiles(nl, prec):
+    """Sight lines in every direction and a bundle of parallel ones, below and
+    above the size from which a tile's lines may run together; seven columns.  Each line's bits are the same alone (a
+    call of one) and among the others."""
+    arrs, cols = particles(20_000, 15)
+    rng = np.random.default_rng(16)
+    cols = cols + [rng.random(20_000) for _ in range(3)]
+    o = rng.uniform(-0.2, 1.2, (3, nl))
+    d = rng.standard_normal((3, nl))
+    d /= np.linalg.norm(d, axis=0)
+    d[:, nl // 4:nl // 2] = [[0.0], [0.6], [0.8]]
+    o[:, nl // 4:nl // 2] *= 0.1  # close to one another
+    spec = dict(scalars=list(range(7)), shepard=[0, 1, 1, 1, 0, 1, 0])
+    orc = O.Oracle(*arrs, cols=cols)
+    ctx = context(arrs, cols)
+    cat = CatalogC(**spec)
+    got = ctx.interp_lines(tuple(o), tuple(d), cat, prec=prec)
+    pairs = ctx.last_stats.pairs
+    m = min(nl, 2000)
+    at = rng.choice(nl, m, replace=False)
+    ref = orc.interp_lines(tuple(o[:, at]), tuple(d[:, at]), scalars=spec["scalars"], shepard=spec["shepard"],
+                           strategy=O.SCATTER, hmode=O.H_PER_SAMPLE, hs=None)
+    tol = FP64_TOL if prec == L.PSB_PREC_FP64 else 4e-6  # the parity tests' bounds
+    if nl > 1:
+        for k in range(cat.L):
+            assert rel_err(got[k][at], ref[k]) <= tol, k
+    if nl <= 1000:
+        count, _, _ = orc.digest(tuple(o), tuple(d), strategy=O.SCATTER, hmode=O.H_PER_SAMPLE)
+        assert pairs == int(count.sum())
+    for i in at[:20]:
+        one = ctx.interp_lines(tuple(o[:, i:i + 1]), tuple(d[:, i:i + 1]), cat, prec=prec)
+        for k in range(cat.L):
+            assert np.array_equal(one[k], got[k][i:i + 1], equal_nan=True), (i, k)
+
+
+def test_lines_that_are_not_unit_vectors():
+    """The formula D^2 - (D.m)^2 holds for any m: the reference's pairs, in FP64."""
+    arrs, cols = particles(5000, 17)
+    rng = np.random.default_rng(18)
+    o, d = rng.random((3, 50)), rng.standard_normal((3, 50))
+    d *= rng.uniform(0.9, 0.999, 50) / np.linalg.norm(d, axis=0)
+    orc = O.Oracle(*arrs, cols=cols)
+    ctx = context(arrs, cols)
+    got = ctx.interp_lines(tuple(o), tuple(d), CatalogC(scalars=[0, 1], shepard=[0, 1]))
+    count, _, _ = orc.digest(tuple(o), tuple(d), strategy=O.SCATTER, hmode=O.H_PER_SAMPLE)
+    ref = orc.interp_lines(tuple(o), tuple(d), scalars=[0, 1], shepard=[0, 1], strategy=O.SCATTER,
+                           hmode=O.H_PER_SAMPLE, hs=None)
+    assert ctx.last_stats.pairs == int(count.sum())
+    for k in range(2):
+        assert rel_err(got[k], ref[k]) <= FP64_TOL, k
