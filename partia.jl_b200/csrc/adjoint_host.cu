@@ -6,6 +6,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <type_traits>
 #include <vector>
 
 #include "k_adjoint.cuh"
@@ -49,56 +50,62 @@ __global__ void k_adj_tile_keys(const double* x, const double* y, const double* 
 
 // pass: 0 = k_adj_points (whole tiles, or the listed ones), 1 = its pair-list
 // form (COL), 2 = k_adj_bodies (grid over list blocks), 3 = k_adj_combine
-template <int KC, bool SCAL, int KF>
+template <int KC, bool SCAL, bool DG, int KF>
 static void launch_adj_points_ks(const AdjArgs& a, int st, int pass, unsigned g, cudaStream_t s) {
     if (pass == 1) {
         if (st == ST_GATHER) k_adj_points<ST_GATHER, 1, true, KF, true><<<g, 128, 0, s>>>(a);
         else if (st == ST_SCATTER) k_adj_points<ST_SCATTER, 1, true, KF, true><<<g, 128, 0, s>>>(a);
         else k_adj_points<ST_SYMMETRIC, 1, true, KF, true><<<g, 128, 0, s>>>(a);
     } else if (pass == 2) {
-        if (st == ST_GATHER) k_adj_bodies<ST_GATHER, KC, SCAL, KF><<<g, 128, 0, s>>>(a);
-        else if (st == ST_SCATTER) k_adj_bodies<ST_SCATTER, KC, SCAL, KF><<<g, 128, 0, s>>>(a);
-        else k_adj_bodies<ST_SYMMETRIC, KC, SCAL, KF><<<g, 128, 0, s>>>(a);
+        if (st == ST_GATHER) k_adj_bodies<ST_GATHER, KC, SCAL, DG, KF><<<g, ADJ_BODY_THREADS, 0, s>>>(a);
+        else if (st == ST_SCATTER) k_adj_bodies<ST_SCATTER, KC, SCAL, DG, KF><<<g, ADJ_BODY_THREADS, 0, s>>>(a);
+        else k_adj_bodies<ST_SYMMETRIC, KC, SCAL, DG, KF><<<g, ADJ_BODY_THREADS, 0, s>>>(a);
     } else if (pass == 3) {
-        k_adj_combine<KC><<<g, 128, 0, s>>>(a);
+        k_adj_combine<KC, DG><<<g, 128, 0, s>>>(a);
     } else {
         if (st == ST_GATHER) k_adj_points<ST_GATHER, KC, SCAL, KF><<<g, 128, 0, s>>>(a);
         else if (st == ST_SCATTER) k_adj_points<ST_SCATTER, KC, SCAL, KF><<<g, 128, 0, s>>>(a);
         else k_adj_points<ST_SYMMETRIC, KC, SCAL, KF><<<g, 128, 0, s>>>(a);
     }
 }
+// The terms a catalog needs: scalars only, gradients, or the density gradient too
+enum { ADJ_SCAL = 0, ADJ_GRAD = 1, ADJ_FULL = 2 };
 // kf: 0 = the M4 code, 1 = the other kernel families
+template <int KC, int KF>
+static void launch_adj_points_k(const AdjArgs& a, int st, int mode, int pass, unsigned g, cudaStream_t s) {
+    if (mode == ADJ_SCAL) launch_adj_points_ks<KC, true, false, KF>(a, st, pass, g, s);
+    else if (mode == ADJ_GRAD) launch_adj_points_ks<KC, false, false, KF>(a, st, pass, g, s);
+    else launch_adj_points_ks<KC, false, true, KF>(a, st, pass, g, s);
+}
 template <int KC>
-static void launch_adj_points_k(const AdjArgs& a, int st, bool scal, int kf, int pass, unsigned g, cudaStream_t s) {
-    if (kf == 0) {
-        if (scal) launch_adj_points_ks<KC, true, 0>(a, st, pass, g, s);
-        else launch_adj_points_ks<KC, false, 0>(a, st, pass, g, s);
-    } else {
-        if (scal) launch_adj_points_ks<KC, true, 1>(a, st, pass, g, s);
-        else launch_adj_points_ks<KC, false, 1>(a, st, pass, g, s);
-    }
-}
-static void launch_adj_rows(int kcl, bool scal, const double* lam, int64_t ns, int kc, const TreeView<double>& sv,
-                            double* rec, cudaStream_t s) {
+static int launch_adj_rows_k(int mode, const double* lam, int64_t ns, int kc, const TreeView<double>& sv, double* rec,
+                             cudaStream_t s) {
     const unsigned g = (unsigned)((ns + 255) / 256);
-    if (scal) {
-        if (kcl == 1) k_adj_rows<1, true><<<g, 256, 0, s>>>(lam, ns, kc, sv, rec);
-        else if (kcl == 2) k_adj_rows<2, true><<<g, 256, 0, s>>>(lam, ns, kc, sv, rec);
-        else if (kcl == 4) k_adj_rows<4, true><<<g, 256, 0, s>>>(lam, ns, kc, sv, rec);
-        else k_adj_rows<8, true><<<g, 256, 0, s>>>(lam, ns, kc, sv, rec);
-    } else {
-        if (kcl == 1) k_adj_rows<1, false><<<g, 256, 0, s>>>(lam, ns, kc, sv, rec);
-        else if (kcl == 2) k_adj_rows<2, false><<<g, 256, 0, s>>>(lam, ns, kc, sv, rec);
-        else if (kcl == 4) k_adj_rows<4, false><<<g, 256, 0, s>>>(lam, ns, kc, sv, rec);
-        else k_adj_rows<8, false><<<g, 256, 0, s>>>(lam, ns, kc, sv, rec);
+    if (rec) {
+        if (mode == ADJ_SCAL) k_adj_rows<KC, true, false><<<g, 256, 0, s>>>(lam, ns, kc, sv, rec);
+        else if (mode == ADJ_GRAD) k_adj_rows<KC, false, false><<<g, 256, 0, s>>>(lam, ns, kc, sv, rec);
+        else k_adj_rows<KC, false, true><<<g, 256, 0, s>>>(lam, ns, kc, sv, rec);
     }
+    return mode == ADJ_SCAL ? AdjRec<KC, true, false>::N : (mode == ADJ_GRAD ? AdjRec<KC, false, false>::N : AdjRec<KC, false, true>::N);
 }
-static void launch_adj_points(const AdjArgs& a, int kcl, int st, bool scal, int kf, int pass, unsigned g,
+// returns the doubles of a record (rec null: nothing is launched)
+static int launch_adj_rows(int kcl, int mode, const double* lam, int64_t ns, int kc, const TreeView<double>& sv,
+                           double* rec, cudaStream_t s) {
+    if (kcl == 1) return launch_adj_rows_k<1>(mode, lam, ns, kc, sv, rec, s);
+    if (kcl == 2) return launch_adj_rows_k<2>(mode, lam, ns, kc, sv, rec, s);
+    if (kcl == 4) return launch_adj_rows_k<4>(mode, lam, ns, kc, sv, rec, s);
+    return launch_adj_rows_k<8>(mode, lam, ns, kc, sv, rec, s);
+}
+static void launch_adj_points(const AdjArgs& a, int kcl, int st, int mode, int kf, int pass, unsigned g,
                               cudaStream_t s) {
-    if (kcl == 1) launch_adj_points_k<1>(a, st, scal, kf, pass, g, s);
-    else if (kcl == 2) launch_adj_points_k<2>(a, st, scal, kf, pass, g, s);
-    else if (kcl == 4) launch_adj_points_k<4>(a, st, scal, kf, pass, g, s);
-    else launch_adj_points_k<8>(a, st, scal, kf, pass, g, s);
+    auto go = [&](auto kc) {
+        if (kf == 0) launch_adj_points_k<decltype(kc)::value, 0>(a, st, mode, pass, g, s);
+        else launch_adj_points_k<decltype(kc)::value, 1>(a, st, mode, pass, g, s);
+    };
+    if (kcl == 1) go(std::integral_constant<int, 1>());
+    else if (kcl == 2) go(std::integral_constant<int, 2>());
+    else if (kcl == 4) go(std::integral_constant<int, 4>());
+    else go(std::integral_constant<int, 8>());
 }
 template <int KC>
 static void launch_adj_beam_k(const AdjArgs& a, int st, unsigned g, cudaStream_t s) {
@@ -334,6 +341,7 @@ int run_adjoint(psb_ctx* c, const SampleReq& rq0, int hmode, const void* hs, int
             J.lam = lams;
             const unsigned g = (unsigned)((n + 127) / 128);
             const int kf = (c->kern == PSB_KERNEL_M4) ? 0 : 1;
+            const int mode = scal ? ADJ_SCAL : (rec.need_dg ? ADJ_FULL : ADJ_GRAD);
             if (c->adj_split) {
                 // Two kernels and a combine: the walk writes each particle
                 // tile's pair lists into blocks of a pool (k_adj_points in its
@@ -346,16 +354,15 @@ int run_adjoint(psb_ctx* c, const SampleReq& rq0, int hmode, const void* hs, int
                 // tiles still left run in k_adj_points.  A call grows the pool
                 // for the next; it starts at two blocks per tile.
                 const int64_t ntiles = (n + 31) / 32;
-                const int nf = 8 + kcl;  // AdjAcc<kcl>::NF
+                const int nf = 4 + kcl + (mode == ADJ_FULL ? 4 : 0);  // AdjAcc::NF
                 const int64_t per_block = (int64_t)ADJ_CH * 32 * 8 + 32 + 8 + (int64_t)nf * 32 * 8;
                 const int64_t cap = (int64_t)(32ll << 30) / per_block;
                 if (c->adj_blocks <= 0) c->adj_blocks = std::min<int64_t>(cap, 2 * ntiles + 64);
-                const int nqc = scal ? 1 + kcl : 8 + 4 * kcl;
-                const int nrec = 6 + ((nqc + 1) & ~1);  // AdjRec<kcl, scal>::N
+                const int nrec = launch_adj_rows(kcl, mode, nullptr, 0, kc, J.sv, nullptr, s);
                 double* recs = (double*)scratch(c, 88, sizeof(double) * (size_t)nrec * ns);
                 if (!recs) return fail(c, PSB_ENOMEM, "scratch allocation failed (adjoint records)");
                 J.lamT = recs;
-                launch_adj_rows(kcl, scal, lams, ns, kc, J.sv, recs, s);
+                launch_adj_rows(kcl, mode, lams, ns, kc, J.sv, recs, s);
                 AdjLists& al = J.al;
                 unsigned ptop = 0, povf = 0;
                 // The walk takes its tiles heaviest first (and with them the pool's
@@ -401,7 +408,7 @@ int run_adjoint(psb_ctx* c, const SampleReq& rq0, int hmode, const void* hs, int
                     al.nblocks = nb;
                     PSB_CUDA_TRY(c, cudaMemsetAsync(al.top, 0, 2 * sizeof(unsigned), s), "memset pool counters");
                     W.al = al;
-                    launch_adj_points(W, kcl, st, scal, kf, 1, g, s);
+                    launch_adj_points(W, kcl, st, mode, kf, 1, g, s);
                     PSB_CUDA_TRY(c, cudaGetLastError(), "adjoint walk launch");
                     unsigned hc[2] = {0, 0};
                     PSB_CUDA_TRY(c, cudaMemcpyAsync(hc, al.top, sizeof(hc), cudaMemcpyDeviceToHost, s), "pool D2H");
@@ -414,13 +421,13 @@ int run_adjoint(psb_ctx* c, const SampleReq& rq0, int hmode, const void* hs, int
                     c->adj_blocks = std::min<int64_t>(cap, std::max<int64_t>(2 * nb, (int64_t)ptop + ptop / 4 + 64));
                 }
                 const int64_t used = std::min<int64_t>((int64_t)ptop, c->adj_blocks);
-                if (used > 0) launch_adj_points(J, kcl, st, scal, kf, 2, (unsigned)((used + 3) / 4), s);
-                launch_adj_points(J, kcl, st, scal, kf, 3, g, s);
+                if (used > 0) launch_adj_points(J, kcl, st, mode, kf, 2, (unsigned)((used + ADJ_BODY_THREADS / 32 - 1) / (ADJ_BODY_THREADS / 32)), s);
+                launch_adj_points(J, kcl, st, mode, kf, 3, g, s);
                 if (povf) {  // tiles the largest pool could not hold
                     AdjArgs F = J;
                     F.tile_list = al.ovf_tiles;
                     F.tile_count = al.ovf_count;
-                    launch_adj_points(F, kcl, st, scal, kf, 0, g, s);
+                    launch_adj_points(F, kcl, st, mode, kf, 0, g, s);
                     ++launches;
                 }
                 PSB_CUDA_TRY(c, cudaGetLastError(), "adjoint kernel launch");
@@ -428,7 +435,7 @@ int run_adjoint(psb_ctx* c, const SampleReq& rq0, int hmode, const void* hs, int
                     c->adj_blocks = std::min<int64_t>(cap, (int64_t)ptop + ptop / 4 + 64);
                 launches += 3;
             } else {
-                launch_adj_points(J, kcl, st, scal, kf, 0, g, s);
+                launch_adj_points(J, kcl, st, mode, kf, 0, g, s);
                 PSB_CUDA_TRY(c, cudaGetLastError(), "adjoint kernel launch");
                 launches += 2;
             }

@@ -42,7 +42,7 @@ struct AdjLists {
     uint8_t* bcnt;        // [block][32]: entries of each lane in the block
     int32_t* bnext;       // [block]: the tile's next block, -1 after its last
     int32_t* btile;       // [block]: the block's tile
-    double* part;         // [block][8 + KC][32]: the block's partial sums (AdjAcc fields)
+    double* part;         // [block][AdjAcc::NF][32]: the block's partial sums
     int32_t* head;        // [tile]: first block, -1 without pairs, -2 overflowed
     unsigned* top;        // blocks taken
     int64_t nblocks;      // pool size
@@ -78,15 +78,15 @@ struct AdjArgs {
     const unsigned* tile_count;
 };
 
-// M4 at delta = x_s - x_b: W, gradW = sigma/h^5 g1(q) delta and the Hessian
-// (xx, yy, zz, xy, xz, yz) = sigma/h^5 (g1 I + g2 q delta delta^T / r^2), with
-// g1 = f'(q)/q and g2 = d g1/dq (kernels/M4_spline.jl:13-36).  r = |delta|,
-// ir = 1/r (0 at r = 0), h and invh = 1/h: 1/q = h ir, so no pair needs a
-// division.  HESS = false leaves H untouched (scalar catalogs need W and
-// gradW only).
-template <bool HESS = true>
-__device__ __forceinline__ void m4_whess(const double dl[3], double r, double ir, double h, double invh, double& W,
-                                         double g[3], double H[6]) {
+// The kernel at delta = x_s - x_b as three numbers: W, gradW = c delta and
+// (with HESS) the Hessian c I + e delta delta^T, with c = sigma/h^5 g1(q),
+// e = sigma/h^5 g2(q) q / r^2, g1 = f'(q)/q and g2 = d g1/dq
+// (kernels/M4_spline.jl:13-36).  r = |delta|, ir = 1/r (0 at r = 0), h and
+// invh = 1/h: 1/q = h ir, so no pair needs a division.  The pair terms need
+// the Hessian only in products with vectors, H v = c v + e (delta . v) delta,
+// so it is never formed.
+template <bool HESS>
+__device__ __forceinline__ void m4_wce(double r, double ir, double h, double invh, double& W, double& c, double& e) {
     const double q = r * invh;
     const double iq = h * ir;
     const double sig = inv_pi<double>();
@@ -96,64 +96,49 @@ __device__ __forceinline__ void m4_whess(const double dl[3], double r, double ir
         f = 1.0 + q * q * (0.75 * q - 1.5);
         g1 = 2.25 * q - 3.0;
         g2 = 2.25;
-    } else if (q < 2.0) {
-        const double a = 2.0 - q;
+    } else {
+        const double a = fmax(2.0 - q, 0.0);
         f = 0.25 * a * a * a;
         g1 = -0.75 * a * a * iq;
         g2 = 0.75 * a * (q + 2.0) * (iq * iq);
-    } else {
-        f = 0.0; g1 = 0.0; g2 = 0.0;
     }
     W = sig * ih3 * f;
-    const double c = sig * ih5 * g1;
-    g[0] = c * dl[0]; g[1] = c * dl[1]; g[2] = c * dl[2];
-    if (!HESS) return;
-    const double e = sig * ih5 * g2 * q * (ir * ir);  // 0 at r = 0 (ir = 0)
-    H[0] = c + e * dl[0] * dl[0]; H[1] = c + e * dl[1] * dl[1]; H[2] = c + e * dl[2] * dl[2];
-    H[3] = e * dl[0] * dl[1]; H[4] = e * dl[0] * dl[2]; H[5] = e * dl[1] * dl[2];
+    c = sig * ih5 * g1;
+    e = HESS ? sig * ih5 * g2 * q * (ir * ir) : 0.0;  // 0 at r = 0 (ir = 0)
 }
 
 // The same for a kernel other than M4 (id k, 3D norm sig): f from kern_fdf,
 // g1 = f'(q)/q and g2 = d g1/dq from kern_g12, with 1/q = h ir.
-template <bool HESS = true>
-__device__ __forceinline__ void kern_whess(int k, double sig, const double dl[3], double r, double ir, double h,
-                                           double invh, double& W, double g[3], double H[6]) {
+template <bool HESS>
+__device__ __forceinline__ void kern_wce(int k, double sig, double r, double ir, double h, double invh, double& W,
+                                         double& c, double& e) {
     const double q = r * invh;
     double f, df, g1, g2;
     kern_fdf<double>(k, q, f, df);
     kern_g12(k, q, h * ir, g1, g2);
     const double ih3 = invh * invh * invh, ih5 = ih3 * invh * invh;
     W = sig * ih3 * f;
-    const double c = sig * ih5 * g1;
-    g[0] = c * dl[0]; g[1] = c * dl[1]; g[2] = c * dl[2];
-    if (!HESS) return;
-    const double e = sig * ih5 * g2 * q * (ir * ir);  // 0 at r = 0 (ir = 0)
-    H[0] = c + e * dl[0] * dl[0]; H[1] = c + e * dl[1] * dl[1]; H[2] = c + e * dl[2] * dl[2];
-    H[3] = e * dl[0] * dl[1]; H[4] = e * dl[0] * dl[2]; H[5] = e * dl[1] * dl[2];
+    c = sig * ih5 * g1;
+    e = HESS ? sig * ih5 * g2 * q * (ir * ir) : 0.0;
 }
 
-// W, gradW (and H) of the context's kernel: KF = 0 is the M4 code, KF = 1 any
+// W, c (and e) of the context's kernel: KF = 0 is the M4 code, KF = 1 any
 // other family (the warp-uniform id in pt.kern)
 template <int KF, bool HESS>
-__device__ __forceinline__ void whess(const TreeView<double>& pt, const double dl[3], double r, double ir, double h,
-                                      double invh, double& W, double g[3], double H[6]) {
-    if constexpr (KF == 0) m4_whess<HESS>(dl, r, ir, h, invh, W, g, H);
-    else kern_whess<HESS>(pt.kern, (double)pt.sig, dl, r, ir, h, invh, W, g, H);
-}
-
-__device__ __forceinline__ void hmul(const double H[6], const double v[3], double o[3]) {
-    o[0] = H[0] * v[0] + H[3] * v[1] + H[4] * v[2];
-    o[1] = H[3] * v[0] + H[1] * v[1] + H[5] * v[2];
-    o[2] = H[4] * v[0] + H[5] * v[1] + H[2] * v[2];
+__device__ __forceinline__ void wce(const TreeView<double>& pt, double r, double ir, double h, double invh, double& W,
+                                    double& c, double& e) {
+    if constexpr (KF == 0) m4_wce<HESS>(r, ir, h, invh, W, c, e);
+    else kern_wce<HESS>(pt.kern, (double)pt.sig, r, ir, h, invh, W, c, e);
 }
 
 // Per-particle sums of the pair terms; the particle's factors 1/rho_b,
 // m_b/rho_b and m_b are applied once after its last pair:
 // dL/dm_b = sW / rho_b + sD, dL/dA_c,b = m_b/rho_b sA_c,
 // dL/dx_b = -(m_b/rho_b vS + m_b vD)
-template <int KC> struct AdjAcc {
-    static constexpr int NF = 8 + KC;  // fields, in the order of f()
-    double sW, sD, vS[3], vD[3], sA[KC];
+// (DG: the catalog has a density gradient; without one sD and vD are 0)
+template <int KC, bool DG> struct AdjAcc {
+    static constexpr int NF = 4 + KC + (DG ? 4 : 0);  // fields, in the order of f()
+    double sW, vS[3], sA[KC], sD, vD[3];
     __device__ __forceinline__ void zero() {
         sW = 0.0; sD = 0.0;
 #pragma unroll
@@ -161,9 +146,9 @@ template <int KC> struct AdjAcc {
 #pragma unroll
         for (int c = 0; c < KC; ++c) sA[c] = 0.0;
     }
-    // field i: sW, sD, vS (3), vD (3), sA (KC)
+    // field i: sW, vS (3), sA (KC), sD, vD (3)
     __device__ __forceinline__ double& f(int i) {
-        return i == 0 ? sW : (i == 1 ? sD : (i < 5 ? vS[i - 2] : (i < 8 ? vD[i - 5] : sA[i - 8])));
+        return i == 0 ? sW : (i < 4 ? vS[i - 1] : (i < 4 + KC ? sA[i - 4] : (i == 4 + KC ? sD : vD[i - 5 - KC])));
     }
 };
 
@@ -183,91 +168,95 @@ struct RowsStrided {
     template <bool SCAL> __device__ __forceinline__ double Sw(int c) const { return ls[((SCAL ? 1 : 8) + c) * rs]; }
     __device__ __forceinline__ double Sg(int c, int d) const { return ls[(8 + kc + 3 * c + d) * rs]; }
 };
-// Per-sample records of k_adj_bodies: x, y, z, h_a, 1/h_a, 0, then the sum
+// Per-sample records of k_adj_bodies: x, y, z, h_a, 1/h_a, then the sum
 // cotangents with the columns at fixed places for KC columns (those past the
 // catalog's kc are 0), padded to whole 16-byte pairs: one record is read with
 // 128-bit loads, where separate arrays would take a 32-byte sector per value.
-template <int KC, bool SCAL> struct AdjRec {
-    static constexpr int NQ = SCAL ? 1 + KC : 8 + 4 * KC;
-    static constexpr int N = 6 + ((NQ + 1) & ~1);  // doubles per record
+// Order: S1, G (3, not SCAL), Sw_c, Sg_c (3 per column, not SCAL), then with a
+// density gradient Dm, Dg (3).
+template <int KC, bool SCAL, bool DG> struct AdjRec {
+    static constexpr int SW = SCAL ? 1 : 4, SG = SW + KC, DM = SG + (SCAL ? 0 : 3 * KC);
+    static constexpr int NQ = DM + (DG ? 4 : 0);
+    static constexpr int N = (5 + NQ + 1) & ~1;  // doubles per record
 };
-template <int KC, bool SCAL> struct RowsRec {
-    double q[AdjRec<KC, SCAL>::N - 6];
-    template <bool S> __device__ __forceinline__ double S1() const { return q[0]; }
-    __device__ __forceinline__ double G(int d) const { return q[1 + d]; }
-    __device__ __forceinline__ double Dm() const { return q[4]; }
-    __device__ __forceinline__ double Dg(int d) const { return q[5 + d]; }
-    template <bool S> __device__ __forceinline__ double Sw(int c) const { return q[(S ? 1 : 8) + c]; }
-    __device__ __forceinline__ double Sg(int c, int d) const { return q[8 + KC + 3 * c + d]; }
+template <int KC, bool SCAL, bool DG> struct RowsRec {
+    using RC = AdjRec<KC, SCAL, DG>;
+    double q[RC::N];  // the whole record, cotangents from q[5]
+    template <bool S> __device__ __forceinline__ double S1() const { return q[5]; }
+    __device__ __forceinline__ double G(int d) const { return q[6 + d]; }
+    __device__ __forceinline__ double Dm() const { return q[5 + RC::DM]; }
+    __device__ __forceinline__ double Dg(int d) const { return q[6 + RC::DM + d]; }
+    template <bool S> __device__ __forceinline__ double Sw(int c) const { return q[5 + RC::SW + c]; }
+    __device__ __forceinline__ double Sg(int c, int d) const { return q[5 + RC::SG + 3 * c + d]; }
 };
 
 // The terms of one pair (sample at (sxv, syv, szv) with h_a = ha, 1/ha = iha;
 // particle xb, hb, ihb = 1/hb, columns Ab) with the sample's sum cotangents R.
-template <int ST, int KC, bool SCAL, int KF, class Rows>
+template <int ST, int KC, bool SCAL, bool DG, int KF, class Rows>
 __device__ __forceinline__ void adj_pair(const TreeView<double>& pt, const double xb[3], double hb, double ihb,
                                          const double (&Ab)[KC], int kc, double sxv, double syv, double szv, double ha,
-                                         double iha, const Rows& R, AdjAcc<KC>& S) {
+                                         double iha, const Rows& R, AdjAcc<KC, DG>& S) {
     const double dl[3] = {sxv - xb[0], syv - xb[1], szv - xb[2]};
     const double r2 = dl[0] * dl[0] + dl[1] * dl[1] + dl[2] * dl[2];
     const double ir = (r2 > 0.0) ? rsqrt(r2) : 0.0;
     const double r = r2 * ir;
-    double W, g[3], H[6];
+    double W, c, e;
     if (ST == ST_GATHER) {
-        whess<KF, !SCAL>(pt, dl, r, ir, ha, iha, W, g, H);
+        wce<KF, !SCAL>(pt, r, ir, ha, iha, W, c, e);
     } else if (ST == ST_SCATTER) {
-        whess<KF, !SCAL>(pt, dl, r, ir, hb, ihb, W, g, H);
+        wce<KF, !SCAL>(pt, r, ir, hb, ihb, W, c, e);
     } else {
-        double Wa, ga3[3], Ha[6], Wb, gb3[3], Hb[6];
-        whess<KF, !SCAL>(pt, dl, r, ir, ha, iha, Wa, ga3, Ha);
-        whess<KF, !SCAL>(pt, dl, r, ir, hb, ihb, Wb, gb3, Hb);
-        W = 0.5 * (Wa + Wb);
-        for (int d = 0; d < 3; ++d) g[d] = 0.5 * (ga3[d] + gb3[d]);
-        if (!SCAL)
-            for (int d = 0; d < 6; ++d) H[d] = 0.5 * (Ha[d] + Hb[d]);
+        double Wb, cb, eb;
+        wce<KF, !SCAL>(pt, r, ir, ha, iha, W, c, e);
+        wce<KF, !SCAL>(pt, r, ir, hb, ihb, Wb, cb, eb);
+        W = 0.5 * (W + Wb);
+        c = 0.5 * (c + cb);
+        e = 0.5 * (e + eb);
     }
+    double aS = R.template S1<SCAL>();
     if constexpr (SCAL) {
-        double aS = R.template S1<SCAL>();
 #pragma unroll
-        for (int c = 0; c < KC; ++c) {
-            if (c < kc) {
-                const double lsw = R.template Sw<SCAL>(c);
-                aS += lsw * Ab[c];
-                S.sA[c] += lsw * W;
+        for (int q = 0; q < KC; ++q) {
+            if (q < kc) {
+                const double lsw = R.template Sw<SCAL>(q);
+                aS += lsw * Ab[q];
+                S.sA[q] += lsw * W;
             }
         }
         S.sW += aS * W;
-        for (int d = 0; d < 3; ++d) S.vS[d] += aS * g[d];
+        const double ac = aS * c;
+        for (int d = 0; d < 3; ++d) S.vS[d] += ac * dl[d];
         return;
     }
-    const double lS1 = R.template S1<SCAL>();
-    const double lG[3] = {R.G(0), R.G(1), R.G(2)};
-    const double lDm = R.Dm();
-    const double lDg[3] = {R.Dg(0), R.Dg(1), R.Dg(2)};
-    double aS = lS1, aG[3] = {lG[0], lG[1], lG[2]};
+    double aG[3] = {R.G(0), R.G(1), R.G(2)};
 #pragma unroll
-    for (int c = 0; c < KC; ++c) {
-        if (c < kc) {
-            const double lsw = R.template Sw<SCAL>(c);
-            const double lsg[3] = {R.Sg(c, 0), R.Sg(c, 1), R.Sg(c, 2)};
-            aS += lsw * Ab[c];
-            aG[0] += Ab[c] * lsg[0]; aG[1] += Ab[c] * lsg[1]; aG[2] += Ab[c] * lsg[2];
-            S.sA[c] += lsw * W + lsg[0] * g[0] + lsg[1] * g[1] + lsg[2] * g[2];
+    for (int q = 0; q < KC; ++q) {
+        if (q < kc) {
+            const double lsw = R.template Sw<SCAL>(q);
+            const double lsg[3] = {R.Sg(q, 0), R.Sg(q, 1), R.Sg(q, 2)};
+            aS += lsw * Ab[q];
+            aG[0] += Ab[q] * lsg[0]; aG[1] += Ab[q] * lsg[1]; aG[2] += Ab[q] * lsg[2];
+            S.sA[q] += lsw * W + c * (lsg[0] * dl[0] + lsg[1] * dl[1] + lsg[2] * dl[2]);
         }
     }
-    S.sW += aS * W + aG[0] * g[0] + aG[1] * g[1] + aG[2] * g[2];
-    S.sD += lDm * W + lDg[0] * g[0] + lDg[1] * g[1] + lDg[2] * g[2];
-    double Ha[3], Hd[3];
-    hmul(H, aG, Ha);
-    hmul(H, lDg, Hd);
-    for (int d = 0; d < 3; ++d) {
-        S.vS[d] += aS * g[d] + Ha[d];
-        S.vD[d] += lDm * g[d] + Hd[d];
+    // v . gradW = c (delta . v), H v = c v + e (delta . v) delta
+    const double dG = aG[0] * dl[0] + aG[1] * dl[1] + aG[2] * dl[2];
+    S.sW += aS * W + c * dG;
+    const double k = aS * c + e * dG;
+    for (int d = 0; d < 3; ++d) S.vS[d] += k * dl[d] + c * aG[d];
+    if constexpr (DG) {
+        const double lDm = R.Dm();
+        const double lDg[3] = {R.Dg(0), R.Dg(1), R.Dg(2)};
+        const double dD = lDg[0] * dl[0] + lDg[1] * dl[1] + lDg[2] * dl[2];
+        S.sD += lDm * W + c * dD;
+        const double kd = lDm * c + e * dD;
+        for (int d = 0; d < 3; ++d) S.vD[d] += kd * dl[d] + c * lDg[d];
     }
 }
 
 // the gradients of particle b (Morton position) from its sums
-template <int KC>
-__device__ __forceinline__ void adj_write(const AdjArgs& A, int64_t b, const AdjAcc<KC>& S, double mb, double rhob,
+template <int KC, bool DG>
+__device__ __forceinline__ void adj_write(const AdjArgs& A, int64_t b, const AdjAcc<KC, DG>& S, double mb, double rhob,
                                           int kc) {
     const double mr = mb / rhob;
     const int64_t o = A.porder[b];
@@ -365,7 +354,7 @@ __global__ void __launch_bounds__(128, (COL || SCAL) ? 8 : 4) k_adj_points(const
         rbmax = fmaxf(rbmax, __shfl_xor_sync(PSB_FULL, rbmax, o));
     }
     const double ihb = 1.0 / hb;
-    AdjAcc<KC> S;
+    AdjAcc<KC, !SCAL> S;
     S.zero();
     const int kc = A.kc;
     const int64_t L = A.lam_stride;
@@ -378,7 +367,7 @@ __global__ void __launch_bounds__(128, (COL || SCAL) ? 8 : 4) k_adj_points(const
         ++n_pairs;
         // row r of this sample: staged, or from global memory
         const RowsStrided R{STAGE ? lst + jj : A.lam + li, STAGE ? (int64_t)SPAN : L, kc};
-        adj_pair<ST, KC, SCAL, KF>(pt, xb, hb, ihb, Ab, kc, sxv, syv, szv, ha, iha, R, S);
+        adj_pair<ST, KC, SCAL, !SCAL, KF>(pt, xb, hb, ihb, Ab, kc, sxv, syv, szv, ha, iha, R, S);
     };
 
     // COL: this tile's chain of list blocks (block, this lane's entries in it)
@@ -551,7 +540,7 @@ __global__ void __launch_bounds__(128, (COL || SCAL) ? 8 : 4) k_adj_points(const
             A.al.head[tile] = -1;
         }
     } else if (valid) {
-        adj_write<KC>(A, b, S, mb, rhob, kc);
+        adj_write<KC, !SCAL>(A, b, S, mb, rhob, kc);
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) n_pairs += __shfl_xor_sync(PSB_FULL, n_pairs, o);
@@ -566,89 +555,168 @@ __global__ void __launch_bounds__(128, (COL || SCAL) ? 8 : 4) k_adj_points(const
     if (!ok && lane == 0) atomicOr(A.err, PSB_DERR_TRAVERSAL);
 }
 
-// The pair terms of the two-kernel path, one list block per warp: lane j
-// sums the pairs of the block's entries of particle j of the block's tile
-// (its own partial sums, from zero) and stores them with the block.  A block
-// holds at most ADJ_CH entries per lane, so the work items are of like size
-// however long a particle's list is: a tile of large-h particles in the
-// outskirts (pair lists 60 times the mean tile's) spreads over as many warps
-// as it has blocks, where one warp per tile left it running long after the
-// others.  Each pair reads its sample as one record (AdjRec) with 128-bit
-// loads.
-template <int ST, int KC, bool SCAL, int KF>
-__global__ void __launch_bounds__(128, 4) k_adj_bodies(const AdjArgs A) {
+// The pair terms of the two-kernel path, one list block per warp.  A block
+// holds at most ADJ_CH entries for each of its tile's 32 particles, so the work
+// items are of like size however long a particle's list is; but within one
+// the particles' pairs are few or many (one particle per lane kept 12 of 32
+// lanes busy).  So the block's pairs, particle after particle, are dealt out
+// in 32 equal runs: a lane sums its run particle by particle, writes what it
+// holds alone, and leaves what it shares with its neighbours (its first and
+// last particle) in shared memory, where each particle's shares are then added
+// in the order of the lanes.  Runs and order follow from the block alone.
+// Each pair reads its sample as one record (AdjRec) with 128-bit loads.
+// Bound by FP64 issue and the records' L1 traffic: 2M Plummer particles,
+// 128^3 grid, 8 fields: 10.1 -> 5.4 ms.  CTAs of one warp, 16 per SM (4 of four: 6.0 ms, a CTA lasts as
+// long as its longest warp; 20 at fewer registers: slower).
+constexpr int ADJ_BODY_THREADS = 32, ADJ_BODY_CTAS = 16;
+template <int ST, int KC, bool SCAL, bool DG, int KF>
+__global__ void __launch_bounds__(ADJ_BODY_THREADS, ADJ_BODY_CTAS) k_adj_bodies(const __grid_constant__ AdjArgs A) {
+    using Acc = AdjAcc<KC, DG>;
+    using RC = AdjRec<KC, SCAL, DG>;
+    struct Stage {
+        double pd[5 + KC][32];          // particles: x, y, z, h, 1/h, columns
+        double seg[2][Acc::NF][32];     // a lane's first and last particle
+        int off[33];                    // pairs before each particle
+    };
+    __shared__ Stage stage_all[ADJ_BODY_THREADS / 32];
     const TreeView<double>& pt = A.pt;
     const int lane = threadIdx.x & 31;
+    Stage& st = stage_all[threadIdx.x >> 5];
     const int64_t blk = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     const int64_t used = (int64_t)*A.al.top;
     if (blk >= (used < A.al.nblocks ? used : A.al.nblocks)) return;  // warp-uniform
     const int64_t tile = A.al.btile[blk];
     // A tile the pool ran out on is k_adj_points' (its last block's counts
     // were never written): skip its blocks.
-    if (A.al.head[tile] == -2) return;  // warp-uniform
-    const int64_t b = tile * 32 + lane;
-    const bool valid = b < pt.n;
+    const int32_t head = A.al.head[tile];
+    if (head == -2) return;  // warp-uniform
+    // a tile's only block holds its particles' sums (k_adj_combine starts from
+    // the first block's sums, so both give the same bits)
+    const bool single = head == blk && A.al.bnext[blk] < 0;
     const int kc = A.kc;
-    double xb[3] = {0.0, 0.0, 0.0}, hb = 1.0, Ab[KC];
+    const uint2* ent = A.al.ent + (size_t)blk * ADJ_CH * 32;
+    int cnt = 0;  // pairs of particle `lane` in the block
+    {
+        const int64_t b = tile * 32 + lane;
+        const bool valid = b < pt.n;
+        const double hb = valid ? pt.h[b] : 1.0;
+        st.pd[0][lane] = valid ? pt.x[b] : 0.0;
+        st.pd[1][lane] = valid ? pt.y[b] : 0.0;
+        st.pd[2][lane] = valid ? pt.z[b] : 0.0;
+        st.pd[3][lane] = hb;
+        st.pd[4][lane] = 1.0 / hb;
 #pragma unroll
-    for (int c = 0; c < KC; ++c) Ab[c] = 0.0;
-    if (valid) {
-        xb[0] = pt.x[b]; xb[1] = pt.y[b]; xb[2] = pt.z[b];
-        hb = pt.h[b];
+        for (int c = 0; c < KC; ++c) st.pd[5 + c][lane] = (valid && c < kc) ? A.colT[c][b] : 0.0;
+        const int ne = valid ? A.al.bcnt[blk * 32 + lane] : 0;
+        for (int e = 0; e < ne; ++e) cnt += __popc(ent[e * 32 + lane].y);
+        int s = cnt;
 #pragma unroll
-        for (int c = 0; c < KC; ++c)
-            if (c < kc) Ab[c] = A.colT[c][b];
-    }
-    const double ihb = 1.0 / hb;
-    AdjAcc<KC> P;
-    P.zero();
-    const int ne = valid ? A.al.bcnt[blk * 32 + lane] : 0;
-    int e = 0;
-    unsigned m = 0;
-    int64_t lo = 0;
-    auto next = [&]() -> bool {  // the next pair: sample lo + ffs(m) - 1
-        while (m == 0) {
-            if (e >= ne) return false;
-            const uint2 q = A.al.ent[((size_t)blk * ADJ_CH + e) * 32 + lane];
-            lo = (int64_t)q.x;
-            m = q.y;
-            ++e;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int t = __shfl_up_sync(PSB_FULL, s, o);
+            if (lane >= o) s += t;
         }
-        return true;
+        st.off[lane + 1] = s;
+        if (lane == 0) st.off[0] = 0;
+    }
+    __syncwarp();
+    const int P = st.off[32];
+    auto emit = [&](int q, Acc& S) {  // the block's sums of particle q
+        if (single) {
+            const int64_t b = tile * 32 + q;
+            if (b < pt.n) adj_write<KC, DG>(A, b, S, pt.m[b], pt.rho[b], kc);
+        } else {
+            double* o = A.al.part + (size_t)blk * Acc::NF * 32 + q;
+#pragma unroll
+            for (int f = 0; f < Acc::NF; ++f) o[(size_t)f * 32] = S.f(f);
+        }
     };
-    unsigned long long n_pairs = 0;
-    bool has = next();
-    while (__any_sync(PSB_FULL, has)) {
-        if (has) {
-            const int64_t s = lo + __ffs(m) - 1;
-            m &= m - 1;
-            ++n_pairs;
-            using RC = AdjRec<KC, SCAL>;
-            const double2* rp = reinterpret_cast<const double2*>(A.lamT + s * RC::N);
-            const double2 h0 = __ldg(rp), h1 = __ldg(rp + 1), h2 = __ldg(rp + 2);
-            RowsRec<KC, SCAL> R;
+    Acc S;
+    S.zero();
+    {
+        const int i0 = P * lane / 32, i1 = P * (lane + 1) / 32;  // this lane's run
+        if (i0 < i1) {
+            int p = 0;  // the particle of pair i0: the last one with off[p] <= i0
 #pragma unroll
-            for (int k = 0; k < (RC::N - 6) / 2; ++k) {
-                const double2 v = __ldg(rp + 3 + k);
-                R.q[2 * k] = v.x;
-                R.q[2 * k + 1] = v.y;
+            for (int o = 16; o > 0; o >>= 1)
+                if (st.off[p + o] <= i0) p += o;
+            double xb[3], hb, ihb, Ab[KC];
+            auto load = [&]() {
+                xb[0] = st.pd[0][p]; xb[1] = st.pd[1][p]; xb[2] = st.pd[2][p];
+                hb = st.pd[3][p]; ihb = st.pd[4][p];
+#pragma unroll
+                for (int c = 0; c < KC; ++c) Ab[c] = st.pd[5 + c][p];
+            };
+            load();
+            int skip = i0 - st.off[p], e = 0, end = st.off[p + 1];
+            uint2 q = ent[p];
+            while (skip >= __popc(q.y)) {
+                skip -= __popc(q.y);
+                ++e;
+                q = ent[e * 32 + p];
             }
-            adj_pair<ST, KC, SCAL, KF>(pt, xb, hb, ihb, Ab, kc, h0.x, h0.y, h1.x, h1.y, h2.x, R, P);
-            has = next();
+            for (; skip > 0; --skip) q.y &= q.y - 1;
+            bool first = true;  // the lane's first particle
+            for (int i = i0; i < i1; ++i) {
+                const double2* rp = reinterpret_cast<const double2*>(
+                    A.lamT + (int64_t)(q.x + (unsigned)__ffs(q.y) - 1u) * RC::N);
+                q.y &= q.y - 1;
+                RowsRec<KC, SCAL, DG> R;
+#pragma unroll
+                for (int k = 0; k < RC::N / 2; ++k) {
+                    const double2 v = __ldg(rp + k);
+                    R.q[2 * k] = v.x;
+                    R.q[2 * k + 1] = v.y;
+                }
+                adj_pair<ST, KC, SCAL, DG, KF>(pt, xb, hb, ihb, Ab, kc, R.q[0], R.q[1], R.q[2], R.q[3], R.q[4], R, S);
+                if (i + 1 == end) {  // the particle's last pair
+                    if (first) {
+#pragma unroll
+                        for (int f = 0; f < Acc::NF; ++f) st.seg[0][f][lane] = S.f(f);
+                    } else {
+                        emit(p, S);
+                    }
+                    first = false;
+                    S.zero();
+                    if (i + 1 < i1) {
+                        do ++p;
+                        while (st.off[p + 1] == end);
+                        end = st.off[p + 1];
+                        load();
+                        e = 0;
+                        q = ent[p];
+                    }
+                } else if (q.y == 0) {
+                    ++e;
+                    q = ent[e * 32 + p];
+                }
+            }
+            if (i1 != end) {  // the particle goes on in the next lane
+#pragma unroll
+                for (int f = 0; f < Acc::NF; ++f) st.seg[first ? 0 : 1][f][lane] = S.f(f);
+            }
         }
     }
-    if (A.al.head[tile] == blk && A.al.bnext[blk] < 0) {
-        // the tile's only block: its sums are the particles' (k_adj_combine
-        // starts from the first block's sums, so both give the same bits)
-        if (valid) adj_write<KC>(A, b, P, pt.m[b], pt.rho[b], kc);
+    __syncwarp();
+    // lane q: particle q, unless one lane held all of it and more before it
+    const int o0 = st.off[lane], o1 = st.off[lane + 1];
+    if (o1 > o0) {
+        const int a = (32 * (o0 + 1) + P - 1) / P - 1, b = (32 * o1 + P - 1) / P - 1;  // lanes of its first and last pair
+        const bool mid = P * a / 32 < o0;  // lane a began with another particle
+        if (!(a == b && mid)) {
+#pragma unroll
+            for (int f = 0; f < Acc::NF; ++f) S.f(f) = st.seg[mid ? 1 : 0][f][a];
+            for (int l = a + 1; l <= b; ++l) {
+                if (P * l / 32 == P * (l + 1) / 32) continue;
+#pragma unroll
+                for (int f = 0; f < Acc::NF; ++f) S.f(f) += st.seg[0][f][l];
+            }
+            emit(lane, S);
+        }
     } else {
-        double* o = A.al.part + (size_t)blk * AdjAcc<KC>::NF * 32 + lane;
-#pragma unroll
-        for (int f = 0; f < AdjAcc<KC>::NF; ++f) o[(size_t)f * 32] = P.f(f);
+        S.zero();
+        emit(lane, S);
     }
-#pragma unroll
-    for (int q = 16; q > 0; q >>= 1) n_pairs += __shfl_xor_sync(PSB_FULL, n_pairs, q);
-    if (lane == 0 && A.stats) atomicAdd(&A.stats[6], n_pairs);
+    if (lane == 0 && A.stats) atomicAdd(&A.stats[6], (unsigned long long)P);
 }
 
 // The gradients of each particle of a tile of several blocks (and zeros for
@@ -657,8 +725,9 @@ __global__ void __launch_bounds__(128, 4) k_adj_bodies(const AdjArgs A) {
 // factors (adj_write).  The blocks' boundaries follow from the
 // walk, so the result does not depend on the pool or on which block landed
 // where in it.
-template <int KC>
-__global__ void __launch_bounds__(128) k_adj_combine(const AdjArgs A) {
+template <int KC, bool DG>
+__global__ void __launch_bounds__(128) k_adj_combine(const __grid_constant__ AdjArgs A) {
+    using Acc = AdjAcc<KC, DG>;
     const TreeView<double>& pt = A.pt;
     const int lane = threadIdx.x & 31;
     const int64_t tile = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -667,47 +736,52 @@ __global__ void __launch_bounds__(128) k_adj_combine(const AdjArgs A) {
     if (b >= pt.n) return;
     int64_t blk = A.al.head[tile];
     if (blk == -2) return;  // overflowed: k_adj_points owns the tile
-    AdjAcc<KC> T;
+    Acc T;
     T.zero();
     if (blk >= 0) {
         int64_t nxt = A.al.bnext[blk];
         if (nxt < 0) return;  // one block: k_adj_bodies wrote the gradients
-        const double* o = A.al.part + (size_t)blk * AdjAcc<KC>::NF * 32 + lane;
+        const double* o = A.al.part + (size_t)blk * Acc::NF * 32 + lane;
 #pragma unroll
-        for (int f = 0; f < AdjAcc<KC>::NF; ++f) T.f(f) = o[(size_t)f * 32];
+        for (int f = 0; f < Acc::NF; ++f) T.f(f) = o[(size_t)f * 32];
         for (blk = nxt; blk >= 0; blk = A.al.bnext[blk]) {
-            o = A.al.part + (size_t)blk * AdjAcc<KC>::NF * 32 + lane;
+            o = A.al.part + (size_t)blk * Acc::NF * 32 + lane;
 #pragma unroll
-            for (int f = 0; f < AdjAcc<KC>::NF; ++f) T.f(f) += o[(size_t)f * 32];
+            for (int f = 0; f < Acc::NF; ++f) T.f(f) += o[(size_t)f * 32];
         }
     }
-    adj_write<KC>(A, b, T, pt.m[b], pt.rho[b], A.kc);
+    adj_write<KC, DG>(A, b, T, pt.m[b], pt.rho[b], A.kc);
 }
 
 // The records of k_adj_bodies (AdjRec), one per sample of the sample tree:
 // position, h_a, 1/h_a and the sum cotangents (lam: rows [q][sample] in the
 // tree's order) at the record's fixed places.
-template <int KC, bool SCAL>
+template <int KC, bool SCAL, bool DG>
 __global__ void k_adj_rows(const double* lam, int64_t ns, int kc, const TreeView<double> sv, double* rec) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= ns) return;
-    using RC = AdjRec<KC, SCAL>;
-    double* o = rec + i * RC::N;
+    using RC = AdjRec<KC, SCAL, DG>;
+    double v[RC::N];
     const double h = sv.h[i];
-    o[0] = sv.x[i]; o[1] = sv.y[i]; o[2] = sv.z[i]; o[3] = h; o[4] = 1.0 / h;
-    for (int r = 5; r < RC::N; ++r) o[r] = 0.0;
-    double* q = o + 6;
+#pragma unroll
+    for (int r = 0; r < RC::N; ++r) v[r] = 0.0;
+    v[0] = sv.x[i]; v[1] = sv.y[i]; v[2] = sv.z[i]; v[3] = h; v[4] = 1.0 / h;
     auto row = [&](int r) { return lam[(int64_t)r * ns + i]; };  // compact row r (kc columns)
-    if (SCAL) {
-        q[0] = row(0);
-        for (int c = 0; c < kc; ++c) q[1 + c] = row(8 + c);  // lambda_Sw_c
-    } else {
-        for (int r = 0; r < 8; ++r) q[r] = row(r);
-        for (int c = 0; c < kc; ++c) {
-            q[8 + c] = row(8 + c);
-            for (int d = 0; d < 3; ++d) q[8 + KC + 3 * c + d] = row(8 + kc + 3 * c + d);
-        }
+    v[5] = row(0);
+#pragma unroll
+    for (int c = 0; c < KC; ++c) {
+        if (c >= kc) continue;
+        v[5 + RC::SW + c] = row(8 + c);
+        if (!SCAL)
+            for (int d = 0; d < 3; ++d) v[5 + RC::SG + 3 * c + d] = row(8 + kc + 3 * c + d);
     }
+    if (!SCAL)
+        for (int d = 0; d < 3; ++d) v[6 + d] = row(1 + d);
+    if (DG)
+        for (int d = 0; d < 4; ++d) v[5 + RC::DM + d] = row(4 + d);
+    double2* o = reinterpret_cast<double2*>(rec + i * RC::N);
+#pragma unroll
+    for (int r = 0; r < RC::N / 2; ++r) o[r] = make_double2(v[2 * r], v[2 * r + 1]);
 }
 
 // line-integrated kernel and its r-derivative: the slope of the table segment
