@@ -19,9 +19,10 @@
 // LBVH built over the samples (node scale = subtree max of h_a) with the
 // forward's radius rules seen from the particle, and re-decides every pair
 // with the forward's exact arithmetic, so the pair set is the forward's.
-// Parallel-beam lines: one thread per particle visits the pixels whose lines
-// can pass within its support (the particle projected onto the frame plane)
-// and re-decides each pair with the forward's line distance.
+// Parallel-beam lines: the pixels whose lines can pass within a particle's
+// support (the particle projected onto the frame plane) are visited by a
+// lane, eight lanes or a warp, after their number, and each pair is re-decided
+// with the forward's line distance.
 #pragma once
 
 #include "k_points.cuh"
@@ -785,108 +786,223 @@ __global__ void k_adj_rows(const double* lam, int64_t ns, int kc, const TreeView
 }
 
 // line-integrated kernel and its r-derivative: the slope of the table segment
-// that line_W interpolates on (LUT_N entries over [0, K], K the support)
-__device__ __forceinline__ void line_Wd(double r, double h, const double* lut, double K, double& W, double& dW) {
-    const double invh = 1.0 / h;
+// that line_W interpolates on (LUT_N entries over [0, K], K the support,
+// idq = 1/spacing)
+__device__ __forceinline__ void line_Wd(double r, double invh, const double* lut, double K, double idq, double& W,
+                                        double& dW) {
     const double q = r * invh;
     if (q >= K) { W = 0.0; dW = 0.0; return; }
-    const double dq = K / (double)(LUT_N - 1);
-    const double idxf = q / dq + 1.0;
+    const double idxf = q * idq + 1.0;
     int i = (int)idxf;
     i = i < 1 ? 1 : (i > LUT_N - 1 ? LUT_N - 1 : i);
     const double t = idxf - (double)i;
-    W = invh * (lut[i - 1] * (1.0 - t) + lut[i] * t);
-    dW = invh * invh * (lut[i] - lut[i - 1]) / dq;
+    const double l0 = __ldg(&lut[i - 1]), l1 = __ldg(&lut[i]);
+    W = invh * (l0 * (1.0 - t) + l1 * t);
+    dW = invh * invh * (l1 - l0) * idq;
 }
 
-template <int ST, int KC>
-__global__ void __launch_bounds__(128) k_adj_beam(const AdjArgs A) {
-    const TreeView<double>& pt = A.pt;
-    const int64_t b = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (b >= pt.n) return;
-    const double xb[3] = {pt.x[b], pt.y[b], pt.z[b]};
-    const double hb = pt.h[b], mb = pt.m[b], rhob = pt.rho[b], mr = mb / rhob;
-    const int kc = A.kc;
-    double Ab[KC];
+// A particle of the beam adjoint and the pixels its support can reach.
+template <int KC> struct BeamPart {
+    double x[3], h, ih, mr;
+    double A[KC];
+    double u, w, ru, rw;   // centre and half widths on the frame plane, in pixels
+    int i0, i1, j0, j1;    // pixels inside those (empty: i1 < i0 or j1 < j0)
+};
+// Partial gradients: sum aS W, sum s (D - (D.m) m), sum lambda_Sw_c W
+template <int KC> struct BeamAcc {
+    double m, x[3], A[KC];
+    __device__ __forceinline__ void zero() {
+        m = 0.0;
+        for (int d = 0; d < 3; ++d) x[d] = 0.0;
 #pragma unroll
-    for (int c = 0; c < KC; ++c) Ab[c] = (c < kc) ? A.colT[c][b] : 0.0;
+        for (int c = 0; c < KC; ++c) A[c] = 0.0;
+    }
+    __device__ __forceinline__ void add_xor(int o) {
+        m += __shfl_xor_sync(PSB_FULL, m, o);
+#pragma unroll
+        for (int d = 0; d < 3; ++d) x[d] += __shfl_xor_sync(PSB_FULL, x[d], o);
+#pragma unroll
+        for (int c = 0; c < KC; ++c) A[c] += __shfl_xor_sync(PSB_FULL, A[c], o);
+    }
+};
+
+// One warp per 32 particles.  A particle's pixels are those of the bounding
+// rectangle of its support on the frame plane, re-decided with the forward's
+// line distance.  A particle of at most BEAM_LANE pixels is one lane's; up to
+// BEAM_GROUP eight lanes share it (4 x 2 pixels at a time, four particles
+// side by side), larger ones the warp (8 x 4).  One thread per particle kept
+// 17 of 32 lanes active (supports span decades in pixels), visited a pixel
+// more than needed on every side, and divided four times a pair: 1M clump
+// particles, 512^2 beam: 10.0 -> 3.1 ms.
+constexpr int BEAM_LANE = 12, BEAM_GROUP = 160;
+template <int ST, int KC>
+__global__ void __launch_bounds__(128, 4) k_adj_beam(const __grid_constant__ AdjArgs A) {
+    const TreeView<double>& pt = A.pt;
+    const int lane = threadIdx.x & 31;
+    const int64_t b = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (b - lane >= pt.n) return;  // warp-uniform
+    const bool valid = b < pt.n;
+    const int kc = A.kc;
     const SampleSrc<double>& B = A.beam;
     const double* f = B.frame;
-    // the particle on the frame plane (frame axes orthonormal)
-    const double v[3] = {xb[0] - f[0], xb[1] - f[1], xb[2] - f[2]};
-    const double xi = v[0] * f[3] + v[1] * f[4] + v[2] * f[5];
-    const double eta = v[0] * f[6] + v[1] * f[7] + v[2] * f[8];
     const double K = pt.Kd;  // the support (2 for M4)
-    const double R = K * fmax(hb, A.ha_max) * (1.0 + 1e-9) + 1e-300;
-    const double dxi = (B.params[1] - B.params[0]) / (double)(B.nx - 1);
-    const double deta = (B.params[3] - B.params[2]) / (double)(B.ny - 1);
-    auto range = [](double c, double R, double lo0, double d, int64_t n, int64_t& a, int64_t& z) {
-        double u0 = (c - R - lo0) / d, u1 = (c + R - lo0) / d;
-        if (u0 > u1) { double t = u0; u0 = u1; u1 = t; }
-        u0 = floor(u0) - 1.0;
-        u1 = ceil(u1) + 1.0;
-        a = u0 < 0.0 ? 0 : (u0 > (double)(n - 1) ? n : (int64_t)u0);
-        z = u1 > (double)(n - 1) ? n - 1 : (u1 < 0.0 ? -1 : (int64_t)u1);
-    };
-    int64_t i0, i1, j0, j1;
-    range(xi, R, B.params[0], dxi, B.nx, i0, i1);
-    range(eta, R, B.params[2], deta, B.ny, j0, j1);
-    double gm = 0.0, gx[3] = {0.0, 0.0, 0.0}, ga[KC];
-#pragma unroll
-    for (int c = 0; c < KC; ++c) ga[c] = 0.0;
+    const double idq = (double)(LUT_N - 1) / K;
+    const double dxi = X<double>::div(X<double>::sub(B.params[1], B.params[0]), (double)(B.nx - 1));
+    const double deta = X<double>::div(X<double>::sub(B.params[3], B.params[2]), (double)(B.ny - 1));
     const int64_t L = A.lam_stride;
-    unsigned long long n_pairs = 0;
-    for (int64_t j = j0; j <= j1; ++j) {
-        for (int64_t i = i0; i <= i1; ++i) {
-            const int64_t k = i + B.nx * j;
-            double o[3], m[3];
-            sample_coords(B, k, o, m);
-            double ha = 0.0;
-            if (ST != ST_SCATTER) ha = (A.hmode == PSB_H_PER_SAMPLE) ? A.hs[k] : A.hs[0];
-            const double ra = X<double>::mul(K, ha);
-            const double ra2 = X<double>::mul(ra, ra);
-            const double e2 = ex_d2_line<double>(o, m, xb[0], xb[1], xb[2]);
-            if (!(e2 <= ex_r2<ST, double>(ra2, hb, K))) continue;
-            ++n_pairs;
-            const double dr = sqrt(e2 < 0.0 ? 0.0 : e2);
-            double W, dW;
-            if (ST == ST_GATHER) {
-                line_Wd(dr, ha, A.lut, K, W, dW);
-            } else if (ST == ST_SCATTER) {
-                line_Wd(dr, hb, A.lut, K, W, dW);
-            } else {
-                double Wa, da, Wb, db;
-                line_Wd(dr, ha, A.lut, K, Wa, da);
-                line_Wd(dr, hb, A.lut, K, Wb, db);
-                W = 0.5 * (Wa + Wb);
-                dW = 0.5 * (da + db);
-            }
-            double aS = __ldg(&A.lam[k]);
+    unsigned n_pairs = 0;
+
+    BeamPart<KC> P;
+    P.i0 = P.j0 = 0;
+    P.i1 = P.j1 = -1;
+    if (valid) {
+        P.x[0] = pt.x[b]; P.x[1] = pt.y[b]; P.x[2] = pt.z[b];
+        P.h = pt.h[b];
+        P.ih = 1.0 / P.h;
+        P.mr = pt.m[b] / pt.rho[b];
 #pragma unroll
-            for (int c = 0; c < KC; ++c) {
-                if (c < kc) {
-                    const double lsw = __ldg(&A.lam[(1 + c) * L + k]);
-                    aS += lsw * Ab[c];
-                    ga[c] += mr * lsw * W;
-                }
-            }
-            gm += aS * W / rhob;
-            if (dr > 0.0) {
-                // d r_perp / d x_b = (D - (D.m) m) / r_perp, D = x_b - o
-                const double D[3] = {xb[0] - o[0], xb[1] - o[1], xb[2] - o[2]};
-                const double Dm = D[0] * m[0] + D[1] * m[1] + D[2] * m[2];
-                const double s = mr * aS * dW / dr;
-                for (int d = 0; d < 3; ++d) gx[d] += s * (D[d] - Dm * m[d]);
-            }
+        for (int c = 0; c < KC; ++c) P.A[c] = (c < kc) ? A.colT[c][b] : 0.0;
+        // the particle on the frame plane (frame axes orthonormal), in pixels
+        const double v[3] = {P.x[0] - f[0], P.x[1] - f[1], P.x[2] - f[2]};
+        const double R = K * fmax(fabs(P.h), A.ha_max);
+        P.u = (v[0] * f[3] + v[1] * f[4] + v[2] * f[5] - B.params[0]) / dxi;
+        P.w = (v[0] * f[6] + v[1] * f[7] + v[2] * f[8] - B.params[2]) / deta;
+        // a frame orthonormal to 1e-9 and the roundings of the projection
+        const double slack = 1e-7 * (fabs(v[0]) + fabs(v[1]) + fabs(v[2]) + R);
+        P.ru = (R + slack) / fabs(dxi);
+        P.rw = (R + slack) / fabs(deta);
+        auto range = [](double c, double r, int64_t n, int& a, int& z) {
+            const double lo = ceil(c - r), hi = floor(c + r);
+            a = lo > 0.0 ? (lo < (double)n ? (int)lo : (int)n) : 0;
+            z = hi < (double)(n - 1) ? (hi >= 0.0 ? (int)hi : -1) : (int)(n - 1);
+        };
+        if (P.u == P.u && P.w == P.w && P.ru == P.ru && P.rw == P.rw) {
+            range(P.u, P.ru, B.nx, P.i0, P.i1);
+            range(P.w, P.rw, B.ny, P.j0, P.j1);
         }
     }
-    const int64_t ob = A.porder[b];
-    A.gm[ob] = gm;
-    A.gx[ob] = gx[0]; A.gy[ob] = gx[1]; A.gz[ob] = gx[2];
+    // pixel (i, j) of particle q
+    auto pixel = [&](const BeamPart<KC>& q, BeamAcc<KC>& S, int i, int j) {
+        // the forward's sample coordinates (sample_coords) and line distance
+        const double xi = X<double>::add(B.params[0], X<double>::mul((double)i, dxi));
+        const double eta = X<double>::add(B.params[2], X<double>::mul((double)j, deta));
+        double o[3];
 #pragma unroll
-    for (int c = 0; c < KC; ++c)
-        if (c < kc && A.gcol[c]) A.gcol[c][ob] = ga[c];
-    if (A.stats && n_pairs) atomicAdd(&A.stats[0], n_pairs);
+        for (int c = 0; c < 3; ++c)
+            o[c] = X<double>::add(X<double>::add(f[c], X<double>::mul(xi, f[3 + c])), X<double>::mul(eta, f[6 + c]));
+        const double* m = f + 9;
+        const int64_t k = i + B.nx * (int64_t)j;
+        double ha = 0.0;
+        if (ST != ST_SCATTER) ha = (A.hmode == PSB_H_PER_SAMPLE) ? A.hs[k] : A.hs[0];
+        const double ra = X<double>::mul(K, ha);
+        const double e2 = ex_d2_line<double>(o, m, q.x[0], q.x[1], q.x[2]);
+        if (!(e2 <= ex_r2<ST, double>(X<double>::mul(ra, ra), q.h, K))) return;
+        ++n_pairs;
+        const double ir = e2 > 0.0 ? rsqrt(e2) : 0.0;
+        const double dr = e2 > 0.0 ? e2 * ir : 0.0;
+        double W, dW;
+        if (ST == ST_GATHER) {
+            line_Wd(dr, 1.0 / ha, A.lut, K, idq, W, dW);
+        } else if (ST == ST_SCATTER) {
+            line_Wd(dr, q.ih, A.lut, K, idq, W, dW);
+        } else {
+            double Wb, db;
+            line_Wd(dr, 1.0 / ha, A.lut, K, idq, W, dW);
+            line_Wd(dr, q.ih, A.lut, K, idq, Wb, db);
+            W = 0.5 * (W + Wb);
+            dW = 0.5 * (dW + db);
+        }
+        double aS = __ldg(&A.lam[k]);
+#pragma unroll
+        for (int c = 0; c < KC; ++c) {
+            if (c < kc) {
+                const double lsw = __ldg(&A.lam[(1 + c) * L + k]);
+                aS += lsw * q.A[c];
+                S.A[c] += lsw * W;
+            }
+        }
+        S.m += aS * W;
+        // d r_perp / d x_b = (D - (D.m) m) / r_perp, D = x_b - o (0 at r_perp = 0: ir = 0)
+        const double D[3] = {q.x[0] - o[0], q.x[1] - o[1], q.x[2] - o[2]};
+        const double Dm = D[0] * m[0] + D[1] * m[1] + D[2] * m[2];
+        const double s = aS * dW * ir;
+#pragma unroll
+        for (int d = 0; d < 3; ++d) S.x[d] += s * (D[d] - Dm * m[d]);
+    };
+    auto write = [&](int64_t q, const BeamAcc<KC>& S, double mr) {
+        const int64_t ob = A.porder[q];
+        A.gm[ob] = S.m / pt.rho[q];
+        A.gx[ob] = mr * S.x[0]; A.gy[ob] = mr * S.x[1]; A.gz[ob] = mr * S.x[2];
+#pragma unroll
+        for (int c = 0; c < KC; ++c)
+            if (c < kc && A.gcol[c]) A.gcol[c][ob] = mr * S.A[c];
+    };
+    const int64_t npix = valid ? (int64_t)max(P.i1 - P.i0 + 1, 0) * max(P.j1 - P.j0 + 1, 0) : 0;
+    BeamAcc<KC> S;
+    S.zero();
+    if (valid && npix <= BEAM_LANE) {
+        for (int j = P.j0; j <= P.j1; ++j)
+            for (int i = P.i0; i <= P.i1; ++i) pixel(P, S, i, j);
+        write(b, S, P.mr);
+    }
+    // particle `from` of the warp, in every lane of a group
+    auto fetch = [&](int from) -> BeamPart<KC> {
+        BeamPart<KC> q;
+#pragma unroll
+        for (int d = 0; d < 3; ++d) q.x[d] = __shfl_sync(PSB_FULL, P.x[d], from);
+        q.h = __shfl_sync(PSB_FULL, P.h, from);
+        q.ih = __shfl_sync(PSB_FULL, P.ih, from);
+        q.mr = __shfl_sync(PSB_FULL, P.mr, from);
+#pragma unroll
+        for (int c = 0; c < KC; ++c) q.A[c] = __shfl_sync(PSB_FULL, P.A[c], from);
+        q.u = __shfl_sync(PSB_FULL, P.u, from);
+        q.w = __shfl_sync(PSB_FULL, P.w, from);
+        q.ru = __shfl_sync(PSB_FULL, P.ru, from);
+        q.rw = __shfl_sync(PSB_FULL, P.rw, from);
+        q.i0 = __shfl_sync(PSB_FULL, P.i0, from);
+        q.i1 = __shfl_sync(PSB_FULL, P.i1, from);
+        q.j0 = __shfl_sync(PSB_FULL, P.j0, from);
+        q.j1 = __shfl_sync(PSB_FULL, P.j1, from);
+        return q;
+    };
+    // the pixels of row j inside the support's ellipse
+    auto row = [&](const BeamPart<KC>& q, int j, int& a, int& z) {
+        const double t = ((double)j - q.w) / q.rw, c = q.ru * sqrt(fmax(1.0 - t * t, 0.0)) + 1e-6;
+        a = max(q.i0, (int)fmax(ceil(q.u - c), -1.0));
+        z = min(q.i1, (int)fmin(floor(q.u + c), 2147483000.0));
+    };
+    unsigned todo = __ballot_sync(PSB_FULL, valid && npix > BEAM_LANE && npix <= BEAM_GROUP);
+    while (todo) {  // eight lanes per particle, four particles at a time
+        const int g = lane >> 3;
+        unsigned t = todo;
+        for (int k = 0; k < g; ++k) t &= t - 1;
+        const int from = t ? __ffs(t) - 1 : 0;
+        const BeamPart<KC> q = fetch(from);
+        S.zero();
+        if (t)
+            for (int j = q.j0 + ((lane >> 2) & 1); j <= q.j1; j += 2)
+                for (int i = q.i0 + (lane & 3); i <= q.i1; i += 4) pixel(q, S, i, j);
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) S.add_xor(o);
+        if (t && (lane & 7) == 0) write(b - lane + from, S, q.mr);
+        for (int k = 0; k < 4; ++k) todo &= todo - 1;
+    }
+    for (todo = __ballot_sync(PSB_FULL, valid && npix > BEAM_GROUP); todo; todo &= todo - 1) {  // the whole warp
+        const int from = __ffs(todo) - 1;
+        const BeamPart<KC> q = fetch(from);
+        S.zero();
+        for (int j = q.j0 + (lane >> 3); j <= q.j1; j += 4) {
+            int a, z;
+            row(q, j, a, z);
+            for (int i = a + (lane & 7); i <= z; i += 8) pixel(q, S, i, j);
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) S.add_xor(o);
+        if (lane == 0) write(b - lane + from, S, q.mr);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) n_pairs += __shfl_xor_sync(PSB_FULL, n_pairs, o);
+    if (lane == 0 && A.stats && n_pairs) atomicAdd(&A.stats[0], (unsigned long long)n_pairs);
 }
 
 // sample coordinates of every sample of a source (grid, box) as arrays

@@ -58,3 +58,36 @@ def test_runs_match_one_lane_per_particle(cat, n, ns, strategy):
             assert np.abs(got[key] - ref[key]).max() <= 1e-10 * np.abs(ref[key]).max(), key
     for a, b in zip(got["cols"], one["cols"]):
         assert np.abs(a - b).max() <= 1e-12 * max(np.abs(b).max(), 1e-300)
+
+
+@pytest.mark.parametrize("strategy", [L.PSB_SCATTER, L.PSB_SYMMETRIC])
+@pytest.mark.parametrize("nx,ny", [(2, 2), (64, 40), (33, 130)])
+def test_beam_supports_of_every_size(nx, ny, strategy):
+    """Supports from a tenth of a pixel to most of the image, inside, across its
+    edges and outside: a lane's, eight lanes' and a warp's particles."""
+    rng = np.random.default_rng(nx)
+    n = 400
+    x, y, z = rng.uniform(-0.7, 0.7, n), rng.uniform(-0.7, 0.7, n), rng.uniform(-1, 1, n)
+    m, rho = rng.uniform(0.5, 1.5, n) / n, rng.uniform(0.5, 2.0, n)
+    h = np.exp(rng.uniform(np.log(0.001), np.log(0.3), n))
+    cols = [rng.standard_normal(n) for _ in range(3)]
+    c, s = np.cos(0.4), np.sin(0.4)
+    frame = np.array([0.05, -0.02, 0.1, c, s, 0, -s, c, 0, 0, 0, 1.0])
+    prm = np.array([-0.5, 0.5, -0.4, 0.45])
+    scal, shep = [0, 2], [0, 1]
+    gout = [rng.standard_normal(nx * ny) for _ in scal]
+    hs = np.array([0.02])
+    ctx = Context(0)
+    ctx.set_particles(x, y, z, m, h, rho, cols)
+    ctx.build(want_perm=False)
+    got = ctx.adjoint_beam(frame, prm, nx, ny, CatalogC(scalars=scal, shepard=shep), gout, strategy=strategy,
+                           hmode=L.PSB_H_CONSTANT, hs=hs)
+    from partia_b200 import workloads as W
+    o = W.plane_coordinates(frame, (prm[0], prm[1], nx), (prm[2], prm[3], ny))
+    d = tuple(np.full(nx * ny, frame[9 + k]) for k in range(3))
+    ref = O.Oracle(x, y, z, m, h, rho, cols=cols).adjoint_lines(o, d, scal, gout, shepard=shep, strategy=strategy,
+                                                               hmode=O.H_CONSTANT, hs=hs)
+    for key in ("m", "x", "y", "z"):
+        assert np.abs(got[key] - ref[key]).max() <= 1e-10 * np.abs(ref[key]).max(), key
+    for k in scal:
+        assert np.abs(got["cols"][k] - ref["cols"][k]).max() <= 1e-10 * np.abs(ref["cols"][k]).max(), k
