@@ -155,7 +155,7 @@ static int run_split(psb_ctx* c, Args<T>& A, int prec, int st, int* launches, in
     // other than M4 (span_shift; slots 80-86)
     const int kc = A.rec.kc;
     const bool shifts = sizeof(T) == 8 && prec == PREC_FP32C && kc > 0 && c->kern != PSB_KERNEL_M4;
-    const int kcl = kc <= 1 ? 1 : (kc <= 2 ? 2 : (kc <= 4 ? 4 : 8));
+    const int kcl = kc <= 1 ? 1 : (kc <= 2 ? 2 : (kc <= 4 ? 4 : (kc <= 6 ? kc : 8)));
     const int nf = what == WHAT_DENSITY ? 1 : 8 + 4 * kcl;
     const bool seq = sizeof(T) == 8 && prec == PREC_FP32C;  // samples of several parts go to k_seq
     // The chunk pool: a quarter of a chunk per sample for the kernels of support 2 h

@@ -16,6 +16,8 @@
 
 namespace psb {
 
+constexpr int BODY_THREADS = 128, WALK_THREADS = 128;  // threads of a block of the pair sums and of the walk
+
 // Per-warp shared memory of the walk.
 constexpr int WQ = 192;  // stack of the walk
 template <class T> struct CStage {
@@ -152,9 +154,9 @@ __device__ __forceinline__ bool window_walk(const TreeView<T>& tv, int32_t* q, N
 // step: 5.45 and 2.97 ms; FP64 on 500k particles and a 101 x 67 x 53 grid,
 // which walked in double, 4.05 -> 1.66 ms; 37 points 4.7 -> 0.37 ms.
 template <class T, int ST>
-__global__ void __launch_bounds__(128, 10) k_collect(const __grid_constant__ Args<T> A) {
+__global__ void __launch_bounds__(WALK_THREADS, 1280 / WALK_THREADS) k_collect(const __grid_constant__ Args<T> A) {
     constexpr bool BAND = sizeof(T) == 8;
-    __shared__ CStage<T> stage_all[4];
+    __shared__ CStage<T> stage_all[WALK_THREADS / 32];
     const TreeView<T>& tv = A.tv;
     const int lane = threadIdx.x & 31;
     const int wib = threadIdx.x >> 5;
@@ -825,8 +827,8 @@ template <int KC> struct PairData<double, PREC_FP32C, KC> {
 };
 
 // The list part of a thread of the pair-sum kernels.  Blocks below `nlist` take
-// four tiles' lists (one lane per sample), the blocks after them 128 chunks of
-// the pool each.
+// some tiles' lists (a warp per tile, one lane per sample), the blocks after
+// them a chunk of the pool per thread.
 struct ListPart {
     int64_t bt;      // the sample's tile in the batch
     int lane;        // and its lane there
@@ -880,7 +882,8 @@ __device__ __forceinline__ ListPart list_part(const SplitBufs& sp, unsigned nlis
 }
 
 template <class T, int PREC, int ST, int KC, int KF, bool DG>
-__global__ void __launch_bounds__(128, (KC <= 4) ? 4 : 2) k_bodies(const Args<T> A, unsigned nlist) {
+__global__ void __launch_bounds__(BODY_THREADS, 128 / BODY_THREADS * ((KC <= 4 || (KC == 5 && sizeof(T) == 4)) ? 4 : (KC <= 6 ? 3 : 2)))
+    k_bodies(const Args<T> A, unsigned nlist) {
     using CT = typename std::conditional<PREC == PREC_FP64, double, float>::type;
     using Acc = typename std::conditional<PREC == PREC_FP64, PlainD, KahanF>::type;
     constexpr bool BAND = (PREC == PREC_FP32C) && (sizeof(T) == 8);
@@ -1076,7 +1079,7 @@ __global__ void __launch_bounds__(128, (KC <= 4) ? 4 : 2) k_bodies(const Args<T>
 // (1M clump particles, gather at the particles: 10.4 ms in k_points; now the
 // walk, k_heavy and this kernel take 3.5 ms).
 template <class T, int PREC, int ST, int KF>
-__global__ void __launch_bounds__(128, 8) k_density(const Args<T> A, unsigned nlist) {
+__global__ void __launch_bounds__(BODY_THREADS, 1024 / BODY_THREADS) k_density(const Args<T> A, unsigned nlist) {
     using CT = typename std::conditional<PREC == PREC_FP64, double, float>::type;
     using Acc = typename std::conditional<PREC == PREC_FP64, PlainD, KahanF>::type;
     constexpr bool BAND = (PREC == PREC_FP32C) && (sizeof(T) == 8);

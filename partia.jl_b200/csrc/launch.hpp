@@ -112,10 +112,12 @@ static cudaError_t dispatch_line_warp(const Args<double>& a, int st, cudaStream_
 enum { SPLIT_WALK = 0, SPLIT_FIELDS = 1, SPLIT_DENSITY = 2, SPLIT_FOLD = 3, SPLIT_FOLD_DENSITY = 4, SPLIT_HEAVY = 5 };
 template <class T, int P, int S, int KF, bool DG>
 static void dispatch_bodies_kfd(const Args<T>& a, int kc, unsigned g, unsigned gc, cudaStream_t s) {
-    if (kc <= 1) k_bodies<T, P, S, 1, KF, DG><<<g + gc, 128, 0, s>>>(a, g);
-    else if (kc <= 2) k_bodies<T, P, S, 2, KF, DG><<<g + gc, 128, 0, s>>>(a, g);
-    else if (kc <= 4) k_bodies<T, P, S, 4, KF, DG><<<g + gc, 128, 0, s>>>(a, g);
-    else k_bodies<T, P, S, 8, KF, DG><<<g + gc, 128, 0, s>>>(a, g);
+    if (kc <= 1) k_bodies<T, P, S, 1, KF, DG><<<g + gc, BODY_THREADS, 0, s>>>(a, g);
+    else if (kc <= 2) k_bodies<T, P, S, 2, KF, DG><<<g + gc, BODY_THREADS, 0, s>>>(a, g);
+    else if (kc <= 4) k_bodies<T, P, S, 4, KF, DG><<<g + gc, BODY_THREADS, 0, s>>>(a, g);
+    else if (kc == 5) k_bodies<T, P, S, 5, KF, DG><<<g + gc, BODY_THREADS, 0, s>>>(a, g);
+    else if (kc <= 6) k_bodies<T, P, S, 6, KF, DG><<<g + gc, BODY_THREADS, 0, s>>>(a, g);
+    else k_bodies<T, P, S, 8, KF, DG><<<g + gc, BODY_THREADS, 0, s>>>(a, g);
 }
 // DG: the catalog has a density gradient (its sums and the masses in
 // registers only where they are used)
@@ -132,8 +134,8 @@ static void dispatch_bodies_k(const Args<T>& a, int kc, unsigned g, unsigned gc,
 
 template <class T, int P, int S>
 static void dispatch_density_k(const Args<T>& a, unsigned g, unsigned gc, cudaStream_t s) {
-    if (a.tv.kern == KERN_M4) k_density<T, P, S, 0><<<g + gc, 128, 0, s>>>(a, g);
-    else k_density<T, P, S, 1><<<g + gc, 128, 0, s>>>(a, g);
+    if (a.tv.kern == KERN_M4) k_density<T, P, S, 0><<<g + gc, BODY_THREADS, 0, s>>>(a, g);
+    else k_density<T, P, S, 1><<<g + gc, BODY_THREADS, 0, s>>>(a, g);
 }
 
 // k_seq: enough warps to fill the GPU, each takes samples until none is left
@@ -159,17 +161,21 @@ template <class T, int P>
 static cudaError_t dispatch_split_p(const Args<T>& a, int st, int kc, int pass, cudaStream_t s) {
     // blocks of the tiles' lists and of the chunk pool
     constexpr bool SEQ = sizeof(T) == 8 && P == PREC_FP32C;
-    const unsigned g = (unsigned)((a.sp.ntiles + 3) / 4), gc = SEQ ? 0 : (a.sp.ncap + 127) / 128;
+    constexpr int BW = BODY_THREADS / 32, WW = WALK_THREADS / 32;
+    const unsigned g = (unsigned)((a.sp.ntiles + BW - 1) / BW), gc = SEQ ? 0 : (a.sp.ncap + BODY_THREADS - 1) / BODY_THREADS;
+    const unsigned gf = (a.sp.ncap + 127) / 128;
     if (g == 0) return cudaSuccess;
     if (pass == SPLIT_FOLD || pass == SPLIT_FOLD_DENSITY) {
         if constexpr (SEQ) {
             dispatch_seq(a, st, pass == SPLIT_FOLD_DENSITY, s);
         } else {
-            if (pass == SPLIT_FOLD_DENSITY) k_fold<T, P, 1, WHAT_DENSITY><<<gc, 128, 0, s>>>(a);
-            else if (kc <= 1) k_fold<T, P, 1, WHAT_INTERP><<<gc, 128, 0, s>>>(a);
-            else if (kc <= 2) k_fold<T, P, 2, WHAT_INTERP><<<gc, 128, 0, s>>>(a);
-            else if (kc <= 4) k_fold<T, P, 4, WHAT_INTERP><<<gc, 128, 0, s>>>(a);
-            else k_fold<T, P, 8, WHAT_INTERP><<<gc, 128, 0, s>>>(a);
+            if (pass == SPLIT_FOLD_DENSITY) k_fold<T, P, 1, WHAT_DENSITY><<<gf, 128, 0, s>>>(a);
+            else if (kc <= 1) k_fold<T, P, 1, WHAT_INTERP><<<gf, 128, 0, s>>>(a);
+            else if (kc <= 2) k_fold<T, P, 2, WHAT_INTERP><<<gf, 128, 0, s>>>(a);
+            else if (kc <= 4) k_fold<T, P, 4, WHAT_INTERP><<<gf, 128, 0, s>>>(a);
+            else if (kc == 5) k_fold<T, P, 5, WHAT_INTERP><<<gf, 128, 0, s>>>(a);
+            else if (kc <= 6) k_fold<T, P, 6, WHAT_INTERP><<<gf, 128, 0, s>>>(a);
+            else k_fold<T, P, 8, WHAT_INTERP><<<gf, 128, 0, s>>>(a);
         }
     } else if (pass == SPLIT_HEAVY) {
         auto kern = st == ST_GATHER ? k_heavy<T, ST_GATHER> : (st == ST_SCATTER ? k_heavy<T, ST_SCATTER> : k_heavy<T, ST_SYMMETRIC>);
@@ -177,10 +183,10 @@ static cudaError_t dispatch_split_p(const Args<T>& a, int st, int kc, int pass, 
         if (e != cudaSuccess) return e;
         kern<<<std::min(2 * 148u, a.sp.hcap), HEAVY_THREADS, HEAVY_SMEM, s>>>(a);
     } else if (pass == SPLIT_WALK) {
-        const unsigned gw = (unsigned)(((a.sp.ntiles << (5 - a.sp.lspt)) + 3) / 4);
-        if (st == ST_GATHER) k_collect<T, ST_GATHER><<<gw, 128, 0, s>>>(a);
-        else if (st == ST_SCATTER) k_collect<T, ST_SCATTER><<<gw, 128, 0, s>>>(a);
-        else k_collect<T, ST_SYMMETRIC><<<gw, 128, 0, s>>>(a);
+        const unsigned gw = (unsigned)(((a.sp.ntiles << (5 - a.sp.lspt)) + WW - 1) / WW);
+        if (st == ST_GATHER) k_collect<T, ST_GATHER><<<gw, WALK_THREADS, 0, s>>>(a);
+        else if (st == ST_SCATTER) k_collect<T, ST_SCATTER><<<gw, WALK_THREADS, 0, s>>>(a);
+        else k_collect<T, ST_SYMMETRIC><<<gw, WALK_THREADS, 0, s>>>(a);
     } else if (pass == SPLIT_DENSITY) {
         if (st == ST_GATHER) dispatch_density_k<T, P, ST_GATHER>(a, g, gc, s);
         else if (st == ST_SCATTER) dispatch_density_k<T, P, ST_SCATTER>(a, g, gc, s);

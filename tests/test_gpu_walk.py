@@ -216,3 +216,25 @@ def test_lines_that_are_not_unit_vectors():
     assert ctx.last_stats.pairs == int(count.sum())
     for k in range(2):
         assert rel_err(got[k], ref[k]) <= FP64_TOL, k
+
+
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("kc", [3, 5, 6, 7])
+def test_column_counts(kc, dtype):
+    """Every column count that has pair sums of its own: equal to the single kernel's."""
+    arrs, cols = particles(3000, 19, dtype)
+    rng = np.random.default_rng(20)
+    cols = [rng.standard_normal(3000).astype(dtype) for _ in range(kc)]
+    s = tuple(rng.random(500).astype(dtype) for _ in range(3))
+    ctx = context(arrs, cols)
+    cat = CatalogC(scalars=list(range(kc)), shepard=[k % 2 for k in range(kc)], grads=[-1, kc - 1])
+    for prec in (L.PSB_PREC_FP64, L.PSB_PREC_FP32C):
+        got = ctx.interp_points(*s, cat, strategy=L.PSB_SYMMETRIC, prec=prec)
+        ctx.extra_flags = L.PSB_FLAG_SINGLE_KERNEL
+        one = ctx.interp_points(*s, cat, strategy=L.PSB_SYMMETRIC, prec=prec)
+        ctx.extra_flags = 0
+        for k in range(cat.L):
+            if dtype == np.float64:
+                assert np.array_equal(got[k], one[k], equal_nan=True), (prec, k)
+            else:  # (the parity tests' bound between the two for float inputs)
+                assert rel_err(got[k], one[k]) <= 1e-6, (prec, k)
