@@ -20,15 +20,66 @@ constexpr int BODY_THREADS = 128, WALK_THREADS = 128;  // threads of a block of 
 
 // Per-warp shared memory of the walk.
 constexpr int WQ = 192;  // stack of the walk
-template <class T> struct CStage {
-    float4 Q[SPAN];   // leaves: position relative to the warp anchor and h (double inputs), or as they
-                      // are and the squared radius (float inputs)
-    float4 P[SPAN];   // samples: position relative to the warp anchor and its error bound, or as they are
-    float2 AB[SPAN];  // double inputs: per-span squared thresholds of each leaf
-    float2 SAB[SPAN]; // per-span squared thresholds of each sample; float inputs: (squared radius, -)
+// Two leaves' negated positions (relative to the warp anchor for double inputs,
+// as they are for float ones) and squared radii: one packed operation takes
+// both leaves.
+struct LeafPair {
+    float2 x, y, z, T;
+};
+struct CStage {
+    LeafPair L[SPAN / 2];
+    float4 P[SPAN];   // samples: position as the leaves', squared radius or nearest candidate bound
     float4 W[SPAN];   // samples: float position and squared radius bound, for node tests one by one
     int32_t q[WQ];
+    // leaf j of the span (all 32 lanes call; a last odd leaf is paired with one out of reach)
+    __device__ __forceinline__ void put(int j, int cnt, float x, float y, float z, float T) {
+        if (j < cnt || j == cnt) {
+            const bool pad = j == cnt;
+            if (pad && !(cnt & 1)) return;
+            float* o = (float*)&L[j >> 1] + (j & 1);
+            o[0] = pad ? 1e18f : -x;
+            o[2] = pad ? 1e18f : -y;
+            o[4] = pad ? 1e18f : -z;
+            o[6] = pad ? 0.f : T;
+        }
+    }
 };
+__device__ __forceinline__ uint64_t pk(float a, float b) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ float2 unpk(uint64_t v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+// Squared distances of a sample (x, y, z packed twice) from a pair of leaves:
+// fused for the float tests, in the reference's operation order (EXACT) for
+// float inputs.
+template <bool EXACT>
+__device__ __forceinline__ float2 pair_d2(uint64_t px, uint64_t py, uint64_t pz, const LeafPair& q) {
+    const uint64_t dx = add2(px, pk(q.x.x, q.x.y)), dy = add2(py, pk(q.y.x, q.y.y)), dz = add2(pz, pk(q.z.x, q.z.y));
+    if (EXACT) return unpk(add2(add2(mul2(dx, dx), mul2(dy, dy)), mul2(dz, dz)));
+    return unpk(fma2(dz, dz, fma2(dy, dy, mul2(dx, dx))));
+}
+// v's sign bit shifted into m from below
+__device__ __forceinline__ unsigned push_sign(unsigned m, float v) { return __funnelshift_l(__float_as_uint(v), m, 1); }
 // found spans that reached none of the warp's samples, after which its node
 // tests go sample by sample
 constexpr int WALK_MISSES = 12;
@@ -152,11 +203,14 @@ __device__ __forceinline__ bool window_walk(const TreeView<T>& tv, int32_t* q, N
 // take 4.75 / 4.68 / 4.78 ms on the 2M-particle 128^3 grid (FP32C, 8 fields)
 // and 2.79 / 2.72 / 2.82 ms on 700k unordered points.  Before, with one node a
 // step: 5.45 and 2.97 ms; FP64 on 500k particles and a 101 x 67 x 53 grid,
-// which walked in double, 4.05 -> 1.66 ms; 37 points 4.7 -> 0.37 ms.
+// which walked in double, 4.05 -> 1.66 ms; 37 points 4.7 -> 0.37 ms.  The leaf
+// tests then took two leaves an instruction, the sign of d^2 - r^2 as the
+// decision and one tolerance per span, in place of two thresholds compared per
+// leaf: 4.70 -> 4.49 ms (FP32C), 1.66 -> 1.40 ms (FP64).
 template <class T, int ST>
 __global__ void __launch_bounds__(WALK_THREADS, 1280 / WALK_THREADS) k_collect(const __grid_constant__ Args<T> A) {
     constexpr bool BAND = sizeof(T) == 8;
-    __shared__ CStage<T> stage_all[WALK_THREADS / 32];
+    __shared__ CStage stage_all[WALK_THREADS / 32];
     const TreeView<T>& tv = A.tv;
     const int lane = threadIdx.x & 31;
     const int wib = threadIdx.x >> 5;
@@ -294,7 +348,8 @@ __global__ void __launch_bounds__(WALK_THREADS, 1280 / WALK_THREADS) k_collect(c
                 span_of(id, lo, cnt);
                 // candidates: float d2 not above (sqrt(best) + error)^2, or exactly not above best
                 float thr;
-                __syncwarp();
+                float4 L = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (lane < cnt) L = __ldg(&tv.leaf4[lo + lane]);
                 if constexpr (BAND) {
                     float o[3];
                     const float eqm = anchor(lo, o, __ldg(&tv.spanb[lo]).x);
@@ -302,34 +357,38 @@ __global__ void __launch_bounds__(WALK_THREADS, 1280 / WALK_THREADS) k_collect(c
                     const float e = 1.7320508f * (esmax + eqm) + 4.f * U1 * bs + 1e-18f;
                     const float t = (bs + e) * (1.f + 4.f * U1);
                     thr = isinf(best) ? INFINITY : t * t;
-                    if (lane < cnt) {
-                        const float4 L = __ldg(&tv.leaf4[lo + lane]);
-                        st.Q[lane] = make_float4(L.x + o[0], L.y + o[1], L.z + o[2], L.w);
-                    }
+                    L.x += o[0]; L.y += o[1]; L.z += o[2];
                 } else {
                     thr = (float)best;  // a float distance: exact
-                    if (lane < cnt) st.Q[lane] = __ldg(&tv.leaf4[lo + lane]);
                 }
                 const bool by_sample = 3 * __popc(parts) >= 2 * cnt;
-                if (!by_sample) st.SAB[lane].x = thr;
-                __syncwarp();
-                auto d2_of = [&](const float4& P, const float4& Q) -> float {
-                    const float dx = P.x - Q.x, dy = P.y - Q.y, dz = P.z - Q.z;
-                    if constexpr (BAND) return dx * dx + dy * dy + dz * dz;
-                    return __fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz));
-                };
                 unsigned cand = 0;
+                __syncwarp();
                 if (by_sample) {  // each taking lane tests its sample against every leaf
+                    st.put(lane, cnt, L.x, L.y, L.z, 0.f);
+                    __syncwarp();
                     if (part) {
                         const float4 P = st.P[lane];
-#pragma unroll 4
-                        for (int j = 0; j < cnt; ++j) cand |= (unsigned)(d2_of(P, st.Q[j]) <= thr) << j;
+                        const uint64_t px = pk(P.x, P.x), py = pk(P.y, P.y), pz = pk(P.z, P.z);
+                        unsigned out = 0;
+#pragma unroll 2
+                        for (int j = (cnt - 1) >> 1; j >= 0; --j) {
+                            const float2 d2 = pair_d2<!BAND>(px, py, pz, st.L[j]);
+                            out = push_sign(push_sign(out, thr - d2.y), thr - d2.x);
+                        }
+                        cand = ~out & (0xffffffffu >> (32 - cnt));
                     }
                 } else {  // lane j tests leaf j against each taking sample
-                    const float4 Q = st.Q[lane < cnt ? lane : 0];
+                    st.P[lane].w = thr;
+                    __syncwarp();
                     for (unsigned pp = parts; pp; pp &= pp - 1) {
                         const int s = __ffs(pp) - 1;
-                        const unsigned b = __ballot_sync(PSB_FULL, lane < cnt && d2_of(st.P[s], Q) <= st.SAB[s].x);
+                        const float4 P = st.P[s];
+                        const float dx = P.x - L.x, dy = P.y - L.y, dz = P.z - L.z;
+                        float d2;
+                        if constexpr (BAND) d2 = dx * dx + dy * dy + dz * dz;
+                        else d2 = __fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz));
+                        const unsigned b = __ballot_sync(PSB_FULL, lane < cnt && d2 <= P.w);
                         if (lane == s) cand = b;
                     }
                 }
@@ -350,9 +409,8 @@ __global__ void __launch_bounds__(WALK_THREADS, 1280 / WALK_THREADS) k_collect(c
     const T Kt = (T)tv.Kd;
     const T ra = X<T>::mul(Kt, ha);
     const T ra2 = X<T>::mul(ra, ra);
-    float ra2_hi = 0.f, ralo = 0.f, rahi = 0.f;
+    float ra2_hi = 0.f, rahi = 0.f;
     if (ST != ST_SCATTER) {
-        ralo = __double2float_rd(fabs((double)ra)) * (1.f - 2.f * U1);
         rahi = __double2float_ru(fabs((double)ra)) * (1.f + 2.f * U1);
         ra2_hi = valid ? __double2float_ru((double)ra2) * (1.f + RELM) + 1e-36f : 0.f;
     }
@@ -429,8 +487,10 @@ __global__ void __launch_bounds__(WALK_THREADS, 1280 / WALK_THREADS) k_collect(c
         // few samples take part: lane j tests leaf j against each of them;
         // otherwise each taking lane tests its sample against every leaf
         const bool by_sample = 3 * __popc(parts) >= 2 * cnt;  // warp-uniform
-        unsigned myacc = 0;
-        __syncwarp();
+        // the leaf of this lane with its squared radius (K hb)^2
+        float4 L = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (lane < cnt) L = __ldg(&tv.leaf4[lo + lane]);
+        float tol = -1.f;  // a pair within it of its squared radius is undecided (double inputs)
         if constexpr (BAND) {
             // one error bound E for every float distance of the span
             float o[3];
@@ -440,95 +500,73 @@ __global__ void __launch_bounds__(WALK_THREADS, 1280 / WALK_THREADS) k_collect(c
             float rmax = rahimax;
             if (ST != ST_GATHER) rmax = fmaxf(rmax, tv.Kf * sb.y * (1.f + 3.f * U1));
             const float E = 1.7320508f * (esmax + eqm) + 4.f * U1 * rmax + 1e-18f;
-            // this lane's sample thresholds
-            float As = 0.f, Bs = 0.f;
-            if (ST != ST_SCATTER) {
-                const float il = fmaxf((ralo - E) * (1.f - 4.f * U1), 0.f), ih2 = (rahi + E) * (1.f + 4.f * U1);
-                As = il * il;
-                Bs = ih2 * ih2;
-            }
-            // the span's leaves (and their radius thresholds) in shared memory
-            float4 Qme = make_float4(0.f, 0.f, 0.f, 0.f);
-            float Aj = 0.f, Bj = 0.f;
-            if (lane < cnt) {
-                const float4 L = __ldg(&tv.leaf4[lo + lane]);
-                Qme = make_float4(L.x + o[0], L.y + o[1], L.z + o[2], L.w);
-                st.Q[lane] = Qme;
-                if (ST != ST_GATHER) {
-                    const float rbhi = tv.Kf * L.w * (1.f + 3.f * U1), rblo = tv.Kf * L.w * (1.f - 3.f * U1);
-                    const float il = fmaxf((rblo - E) * (1.f - 4.f * U1), 0.f), ih2 = (rbhi + E) * (1.f + 4.f * U1);
-                    Aj = il * il;
-                    Bj = ih2 * ih2;
-                    st.AB[lane] = make_float2(Aj, Bj);
-                }
-            }
-            if (!by_sample) st.SAB[lane] = make_float2(As, Bs);
+            // |d - d_exact| <= E, so d^2 and the exact distance lie on the same side of r^2 unless
+            // |d^2 - r^2| <= 2 r E + E^2 (and the roundings of r^2 and of the difference)
+            tol = ((2.f * rmax + E) * E + 8.f * U1 * rmax * rmax) * (1.f + 1e-3f);
+            L.x += o[0]; L.y += o[1]; L.z += o[2];
+            const float kb = tv.Kf * L.w;
+            L.w = kb * kb;
+        } else if (ST != ST_GATHER) {
+            L.w = ex_r2<ST_SCATTER, float>(0.f, L.w, (float)Kt);
+        }
+        const float Ts = (float)ra2;  // the sample's squared radius
+        unsigned myacc = 0;
+        float near = INFINITY;  // smallest |d^2 - r^2| of this lane's tests
+        __syncwarp();
+        if (by_sample) {
+            st.put(lane, cnt, L.x, L.y, L.z, L.w);
             __syncwarp();
-            // surely in: d2 < A; maybe in: d2 <= B (undecided = maybe and not surely)
-            unsigned mymaybe = 0;
-            if (!by_sample) {
-                for (unsigned pp = parts; pp; pp &= pp - 1) {
-                    const int s = __ffs(pp) - 1;
-                    const float4 Ps = st.P[s];
-                    const float2 sab = st.SAB[s];
-                    const float dx = Ps.x - Qme.x, dy = Ps.y - Qme.y, dz = Ps.z - Qme.z;
-                    const float d2 = dx * dx + dy * dy + dz * dz;
-                    const float At = (ST == ST_GATHER) ? sab.x : ((ST == ST_SCATTER) ? Aj : fmaxf(sab.x, Aj));
-                    const float Bt = (ST == ST_GATHER) ? sab.y : ((ST == ST_SCATTER) ? Bj : fmaxf(sab.y, Bj));
-                    const unsigned bi = __ballot_sync(PSB_FULL, lane < cnt && d2 < At);
-                    const unsigned bm = __ballot_sync(PSB_FULL, lane < cnt && d2 <= Bt);
-                    if (lane == s) { myacc = bi; mymaybe = bm; }
-                }
-            } else if (part) {
-                const float4 Pme = st.P[lane];
-#pragma unroll 4
-                for (int j = 0; j < cnt; ++j) {
-                    const float4 Q = st.Q[j];
-                    const float dx = Pme.x - Q.x, dy = Pme.y - Q.y, dz = Pme.z - Q.z;
-                    const float d2 = dx * dx + dy * dy + dz * dz;
-                    float At = As, Bt = Bs;
-                    if (ST != ST_GATHER) {
-                        const float2 ab = st.AB[j];
-                        At = (ST == ST_SCATTER) ? ab.x : fmaxf(As, ab.x);
-                        Bt = (ST == ST_SCATTER) ? ab.y : fmaxf(Bs, ab.y);
+            if (part) {
+                const float4 P = st.P[lane];
+                const uint64_t px = pk(P.x, P.x), py = pk(P.y, P.y), pz = pk(P.z, P.z);
+                unsigned m = 0;
+#pragma unroll 2
+                for (int j = (cnt - 1) >> 1; j >= 0; --j) {
+                    const LeafPair q = st.L[j];
+                    const float2 d2 = pair_d2<!BAND>(px, py, pz, q);
+                    float T0 = Ts, T1 = Ts;
+                    if (ST == ST_SCATTER) { T0 = q.T.x; T1 = q.T.y; }
+                    if (ST == ST_SYMMETRIC) { T0 = fmaxf(Ts, q.T.x); T1 = fmaxf(Ts, q.T.y); }
+                    if constexpr (BAND) {  // inside: d^2 - r^2 < 0
+                        const float t0 = d2.x - T0, t1 = d2.y - T1;
+                        m = push_sign(push_sign(m, t1), t0);
+                        near = fminf(near, fminf(fabsf(t0), fabsf(t1)));
+                    } else {               // outside: r^2 - d^2 < 0
+                        m = push_sign(push_sign(m, T1 - d2.y), T0 - d2.x);
                     }
-                    myacc |= (unsigned)(d2 < At) << j;
-                    mymaybe |= (unsigned)(d2 <= Bt) << j;
                 }
-            }
-            // undecided pairs: the reference's double test
-            for (unsigned u = mymaybe & ~myacc; u; u &= u - 1) {
-                const int jj = __ffs(u) - 1;
-                const int64_t li = lo + jj;
-                ++n_retest;
-                T e2 = ex_d2_pp<T>(p, tv.x[li], tv.y[li], tv.z[li]);
-                if (e2 <= ex_r2<ST, T>(ra2, tv.h[li], Kt)) myacc |= 1u << jj;
+                myacc = (BAND ? m : ~m) & (0xffffffffu >> (32 - cnt));
             }
         } else {
-            // float inputs: the reference's float arithmetic on the leaf records
-            float4 Qme = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (lane < cnt) {
-                Qme = __ldg(&tv.leaf4[lo + lane]);
-                if (ST != ST_GATHER) Qme.w = ex_r2<ST_SCATTER, float>(0.f, Qme.w, (float)Kt);  // (K hb)^2
-                st.Q[lane] = Qme;
-            }
-            if (!by_sample) st.SAB[lane].x = (float)ra2;
+            st.P[lane].w = Ts;
             __syncwarp();
-            auto inside = [&](const float4& P, const float4& Q, float r2a) -> bool {
-                const float dx = __fsub_rn(P.x, Q.x), dy = __fsub_rn(P.y, Q.y), dz = __fsub_rn(P.z, Q.z);
-                const float e2 = __fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz));
-                return e2 <= ((ST == ST_GATHER) ? r2a : ((ST == ST_SCATTER) ? Q.w : jmax(r2a, Q.w)));
-            };
-            if (!by_sample) {
-                for (unsigned pp = parts; pp; pp &= pp - 1) {
-                    const int s = __ffs(pp) - 1;
-                    const unsigned b = __ballot_sync(PSB_FULL, lane < cnt && inside(st.P[s], Qme, st.SAB[s].x));
-                    if (lane == s) myacc = b;
+            for (unsigned pp = parts; pp; pp &= pp - 1) {
+                const int s = __ffs(pp) - 1;
+                const float4 P = st.P[s];
+                const float dx = P.x - L.x, dy = P.y - L.y, dz = P.z - L.z;
+                const float Tp = (ST == ST_GATHER) ? P.w : ((ST == ST_SCATTER) ? L.w : fmaxf(P.w, L.w));
+                bool in;
+                if constexpr (BAND) {
+                    const float t = dx * dx + dy * dy + dz * dz - Tp;
+                    in = t < 0.f;
+                    if (lane < cnt) near = fminf(near, fabsf(t));
+                } else {
+                    in = __fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz)) <= Tp;
                 }
-            } else if (part) {
-                const float4 Pme = st.P[lane];
-#pragma unroll 4
-                for (int j = 0; j < cnt; ++j) myacc |= (unsigned)inside(Pme, st.Q[j], (float)ra2) << j;
+                const unsigned b = __ballot_sync(PSB_FULL, lane < cnt && in);
+                if (lane == s) myacc = b;
+            }
+        }
+        if (BAND && __any_sync(PSB_FULL, near <= tol)) {
+            // an undecided pair: the reference's double test for the span's (rare)
+            if (part) {
+                n_retest += cnt;
+                myacc = 0;
+                for (int j = 0; j < cnt; ++j) {
+                    const int64_t li = lo + j;
+                    const T e2 = ex_d2_pp<T>(p, __ldg(&tv.x[li]), __ldg(&tv.y[li]), __ldg(&tv.z[li]));
+                    myacc |= (unsigned)(e2 <= ex_r2<ST, T>(ra2, __ldg(&tv.h[li]), Kt)) << j;
+                }
             }
         }
         emit(lo, myacc);
