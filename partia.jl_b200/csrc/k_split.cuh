@@ -59,11 +59,6 @@ __device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
     asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
     return r;
 }
-__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
-    uint64_t r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
 __device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
     uint64_t r;
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
@@ -75,8 +70,14 @@ __device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
 template <bool EXACT>
 __device__ __forceinline__ float2 pair_d2(uint64_t px, uint64_t py, uint64_t pz, const LeafPair& q) {
     const uint64_t dx = add2(px, pk(q.x.x, q.x.y)), dy = add2(py, pk(q.y.x, q.y.y)), dz = add2(pz, pk(q.z.x, q.z.y));
-    if (EXACT) return unpk(add2(add2(mul2(dx, dx), mul2(dy, dy)), mul2(dz, dz)));
-    return unpk(fma2(dz, dz, fma2(dy, dy, mul2(dx, dx))));
+    if (EXACT) {
+        // the products one by one: a packed product may be merged into the packed sum behind it
+        const float2 x = unpk(dx), y = unpk(dy), z = unpk(dz);
+        const uint64_t xx = pk(__fmul_rn(x.x, x.x), __fmul_rn(x.y, x.y)), yy = pk(__fmul_rn(y.x, y.x), __fmul_rn(y.y, y.y)),
+                       zz = pk(__fmul_rn(z.x, z.x), __fmul_rn(z.y, z.y));
+        return unpk(add2(add2(xx, yy), zz));
+    }
+    return unpk(fma2(dz, dz, fma2(dy, dy, fma2(dx, dx, 0ull))));
 }
 // v's sign bit shifted into m from below
 __device__ __forceinline__ unsigned push_sign(unsigned m, float v) { return __funnelshift_l(__float_as_uint(v), m, 1); }

@@ -238,3 +238,23 @@ def test_column_counts(kc, dtype):
                 assert np.array_equal(got[k], one[k], equal_nan=True), (prec, k)
             else:  # (the parity tests' bound between the two for float inputs)
                 assert rel_err(got[k], one[k]) <= 1e-6, (prec, k)
+
+
+def test_float_decisions_on_the_support_edge():
+    """Float particles on a lattice with radii that are its distances: the sum
+    of squares rounds at every step, and a fused one decides otherwise."""
+    g = np.arange(12, dtype=np.float32) * np.float32(0.1)
+    x, y, z = (a.ravel().astype(np.float32) for a in np.meshgrid(g, g, g, indexing="ij"))
+    n = len(x)
+    one = np.ones(n, dtype=np.float32)
+    rng = np.random.default_rng(21)
+    h = (np.float32(0.05) * np.sqrt(rng.integers(1, 9, n))).astype(np.float32)
+    ctx = context([x, y, z, one / n, h, one], [one])
+    s = tuple(np.concatenate([a[::3], a[1::7]]) for a in (x, y, z))
+    orc = O.Oracle(x, y, z, one / n, h, one, cols=[one], dtype=np.float32)
+    for strategy in (L.PSB_GATHER, L.PSB_SCATTER, L.PSB_SYMMETRIC):
+        for hs in ([0.05], [0.0707106781], [0.1], [0.111803398]):
+            kw = dict(strategy=strategy, hmode=L.PSB_H_CONSTANT, hs=np.array(hs, dtype=np.float32))
+            ctx.interp_points(*s, CatalogC(scalars=[0], shepard=[0]), **kw)
+            count, _, _ = orc.digest(s, **kw)
+            assert ctx.last_stats.pairs == int(count.sum()), (strategy, hs)
