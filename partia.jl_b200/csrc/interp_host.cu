@@ -152,11 +152,13 @@ static int run_split(psb_ctx* c, Args<T>& A, int prec, int st, int* launches, in
         int32_t* ovf_tiles; uint32_t* own; int32_t* next; uint8_t* ccnt; double* part; uint32_t* hlist; uint32_t* mlist;
     };
     // FP32C sums of double inputs take per-entry column shifts for the kernels
-    // other than M4 (span_shift; slots 80-86)
+    // other than M4 (span_shift)
     const int kc = A.rec.kc;
     const bool shifts = sizeof(T) == 8 && prec == PREC_FP32C && kc > 0 && c->kern != PSB_KERNEL_M4;
     const int kcl = kc <= 1 ? 1 : (kc <= 2 ? 2 : (kc <= 4 ? 4 : (kc <= 6 ? kc : 8)));
     const int nf = what == WHAT_DENSITY ? 1 : 8 + 4 * kcl;
+    A.sp.seq_all = A.src.ns <= SEQ_ALL ? 1 : 0;
+    A.sp.kcl = kcl;
     const bool seq = sizeof(T) == 8 && prec == PREC_FP32C;  // samples of several parts go to k_seq
     // The chunk pool: a quarter of a chunk per sample for the kernels of support 2 h
     // (neighbourhoods of more than RCAP spans are rare there), one per
@@ -168,36 +170,41 @@ static int run_split(psb_ctx* c, Args<T>& A, int prec, int st, int* launches, in
     const unsigned ncap = (unsigned)std::min<int64_t>(std::max<int64_t>(65536, A.tv.Kd > 2.0 ? lanes : lanes / 4), most);
     constexpr unsigned HCAP = 4096;  // samples of a batch for k_heavy (the rest stay in their tiles' walks)
     Lists ls[SPLIT_STREAMS];
-    for (int k = 0; k < nsets; ++k) {
-        // scratch slots 16-20 (+ slot_off), 48-52, 37-41 and 42-46 (clear of the
-        // build, sort, sample-order and adjoint slots), and 80-86 and 96-102
-        static const int set_off[SPLIT_STREAMS] = {0, 32, 21, 26};
-        const int so = slot_off + set_off[k];
-        const int es_slot = slot_off == 0 ? k : (slot_off == 32 ? 4 : (slot_off == 14 ? 5 : 6));
+    {
+        // One block for all the streams' lists (slots 96-99): a context's first
+        // call pays for the number of allocations.
+        const int slot = 96 + (slot_off == 0 ? 0 : (slot_off == 32 ? 1 : (slot_off == 14 ? 2 : 3)));
         const size_t nent = (size_t)RCAP * 32 * B + (size_t)RCAP * ncap;
-        ls[k].ent4 = (float4*)scratch(c, 16 + so, sizeof(float4) * nent);
-        ls[k].emask = (uint32_t*)scratch(c, 20 + so, sizeof(uint32_t) * nent);
-        ls[k].eshift = nullptr;
-        if (shifts) {
-            ls[k].eshift = (float*)scratch(c, 80 + es_slot, sizeof(float) * nent * kc);
-            if (!ls[k].eshift) return fail(c, PSB_ENOMEM, "scratch allocation failed (pair-list shifts)");
+        size_t size = 0;
+        auto take = [&](size_t bytes) {
+            const size_t at = size;
+            size += (bytes + 255) & ~(size_t)255;
+            return at;
+        };
+        const size_t ent4 = take(sizeof(float4) * nent), emask = take(sizeof(uint32_t) * nent);
+        const size_t eshift = take(shifts ? sizeof(float) * nent * kc : 0);
+        const size_t hab = take(sizeof(double) * lanes), head = take(sizeof(int32_t) * lanes), cnt = take(lanes);
+        const size_t part = take((seq ? sizeof(uint32_t) : sizeof(double) * 2 * nf) * (size_t)ncap);
+        const size_t own = take(sizeof(uint32_t) * ncap), next = take(sizeof(int32_t) * ncap), ccnt = take(ncap);
+        const size_t hlist = take(sizeof(uint32_t) * HCAP), ovf = take(sizeof(int32_t) * (size_t)B), ctr = take(256);
+        char* base = (char*)scratch(c, slot, size * nsets);
+        if (!base) return fail(c, PSB_ENOMEM, "scratch allocation failed (pair lists)");
+        for (int k = 0; k < nsets; ++k, base += size) {
+            ls[k].ent4 = (float4*)(base + ent4);
+            ls[k].emask = (uint32_t*)(base + emask);
+            ls[k].eshift = shifts ? (float*)(base + eshift) : nullptr;
+            ls[k].hab = base + hab;
+            ls[k].head = (int32_t*)(base + head);
+            ls[k].cnt = (uint8_t*)(base + cnt);
+            ls[k].part = seq ? nullptr : (double*)(base + part);
+            ls[k].mlist = seq ? (uint32_t*)(base + part) : nullptr;
+            ls[k].own = (uint32_t*)(base + own);
+            ls[k].next = (int32_t*)(base + next);
+            ls[k].ccnt = (uint8_t*)(base + ccnt);
+            ls[k].hlist = (uint32_t*)(base + hlist);
+            ls[k].ovf_tiles = (int32_t*)(base + ovf);
+            ls[k].ctr = (unsigned*)(base + ctr);
         }
-        char* cnt = (char*)scratch(c, 17 + so, (size_t)(1 + sizeof(int32_t)) * lanes);
-        ls[k].hab = scratch(c, 18 + so, sizeof(double) * 32 * (size_t)B);
-        char* ovf = (char*)scratch(c, 19 + so, 256 + sizeof(int32_t) * ((size_t)B * 33 + HCAP));
-        char* pool = (char*)scratch(c, 96 + es_slot, (size_t)ncap * ((seq ? sizeof(uint32_t) : sizeof(double) * 2 * nf) + 2 * sizeof(int32_t) + 1));
-        if (!ls[k].ent4 || !ls[k].emask || !cnt || !ls[k].hab || !ovf || !pool)
-            return fail(c, PSB_ENOMEM, "scratch allocation failed (pair lists)");
-        ls[k].head = (int32_t*)cnt;
-        ls[k].cnt = (uint8_t*)(cnt + sizeof(int32_t) * lanes);
-        ls[k].ctr = (unsigned*)ovf;
-        ls[k].hlist = (uint32_t*)(ovf + 256);
-        ls[k].ovf_tiles = (int32_t*)(ls[k].hlist + HCAP);
-        ls[k].part = seq ? nullptr : (double*)pool;
-        ls[k].mlist = seq ? (uint32_t*)pool : nullptr;
-        ls[k].own = (uint32_t*)(pool + (seq ? sizeof(uint32_t) : sizeof(double) * 2 * nf) * (size_t)ncap);
-        ls[k].next = (int32_t*)(ls[k].own + ncap);
-        ls[k].ccnt = (uint8_t*)(ls[k].next + ncap);
     }
     A.sp.ncap = ncap;
     A.sp.ebase = (uint32_t)((int64_t)RCAP * 32 * B);
@@ -223,14 +230,15 @@ static int run_split(psb_ctx* c, Args<T>& A, int prec, int st, int* launches, in
         const bool dens = what == WHAT_DENSITY;
         PSB_CUDA_TRY(c, launch_split(A, prec, st, kc, SPLIT_WALK, sk), "pair-list kernel launch");
         PSB_CUDA_TRY(c, launch_split(A, prec, st, kc, SPLIT_HEAVY, sk), "heavy-sample kernel launch");
-        PSB_CUDA_TRY(c, launch_split(A, prec, st, kc, dens ? SPLIT_DENSITY : SPLIT_FIELDS, sk), "pair-sum kernel launch");
+        if (!(seq && A.sp.seq_all))
+            PSB_CUDA_TRY(c, launch_split(A, prec, st, kc, dens ? SPLIT_DENSITY : SPLIT_FIELDS, sk), "pair-sum kernel launch");
         PSB_CUDA_TRY(c, launch_split(A, prec, st, kc, dens ? SPLIT_FOLD_DENSITY : SPLIT_FOLD, sk), "fold kernel launch");
         Args<T> F = A;
         F.tile_list = ls[k].ovf_tiles;
         F.tile_count = ls[k].ctr;
         F.src.ntiles = nb;  // grid of the list pass: at most nb tiles
         PSB_CUDA_TRY(c, launch_points<T>(F, prec, st, A.rec.kc, what, sk), "overflow pass launch");
-        *launches += 5;
+        *launches += seq && A.sp.seq_all ? 4 : 5;
     }
     for (int k = 1; k < nsets; ++k) {  // the call's later work on s follows every stream
         PSB_CUDA_TRY(c, cudaEventRecord(c->sev[k], ss[k]), "event");

@@ -70,9 +70,11 @@ struct SplitBufs {
     unsigned* hcount;
     uint32_t* hlist;     // tile in the batch * 32 + lane
     unsigned hcap;
-    // FP32C of double particles: the samples of several parts, for k_seq (null otherwise)
+    // the samples of several parts for k_seq (FP32C of double particles; null otherwise)
     unsigned* mcount;
     uint32_t* mlist;     // first chunk of each
+    int seq_all;         // k_seq takes every sample (a small call)
+    int kcl;             // columns of the partial sums' layout (the KC of k_fold)
 };
 constexpr uint8_t CNT_DEAD = 0xFF;   // the tile is the single-kernel pass's
 constexpr uint8_t CNT_HEAVY = 0xFE;  // the sample's entries are k_heavy's

@@ -1251,20 +1251,34 @@ __global__ void __launch_bounds__(128) k_fold(const Args<T> A) {
     write_interp_outputs<T, PlainD, CT, KC>(A, k, S1, G, Sw, Sg, Dm, Dg, a0);
 }
 
-// The FP32C sums of double particles' samples of several list parts: one warp
-// per sample, the parts in order.  Lane j of an entry evaluates the weights of
-// the entry's leaf j, with k_bodies' arithmetic; then each compensated sum runs
-// through the entry's pairs in leaf order in a lane of its own (4 + 4 kc sums,
-// 4 more with a density gradient, two to a lane past 32).  The sums have the
-// bits of one lane adding pair after pair, without its other 31 lanes idle.
-constexpr int SEQ_COMP = 8;              // weights of a pair: w, w d (3); with a density gradient m W, m W' d (3)
-constexpr int SEQ_ROWS = SEQ_COMP + MAX_KC;
-template <int ST, int KF, int WHAT>
-__global__ void __launch_bounds__(128) k_seq(const __grid_constant__ Args<double> A) {
-    constexpr bool EXS = KF == 1;
-    __shared__ float rows_all[4][SEQ_ROWS][33];  // [component or column][leaf]
+// One warp per sample: in FP32C of double particles for the samples of several
+// list parts, whose sums run on through the parts, and in small calls for every
+// sample (seq_all; parts of FP64 and float particles' samples are summed apart,
+// as in k_bodies).  Lane j of an entry evaluates the weights of the entry's
+// leaf j, with k_bodies' arithmetic; then each sum runs through the entry's
+// pairs in leaf order in a lane of its own (4 + 4 kc sums, 4 more with a
+// density gradient, two to a lane past 32).  The sums have the bits of one lane
+// adding pair after pair.
+//
+// A small call is as long as its longest lane: 37 points waited 230 us for
+// k_bodies.  With this, 1M uniform particles, scatter, 12 FP64 outputs: 32
+// points take 132 us a call (k_bodies 162), 1024 212 (241), 4096 293 (316),
+// 8192 416 (400), 65,536 1000 (571); the density alone 129 (150), 204 (231),
+// 241 (298), 341 (381), 622 (521).  FP32C and float particles cross between
+// 4096 and 8192 points as well.
+constexpr int SEQ_COMP = 8;  // weights of a pair: w, w d (3); with a density gradient W, d (3); then the columns, m, m W'
+constexpr int SEQ_ROWS = SEQ_COMP + MAX_KC + 2;
+constexpr int64_t SEQ_ALL = 4096;  // samples of a call up to which k_seq takes all
+template <class T, int PREC, int ST, int KF, int WHAT>
+__global__ void __launch_bounds__(128) k_seq(const __grid_constant__ Args<T> A) {
+    using CT = typename std::conditional<PREC == PREC_FP64, double, float>::type;
+    using Acc = typename std::conditional<PREC == PREC_FP64, PlainD, KahanF>::type;
+    constexpr bool BAND = PREC == PREC_FP32C && sizeof(T) == 8;
+    constexpr bool SHIFT = PREC == PREC_FP32C, EXS = BAND && KF == 1;
+    constexpr bool FOLD = !BAND;  // the parts are summed apart and added up by k_fold
+    __shared__ CT rows_all[4][SEQ_ROWS][33];  // [component or column][leaf]
     __shared__ double sums_all[4][8 + 4 * MAX_KC];
-    const TreeView<double>& tv = A.tv;
+    const TreeView<T>& tv = A.tv;
     const SplitBufs& sp = A.sp;
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     auto& rows = rows_all[wib];
@@ -1284,43 +1298,53 @@ __global__ void __launch_bounds__(128) k_seq(const __grid_constant__ Args<double
         else if (q < 4 + 4 * kc) {
             const int c = (q - 4) >> 2, d = (q - 4) & 3;
             ra[u] = d; rb[u] = SEQ_COMP + c;
-            fo[u] = d == 0 ? 8 + c : 8 + MAX_KC + 3 * c + d - 1;
-        } else { ra[u] = 4 + (q - 4 - 4 * kc); fo[u] = 4 + (q - 4 - 4 * kc); }
+            fo[u] = d == 0 ? 8 + c : 8 + sp.kcl + 3 * c + d - 1;
+        } else {  // m W, then (m W') d
+            const int d = q - 4 - 4 * kc;
+            ra[u] = 4 + d; rb[u] = SEQ_COMP + MAX_KC + (d ? 1 : 0);
+            fo[u] = 4 + d;
+        }
+        if (WHAT == WHAT_DENSITY) rb[u] = 1;
     }
     const bool two = nsum > 32;
-    const unsigned nm = min(*sp.mcount, sp.ncap);
+    // the tiles' lists (seq_all), then the chunks, or (FP32C of double particles) the samples of several parts
+    const unsigned n1 = sp.seq_all ? (unsigned)sp.ntiles * 32u : 0u;
+    const unsigned nm = min(FOLD ? *sp.top : *sp.mcount, sp.ncap);
     const unsigned nw = gridDim.x * (blockDim.x >> 5);
-    for (unsigned i = blockIdx.x * (blockDim.x >> 5) + wib; i < nm; i += nw) {
-        const uint32_t c0 = sp.mlist[i];
-        const uint32_t w0 = sp.own[c0], own = w0 & OWN_IDX;
+    for (unsigned i = blockIdx.x * (blockDim.x >> 5) + wib; i < n1 + nm; i += nw) {
+        const int32_t c0 = i < n1 ? -1 : (FOLD ? (int32_t)(i - n1) : (int32_t)sp.mlist[i - n1]);
+        const uint32_t w0 = i < n1 ? i : sp.own[c0], own = w0 & OWN_IDX;
+        if (FOLD && w0 == OWN_NONE) continue;
         const int cn = sp.cnt[own];
-        const bool heavy = (w0 & OWN_HEAVY) != 0;
+        const bool heavy = i >= n1 && (w0 & OWN_HEAVY) != 0;
         if (cn == CNT_DEAD || (cn == CNT_HEAVY) != heavy) continue;  // warp-uniform
+        const int32_t more = i < n1 && cn == RCAP ? sp.head[own] : -1;  // a list of several parts
+        if (!FOLD && more >= 0) continue;
         const int64_t k = sample_of(A.src, sp.tile0 + (own >> 5), own & 31);
         if (k < 0) continue;
-        double p[3], dd[3];
+        T p[3], dd[3];
         sample_coords(A.src, k, p, dd);
-        const double ha = ((const double*)sp.ha)[own];
-        const float sig = (KF == 0) ? inv_pi<float>() : (float)tv.sig;
-        float ia = 0.f, sa3 = 0.f, sa4 = 0.f;
+        const T ha = ((const T*)sp.ha)[own];
+        const CT sig = (KF == 0) ? inv_pi<CT>() : (CT)tv.sig;
+        CT ia = CT(0), sa3 = CT(0), sa4 = CT(0);
         if (ST != ST_SCATTER) {
-            ia = 1.f / (float)ha;
+            ia = CT(1) / (CT)ha;
             sa3 = sig * ia * ia * ia;
             sa4 = sa3 * ia;
         }
-        const double kha = tv.Kd * ha;
+        const double kha = tv.Kd * (double)ha;
         const double fa2 = kha * kha;
-        const double ika = (KF == 1 && ST != ST_SCATTER) ? 0.5 / ha : 0.0;
+        const double ika = (KF == 1 && ST != ST_SCATTER) ? 0.5 / (double)ha : 0.0;
         const float qe = (KF == 0) ? 1.f : tv.qedge;
         const size_t q0 = (size_t)(own >> 5) * RCAP * 32 + (own & 31);
-        const int64_t first = (int64_t)__float_as_int(sp.ent4[q0].w) + __ffs(sp.emask[q0]) - 1;
-        KahanF S[2];
+        const int64_t first = (SHIFT && cn > 0) ? (int64_t)__float_as_int(sp.ent4[q0].w) + __ffs(sp.emask[q0]) - 1 : 0;
+        Acc S[2];
         S[0].zero();
         S[1].zero();
-        // parts: the tile's list (not a heavy sample's), then the chunks
-        int32_t chunk = heavy ? (int32_t)c0 : -1;
+        // the tile's list (not a heavy sample's), then the chunks; with k_fold, one part
+        int32_t chunk = (FOLD || heavy) ? c0 : -1;
         while (true) {
-            const int n = chunk < 0 ? RCAP : sp.ccnt[chunk];
+            const int n = chunk < 0 ? cn : sp.ccnt[chunk];
             const size_t e0 = chunk < 0 ? q0 : (size_t)sp.ebase + (size_t)chunk * RCAP;
             const int est = chunk < 0 ? 32 : 1;
             const float* esh = !EXS || kc == 0 ? nullptr
@@ -1333,53 +1357,90 @@ __global__ void __launch_bounds__(128) k_seq(const __grid_constant__ Args<double
                 __syncwarp();
                 if ((m >> lane) & 1u) {
                     const int64_t li = lo + lane;
-                    const float4 L = __ldg(&tv.leaf4[li]), K = __ldg(&tv.leafK[li]);
-                    const float dx = __fsub_rn(q.x, L.x), dy = __fsub_rn(q.y, L.y), dz = __fsub_rn(q.z, L.z);
-                    float W, c;
-                    f32c_pair_weights<ST, KF>(
-                        tv.kern, tv.Kf, qe, dx, dy, dz, ia, sa3, sa4, fa2, ika, (float)ha, K, L.w,
-                        [&]() {
-                            const double ex = __dsub_rn(p[0], __ldg(&tv.x[li]));
-                            const double ey = __dsub_rn(p[1], __ldg(&tv.y[li]));
-                            const double ez = __dsub_rn(p[2], __ldg(&tv.z[li]));
-                            return __fma_rn(ex, ex, __fma_rn(ey, ey, __dmul_rn(ez, ez)));
-                        },
-                        [&]() { return __dmul_rn(tv.Kd, __ldg(&tv.h[li])); }, W, c);
-                    if (WHAT == WHAT_DENSITY) {
-                        rows[0][lane] = __fmul_rn(unit ? 1.f : __ldg(&tv.mf[li]), W);
+                    CT dx, dy, dz, W, c, mr, mb;
+                    if constexpr (PREC == PREC_FP64) {
+                        const double2 a = __ldg(&tv.leafD[0][li]), b = __ldg(&tv.leafD[1][li]), s = __ldg(&tv.leafD[2][li]);
+                        dx = __dsub_rn((double)p[0], a.x);
+                        dy = __dsub_rn((double)p[1], a.y);
+                        dz = __dsub_rn((double)p[2], b.x);
+                        f64_pair_weights<ST, KF>(tv.kern, dx, dy, dz, ia, sa3, b.y, s.x, W, c);
+                        mr = s.y;
+                        mb = (dg || !unit) ? (CT)__ldg(&tv.m[li]) : CT(1);
                     } else {
-                        const float gc = __fmul_rn(K.w, c);
-                        rows[0][lane] = __fmul_rn(K.w, W);
-                        rows[1][lane] = __fmul_rn(gc, dx);
-                        rows[2][lane] = __fmul_rn(gc, dy);
-                        rows[3][lane] = __fmul_rn(gc, dz);
-                        if (dg) {
-                            const float mb = __ldg(&tv.mf[li]), mc = __fmul_rn(mb, c);
-                            rows[4][lane] = __fmul_rn(mb, W);
-                            rows[5][lane] = __fmul_rn(mc, dx);
-                            rows[6][lane] = __fmul_rn(mc, dy);
-                            rows[7][lane] = __fmul_rn(mc, dz);
+                        const float4 L = __ldg(&tv.leaf4[li]), K = __ldg(&tv.leafK[li]);
+                        if constexpr (BAND) {
+                            dx = __fsub_rn(q.x, L.x);
+                            dy = __fsub_rn(q.y, L.y);
+                            dz = __fsub_rn(q.z, L.z);
+                            f32c_pair_weights<ST, KF>(
+                                tv.kern, tv.Kf, qe, dx, dy, dz, ia, sa3, sa4, fa2, ika, (float)ha, K, L.w,
+                                [&]() {
+                                    const double ex = __dsub_rn(p[0], __ldg(&tv.x[li]));
+                                    const double ey = __dsub_rn(p[1], __ldg(&tv.y[li]));
+                                    const double ez = __dsub_rn(p[2], __ldg(&tv.z[li]));
+                                    return __fma_rn(ex, ex, __fma_rn(ey, ey, __dmul_rn(ez, ez)));
+                                },
+                                [&]() { return __dmul_rn(tv.Kd, __ldg(&tv.h[li])); }, W, c);
+                        } else {
+                            dx = __fsub_rn(p[0], L.x);
+                            dy = __fsub_rn(p[1], L.y);
+                            dz = __fsub_rn(p[2], L.z);
+                            f32_pair_weights<ST, KF>(tv.kern, ex_d2_pp<T>(p, L.x, L.y, L.z), ia, sa3, sa4, K.x, K.y, W, c);
                         }
-                        for (int s = 0; s < kc; ++s)
-                            rows[SEQ_COMP + s][lane] =
-                                EXS ? __fadd_rn(__ldg(&A.colR[s][li]), esh[(e * kc + s) * est])
-                                    : __fsub_rn(__ldg(&A.colF[s][li]), __ldg(&A.colF[s][first]));
+                        mr = K.w;
+                        mb = (dg || !unit) ? __ldg(&tv.mf[li]) : 1.f;
+                    }
+                    if (WHAT == WHAT_DENSITY) {
+                        rows[0][lane] = W;
+                        rows[1][lane] = unit ? CT(1) : mb;
+                    } else {
+                        const CT gc = acc_mul(mr, c);
+                        rows[0][lane] = acc_mul(mr, W);
+                        rows[1][lane] = acc_mul(gc, dx);
+                        rows[2][lane] = acc_mul(gc, dy);
+                        rows[3][lane] = acc_mul(gc, dz);
+                        if (dg) {
+                            const CT mc = acc_mul(mb, c);
+                            rows[4][lane] = W;
+                            rows[5][lane] = dx;
+                            rows[6][lane] = dy;
+                            rows[7][lane] = dz;
+                            rows[SEQ_COMP + MAX_KC][lane] = mb;
+                            rows[SEQ_COMP + MAX_KC + 1][lane] = mc;
+                        }
+                        for (int s = 0; s < kc; ++s) {
+                            CT a;
+                            if constexpr (EXS) a = __fadd_rn(__ldg(&A.colR[s][li]), esh[(e * kc + s) * est]);
+                            else if constexpr (SHIFT) a = __fsub_rn(__ldg(&A.colF[s][li]), __ldg(&A.colF[s][first]));
+                            else a = (CT)__ldg(&A.colT[s][li]);
+                            rows[SEQ_COMP + s][lane] = a;
+                        }
                     }
                 }
                 __syncwarp();
 #pragma unroll 4
                 for (unsigned b = m; b; b &= b - 1) {
                     const int j = __ffs(b) - 1;
-                    const float v = rows[ra[0]][j];
-                    S[0].add(rb[0] < 0 ? v : __fmul_rn(rows[rb[0]][j], v));
+                    const CT v = rows[ra[0]][j];
+                    if (rb[0] < 0) S[0].add(v);
+                    else acc_mac(S[0], rows[rb[0]][j], v);
                     if (two) {
-                        const float v1 = rows[ra[1]][j];
-                        S[1].add(rb[1] < 0 ? v1 : __fmul_rn(rows[rb[1]][j], v1));
+                        const CT v1 = rows[ra[1]][j];
+                        if (rb[1] < 0) S[1].add(v1);
+                        else acc_mac(S[1], rows[rb[1]][j], v1);
                     }
                 }
             }
-            chunk = chunk < 0 ? (int32_t)c0 : sp.next[chunk];
+            if (FOLD || i < n1) break;
+            chunk = chunk < 0 ? c0 : sp.next[chunk];
             if (chunk < 0) break;
+        }
+        if (FOLD && (chunk >= 0 || more >= 0)) {  // a part, for k_fold
+            double* o = sp.part + (chunk >= 0 ? chunk : (size_t)sp.ncap + more);
+#pragma unroll
+            for (int u = 0; u < 2; ++u)
+                if (fo[u] >= 0) o[fo[u] * 2 * (size_t)sp.ncap] = S[u].get();
+            continue;
         }
 #pragma unroll
         for (int u = 0; u < 2; ++u)
@@ -1387,7 +1448,7 @@ __global__ void __launch_bounds__(128) k_seq(const __grid_constant__ Args<double
         __syncwarp();
         if (lane == 0) {
             if (WHAT == WHAT_DENSITY) {
-                A.out[0][k] = (double)(float)sums[0];
+                A.out[0][k] = (PREC == PREC_FP64) ? (T)sums[0] : (T)(CT)sums[0];
             } else {
                 PlainD S1, G[3], Dm, Dg[3], Sw[MAX_KC], Sg[MAX_KC][3];
                 double a0[MAX_KC];
@@ -1400,10 +1461,10 @@ __global__ void __launch_bounds__(128) k_seq(const __grid_constant__ Args<double
                 for (int c = 0; c < MAX_KC; ++c) {
                     const bool on = c < kc;
                     Sw[c].s = on ? sums[8 + c] : 0.0;
-                    for (int d = 0; d < 3; ++d) Sg[c][d].s = on ? sums[8 + MAX_KC + 3 * c + d] : 0.0;
-                    a0[c] = !on ? 0.0 : (EXS ? A.colT[c][first] : (double)A.colF[c][first]);
+                    for (int d = 0; d < 3; ++d) Sg[c][d].s = on ? sums[8 + sp.kcl + 3 * c + d] : 0.0;
+                    a0[c] = (!on || !SHIFT || cn == 0) ? 0.0 : (EXS ? (double)A.colT[c][first] : (double)A.colF[c][first]);
                 }
-                write_interp_outputs<double, PlainD, float, MAX_KC>(A, k, S1, G, Sw, Sg, Dm, Dg, a0);
+                write_interp_outputs<T, PlainD, CT, MAX_KC>(A, k, S1, G, Sw, Sg, Dm, Dg, a0);
             }
         }
         __syncwarp();

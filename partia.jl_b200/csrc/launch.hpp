@@ -139,22 +139,24 @@ static void dispatch_density_k(const Args<T>& a, unsigned g, unsigned gc, cudaSt
 }
 
 // k_seq: enough warps to fill the GPU, each takes samples until none is left
-template <int S>
-static void dispatch_seq_s(const Args<double>& a, bool density, cudaStream_t s) {
-    const unsigned g = std::min(148u * 8u, (a.sp.ncap + 3) / 4);
+template <class T, int P, int S>
+static void dispatch_seq_s(const Args<T>& a, bool density, cudaStream_t s) {
+    const int64_t items = (a.sp.seq_all ? a.sp.ntiles * 32 : 0) + a.sp.ncap;
+    const unsigned g = (unsigned)std::min<int64_t>(148 * 8, (items + 3) / 4);
     const bool m4 = a.tv.kern == KERN_M4;
     if (density) {
-        if (m4) k_seq<S, 0, WHAT_DENSITY><<<g, 128, 0, s>>>(a);
-        else k_seq<S, 1, WHAT_DENSITY><<<g, 128, 0, s>>>(a);
+        if (m4) k_seq<T, P, S, 0, WHAT_DENSITY><<<g, 128, 0, s>>>(a);
+        else k_seq<T, P, S, 1, WHAT_DENSITY><<<g, 128, 0, s>>>(a);
     } else {
-        if (m4) k_seq<S, 0, WHAT_INTERP><<<g, 128, 0, s>>>(a);
-        else k_seq<S, 1, WHAT_INTERP><<<g, 128, 0, s>>>(a);
+        if (m4) k_seq<T, P, S, 0, WHAT_INTERP><<<g, 128, 0, s>>>(a);
+        else k_seq<T, P, S, 1, WHAT_INTERP><<<g, 128, 0, s>>>(a);
     }
 }
-static inline void dispatch_seq(const Args<double>& a, int st, bool density, cudaStream_t s) {
-    if (st == ST_GATHER) dispatch_seq_s<ST_GATHER>(a, density, s);
-    else if (st == ST_SCATTER) dispatch_seq_s<ST_SCATTER>(a, density, s);
-    else dispatch_seq_s<ST_SYMMETRIC>(a, density, s);
+template <class T, int P>
+static void dispatch_seq(const Args<T>& a, int st, bool density, cudaStream_t s) {
+    if (st == ST_GATHER) dispatch_seq_s<T, P, ST_GATHER>(a, density, s);
+    else if (st == ST_SCATTER) dispatch_seq_s<T, P, ST_SCATTER>(a, density, s);
+    else dispatch_seq_s<T, P, ST_SYMMETRIC>(a, density, s);
 }
 
 template <class T, int P>
@@ -167,7 +169,7 @@ static cudaError_t dispatch_split_p(const Args<T>& a, int st, int kc, int pass, 
     if (g == 0) return cudaSuccess;
     if (pass == SPLIT_FOLD || pass == SPLIT_FOLD_DENSITY) {
         if constexpr (SEQ) {
-            dispatch_seq(a, st, pass == SPLIT_FOLD_DENSITY, s);
+            dispatch_seq<T, P>(a, st, pass == SPLIT_FOLD_DENSITY, s);
         } else {
             if (pass == SPLIT_FOLD_DENSITY) k_fold<T, P, 1, WHAT_DENSITY><<<gf, 128, 0, s>>>(a);
             else if (kc <= 1) k_fold<T, P, 1, WHAT_INTERP><<<gf, 128, 0, s>>>(a);
@@ -187,6 +189,8 @@ static cudaError_t dispatch_split_p(const Args<T>& a, int st, int kc, int pass, 
         if (st == ST_GATHER) k_collect<T, ST_GATHER><<<gw, WALK_THREADS, 0, s>>>(a);
         else if (st == ST_SCATTER) k_collect<T, ST_SCATTER><<<gw, WALK_THREADS, 0, s>>>(a);
         else k_collect<T, ST_SYMMETRIC><<<gw, WALK_THREADS, 0, s>>>(a);
+    } else if (a.sp.seq_all) {  // in FP32C of double particles the fold pass takes all samples
+        if constexpr (!SEQ) dispatch_seq<T, P>(a, st, pass == SPLIT_DENSITY, s);
     } else if (pass == SPLIT_DENSITY) {
         if (st == ST_GATHER) dispatch_density_k<T, P, ST_GATHER>(a, g, gc, s);
         else if (st == ST_SCATTER) dispatch_density_k<T, P, ST_SCATTER>(a, g, gc, s);

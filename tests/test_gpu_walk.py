@@ -81,6 +81,29 @@ def test_list_parts_and_heavy_samples(ns, kid, prec, strategy):
     assert np.array_equal(dens, done)
 
 
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("prec", [L.PSB_PREC_FP64, L.PSB_PREC_FP32C])
+@pytest.mark.parametrize("kid", [L.PSB_KERNEL_M4, L.PSB_KERNEL_M5])
+def test_small_calls_have_the_bits_of_large_ones(kid, prec, dtype):
+    """Up to 4096 samples a warp sums each sample, above that a lane: the same
+    pairs, rounded alike and added in the same order, with the same parts."""
+    arrs, cols = particles(20_000, 11, dtype)
+    rng = np.random.default_rng(12)
+    ns = 4097
+    s = tuple(rng.random(ns).astype(dtype) for _ in range(3))
+    hs = rng.choice([0.01, 0.03, 0.06, 0.12, 0.3], ns, p=[0.5, 0.3, 0.15, 0.04, 0.01]).astype(dtype)
+    ctx = context(arrs, cols, kid)
+    cat = CatalogC(**SPEC)
+    for strategy in (L.PSB_GATHER, L.PSB_SCATTER, L.PSB_SYMMETRIC):
+        kw = dict(strategy=strategy, hmode=L.PSB_H_PER_SAMPLE, prec=prec)
+        large = ctx.interp_points(*s, cat, hs=hs, **kw) + [ctx.density(*s, hs=hs, **kw)]
+        for k0, k1 in ((0, 4096), (4094, 4097)):
+            t = tuple(a[k0:k1] for a in s)
+            small = ctx.interp_points(*t, cat, hs=hs[k0:k1], **kw) + [ctx.density(*t, hs=hs[k0:k1], **kw)]
+            for k, (a, b) in enumerate(zip(small, large)):
+                assert np.array_equal(a, b[k0:k1], equal_nan=True), (strategy, k)
+
+
 @pytest.mark.parametrize("prec", [L.PSB_PREC_FP64, L.PSB_PREC_FP32C])
 def test_heavy_samples_of_float_particles(prec):
     """Float particles: equal to the single kernel to a float rounding, whose parts these are."""
