@@ -164,10 +164,15 @@ static int run_split(psb_ctx* c, Args<T>& A, int prec, int st, int* launches, in
     // (neighbourhoods of more than RCAP spans are rare there), one per
     // sample for M5 and M6, whose ordinary samples often take two parts.
     const int64_t lanes = 32 * B;
-    // At least 65536 for calls with a few large neighbourhoods, but no more than
-    // the samples of a small call can fill (a chunk holds RCAP spans of the tree).
+    // For large neighbourhoods eight per sample up to 262144 over the streams, at
+    // least 65536, but no more than the samples of a small call can fill (a chunk
+    // holds RCAP spans of the tree).  A call that finds the pool empty sums the
+    // rest in the single kernel: 65,536 samples of 1M particles of which one in
+    // ten has thousands of neighbours take 48 ms with 65536 chunks, 13 with 262144.
     const int64_t most = std::min<int64_t>(lanes, A.src.ns) * (c->n / 256 + 2);
-    const unsigned ncap = (unsigned)std::min<int64_t>(std::max<int64_t>(65536, A.tv.Kd > 2.0 ? lanes : lanes / 4), most);
+    const unsigned ncap = (unsigned)std::min<int64_t>(
+        std::max<int64_t>(std::max<int64_t>(65536, std::min<int64_t>(262144 / nsets, 8 * lanes)),
+                          A.tv.Kd > 2.0 ? lanes : lanes / 4), most);
     constexpr unsigned HCAP = 4096;  // samples of a batch for k_heavy (the rest stay in their tiles' walks)
     Lists ls[SPLIT_STREAMS];
     {
@@ -186,7 +191,7 @@ static int run_split(psb_ctx* c, Args<T>& A, int prec, int st, int* launches, in
         const size_t hab = take(sizeof(double) * lanes), head = take(sizeof(int32_t) * lanes), cnt = take(lanes);
         const size_t part = take((seq ? sizeof(uint32_t) : sizeof(double) * 2 * nf) * (size_t)ncap);
         const size_t own = take(sizeof(uint32_t) * ncap), next = take(sizeof(int32_t) * ncap), ccnt = take(ncap);
-        const size_t hlist = take(sizeof(uint32_t) * HCAP), ovf = take(sizeof(int32_t) * (size_t)B), ctr = take(256);
+        const size_t hlist = take(sizeof(uint32_t) * HCAP), ovf = take(sizeof(int32_t) * (size_t)B), ctr = take(256 + sizeof(unsigned) * (size_t)B);
         char* base = (char*)scratch(c, slot, size * nsets);
         if (!base) return fail(c, PSB_ENOMEM, "scratch allocation failed (pair lists)");
         for (int k = 0; k < nsets; ++k, base += size) {
@@ -203,7 +208,7 @@ static int run_split(psb_ctx* c, Args<T>& A, int prec, int st, int* launches, in
             ls[k].ccnt = (uint8_t*)(base + ccnt);
             ls[k].hlist = (uint32_t*)(base + hlist);
             ls[k].ovf_tiles = (int32_t*)(base + ovf);
-            ls[k].ctr = (unsigned*)(base + ctr);
+            ls[k].ctr = (unsigned*)(base + ctr);  // then a word per tile, both zeroed for each batch
         }
     }
     A.sp.ncap = ncap;
@@ -219,10 +224,10 @@ static int run_split(psb_ctx* c, Args<T>& A, int prec, int st, int* launches, in
         const int k = (int)(bi % nsets);
         const cudaStream_t sk = ss[k];
         const int64_t nb = std::min<int64_t>(B, nt - t0);
-        PSB_CUDA_TRY(c, cudaMemsetAsync(ls[k].ctr, 0, 4 * sizeof(unsigned), sk), "memset list counters");
+        PSB_CUDA_TRY(c, cudaMemsetAsync(ls[k].ctr, 0, 256 + sizeof(unsigned) * (size_t)nb, sk), "memset list counters");
         A.sp.ent4 = ls[k].ent4; A.sp.emask = ls[k].emask; A.sp.cnt = ls[k].cnt; A.sp.ha = ls[k].hab;
         A.sp.eshift = ls[k].eshift; A.sp.head = ls[k].head;
-        A.sp.ovf_tiles = ls[k].ovf_tiles; A.sp.ovf_count = ls[k].ctr; A.sp.top = ls[k].ctr + 1;
+        A.sp.ovf_tiles = ls[k].ovf_tiles; A.sp.ovf_count = ls[k].ctr; A.sp.dead = ls[k].ctr + 64; A.sp.top = ls[k].ctr + 1;
         A.sp.own = ls[k].own; A.sp.next = ls[k].next; A.sp.ccnt = ls[k].ccnt; A.sp.part = ls[k].part;
         A.sp.hcount = ls[k].ctr + 2; A.sp.hlist = ls[k].hlist; A.sp.hcap = HCAP;
         A.sp.mcount = ls[k].ctr + 3; A.sp.mlist = ls[k].mlist;

@@ -39,9 +39,9 @@ namespace psb {
 // lanes as it has chunks.  k_points sums in the same parts.  (FP32C with
 // double particles: a compensated sum's bits depend on its order to a float
 // rounding of its terms, so there the sums run on through the parts, a warp
-// per sample: k_seq.)  A tile of which
-// a sample finds the pool exhausted is marked (cnt = 0xFF for all its lanes)
-// and listed in ovf_tiles; the single-kernel path computes those tiles.
+// per sample: k_seq.)  The samples
+// of a warp of which one finds the pool exhausted are marked (cnt = CNT_DEAD)
+// and their tile is listed in ovf_tiles; the single-kernel path computes them.
 constexpr int RCAP = 32;
 struct SplitBufs {
     // entries: [tile][RCAP][32] lists, then [chunk][RCAP]
@@ -53,6 +53,7 @@ struct SplitBufs {
     void* ha;            // [tile][32], element type T
     int32_t* head;       // [tile][32]: the sample's first chunk, or -1
     int32_t* ovf_tiles;  // absolute tile ids
+    unsigned* dead;      // [tile]: the samples the single-kernel path computes
     unsigned* ovf_count;
     int64_t tile0;       // first tile of the batch
     int64_t ntiles;      // tiles in the batch
@@ -76,7 +77,7 @@ struct SplitBufs {
     int seq_all;         // k_seq takes every sample (a small call)
     int kcl;             // columns of the partial sums' layout (the KC of k_fold)
 };
-constexpr uint8_t CNT_DEAD = 0xFF;   // the tile is the single-kernel pass's
+constexpr uint8_t CNT_DEAD = 0xFF;   // the sample is the single-kernel pass's
 constexpr uint8_t CNT_HEAVY = 0xFE;  // the sample's entries are k_heavy's
 constexpr uint32_t OWN_LATER = 0x80000000u;  // not the sample's first chunk
 constexpr uint32_t OWN_HEAVY = 0x40000000u;  // a chunk of k_heavy

@@ -324,7 +324,8 @@ __global__ void __launch_bounds__(128) k_points(const Args<T> A) {
         return;  // warp-uniform
     }
 
-    const int64_t k = sample_of(A.src, tile, lane);
+    int64_t k = sample_of(A.src, tile, lane);
+    if (A.tile_list && A.sp.cnt[(tile - A.sp.tile0) * 32 + lane] != CNT_DEAD) k = -1;  // summed from its lists
     const bool valid = k >= 0;
     T p[3] = {T(0), T(0), T(0)}, dd[3];
     if (valid) sample_coords(A.src, k, p, dd);

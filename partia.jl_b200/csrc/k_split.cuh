@@ -110,6 +110,12 @@ static __device__ __noinline__ int2 next_part(const SplitBufs& sp, uint32_t idx,
     return make_int2((int32_t)c, nparts + 1);
 }
 
+// Samples left to the single kernel (their cnt is CNT_DEAD): their tile is
+// listed once, by whoever marks the first of its samples.
+static __device__ __forceinline__ void list_dead(const SplitBufs& sp, uint32_t bt, unsigned mask) {
+    if (atomicOr(&sp.dead[bt], mask) == 0u) sp.ovf_tiles[atomicAdd(sp.ovf_count, 1u)] = (int32_t)(sp.tile0 + bt);
+}
+
 // The walk of one warp: the nodes that reach the warp's samples, found 32 at a
 // time.  The stack holds nodes (id) and found spans (-id) with the leftmost
 // item on top.  A step takes the top items of the stack, one per lane, tests
@@ -231,7 +237,7 @@ __global__ void __launch_bounds__(WALK_THREADS, 1280 / WALK_THREADS) k_collect(c
     T p[3] = {T(0), T(0), T(0)}, dd[3];
     if (valid) sample_coords(A.src, k, p, dd);
     // A sample whose position or h is not finite, or beyond the range of the
-    // float tests, sends its tile to the single kernel.
+    // float tests, sends its warp's samples to the single kernel.
     {
         bool wild = valid && !(fabs((double)p[0]) <= 1e18 && fabs((double)p[1]) <= 1e18 && fabs((double)p[2]) <= 1e18);
         if (ST != ST_SCATTER && A.hmode != PSB_H_NEAREST && valid)
@@ -242,7 +248,7 @@ __global__ void __launch_bounds__(WALK_THREADS, 1280 / WALK_THREADS) k_collect(c
                 A.sp.cnt[slot] = any_wild ? CNT_DEAD : 0;
                 A.sp.head[slot] = -1;
             }
-            if (any_wild && lane == 0) A.sp.ovf_tiles[atomicAdd(A.sp.ovf_count, 1u)] = (int32_t)tile;
+            if (any_wild && lane == 0) list_dead(A.sp, (uint32_t)bt, 0xffffffffu >> (32 - (1 << lspt)) << s0);
             return;
         }
     }
@@ -428,7 +434,7 @@ __global__ void __launch_bounds__(WALK_THREADS, 1280 / WALK_THREADS) k_collect(c
     int nent = 0;         // entries in the current part
     int32_t chunk = -1;   // the current chunk (-1: the tile's list)
     int nparts = 1;       // parts so far; 0: the sample is k_heavy's
-    bool dead = false;    // warp-uniform: the pool ran out, the tile is k_points'
+    bool dead = false;    // warp-uniform: the pool ran out, the samples are k_points'
     auto emit = [&](int64_t lo, unsigned acc) {
         if (__any_sync(PSB_FULL, acc && nent == RCAP)) {
             if (acc && nent == RCAP) {
@@ -611,8 +617,8 @@ __global__ void __launch_bounds__(WALK_THREADS, 1280 / WALK_THREADS) k_collect(c
         }
     }
     if (valid && A.ha_out) A.ha_out[k] = ha;
-    if (dead && lane == 0) A.sp.ovf_tiles[atomicAdd(A.sp.ovf_count, 1u)] = (int32_t)tile;
-    // the single-kernel pass counts the pairs of a dead tile, k_heavy those of its samples
+    if (dead && lane == 0) list_dead(A.sp, (uint32_t)bt, 0xffffffffu >> (32 - (1 << lspt)) << s0);
+    // the single-kernel pass counts the pairs of dead samples, k_heavy those of its samples
     unsigned long long t_pairs = (dead || nparts == 0) ? 0ull : n_pairs, t_retest = n_retest;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
@@ -679,6 +685,19 @@ __global__ void __launch_bounds__(HEAVY_THREADS, 2) k_heavy(const Args<T> A) {
     const unsigned nh = min(*sp.hcount, sp.hcap);
     for (unsigned i = blockIdx.x; i < nh; i += gridDim.x) {
         const uint32_t idx = sp.hlist[i];
+        // a sample whose warp found the pool empty is k_points' already; with
+        // the pool empty no other sample is worth its walk
+        if (tid == 0) s_base = sp.cnt[idx] == CNT_DEAD ? 2u : (atomicAdd(sp.top, 0u) >= sp.ncap ? 1u : 0u);
+        __syncthreads();
+        const unsigned give_up = s_base;
+        __syncthreads();
+        if (give_up) {
+            if (give_up == 1u && tid == 0) {
+                sp.cnt[idx] = CNT_DEAD;
+                list_dead(sp, idx >> 5, 1u << (idx & 31));
+            }
+            continue;
+        }
         const int64_t k = sample_of(A.src, sp.tile0 + (idx >> 5), idx & 31);
         T p[3], dd[3];
         sample_coords(A.src, k, p, dd);
@@ -808,11 +827,9 @@ __global__ void __launch_bounds__(HEAVY_THREADS, 2) k_heavy(const Args<T> A) {
                 if (sp.mlist && tid == 0) sp.mlist[atomicAdd(sp.mcount, 1u)] = base;
             }
         }
-        if (!fits && tid == 0) {  // k_points takes the tile (once)
-            const uint32_t t0 = idx & ~31u;
-            for (int q = 0; q < 32; ++q) sp.cnt[t0 + q] = CNT_DEAD;
-            if (atomicExch(&sp.head[t0], -2) != -2)
-                sp.ovf_tiles[atomicAdd(sp.ovf_count, 1u)] = (int32_t)(sp.tile0 + (idx >> 5));
+        if (!fits && tid == 0) {  // k_points takes the sample
+            sp.cnt[idx] = CNT_DEAD;
+            list_dead(sp, idx >> 5, 1u << (idx & 31));
         }
     }
 }

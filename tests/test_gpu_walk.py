@@ -281,3 +281,48 @@ def test_float_decisions_on_the_support_edge():
             ctx.interp_points(*s, CatalogC(scalars=[0], shepard=[0]), **kw)
             count, _, _ = orc.digest(s, **kw)
             assert ctx.last_stats.pairs == int(count.sum()), (strategy, hs)
+
+
+@pytest.mark.parametrize("ns", [500, 4000, 9000])
+def test_out_of_range_samples_leave_their_neighbours_lists(ns):
+    """Samples outside the float range in every tile and in small calls' warps of
+    a few samples: the single kernel takes them, once each (pairs are counted
+    once), and the others keep their results."""
+    arrs, cols = particles(20_000, 13)
+    rng = np.random.default_rng(14)
+    s = [rng.random(ns) for _ in range(3)]
+    s[1][rng.random(ns) < 0.2] = 1e19
+    hs = np.full(ns, 0.05)
+    ctx = context(arrs, cols)
+    cat = CatalogC(**SPEC)
+    for prec in (L.PSB_PREC_FP64, L.PSB_PREC_FP32C):
+        kw = dict(strategy=L.PSB_GATHER, hmode=L.PSB_H_PER_SAMPLE, hs=hs, prec=prec)
+        ctx.extra_flags = 0
+        got = ctx.interp_points(*s, cat, **kw)
+        pairs = ctx.last_stats.pairs
+        ctx.extra_flags = L.PSB_FLAG_SINGLE_KERNEL
+        one = ctx.interp_points(*s, cat, **kw)
+        assert ctx.last_stats.pairs == pairs
+        for k in range(cat.L):
+            assert np.array_equal(got[k], one[k], equal_nan=True), (prec, k)
+
+
+def test_more_large_neighbourhoods_than_the_pool_holds():
+    """20,000 samples that each reach most of 30,000 particles: more entries than
+    the lists hold, so the single kernel sums the rest; every pair counted once."""
+    arrs, cols = particles(30_000, 15)
+    rng = np.random.default_rng(16)
+    s = [rng.random(20_000) for _ in range(3)]
+    hs = np.full(20_000, 0.3)
+    hs[rng.random(20_000) < 0.3] = 0.02
+    ctx = context(arrs, cols)
+    kw = dict(strategy=L.PSB_GATHER, hmode=L.PSB_H_PER_SAMPLE, hs=hs, prec=L.PSB_PREC_FP32C)
+    cat = CatalogC(scalars=[0, 1], grads=[-1, 1])
+    got, dens = ctx.interp_points(*s, cat, **kw), ctx.density(*s, **kw)
+    pairs = ctx.last_stats.pairs
+    ctx.extra_flags = L.PSB_FLAG_SINGLE_KERNEL
+    one, done = ctx.interp_points(*s, cat, **kw), ctx.density(*s, **kw)
+    assert ctx.last_stats.pairs == pairs
+    for k in range(cat.L):
+        assert np.array_equal(got[k], one[k], equal_nan=True), k
+    assert np.array_equal(dens, done)
