@@ -111,8 +111,7 @@ static float ms_between(cudaEvent_t a, cudaEvent_t b) {
 // lists of a batch, k_bodies sums them, k_fold adds up the samples of several
 // parts, and k_points takes the tiles that found the chunk pool exhausted.  A
 // batch holds at most SPLIT_BATCH tiles, which bounds the lists' memory at
-// SPLIT_BATCH * RCAP * 32 * 20 bytes (640 MiB) per stream, and the pool's at
-// about the same (M5, M6) or a quarter of it.
+// SPLIT_BATCH * RCAP * 32 * 20 bytes (640 MiB) per stream.
 //
 // A direct call (multi_stream) of at least two batches' worth of tiles
 // spreads its batches over up to SPLIT_STREAMS streams (the context stream and
@@ -164,18 +163,19 @@ static int run_split(psb_ctx* c, Args<T>& A, int prec, int st, int* launches, in
     // (neighbourhoods of more than RCAP spans are rare there), one per
     // sample for M5 and M6, whose ordinary samples often take two parts.
     const int64_t lanes = 32 * B;
-    // For large neighbourhoods eight per sample up to 262144 over the streams, at
-    // least 65536, but no more than the samples of a small call can fill (a chunk
+    // For large neighbourhoods eight per sample up to 4M over the streams (5 GB;
+    // the small pool if the device has no room for it), at least 65536, but no more than the samples of a small call can fill (a chunk
     // holds RCAP spans of the tree).  A call that finds the pool empty sums the
     // rest in the single kernel: 65,536 samples of 1M particles of which one in
-    // ten has thousands of neighbours take 48 ms with 65536 chunks, 13 with 262144.
+    // ten has thousands of neighbours take 48 ms with 65536 chunks, 13 with
+    // 262144; 524,288 samples 70 ms with 262144, 42 with 4M.
     const int64_t most = std::min<int64_t>(lanes, A.src.ns) * (c->n / 256 + 2);
-    const unsigned ncap = (unsigned)std::min<int64_t>(
-        std::max<int64_t>(std::max<int64_t>(65536, std::min<int64_t>(262144 / nsets, 8 * lanes)),
+    unsigned ncap = (unsigned)std::min<int64_t>(
+        std::max<int64_t>(std::max<int64_t>(65536, std::min<int64_t>(4194304 / nsets, 8 * lanes)),
                           A.tv.Kd > 2.0 ? lanes : lanes / 4), most);
     constexpr unsigned HCAP = 4096;  // samples of a batch for k_heavy (the rest stay in their tiles' walks)
     Lists ls[SPLIT_STREAMS];
-    {
+    for (bool retry = true;;) {
         // One block for all the streams' lists (slots 96-99): a context's first
         // call pays for the number of allocations.
         const int slot = 96 + (slot_off == 0 ? 0 : (slot_off == 32 ? 1 : (slot_off == 14 ? 2 : 3)));
@@ -193,6 +193,11 @@ static int run_split(psb_ctx* c, Args<T>& A, int prec, int st, int* launches, in
         const size_t own = take(sizeof(uint32_t) * ncap), next = take(sizeof(int32_t) * ncap), ccnt = take(ncap);
         const size_t hlist = take(sizeof(uint32_t) * HCAP), ovf = take(sizeof(int32_t) * (size_t)B), ctr = take(256 + sizeof(unsigned) * (size_t)B);
         char* base = (char*)scratch(c, slot, size * nsets);
+        if (!base && retry && ncap > 65536) {
+            retry = false;
+            ncap = 65536;
+            continue;
+        }
         if (!base) return fail(c, PSB_ENOMEM, "scratch allocation failed (pair lists)");
         for (int k = 0; k < nsets; ++k, base += size) {
             ls[k].ent4 = (float4*)(base + ent4);
@@ -210,6 +215,7 @@ static int run_split(psb_ctx* c, Args<T>& A, int prec, int st, int* launches, in
             ls[k].ovf_tiles = (int32_t*)(base + ovf);
             ls[k].ctr = (unsigned*)(base + ctr);  // then a word per tile, both zeroed for each batch
         }
+        break;
     }
     A.sp.ncap = ncap;
     A.sp.ebase = (uint32_t)((int64_t)RCAP * 32 * B);
