@@ -171,7 +171,7 @@ static int run_split(psb_ctx* c, Args<T>& A, int prec, int st, int* launches, in
     // 262144; 524,288 samples 70 ms with 262144, 42 with 4M.
     const int64_t most = std::min<int64_t>(lanes, A.src.ns) * (c->n / 256 + 2);
     unsigned ncap = (unsigned)std::min<int64_t>(
-        std::max<int64_t>(std::max<int64_t>(65536, std::min<int64_t>(4194304 / nsets, 8 * lanes)),
+        std::max<int64_t>(std::max<int64_t>(65536, std::min<int64_t>(4194304 / (multi_stream ? nsets : SPLIT_STREAMS), 8 * lanes)),
                           A.tv.Kd > 2.0 ? lanes : lanes / 4), most);
     constexpr unsigned HCAP = 4096;  // samples of a batch for k_heavy (the rest stay in their tiles' walks)
     Lists ls[SPLIT_STREAMS];
@@ -747,7 +747,7 @@ static int run_points_pipelined(psb_ctx* c, const SampleReq& rq, int hmode, cons
     char* inb = (char*)scratch(c, 0, es * CH * nin * PIPE_SETS);
     char* outb = (char*)scratch(c, 2, es * CH * (L > 0 ? L : 1) * PIPE_SETS);
     // per set: sample codes and order (slots), the sample sort's scratch
-    // (slot base, 7 slots) and the pair lists (slot offset: slots 16-20 + off)
+    // (slot base, 7 slots) and the pair lists (slots 96-99, by the offset)
     static const int code_slot[PIPE_SETS] = {3, 35, 53, 55};
     static const int sort_slot[PIPE_SETS] = {6, 38, 64, 72};
     static const int list_off[PIPE_SETS] = {0, 32, 14, 41};
