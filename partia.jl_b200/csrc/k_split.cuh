@@ -678,7 +678,8 @@ template <class T, int ST>
 __global__ void __launch_bounds__(HEAVY_THREADS, 2) k_heavy(const Args<T> A) {
     extern __shared__ __align__(16) int32_t hbuf[];
     __shared__ int wt[HEAVY_THREADS / 32];
-    __shared__ unsigned s_base;
+    // two words: a warp may still read one sample's s_base when thread 0 is at the next sample's s_skip
+    __shared__ unsigned s_skip, s_base;
     const TreeView<T>& tv = A.tv;
     const SplitBufs& sp = A.sp;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -687,9 +688,9 @@ __global__ void __launch_bounds__(HEAVY_THREADS, 2) k_heavy(const Args<T> A) {
         const uint32_t idx = sp.hlist[i];
         // a sample whose warp found the pool empty is k_points' already; with
         // the pool empty no other sample is worth its walk
-        if (tid == 0) s_base = sp.cnt[idx] == CNT_DEAD ? 2u : (atomicAdd(sp.top, 0u) >= sp.ncap ? 1u : 0u);
+        if (tid == 0) s_skip = sp.cnt[idx] == CNT_DEAD ? 2u : (atomicAdd(sp.top, 0u) >= sp.ncap ? 1u : 0u);
         __syncthreads();
-        const unsigned give_up = s_base;
+        const unsigned give_up = s_skip;
         __syncthreads();
         if (give_up) {
             if (give_up == 1u && tid == 0) {

@@ -1,0 +1,47 @@
+"""Many samples of large neighbourhoods: k_heavy's blocks take several in turn,
+of different sizes, so that a block's threads that run ahead meet the next
+sample while others still place the last one's entries.  Bit for bit against
+the single kernel, and the oracle's pair counts.
+"""
+import numpy as np
+import pytest
+
+from conftest import has_gpu
+
+pytestmark = pytest.mark.gpu
+
+if not has_gpu():
+    pytest.skip("needs a CUDA GPU", allow_module_level=True)
+
+import oracle as O  # noqa: E402
+from partia_b200 import _lib as L  # noqa: E402
+from partia_b200.engine import CatalogC, Context  # noqa: E402
+
+
+@pytest.mark.parametrize("prec", [L.PSB_PREC_FP64, L.PSB_PREC_FP32C])
+@pytest.mark.parametrize("kid", [L.PSB_KERNEL_M4, L.PSB_KERNEL_M6])
+def test_blocks_take_several_heavy_samples_in_turn(kid, prec):
+    rng = np.random.default_rng(41)
+    n, ns = 20_000, 1500  # five samples to each of k_heavy's blocks
+    x, y, z = rng.random((3, n))
+    m, rho = rng.uniform(0.5, 1.5, n) / n, rng.uniform(0.5, 2.0, n)
+    h = 1.2 * n ** (-1 / 3) * rng.uniform(0.5, 2.0, n)
+    cols = [rng.standard_normal(n) for _ in range(2)]
+    s = tuple(rng.random((3, ns)))
+    hs = rng.uniform(0.1, 0.18, ns) * (2.0 if kid == L.PSB_KERNEL_M4 else 1.4)
+    count, _, _ = O.Oracle(x, y, z, m, h, rho, cols=cols, kernel=kid).digest(
+        s, strategy=O.GATHER, hmode=O.H_PER_SAMPLE, hs=hs)
+    ctx = Context(0)
+    ctx.set_particles(x, y, z, m, h, rho, cols, kernel=kid)
+    ctx.build(want_perm=False)
+    cat = CatalogC(scalars=[0, 1], shepard=[0, 1], grads=[-1, 1])
+    kw = dict(strategy=L.PSB_GATHER, hmode=L.PSB_H_PER_SAMPLE, hs=hs, prec=prec)
+    ctx.extra_flags = L.PSB_FLAG_SINGLE_KERNEL
+    one, done = ctx.interp_points(*s, cat, **kw), ctx.density(*s, **kw)
+    ctx.extra_flags = 0
+    for _ in range(5):
+        got, dens = ctx.interp_points(*s, cat, **kw), ctx.density(*s, **kw)
+        assert ctx.last_stats.pairs == int(count.sum())
+        for k in range(cat.L):
+            assert np.array_equal(got[k], one[k], equal_nan=True), k
+        assert np.array_equal(dens, done)
