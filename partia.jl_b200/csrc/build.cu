@@ -354,10 +354,11 @@ __global__ void k_pack_leaves(int64_t n, const T* x, const T* y, const T* z, con
     const float ih = 1.f / r.w;
     const float s3 = sig * ih * ih * ih;  // sig = the kernel's 3D norm
     leafK[i] = make_float4(ih, s3, s3 * ih, mr);
-    // span bounds: max |offset|_1 and max h, rounded up (non-negative floats
-    // order like their bit patterns); spanb starts at zero
+    // span bounds: max |offset|_1 and max |h| (its square is the radius), rounded
+    // up, without the h that are NaN (non-negative floats order like their bit
+    // patterns); spanb starts at zero
     const float l1 = (fabsf(r.x) + fabsf(r.y) + fabsf(r.z)) * 1.0000005f;
-    const float hu = __double2float_ru((double)h[i]);
+    const float hu = fmaxf(__double2float_ru(fabs((double)h[i])), 0.f);
     atomicMax((int*)&spanb[sfirst[i]].x, __float_as_int(l1));
     atomicMax((int*)&spanb[sfirst[i]].y, __float_as_int(hu));
 }

@@ -117,7 +117,7 @@ template <class T> struct TreeView {
     // FP64 pair sums: (x, y), (z, 1/h) and (sigma/h^3, m/rho) in double
     const double2* leafD[3];
     // at the first leaf of every span: (max over the span of |leaf4.x| +
-    // |leaf4.y| + |leaf4.z|, max h), both rounded up (float error bounds)
+    // |leaf4.y| + |leaf4.z|, max |h|), both rounded up (float error bounds)
     const float2* spanb;
     float coord_err;         // bound on |float coordinate - exact| for node tests
     // kernel family (psb_kernel): support K in units of h (exact in float),

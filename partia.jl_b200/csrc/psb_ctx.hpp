@@ -49,7 +49,7 @@ struct psb_ctx {
     // coordinates and h lie in the range where the float tests of the walk are
     // proven (build_typed); other sets are interpolated by the single kernel
     bool band_ok = false;
-    float2* spanb = nullptr;  // at a span's first leaf: (max |leaf4.xyz|_1, max h) over the span, rounded up
+    float2* spanb = nullptr;  // at a span's first leaf: (max |leaf4.xyz|_1, max |h|) over the span, rounded up
     float* colsf = nullptr;  // float copies of the columns (double inputs), ncol x n
     int32_t* sfirst = nullptr;  // first leaf of each leaf's span (double inputs)
     float* colsr = nullptr;  // columns relative to the span's first leaf, A[i] - A[sfirst[i]] in float, ncol x n
