@@ -289,7 +289,8 @@ __global__ void __launch_bounds__(WALK_THREADS, 1280 / WALK_THREADS) k_collect(c
         for (int s = 0; s < (1 << lspt); ++s) {
             const float4 w = st.W[s];
             const float q[3] = {w.x, w.y, w.z};
-            if (!(lb_d2_pbox(q, pemx, lo, hi) > fmaxf(w.w, r2n))) return true;
+            // (a node whose h is NaN is not left out by it: the box test's answer)
+            if (!(lb_d2_pbox(q, pemx, lo, hi) > (ST == ST_SCATTER ? r2n : fmaxf(w.w, r2n)))) return true;
         }
         return false;
     };

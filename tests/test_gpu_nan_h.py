@@ -66,6 +66,26 @@ def check(orc, ctx, s, dtype, strategy, prec, hmode, hs=None):
 
 
 @pytest.mark.parametrize("prec", PRECS)
+@pytest.mark.parametrize("dtype", [np.float64])
+@pytest.mark.parametrize("strategy", [L.PSB_SCATTER])
+@pytest.mark.parametrize("seed,root_nan", [(57, False), (50, True)])
+def test_particles_without_a_radius(seed, root_nan, strategy, dtype, prec):
+    """Close samples (a tile's samples against every leaf), loose and scattered
+    ones (leaf by leaf, and node tests sample by sample); with a NaN for the
+    largest h of the tree and without."""
+    rng = np.random.default_rng(51)
+    arrs, cols = particles(4000, seed, 0.08, dtype)
+    orc, ctx = pair(arrs, cols, dtype)
+    assert np.isnan(orc.tree()["node_scale"][0]) == root_nan
+    close = tuple((0.35 + 0.3 * rng.random((3, 140_000))).astype(dtype))  # 32 samples a warp
+    loose = tuple(rng.random((3, 700)).astype(dtype))
+    far = tuple(rng.uniform(-1, 2, (3, 700)).astype(dtype))
+    for s in (close, loose, far):
+        check(orc, ctx, s, dtype, strategy, prec, L.PSB_H_CONSTANT, np.array([0.085], dtype=dtype))
+        check(orc, ctx, s, dtype, strategy, prec, L.PSB_H_NEAREST)
+
+
+@pytest.mark.parametrize("prec", PRECS)
 @pytest.mark.parametrize("dtype", [np.float64, np.float32])
 @pytest.mark.parametrize("sign", [1.0, -1.0])
 @pytest.mark.parametrize("strategy", [L.PSB_SCATTER, L.PSB_SYMMETRIC])
