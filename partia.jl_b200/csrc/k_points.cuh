@@ -407,6 +407,7 @@ __global__ void __launch_bounds__(128) k_points(const Args<T> A) {
     const T Kt = (T)tv.Kd;
     const T ra = X<T>::mul(Kt, ha);
     const T ra2 = X<T>::mul(ra, ra);
+    const bool takes = valid && (ST == ST_SCATTER || ra2 == ra2);  // (a radius of NaN: no neighbours)
     if constexpr (BAND) {
         float ralo = 0.f, rahi = 0.f;
         if (ST != ST_SCATTER) {
@@ -760,7 +761,7 @@ __global__ void __launch_bounds__(128) k_points(const Args<T> A) {
             __syncwarp();
             if (nb == NB) flush();  // pair bodies of this span (R0 / R1 belong to it)
         };
-        ok = warp_traverse_spans(start, tv.n, tv.links, tv.escape, valid, node_fn, span_fn, steps) && ok;
+        ok = warp_traverse_spans(start, tv.n, tv.links, tv.escape, takes, node_fn, span_fn, steps) && ok;
         if (nb > 0) flush();
     } else {
         const bool with_cols = (WHAT != WHAT_DIGEST);
@@ -792,7 +793,7 @@ __global__ void __launch_bounds__(128) k_points(const Args<T> A) {
             }
         };
 
-        ok = warp_traverse_spans(start, tv.n, tv.links, tv.escape, valid, node_fn, span_fn, steps) && ok;
+        ok = warp_traverse_spans(start, tv.n, tv.links, tv.escape, takes, node_fn, span_fn, steps) && ok;
     }
 
     // ---- outputs ----

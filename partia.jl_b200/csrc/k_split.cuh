@@ -284,7 +284,7 @@ __global__ void __launch_bounds__(WALK_THREADS, 1280 / WALK_THREADS) k_collect(c
     // such spans a node must also reach one of the samples themselves.
     int misses = 0;  // warp-uniform
     const float pemx = __uint_as_float(__reduce_max_sync(PSB_FULL, valid ? __float_as_uint(pem) : 0u));
-    auto set_sample = [&](float r2) { st.W[lane] = make_float4(valid ? pf[0] : 1e30f, pf[1], pf[2], r2); };
+    auto set_sample = [&](bool on, float r2) { st.W[lane] = make_float4(on ? pf[0] : 1e30f, pf[1], pf[2], r2); };
     auto any_sample = [&](const float4& lo, const float4& hi, float r2n) -> bool {
         for (int s = 0; s < (1 << lspt); ++s) {
             const float4 w = st.W[s];
@@ -336,7 +336,7 @@ __global__ void __launch_bounds__(WALK_THREADS, 1280 / WALK_THREADS) k_collect(c
             int32_t bidx = -1;
             if (valid) nearest_seed<T>(tv, p, best, bidx);
             float bestf = __double2float_ru(best);
-            set_sample(bestf);
+            set_sample(valid, bestf);
             float bmax = __uint_as_float(__reduce_max_sync(PSB_FULL, valid ? __float_as_uint(bestf) : 0u));
             auto node_ok = [&](int ni) -> bool {
                 const float4 lo = __ldg(&tv.node_lo[ni]), hi = __ldg(&tv.node_hi[ni]);
@@ -417,18 +417,21 @@ __global__ void __launch_bounds__(WALK_THREADS, 1280 / WALK_THREADS) k_collect(c
     const T Kt = (T)tv.Kd;
     const T ra = X<T>::mul(Kt, ha);
     const T ra2 = X<T>::mul(ra, ra);
+    // a sample of radius NaN (the nearest particle's h, or none near) has no
+    // neighbours, in the symmetric strategy either (jmax(NaN, r) is NaN)
+    const bool takes = valid && (ST == ST_SCATTER || ra2 == ra2);
     float ra2_hi = 0.f, rahi = 0.f;
     if (ST != ST_SCATTER) {
         rahi = __double2float_ru(fabs((double)ra)) * (1.f + 2.f * U1);
-        ra2_hi = valid ? __double2float_ru((double)ra2) * (1.f + RELM) + 1e-36f : 0.f;
+        ra2_hi = takes ? __double2float_ru((double)ra2) * (1.f + RELM) + 1e-36f : 0.f;
     }
-    // tile-wide maxima (a NaN h, of a set without particles nearby, reaches nothing)
+    // tile-wide maxima (NaN reaches nothing)
     auto warp_max = [&](float v) { return __uint_as_float(__reduce_max_sync(PSB_FULL, v > 0.f ? __float_as_uint(v) : 0u)); };
     const float rahimax = warp_max(rahi);
     float ra2max = warp_max(ra2_hi);
     misses = 0;
     __syncwarp();
-    set_sample(ra2_hi);
+    set_sample(takes, ra2_hi);
 
     // this lane's pair list: the next entry goes to index epos
     uint32_t epos = (uint32_t)bt * (RCAP * 32) + (slot & 31);
@@ -479,7 +482,7 @@ __global__ void __launch_bounds__(WALK_THREADS, 1280 / WALK_THREADS) k_collect(c
         return misses < WALK_MISSES || any_sample(lo, hi, ST == ST_GATHER ? 0.f : hi_r2_node<ST_SCATTER>(0.f, lo.w, tv.Kf));
     };
     auto span_fn = [&](int32_t id) {
-        bool part = valid && nparts > 0 && !dead;
+        bool part = takes && nparts > 0 && !dead;
         if (id < (int32_t)tv.n) {
             const float4 lo = __ldg(&tv.node_lo[id - 1]), hi = __ldg(&tv.node_hi[id - 1]);
             part = part && !(lb_d2_pbox(pf, pem, lo, hi) > hi_r2_node<ST>(ra2_hi, lo.w, tv.Kf));
@@ -515,7 +518,8 @@ __global__ void __launch_bounds__(WALK_THREADS, 1280 / WALK_THREADS) k_collect(c
             const float kb = tv.Kf * L.w;
             L.w = kb * kb;
         } else if (ST != ST_GATHER) {
-            L.w = ex_r2<ST_SCATTER, float>(0.f, L.w, (float)Kt);
+            // (no pair is within a radius of NaN: staged as one that nothing is within)
+            L.w = fmaxf(ex_r2<ST_SCATTER, float>(0.f, L.w, (float)Kt), -1.f);
         }
         const float Ts = (float)ra2;  // the sample's squared radius
         unsigned myacc = 0;

@@ -66,8 +66,8 @@ def check(orc, ctx, s, dtype, strategy, prec, hmode, hs=None):
 
 
 @pytest.mark.parametrize("prec", PRECS)
-@pytest.mark.parametrize("dtype", [np.float64])
-@pytest.mark.parametrize("strategy", [L.PSB_SCATTER])
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("strategy", STRATEGIES)
 @pytest.mark.parametrize("seed,root_nan", [(57, False), (50, True)])
 def test_particles_without_a_radius(seed, root_nan, strategy, dtype, prec):
     """Close samples (a tile's samples against every leaf), loose and scattered
@@ -83,6 +83,18 @@ def test_particles_without_a_radius(seed, root_nan, strategy, dtype, prec):
     for s in (close, loose, far):
         check(orc, ctx, s, dtype, strategy, prec, L.PSB_H_CONSTANT, np.array([0.085], dtype=dtype))
         check(orc, ctx, s, dtype, strategy, prec, L.PSB_H_NEAREST)
+
+
+@pytest.mark.parametrize("prec", PRECS)
+@pytest.mark.parametrize("strategy", STRATEGIES)
+def test_samples_without_a_radius(strategy, prec):
+    rng = np.random.default_rng(52)
+    arrs, cols = particles(4000, 53, 0.08, np.float64, share=0.0)
+    orc, ctx = pair(arrs, cols, np.float64)
+    s = tuple(rng.random((3, 3000)))
+    hs = rng.uniform(0.05, 0.1, 3000)
+    hs[::7] = np.nan
+    check(orc, ctx, s, np.float64, strategy, prec, L.PSB_H_PER_SAMPLE, hs)
 
 
 @pytest.mark.parametrize("prec", PRECS)
