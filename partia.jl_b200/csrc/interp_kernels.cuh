@@ -445,6 +445,7 @@ __global__ void __launch_bounds__(128) k_lines(const Args<T> A) {
     const T Kt = (T)tv.Kd;
     const T ra = X<T>::mul(Kt, ha);
     const T ra2 = X<T>::mul(ra, ra);
+    const bool takes = valid && (ST == ST_SCATTER || ra2 == ra2);  // (a radius of NaN: no neighbours)
     float ra2_hi = 0.f, ra2_lo = 0.f;
     if (BAND && ST != ST_SCATTER) {
         ra2_hi = __double2float_ru((double)ra2) * (1.f + RELM);
@@ -536,7 +537,7 @@ __global__ void __launch_bounds__(128) k_lines(const Args<T> A) {
                 body(lo + j, (CT)r, st.ih[j], st.mr[j], cols);
             }
         };
-        ok = warp_traverse_spans(start, tv.n, tv.links, tv.escape, valid, node_fn, span_fn, steps);
+        ok = warp_traverse_spans(start, tv.n, tv.links, tv.escape, takes, node_fn, span_fn, steps);
     } else {
         auto node_fn = [&](int ni) -> bool {
             ++steps;
@@ -555,7 +556,7 @@ __global__ void __launch_bounds__(128) k_lines(const Args<T> A) {
             const CT s2 = (CT)e2;
             body(li, sqrt(s2 < CT(0) ? CT(0) : s2), CT(1) / (CT)hb, mr, cols);
         };
-        ok = warp_traverse(start, tv.n, tv.left, tv.escape, valid, node_fn, leaf_fn);
+        ok = warp_traverse(start, tv.n, tv.left, tv.escape, takes, node_fn, leaf_fn);
     }
 
     if (valid) {

@@ -262,6 +262,7 @@ __global__ void __launch_bounds__(128, KC <= 1 ? 8 : 6) k_line_tile(const __grid
     if (ST != ST_SCATTER && valid) ha = (A.hmode == PSB_H_PER_SAMPLE) ? A.hs[k] : A.hs[0];
     const double ra = X<double>::mul(tv.Kd, ha);
     const double ra2 = X<double>::mul(ra, ra);
+    const bool takes = valid && (ST == ST_SCATTER || ra2 == ra2);  // (a radius of NaN: no neighbours)
     float ra2_hi = 0.f, ra2_lo = 0.f, ra2max = 0.f;
     if (ST != ST_SCATTER) {
         ra2_hi = __double2float_ru(ra2) * (1.f + RELM) + 1e-36f;
@@ -365,7 +366,7 @@ __global__ void __launch_bounds__(128, KC <= 1 ? 8 : 6) k_line_tile(const __grid
         }
         __syncwarp();
         unsigned acc = 0, maybe = 0;
-        if (valid) {
+        if (takes) {
 #pragma unroll 4
             for (int j = g; j < ns; j += G) {
                 const float fs = line_fs_f32(st.L[j], cf, mf3);

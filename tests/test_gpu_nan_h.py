@@ -122,3 +122,27 @@ def test_edge_of_the_support_beside_them(strategy, sign, dtype, prec):
         ctx.interp_points(*s, CatalogC(scalars=[0], shepard=[0]), strategy=strategy, hmode=L.PSB_H_CONSTANT, hs=hs,
                           prec=prec)
         assert ctx.last_stats.pairs == int(count.sum()), k
+
+
+@pytest.mark.parametrize("prec", PRECS)
+@pytest.mark.parametrize("nl", [300, 20_000])
+@pytest.mark.parametrize("strategy", STRATEGIES)
+def test_lines_without_a_radius(strategy, nl, prec):
+    """Lines and particles with a NaN h: sight lines, and lines that run in tiles."""
+    rng = np.random.default_rng(55)
+    arrs, cols = particles(4000, 56, 0.08, np.float64)
+    orc, ctx = pair(arrs, cols, np.float64)
+    o = rng.uniform(0, 1, (3, nl))
+    d = np.empty((3, nl))
+    d[:] = [[0.0], [0.6], [0.8]]
+    d[:, : nl // 4] = rng.standard_normal((3, nl // 4))
+    d /= np.linalg.norm(d, axis=0)
+    hs = rng.uniform(0.08, 0.1, nl)
+    hs[::7] = np.nan
+    count, _, _ = orc.digest(tuple(o), tuple(d), strategy=strategy, hmode=O.H_PER_SAMPLE, hs=hs)
+    ctx.interp_lines(tuple(o), tuple(d), CatalogC(scalars=[0], shepard=[0]), strategy=strategy,
+                     hmode=L.PSB_H_PER_SAMPLE, hs=hs, prec=prec)
+    assert ctx.last_stats.pairs == int(count.sum())
+    got, _, _ = ctx.digest(tuple(o), tuple(d), strategy=strategy, hmode=L.PSB_H_PER_SAMPLE, hs=hs,
+                            fp32c=prec == L.PSB_PREC_FP32C)
+    assert np.array_equal(got, count)
