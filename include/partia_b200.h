@@ -409,6 +409,14 @@ int psb_test_loop_escapes(psb_ctx* ctx);
  * tiles that do not fit run in the single-kernel walk. */
 int psb_test_adjoint_pool(psb_ctx* ctx, int64_t blocks, int32_t split);
 
+/* No counterpart in the reference.  For tests of the point path's pair lists:
+ * chunks > 0 is the chunk pool's size in the following calls (per batch of
+ * lists; 0: by need again), whose samples of large neighbourhoods beyond it are
+ * summed by the single kernel; refuse is the number of following requests for
+ * list memory that are answered as if the device had no room.  The results do
+ * not depend on the pool. */
+int psb_test_list_pool(psb_ctx* ctx, int64_t chunks, int32_t refuse);
+
 /* ---- interpolation without device allocation -------------------------------- */
 
 /* No counterpart in the reference: an addition of this library.

@@ -447,6 +447,16 @@ PSB_API int psb_test_adjoint_pool(psb_ctx* c, int64_t blocks, int32_t split) {
     return PSB_OK;
 }
 
+PSB_API int psb_test_list_pool(psb_ctx* c, int64_t chunks, int32_t refuse) {
+    if (!c) return PSB_EINVAL;
+    c->err.clear();
+    if (chunks < 0 || chunks > (int64_t(1) << 24) || refuse < 0)
+        return fail(c, PSB_EINVAL, "chunks must be 0 to 2^24, refuse non-negative");
+    c->pool_fixed = chunks;
+    c->pool_refuse = refuse;
+    return PSB_OK;
+}
+
 PSB_API int psb_get_tree(psb_ctx* c, int32_t* root, int32_t* left, int32_t* right, int32_t* escape, int32_t* parent,
                          double* node_min, double* node_max, double* node_scale) {
     if (!c) return PSB_EINVAL;

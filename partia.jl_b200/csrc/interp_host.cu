@@ -109,9 +109,11 @@ static float ms_between(cudaEvent_t a, cudaEvent_t b) {
 
 // Two-kernel point path over batches of tiles: k_collect writes the pair
 // lists of a batch, k_bodies sums them, k_fold adds up the samples of several
-// parts, and k_points takes the tiles that found the chunk pool exhausted.  A
-// batch holds at most SPLIT_BATCH tiles, which bounds the lists' memory at
-// SPLIT_BATCH * RCAP * 32 * 20 bytes (640 MiB) per stream.
+// parts, and k_points takes the samples that found the chunk pool exhausted.  A
+// batch holds at most SPLIT_BATCH tiles, whose lists take SPLIT_BATCH * RCAP *
+// 32 * 20 bytes (640 MiB) per stream, 4 bytes more per entry and column for the
+// FP32C sums of the kernels other than M4 (eshift).  The chunk pool is beside
+// them (list_pool).
 //
 // A direct call (multi_stream) of at least two batches' worth of tiles
 // spreads its batches over up to SPLIT_STREAMS streams (the context stream and
@@ -122,6 +124,46 @@ static float ms_between(cudaEvent_t a, cudaEvent_t b) {
 // to 5.9 ms and the FP64 step from 12.0 to 8.0 ms.
 constexpr int64_t SPLIT_BATCH = 32768;
 constexpr int SPLIT_STREAMS = 4;
+
+// The chunk pool, in chunks per batch of lists.  Most sets need next to none:
+// at 50 to 100 neighbours a sample takes its tile's list alone (uniform and
+// Plummer sets 0 to 0.02 chunks a sample, M4 to M6), clumps 0.05 (densities at
+// the particles) to 0.9 (M4), 1.7 (M5) and 2.8 (M6, points spread about the
+// clumps).  A context's first calls take an eighth of a chunk per sample, at
+// least 65536 (43 to 68 MB); one that runs out leaves the rest to the single kernel, which
+// counts what they lacked, and the following calls' pool has room for it and a
+// quarter more.  It grows to a sixteenth of the memory that was free when the
+// context first asked for more, and after a refused request no further.
+//
+// 1M samples, FP64, four columns: 5.2 GB with eight chunks a sample whatever the
+// set (4M at most), 0.8 GB so.  4096 is the least that a refused allocation leaves.
+constexpr int64_t LIST_POOL_MIN = 4096;
+static int64_t list_pool_first(int64_t lanes, int sets) {
+    return std::max<int64_t>(lanes / 8, 65536 / sets);
+}
+static int64_t list_pool(psb_ctx* c, int64_t lanes, int sets, size_t per_chunk) {
+    if (c->pool_fixed > 0) return c->pool_fixed;
+    if (c->pool_limit == 2) return LIST_POOL_MIN;
+    const int64_t first = list_pool_first(lanes, sets);
+    int64_t want = std::min(c->pool_need, (int64_t)(c->pool_per_sample * (double)lanes));
+    if (want <= first || c->pool_limit == 1) return first;
+    if (c->pool_limit == 0) {
+        size_t free = 0, total = 0;
+        if (cudaMemGetInfo(&free, &total) != cudaSuccess) cudaGetLastError();
+        c->pool_limit = std::max<size_t>(free / 16, 3);
+    }
+    want = std::min<int64_t>(want, (int64_t)(c->pool_limit / (per_chunk * sets)));
+    return std::max(first, std::min<int64_t>(want, (int64_t)OWN_IDX / RCAP));
+}
+// After a call: `need` chunks of one batch, or 0 if no batch ran out.
+static void list_pool_learn(psb_ctx* c, int64_t need) {
+    const int64_t chunks = c->pool_chunks, lanes = c->pool_lanes;
+    c->pool_chunks = c->pool_lanes = 0;
+    if (need <= 0 || lanes <= 0) return;
+    const int64_t want = std::max(need + need / 4, 2 * chunks);  // (at least twice: the count is of one batch)
+    c->pool_need = std::max(c->pool_need, want);
+    c->pool_per_sample = std::max(c->pool_per_sample, (double)want / (double)lanes);
+}
 template <class T>
 static int run_split(psb_ctx* c, Args<T>& A, int prec, int st, int* launches, int what = WHAT_INTERP,
                      int slot_off = 0, bool multi_stream = true) {
@@ -159,26 +201,20 @@ static int run_split(psb_ctx* c, Args<T>& A, int prec, int st, int* launches, in
     A.sp.seq_all = A.src.ns <= SEQ_ALL ? 1 : 0;
     A.sp.kcl = kcl;
     const bool seq = sizeof(T) == 8 && prec == PREC_FP32C;  // samples of several parts go to k_seq
-    // The chunk pool: a quarter of a chunk per sample for the kernels of support 2 h
-    // (neighbourhoods of more than RCAP spans are rare there), one per
-    // sample for M5 and M6, whose ordinary samples often take two parts.
     const int64_t lanes = 32 * B;
-    // For large neighbourhoods eight per sample up to 4M over the streams (5 GB;
-    // the small pool if the device has no room for it), at least 65536, but no more than the samples of a small call can fill (a chunk
-    // holds RCAP spans of the tree).  A call that finds the pool empty sums the
-    // rest in the single kernel: 65,536 samples of 1M particles of which one in
-    // ten has thousands of neighbours take 48 ms with 65536 chunks, 13 with
-    // 262144; 524,288 samples 70 ms with 262144, 42 with 4M.
-    const int64_t most = std::min<int64_t>(lanes, A.src.ns) * (c->n / 256 + 2);
-    unsigned ncap = (unsigned)std::min<int64_t>(
-        std::max<int64_t>(std::max<int64_t>(65536, std::min<int64_t>(4194304 / (multi_stream ? nsets : SPLIT_STREAMS), 8 * lanes)),
-                          A.tv.Kd > 2.0 ? lanes : lanes / 4), most);
+    // bytes of a chunk: its entries, sums and links
+    const size_t per_chunk = (size_t)RCAP * (sizeof(float4) + sizeof(uint32_t) + (shifts ? sizeof(float) * kc : 0)) +
+                             (seq ? sizeof(uint32_t) : sizeof(double) * 2 * nf) + 9;
+    const int sets = multi_stream ? nsets : SPLIT_STREAMS;  // (the chunked host calls run four)
+    int64_t pool = list_pool(c, lanes, sets, per_chunk);
     constexpr unsigned HCAP = 4096;  // samples of a batch for k_heavy (the rest stay in their tiles' walks)
     Lists ls[SPLIT_STREAMS];
-    for (bool retry = true;;) {
+    unsigned ncap = 0;
+    for (;;) {
         // One block for all the streams' lists (slots 96-99): a context's first
         // call pays for the number of allocations.
         const int slot = 96 + (slot_off == 0 ? 0 : (slot_off == 32 ? 1 : (slot_off == 14 ? 2 : 3)));
+        ncap = (unsigned)pool;
         const size_t nent = (size_t)RCAP * 32 * B + (size_t)RCAP * ncap;
         size_t size = 0;
         auto take = [&](size_t bytes) {
@@ -192,13 +228,17 @@ static int run_split(psb_ctx* c, Args<T>& A, int prec, int st, int* launches, in
         const size_t part = take((seq ? sizeof(uint32_t) : sizeof(double) * 2 * nf) * (size_t)ncap);
         const size_t own = take(sizeof(uint32_t) * ncap), next = take(sizeof(int32_t) * ncap), ccnt = take(ncap);
         const size_t hlist = take(sizeof(uint32_t) * HCAP), ovf = take(sizeof(int32_t) * (size_t)B), ctr = take(256 + sizeof(unsigned) * (size_t)B);
-        char* base = (char*)scratch(c, slot, size * nsets);
-        if (!base && retry && ncap > 65536) {
-            retry = false;
-            ncap = 65536;
+        char* base = nullptr;
+        if (c->pool_refuse > 0) --c->pool_refuse;
+        else base = (char*)scratch(c, slot, size * nsets);
+        if (!base) {
+            // no room: the pool a first call takes, then the least, from now on
+            const int64_t first = list_pool_first(lanes, sets), less = pool > first ? first : LIST_POOL_MIN;
+            if (pool <= less) return fail(c, PSB_ENOMEM, "scratch allocation failed (pair lists)");
+            c->pool_limit = pool > first ? 1 : 2;
+            pool = less;
             continue;
         }
-        if (!base) return fail(c, PSB_ENOMEM, "scratch allocation failed (pair lists)");
         for (int k = 0; k < nsets; ++k, base += size) {
             ls[k].ent4 = (float4*)(base + ent4);
             ls[k].emask = (uint32_t*)(base + emask);
@@ -217,6 +257,8 @@ static int run_split(psb_ctx* c, Args<T>& A, int prec, int st, int* launches, in
         }
         break;
     }
+    c->pool_chunks = std::max<int64_t>(c->pool_chunks, ncap);
+    c->pool_lanes = std::max(c->pool_lanes, lanes);
     A.sp.ncap = ncap;
     A.sp.ebase = (uint32_t)((int64_t)RCAP * 32 * B);
     A.sp.fp64 = prec == PREC_FP64 ? 1 : 0;
@@ -236,7 +278,7 @@ static int run_split(psb_ctx* c, Args<T>& A, int prec, int st, int* launches, in
         A.sp.ovf_tiles = ls[k].ovf_tiles; A.sp.ovf_count = ls[k].ctr; A.sp.dead = ls[k].ctr + 64; A.sp.top = ls[k].ctr + 1;
         A.sp.own = ls[k].own; A.sp.next = ls[k].next; A.sp.ccnt = ls[k].ccnt; A.sp.part = ls[k].part;
         A.sp.hcount = ls[k].ctr + 2; A.sp.hlist = ls[k].hlist; A.sp.hcap = HCAP;
-        A.sp.mcount = ls[k].ctr + 3; A.sp.mlist = ls[k].mlist;
+        A.sp.mcount = ls[k].ctr + 3; A.sp.mlist = ls[k].mlist; A.sp.need = ls[k].ctr + 4;
         A.sp.tile0 = t0; A.sp.ntiles = nb;
         const bool dens = what == WHAT_DENSITY;
         PSB_CUDA_TRY(c, launch_split(A, prec, st, kc, SPLIT_WALK, sk), "pair-list kernel launch");
@@ -641,6 +683,7 @@ static int run_typed(psb_ctx* c, const SampleReq& rq, int hmode, const void* hs,
     PSB_CUDA_TRY(c, cudaMemcpyAsync(hst, dstats, sizeof(hst), cudaMemcpyDeviceToHost, s), "stats D2H");
     PSB_CUDA_TRY(c, cudaMemcpyAsync(&herr, c->d_err, sizeof(herr), cudaMemcpyDeviceToHost, s), "error D2H");
     PSB_CUDA_TRY(c, cudaStreamSynchronize(s), "synchronize");
+    list_pool_learn(c, (int64_t)hst[7]);
     if (herr) {
         cudaMemsetAsync(c->d_err, 0, sizeof(unsigned), s);
         cudaStreamSynchronize(s);
@@ -839,6 +882,7 @@ static int run_points_pipelined(psb_ctx* c, const SampleReq& rq, int hmode, cons
     PSB_CUDA_TRY(c, cudaMemcpyAsync(hst, dstats, sizeof(hst), cudaMemcpyDeviceToHost, s), "stats D2H");
     PSB_CUDA_TRY(c, cudaMemcpyAsync(&herr, c->d_err, sizeof(herr), cudaMemcpyDeviceToHost, s), "error D2H");
     PSB_CUDA_TRY(c, cudaStreamSynchronize(s), "synchronize");
+    list_pool_learn(c, (int64_t)hst[7]);
     if (herr) {
         cudaMemsetAsync(c->d_err, 0, sizeof(unsigned), s);
         cudaStreamSynchronize(s);

@@ -71,6 +71,7 @@ struct SplitBufs {
     unsigned* hcount;
     uint32_t* hlist;     // tile in the batch * 32 + lane
     unsigned hcap;
+    unsigned* need;      // chunks that the samples left to the single kernel would have taken (counted if the pool ran out)
     // the samples of several parts for k_seq (FP32C of double particles; null otherwise)
     unsigned* mcount;
     uint32_t* mlist;     // first chunk of each

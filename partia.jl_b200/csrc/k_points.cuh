@@ -459,6 +459,7 @@ __global__ void __launch_bounds__(128) k_points(const Args<T> A) {
     double tot[NF];
     int nent = 0;
     bool folded = false;
+    uint32_t n_ent = 0;  // entries in all
     auto get_part = [&](double* v) {
         if (WHAT == WHAT_DENSITY) {
             v[0] = Dm.get();
@@ -476,6 +477,7 @@ __global__ void __launch_bounds__(128) k_points(const Args<T> A) {
         }
     };
     auto count_entry = [&]() {
+        ++n_ent;
         if (WHAT == WHAT_DIGEST || BAND) return;
         if (nent == RCAP) {
             double v[NF];
@@ -657,6 +659,7 @@ __global__ void __launch_bounds__(128) k_points(const Args<T> A) {
             }
             unc0 = unc1 = unc2 = unc3 = 0;
             n_bodyit += __reduce_max_sync(PSB_FULL, (unsigned)(__popc(acc0) + __popc(acc1) + __popc(acc2) + __popc(acc3)));
+            if (acc0 | acc1 | acc2 | acc3) count_entry();
             // one flattened loop over the pairs of all batched spans, in leaf order
             while (true) {
                 int b;
@@ -848,6 +851,11 @@ __global__ void __launch_bounds__(128) k_points(const Args<T> A) {
         atomicAdd(&A.stats[3], n_spans);
         atomicAdd(&A.stats[4], n_parts);
         atomicAdd(&A.stats[5], n_bodyit);
+    }
+    if (WHAT != WHAT_DIGEST && A.tile_list) {  // what these samples' lists lacked, if it was the pool
+        const unsigned lack = __reduce_add_sync(PSB_FULL, n_ent > RCAP ? (n_ent + RCAP - 1) / RCAP + HEAVY_PARTS : 0u);
+        if (lane == 0 && lack && *A.sp.top > A.sp.ncap)
+            atomicMax(&A.stats[7], (unsigned long long)A.sp.ncap + atomicAdd(A.sp.need, lack) + lack);
     }
     if (!ok && lane == 0) atomicOr(A.err, PSB_DERR_TRAVERSAL);
 }

@@ -83,6 +83,16 @@ struct psb_ctx {
     int64_t adj_blocks = 0;           // list-block pool of the two-kernel point adjoint (grown to the last need)
     int adj_split = 1;                // 0: k_adj_points alone; 2: the pool keeps its size (psb_test_adjoint_pool)
 
+    // chunk pool of the point path's pair lists (run_split): what calls turned
+    // out to need, the bytes it may grow to (0: not asked for yet; after a refused
+    // request 1, no growth, or 2, the least pool), and the last call's pool and samples per batch
+    int64_t pool_need = 0;
+    double pool_per_sample = 0.0;
+    size_t pool_limit = 0;
+    int64_t pool_chunks = 0, pool_lanes = 0;
+    int64_t pool_fixed = 0;  // psb_test_list_pool: the pool's size, kept
+    int pool_refuse = 0;     // and the requests for list memory still to be refused
+
     cudaEvent_t ev[8] = {};
     // copy streams (in, out) and three more compute streams of the chunked
     // host-memory path (created on first use)
