@@ -1277,18 +1277,27 @@ __global__ void __launch_bounds__(128) k_fold(const Args<T> A) {
 // One warp per sample: in FP32C of double particles for the samples of several
 // list parts, whose sums run on through the parts, and in small calls for every
 // sample (seq_all; parts of FP64 and float particles' samples are summed apart,
-// as in k_bodies).  Lane j of an entry evaluates the weights of the entry's
-// leaf j, with k_bodies' arithmetic; then each sum runs through the entry's
-// pairs in leaf order in a lane of its own (4 + 4 kc sums, 4 more with a
-// density gradient, two to a lane past 32).  The sums have the bits of one lane
-// adding pair after pair.
+// as in k_bodies).  A part's pairs are taken 32 at a time, whatever entries they
+// come from: lane j evaluates the weights of pair j, with k_bodies' arithmetic;
+// then each sum runs through those pairs in order in a lane of its own (4 + 4 kc
+// sums, 4 more with a density gradient, two to a lane past 32).  The sums have
+// the bits of one lane adding pair after pair.
+//
+// Bound by the latency of the records and of the compensated chain (four
+// dependent operations a pair).  FP32C of samples of several parts, 4 columns:
+// taken entry by entry, with the lanes of an entry's accepted leaves (some 16 of
+// 32) at work, 524,288 samples of 1922 neighbours on average (a tenth of them
+// have most, up to 45,000) took 82 ms a call, in windows 51; the tiles' walk
+// and single kernel that such samples took before there were parts, 53.  M6: 154, 99,
+// 92; 500,000 points about clumps (M6) 72, 40, 104.  A lane per sample through
+// all its parts: 93 and 163, 90.
 //
 // A small call is as long as its longest lane: 37 points waited 230 us for
-// k_bodies.  With this, 1M uniform particles, scatter, 12 FP64 outputs: 32
-// points take 132 us a call (k_bodies 162), 1024 212 (241), 4096 293 (316),
-// 8192 416 (400), 65,536 1000 (571); the density alone 129 (150), 204 (231),
-// 241 (298), 341 (381), 622 (521).  FP32C and float particles cross between
-// 4096 and 8192 points as well.
+// k_bodies.  1M uniform particles, scatter, 12 FP64 outputs, a call of 32
+// points takes 126 us (k_bodies 170), 1024 202 (241), 4096 274 (317), 8192 366
+// (390), 16,384 420 (418), 65,536 753 (559); the density alone 123 (159), 194
+// (230), 234 (292), 318 (377), 349 (402), 517 (514).  FP32C and float particles
+// cross at 8192 to 16,384 points as well; the line stays below that.
 constexpr int SEQ_COMP = 8;  // weights of a pair: w, w d (3); with a density gradient W, d (3); then the columns, m, m W'
 constexpr int SEQ_ROWS = SEQ_COMP + MAX_KC + 2;
 constexpr int64_t SEQ_ALL = 4096;  // samples of a call up to which k_seq takes all
@@ -1373,13 +1382,39 @@ __global__ void __launch_bounds__(128) k_seq(const __grid_constant__ Args<T> A) 
             const float* esh = !EXS || kc == 0 ? nullptr
                                : chunk < 0 ? sp.eshift + (size_t)(own >> 5) * RCAP * kc * 32 + (own & 31)
                                            : sp.eshift + e0 * kc;
-            for (int e = 0; e < n; ++e) {
-                const float4 q = sp.ent4[e0 + (size_t)e * est];
-                const unsigned m = sp.emask[e0 + (size_t)e * est];
-                const int64_t lo = (int64_t)__float_as_int(q.w);
+            // lane l: entry l of the part, and the pairs up to it
+            float4 en = make_float4(0.f, 0.f, 0.f, 0.f);
+            unsigned em = 0;
+            if (lane < n) {
+                en = sp.ent4[e0 + (size_t)lane * est];
+                em = sp.emask[e0 + (size_t)lane * est];
+            }
+            int upto = __popc(em);
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int t = __shfl_up_sync(PSB_FULL, upto, o);
+                if (lane >= o) upto += t;
+            }
+            const int np = __shfl_sync(PSB_FULL, upto, 31);
+            for (int w = 0; w < np; w += 32) {
+                // lane j: pair w + j of the part, leaf li of entry e
+                const int at = w + lane;
+                int e = 0;
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1)
+                    if (__shfl_sync(PSB_FULL, upto, e + o - 1) <= at) e += o;
+                unsigned m = __shfl_sync(PSB_FULL, em, e);
+                int r = at - (__shfl_sync(PSB_FULL, upto, e) - __popc(m)), bit = 0;  // m's r-th bit
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) {
+                    const int c = __popc(m & ((1u << o) - 1u));
+                    if (r >= c) { r -= c; bit += o; m >>= o; }
+                }
+                const float qx = __shfl_sync(PSB_FULL, en.x, e), qy = __shfl_sync(PSB_FULL, en.y, e),
+                            qz = __shfl_sync(PSB_FULL, en.z, e);
+                const int64_t li = (int64_t)__shfl_sync(PSB_FULL, __float_as_int(en.w), e) + bit;
                 __syncwarp();
-                if ((m >> lane) & 1u) {
-                    const int64_t li = lo + lane;
+                if (at < np) {
                     CT dx, dy, dz, W, c, mr, mb;
                     if constexpr (PREC == PREC_FP64) {
                         const double2 a = __ldg(&tv.leafD[0][li]), b = __ldg(&tv.leafD[1][li]), s = __ldg(&tv.leafD[2][li]);
@@ -1392,9 +1427,9 @@ __global__ void __launch_bounds__(128) k_seq(const __grid_constant__ Args<T> A) 
                     } else {
                         const float4 L = __ldg(&tv.leaf4[li]), K = __ldg(&tv.leafK[li]);
                         if constexpr (BAND) {
-                            dx = __fsub_rn(q.x, L.x);
-                            dy = __fsub_rn(q.y, L.y);
-                            dz = __fsub_rn(q.z, L.z);
+                            dx = __fsub_rn(qx, L.x);
+                            dy = __fsub_rn(qy, L.y);
+                            dz = __fsub_rn(qz, L.z);
                             f32c_pair_weights<ST, KF>(
                                 tv.kern, tv.Kf, qe, dx, dy, dz, ia, sa3, sa4, fa2, ika, (float)ha, K, L.w,
                                 [&]() {
@@ -1441,9 +1476,9 @@ __global__ void __launch_bounds__(128) k_seq(const __grid_constant__ Args<T> A) 
                     }
                 }
                 __syncwarp();
+                const int nj = min(32, np - w);
 #pragma unroll 4
-                for (unsigned b = m; b; b &= b - 1) {
-                    const int j = __ffs(b) - 1;
+                for (int j = 0; j < nj; ++j) {
                     const CT v = rows[ra[0]][j];
                     if (rb[0] < 0) S[0].add(v);
                     else acc_mac(S[0], rows[rb[0]][j], v);

@@ -45,3 +45,38 @@ def test_blocks_take_several_heavy_samples_in_turn(kid, prec):
         for k in range(cat.L):
             assert np.array_equal(got[k], one[k], equal_nan=True), k
         assert np.array_equal(dens, done)
+
+
+@pytest.mark.parametrize("prec", [L.PSB_PREC_FP64, L.PSB_PREC_FP32C])
+@pytest.mark.parametrize("kid", [L.PSB_KERNEL_M4, L.PSB_KERNEL_M5, L.PSB_KERNEL_C4])
+@pytest.mark.parametrize("ns", [40, 6000])
+@pytest.mark.parametrize("kc", [1, 8])
+def test_pair_sums_by_a_warp(kc, ns, kid, prec):
+    """Parts of 1 to 1024 pairs, in windows of 32 pairs whatever entries they
+    come from; up to 40 sums, two to a lane.  Small calls (a warp sums each
+    sample) and the samples of several parts in larger FP32C ones."""
+    rng = np.random.default_rng(43)
+    n = 8000
+    x, y, z = rng.random((3, n))
+    x[:500] = 0.5 + 1e-3 * rng.random(500)  # full spans
+    y[:500] = 0.5 + 1e-3 * rng.random(500)
+    z[:500] = 0.5 + 1e-3 * rng.random(500)
+    m, rho = rng.uniform(0.5, 1.5, n) / n, rng.uniform(0.5, 2.0, n)
+    h = 1.2 * n ** (-1 / 3) * rng.uniform(0.5, 2.0, n)
+    cols = [rng.standard_normal(n) for _ in range(kc)]
+    s = rng.random((3, ns))
+    s[:, ::5] = 0.5 + 1e-2 * rng.standard_normal((3, len(s[0, ::5])))
+    hs = rng.choice([0.005, 0.02, 0.05, 0.1, 0.2], ns)
+    ctx = Context(0)
+    ctx.set_particles(x, y, z, m, h, rho, cols, kernel=kid)
+    ctx.build(want_perm=False)
+    cat = CatalogC(scalars=range(kc), shepard=[0] * kc, grads=[-1, *range(kc)])
+    for strategy in (L.PSB_GATHER, L.PSB_SCATTER, L.PSB_SYMMETRIC):
+        kw = dict(strategy=strategy, hmode=L.PSB_H_PER_SAMPLE, hs=hs, prec=prec)
+        got, dens = ctx.interp_points(*s, cat, **kw), ctx.density(*s, **kw)
+        ctx.extra_flags = L.PSB_FLAG_SINGLE_KERNEL
+        one, done = ctx.interp_points(*s, cat, **kw), ctx.density(*s, **kw)
+        ctx.extra_flags = 0
+        for k in range(cat.L):
+            assert np.array_equal(got[k], one[k], equal_nan=True), (strategy, k)
+        assert np.array_equal(dens, done)
