@@ -555,11 +555,14 @@ static int build_typed(psb_ctx* c) {
     }
     // The float band tests carry absolute floors of 1e-18 (lengths) and 1e-36
     // (squares), so they are exact supersets as long as squares of extents and
-    // radii neither overflow a float nor all lie below those floors; outside
-    // this range the single kernel interpolates.
+    // radii neither overflow a float nor all lie below those floors (the lines'
+    // bounds multiply lengths by the distance of a line's origin too); outside
+    // this range the walk tests in the particles' arithmetic
+    // (k_collect, WIDE) and lines take the general kernel.
     double ext = 0;
     for (int d = 0; d < 3; ++d) ext = std::max(ext, (double)hb[3 + d] - (double)hb[d]);
-    c->band_ok = maxabs <= 1e15 && ext >= 1e-12 && (double)hmax <= 1e15;
+    c->band_ok = maxabs <= 1e18 && ext >= 1e-12 && (double)hmax <= 1e18;
+    c->band_lines = maxabs <= 1e15 && ext >= 1e-12 && (double)hmax <= 1e15;
     // |float(v) - v| <= 2^-24 |v|; the node tests allow twice that
     c->coord_err = (float)(maxabs * 1.1920928955078125e-07);
     c->built = true;

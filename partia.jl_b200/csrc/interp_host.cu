@@ -262,6 +262,7 @@ static int run_split(psb_ctx* c, Args<T>& A, int prec, int st, int* launches, in
     A.sp.ncap = ncap;
     A.sp.ebase = (uint32_t)((int64_t)RCAP * 32 * B);
     A.sp.fp64 = prec == PREC_FP64 ? 1 : 0;
+    A.sp.wide = c->band_ok ? 0 : 1;
     // A warp walks for 32 samples where that leaves enough warps to fill the
     // GPU (4096 of its 7104), for fewer in smaller calls: a call of some
     // probe points is as long as its longest walk.
@@ -563,10 +564,10 @@ static int run_typed(psb_ctx* c, const SampleReq& rq, int hmode, const void* hs,
 
     // ---- launch ----
     if (ns > 0) {
-        const bool split = what != WHAT_DIGEST && !rq.line && c->band_ok && !(flags & PSB_FLAG_SINGLE_KERNEL);
+        const bool split = what != WHAT_DIGEST && !rq.line && !(flags & PSB_FLAG_SINGLE_KERNEL);
         // line integrals of double particles in the float tests' range (a
         // beam's direction must be a unit vector for them)
-        bool line_warp = rq.line && what == WHAT_INTERP && sizeof(T) == 8 && c->band_ok;
+        bool line_warp = rq.line && what == WHAT_INTERP && sizeof(T) == 8 && c->band_lines;
         if (line_warp) {
             A.line_extent = 0.0;
             for (int d = 0; d < 3; ++d) {
@@ -856,7 +857,7 @@ static int run_points_pipelined(psb_ctx* c, const SampleReq& rq, int hmode, cons
             PSB_CUDA_TRY(c, radix_sort_pairs(codes[b], idx[b], cn, c, sort_slot[b], &launches, false, SAMPLE_KEY_BITS), "sample sort");
             S.order = idx[b];
         }
-        const bool split = c->band_ok && !(flags & PSB_FLAG_SINGLE_KERNEL);
+        const bool split = !(flags & PSB_FLAG_SINGLE_KERNEL);
         if (split) {
             rc = run_split(c, A, prec, st, &launches, WHAT_INTERP, list_off[b], false);  // chunks already overlap
             if (rc) return rc;

@@ -58,6 +58,7 @@ struct SplitBufs {
     int64_t tile0;       // first tile of the batch
     int64_t ntiles;      // tiles in the batch
     int fp64;            // the pair sums run in double: entries need no relative positions
+    int wide;            // k_collect tests in the particles' arithmetic (a set outside the float tests' range)
     int lspt;            // k_collect: log2 of the samples a warp walks for (5 but in calls of few samples)
     // the chunk pool
     unsigned* top;       // chunks taken
@@ -235,11 +236,12 @@ __device__ __forceinline__ float lb_d2_pbox(const float pf[3], float pem, float4
     return (tx * tx + ty * ty + tz * tz) * (1.f - RELM);
 }
 
-// upper bound of the node radius^2 (node scale is rounded up; K = support)
+// upper bound of the node radius^2 (node scale is rounded up; K = support; the
+// sum covers squares that fall below the floats' normal range)
 template <int ST> __device__ __forceinline__ float hi_r2_node(float ra2_hi, float scale_up, float Kf) {
     if (ST == ST_GATHER) return ra2_hi;
     float r = Kf * scale_up;
-    float r2 = r * r * (1.f + 2.f * RELM);
+    float r2 = r * r * (1.f + 2.f * RELM) + 1e-36f;
     if (ST == ST_SCATTER) return r2;
     return fmaxf(ra2_hi, r2);
 }

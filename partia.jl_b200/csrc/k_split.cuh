@@ -44,6 +44,12 @@ struct CStage {
         }
     }
 };
+// The walk in the particles' own arithmetic (WIDE): the samples, each with its
+// squared radius or nearest candidate distance (below 0: takes no part).
+template <class T> struct WStage : CStage {
+    T wx[SPAN], wy[SPAN], wz[SPAN], wr2[SPAN];
+    T lx[SPAN], ly[SPAN], lz[SPAN], lr2[SPAN];  // the span's leaves
+};
 __device__ __forceinline__ uint64_t pk(float a, float b) {
     uint64_t r;
     asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
@@ -214,10 +220,18 @@ __device__ __forceinline__ bool window_walk(const TreeView<T>& tv, int32_t* q, N
 // tests then took two leaves an instruction, the sign of d^2 - r^2 as the
 // decision and one tolerance per span, in place of two thresholds compared per
 // leaf: 4.70 -> 4.49 ms (FP32C), 1.66 -> 1.40 ms (FP64).
-template <class T, int ST>
-__global__ void __launch_bounds__(WALK_THREADS, 1280 / WALK_THREADS) k_collect(const __grid_constant__ Args<T> A) {
+//
+// WIDE: particle sets outside the float tests' range (psb_ctx::band_ok), with
+// every test in the reference's arithmetic.  Differences, squares and their sums
+// round monotonically, so the box around the samples is nearer to a node than any
+// of them, and a node than its leaves, in that arithmetic too: no margins.
+// 1M uniform particles, 96^3 grid, FP64 at 4e20: gather 4.5 -> 2.5 ms, symmetric
+// 4.9 -> 2.7 (the single kernel took such sets; in the float tests' range 1.7, 1.8).
+template <class T, int ST, bool WIDE>
+__global__ void __launch_bounds__(WALK_THREADS, (WIDE ? 640 : 1280) / WALK_THREADS)
+    k_collect(const __grid_constant__ Args<T> A) {
     constexpr bool BAND = sizeof(T) == 8;
-    __shared__ CStage stage_all[WALK_THREADS / 32];
+    __shared__ typename std::conditional<WIDE, WStage<T>, CStage>::type stage_all[WALK_THREADS / 32];
     const TreeView<T>& tv = A.tv;
     const int lane = threadIdx.x & 31;
     const int wib = threadIdx.x >> 5;
@@ -236,12 +250,13 @@ __global__ void __launch_bounds__(WALK_THREADS, 1280 / WALK_THREADS) k_collect(c
     const bool valid = k >= 0;
     T p[3] = {T(0), T(0), T(0)}, dd[3];
     if (valid) sample_coords(A.src, k, p, dd);
-    // A sample whose position or h is not finite, or beyond the range of the
-    // float tests, sends its warp's samples to the single kernel.
+    // A sample whose position or h is not finite, or (not WIDE) beyond the range of
+    // the float tests, sends its warp's samples to the single kernel.
     {
-        bool wild = valid && !(fabs((double)p[0]) <= 1e18 && fabs((double)p[1]) <= 1e18 && fabs((double)p[2]) <= 1e18);
+        constexpr double most = WIDE ? 1.7976931348623157e308 : 1e18;
+        bool wild = valid && !(fabs((double)p[0]) <= most && fabs((double)p[1]) <= most && fabs((double)p[2]) <= most);
         if (ST != ST_SCATTER && A.hmode != PSB_H_NEAREST && valid)
-            wild = wild || !(fabs((double)((A.hmode == PSB_H_PER_SAMPLE) ? A.hs[k] : A.hs[0])) <= 1e18);
+            wild = wild || !(fabs((double)((A.hmode == PSB_H_PER_SAMPLE) ? A.hs[k] : A.hs[0])) <= most);
         const bool any_wild = __any_sync(PSB_FULL, wild);
         if (any_wild || !__any_sync(PSB_FULL, valid)) {
             if (mine) {
@@ -295,6 +310,82 @@ __global__ void __launch_bounds__(WALK_THREADS, 1280 / WALK_THREADS) k_collect(c
         return false;
     };
 
+    // WIDE: the samples as they are, the box around them, and the exact squared
+    // distance of that box, and of the samples, from node ni
+    T lob[3] = {T(0), T(0), T(0)}, hib[3] = {T(0), T(0), T(0)};
+    auto wide_max = [&](T v) -> T {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const T u = __shfl_xor_sync(PSB_FULL, v, o);
+            v = u > v ? u : v;
+        }
+        return v;
+    };
+    if constexpr (WIDE) {
+        st.wx[lane] = p[0]; st.wy[lane] = p[1]; st.wz[lane] = p[2];
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            lob[d] = -wide_max(valid ? -p[d] : -(T)INFINITY);
+            hib[d] = wide_max(valid ? p[d] : -(T)INFINITY);
+        }
+    }
+    auto wide_box_d2 = [&](int ni) -> T {
+        T r = T(0);
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            const T a = __ldg(&tv.nmin[d][ni]), b = __ldg(&tv.nmax[d][ni]);
+            const T t = hib[d] < a ? X<T>::sub(a, hib[d]) : (lob[d] > b ? X<T>::sub(lob[d], b) : T(0));
+            r = X<T>::add(r, X<T>::mul(t, t));
+        }
+        return r;
+    };
+    auto wide_any = [&](int ni, bool near) -> bool {
+        if constexpr (WIDE) {
+            const T hn = ST == ST_GATHER || near ? T(0) : __ldg(&tv.nscale[ni]);
+            for (int s = 0; s < (1 << lspt); ++s) {
+                const T r2 = st.wr2[s];
+                const T q[3] = {st.wx[s], st.wy[s], st.wz[s]};
+                if (r2 >= T(0) && !(ex_d2_pbox<T>(q, tv, ni) > (near ? r2 : ex_r2<ST, T>(r2, hn, (T)tv.Kd)))) return true;
+            }
+        }
+        return false;
+    };
+    // The leaves of the span within a taking sample's radius, the particle's
+    // (SA = ST_SCATTER), or the larger one, by the loop with fewer tests.
+    auto wide_leaves = [&](int64_t lo, int cnt, unsigned parts, auto sa) -> unsigned {
+        unsigned mine = 0;
+        if constexpr (WIDE) {
+            constexpr int SA = decltype(sa)::value;
+            auto radius = [&](T r2s, T r2b) { return SA == ST_GATHER ? r2s : (SA == ST_SCATTER ? r2b : jmax(r2s, r2b)); };
+            const bool by_sample = __popc(parts) >= cnt;
+            T lx = T(0), ly = T(0), lz = T(0), r2b = T(0);
+            if (lane < cnt) {
+                lx = __ldg(&tv.x[lo + lane]); ly = __ldg(&tv.y[lo + lane]); lz = __ldg(&tv.z[lo + lane]);
+                if (SA != ST_GATHER) r2b = ex_r2<ST_SCATTER, T>(T(0), __ldg(&tv.h[lo + lane]), (T)tv.Kd);
+            }
+            __syncwarp();
+            if (by_sample) {
+                st.lx[lane] = lx; st.ly[lane] = ly; st.lz[lane] = lz; st.lr2[lane] = r2b;
+                __syncwarp();
+                if ((parts >> lane) & 1u) {
+                    const T r2s = st.wr2[lane];
+#pragma unroll 4
+                    for (int j = 0; j < cnt; ++j)
+                        mine |= (unsigned)(ex_d2_pp<T>(p, st.lx[j], st.ly[j], st.lz[j]) <= radius(r2s, st.lr2[j])) << j;
+                }
+            } else {
+                for (unsigned pp = parts; pp; pp &= pp - 1) {
+                    const int s = __ffs(pp) - 1;
+                    const T q[3] = {st.wx[s], st.wy[s], st.wz[s]};
+                    const unsigned b = __ballot_sync(PSB_FULL, lane < cnt && ex_d2_pp<T>(q, lx, ly, lz) <= radius(st.wr2[s], r2b));
+                    if (lane == s) mine = b;
+                }
+            }
+            __syncwarp();
+        }
+        return mine;
+    };
+
     // the warp anchor (its first sample) and the samples relative to it
     const int first = __ffs(__ballot_sync(PSB_FULL, valid)) - 1;
     const double cw[3] = {__shfl_sync(PSB_FULL, (double)p[0], first), __shfl_sync(PSB_FULL, (double)p[1], first),
@@ -338,13 +429,26 @@ __global__ void __launch_bounds__(WALK_THREADS, 1280 / WALK_THREADS) k_collect(c
             float bestf = __double2float_ru(best);
             set_sample(valid, bestf);
             float bmax = __uint_as_float(__reduce_max_sync(PSB_FULL, valid ? __float_as_uint(bestf) : 0u));
+            T bwide = T(0);  // WIDE: the largest candidate distance (best is one in T)
+            auto set_wide = [&]() {
+                if constexpr (WIDE) {
+                    __syncwarp();
+                    st.wr2[lane] = valid ? (T)best : T(-1);
+                    bwide = wide_max(valid ? (T)best : T(-1));
+                    __syncwarp();
+                }
+            };
+            set_wide();
             auto node_ok = [&](int ni) -> bool {
+                if constexpr (WIDE) return !(wide_box_d2(ni) > bwide) && (misses < WALK_MISSES || wide_any(ni, true));
                 const float4 lo = __ldg(&tv.node_lo[ni]), hi = __ldg(&tv.node_hi[ni]);
                 return !(box_d2(lo, hi) > bmax) && (misses < WALK_MISSES || any_sample(lo, hi, 0.f));
             };
             auto span_fn = [&](int32_t id) {
                 bool part = valid;
-                if (id < (int32_t)tv.n)
+                if (WIDE && id < (int32_t)tv.n)
+                    part = part && !(ex_d2_pbox<T>(p, tv, id - 1) > (T)best);
+                else if (id < (int32_t)tv.n)
                     part = part && !(lb_d2_pbox(pf, pem, __ldg(&tv.node_lo[id - 1]), __ldg(&tv.node_hi[id - 1])) > bestf);
                 const unsigned parts = __ballot_sync(PSB_FULL, part);
                 if (!parts) {
@@ -354,6 +458,15 @@ __global__ void __launch_bounds__(WALK_THREADS, 1280 / WALK_THREADS) k_collect(c
                 int64_t lo;
                 int cnt;
                 span_of(id, lo, cnt);
+                if constexpr (WIDE) {
+                    for (unsigned u = wide_leaves(lo, cnt, parts, std::integral_constant<int, ST_GATHER>()); u; u &= u - 1) {
+                        const int64_t li = lo + __ffs(u) - 1;
+                        const double d2 = (double)ex_d2_pp<T>(p, tv.x[li], tv.y[li], tv.z[li]);
+                        if (d2 < best || (d2 == best && li < bidx)) { best = d2; bidx = (int32_t)li; }
+                    }
+                    set_wide();
+                    return;
+                }
                 // candidates: float d2 not above (sqrt(best) + error)^2, or exactly not above best
                 float thr;
                 float4 L = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -432,6 +545,13 @@ __global__ void __launch_bounds__(WALK_THREADS, 1280 / WALK_THREADS) k_collect(c
     misses = 0;
     __syncwarp();
     set_sample(takes, ra2_hi);
+    const T ra2w = !takes ? T(-1) : (ST == ST_SCATTER ? T(0) : ra2);
+    T ra2wmax = T(-1);  // WIDE: the largest squared radius
+    if constexpr (WIDE) {
+        st.wr2[lane] = ra2w;
+        ra2wmax = wide_max(ra2w);
+        __syncwarp();
+    }
 
     // this lane's pair list: the next entry goes to index epos
     uint32_t epos = (uint32_t)bt * (RCAP * 32) + (slot & 31);
@@ -454,9 +574,13 @@ __global__ void __launch_bounds__(WALK_THREADS, 1280 / WALK_THREADS) k_collect(c
                 acc = 0;
                 ra2_hi = 0.f;
                 st.W[lane].x = 1e30f;
+                if constexpr (WIDE) st.wr2[lane] = T(-1);
             }
             dead = __any_sync(PSB_FULL, acc && nent == RCAP);
-            if (ST == ST_GATHER) ra2max = warp_max(ra2_hi);  // (the other strategies reach nodes by h_b too)
+            if (ST == ST_GATHER) {  // (the other strategies reach nodes by h_b too)
+                if constexpr (WIDE) ra2wmax = wide_max(nparts > 0 ? ra2w : T(-1));
+                else ra2max = warp_max(ra2_hi);
+            }
         }
         if (!acc || dead) return;
         n_pairs += __popc(acc);
@@ -477,13 +601,20 @@ __global__ void __launch_bounds__(WALK_THREADS, 1280 / WALK_THREADS) k_collect(c
 
     auto node_ok = [&](int ni) -> bool {
         if (dead) return false;
+        if constexpr (WIDE) {
+            const T r2 = ST == ST_GATHER ? ra2wmax : ex_r2<ST, T>(ra2wmax, __ldg(&tv.nscale[ni]), Kt);
+            return !(wide_box_d2(ni) > r2) && (misses < WALK_MISSES || wide_any(ni, false));
+        }
         const float4 lo = __ldg(&tv.node_lo[ni]), hi = __ldg(&tv.node_hi[ni]);
         if (box_d2(lo, hi) > hi_r2_node<ST>(ra2max, lo.w, tv.Kf)) return false;
         return misses < WALK_MISSES || any_sample(lo, hi, ST == ST_GATHER ? 0.f : hi_r2_node<ST_SCATTER>(0.f, lo.w, tv.Kf));
     };
     auto span_fn = [&](int32_t id) {
         bool part = takes && nparts > 0 && !dead;
-        if (id < (int32_t)tv.n) {
+        if (WIDE && id < (int32_t)tv.n) {
+            const T r2 = ST == ST_GATHER ? ra2 : ex_r2<ST, T>(ra2, __ldg(&tv.nscale[id - 1]), Kt);
+            part = part && !(ex_d2_pbox<T>(p, tv, id - 1) > r2);
+        } else if (id < (int32_t)tv.n) {
             const float4 lo = __ldg(&tv.node_lo[id - 1]), hi = __ldg(&tv.node_hi[id - 1]);
             part = part && !(lb_d2_pbox(pf, pem, lo, hi) > hi_r2_node<ST>(ra2_hi, lo.w, tv.Kf));
         }
@@ -495,6 +626,12 @@ __global__ void __launch_bounds__(WALK_THREADS, 1280 / WALK_THREADS) k_collect(c
         int64_t lo;
         int cnt;
         span_of(id, lo, cnt);
+        if constexpr (WIDE) {
+            emit(lo, wide_leaves(lo, cnt, parts, std::integral_constant<int, ST>()));
+            ++n_spans;
+            n_parts += __popc(parts);
+            return;
+        }
         // few samples take part: lane j tests leaf j against each of them;
         // otherwise each taking lane tests its sample against every leaf
         const bool by_sample = 3 * __popc(parts) >= 2 * cnt;  // warp-uniform

@@ -186,9 +186,14 @@ static cudaError_t dispatch_split_p(const Args<T>& a, int st, int kc, int pass, 
         kern<<<std::min(2 * 148u, a.sp.hcap), HEAVY_THREADS, HEAVY_SMEM, s>>>(a);
     } else if (pass == SPLIT_WALK) {
         const unsigned gw = (unsigned)(((a.sp.ntiles << (5 - a.sp.lspt)) + WW - 1) / WW);
-        if (st == ST_GATHER) k_collect<T, ST_GATHER><<<gw, WALK_THREADS, 0, s>>>(a);
-        else if (st == ST_SCATTER) k_collect<T, ST_SCATTER><<<gw, WALK_THREADS, 0, s>>>(a);
-        else k_collect<T, ST_SYMMETRIC><<<gw, WALK_THREADS, 0, s>>>(a);
+        auto walk = [&](auto wide) {
+            constexpr bool W = decltype(wide)::value;
+            if (st == ST_GATHER) k_collect<T, ST_GATHER, W><<<gw, WALK_THREADS, 0, s>>>(a);
+            else if (st == ST_SCATTER) k_collect<T, ST_SCATTER, W><<<gw, WALK_THREADS, 0, s>>>(a);
+            else k_collect<T, ST_SYMMETRIC, W><<<gw, WALK_THREADS, 0, s>>>(a);
+        };
+        if (a.sp.wide) walk(std::true_type());
+        else walk(std::false_type());
     } else if (a.sp.seq_all) {  // in FP32C of double particles the fold pass takes all samples
         if constexpr (!SEQ) dispatch_seq<T, P>(a, st, pass == SPLIT_DENSITY, s);
     } else if (pass == SPLIT_DENSITY) {

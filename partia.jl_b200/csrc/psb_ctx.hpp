@@ -47,8 +47,9 @@ struct psb_ctx {
     // FP64 pair sums, per leaf in double: (x, y), (z, 1/h), (sigma/h^3, m/rho)
     double2* leafD[3] = {nullptr, nullptr, nullptr};
     // coordinates and h lie in the range where the float tests of the walk are
-    // proven (build_typed); other sets are interpolated by the single kernel
+    // proven (build_typed); other sets take its form in their own arithmetic
     bool band_ok = false;
+    bool band_lines = false;  // the same for the line kernels
     float2* spanb = nullptr;  // at a span's first leaf: (max |leaf4.xyz|_1, max |h|) over the span, rounded up
     float* colsf = nullptr;  // float copies of the columns (double inputs), ncol x n
     int32_t* sfirst = nullptr;  // first leaf of each leaf's span (double inputs)
