@@ -324,8 +324,7 @@ __global__ void k_span_roots(int64_t n, const int32_t* parent, const int32_t* rl
 template <class T>
 __global__ void k_pack_leaves(int64_t n, const T* x, const T* y, const T* z, const T* h, const T* m, const T* rho,
                               const int32_t* sfirst, float4* leaf4, float* mrho, float* mf, float4* leafK,
-                              float2* spanb, double2* d0, double2* d1, double2* d2, double sigd) {
-    const float sig = (float)sigd;
+                              float2* spanb, float sig) {
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     double ax = 0, ay = 0, az = 0;
@@ -341,15 +340,9 @@ __global__ void k_pack_leaves(int64_t n, const T* x, const T* y, const T* z, con
         r = make_float4((float)x[i], (float)y[i], (float)z[i], (float)h[i]);
     }
     leaf4[i] = r;
-    const double mrd = (double)m[i] / (double)rho[i];
-    const float mr = (float)mrd;
+    const float mr = (float)((double)m[i] / (double)rho[i]);
     mrho[i] = mr;
     mf[i] = (float)m[i];
-    // the same factors for the double pair sums
-    const double ihd = 1.0 / (double)h[i];
-    d0[i] = make_double2((double)x[i], (double)y[i]);
-    d1[i] = make_double2((double)z[i], ihd);
-    d2[i] = make_double2(sigd * ihd * ihd * ihd, mrd);
     // kernel-weight factors of the float pair bodies
     const float ih = 1.f / r.w;
     const float s3 = sig * ih * ih * ih;  // sig = the kernel's 3D norm
@@ -390,8 +383,21 @@ static int pack_columns(psb_ctx* c, cudaStream_t s) {
     return PSB_OK;
 }
 
-// The mass-dependent parts of the leaf records (m/rho, m, leafK.w and leafD[2].y), with
-// k_pack_leaves' arithmetic: a values-only update leaves them as a full
+// Leaf records of the double pair sums.  48 bytes a particle that only calls in
+// FP64 read, so the first of them after a build fills them (double_records).
+template <class T>
+__global__ void k_pack_double(int64_t n, const T* x, const T* y, const T* z, const T* h, const T* m, const T* rho,
+                              double2* d0, double2* d1, double2* d2, double sig) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const double ih = 1.0 / (double)h[i];
+    d0[i] = make_double2((double)x[i], (double)y[i]);
+    d1[i] = make_double2((double)z[i], ih);
+    d2[i] = make_double2(sig * ih * ih * ih, (double)m[i] / (double)rho[i]);
+}
+
+// The mass-dependent parts of the leaf records (m/rho, m, leafK.w, and leafD[2].y
+// if the double records are filled), with k_pack_leaves' and k_pack_double's arithmetic: a values-only update leaves them as a full
 // build over the same particles would.
 template <class T>
 __global__ void k_pack_values(int64_t n, const T* m, const T* rho, float* mrho, float* mf, float4* leafK,
@@ -400,7 +406,7 @@ __global__ void k_pack_values(int64_t n, const T* m, const T* rho, float* mrho, 
     if (i >= n) return;
     const double mrd = (double)m[i] / (double)rho[i];
     const float mr = (float)mrd;
-    d2[i].y = mrd;
+    if (d2) d2[i].y = mrd;
     mrho[i] = mr;
     mf[i] = (float)m[i];
     reinterpret_cast<float*>(leafK + i)[3] = mr;
@@ -513,7 +519,6 @@ static int build_typed(psb_ctx* c) {
     PSB_CUDA_TRY(c, dgrow_t(c, &c->mf, sizeof(float) * n), "cudaMalloc mf");
     PSB_CUDA_TRY(c, dgrow_t(c, &c->leafK, sizeof(float4) * n), "cudaMalloc leafK");
     PSB_CUDA_TRY(c, dgrow_t(c, &c->spanb, sizeof(float2) * n), "cudaMalloc span bounds");
-    for (double2*& d : c->leafD) PSB_CUDA_TRY(c, dgrow_t(c, &d, sizeof(double2) * n), "cudaMalloc double leaf records");
     PSB_CUDA_TRY(c, cudaMemsetAsync(c->spanb, 0, sizeof(float2) * n, s), "memset span bounds");
     if (nint > 0)
         k_pack_nodes<T><<<grid_for(nint), BT, 0, s>>>(nint, (const T*)c->nmin[0], (const T*)c->nmin[1],
@@ -524,8 +529,7 @@ static int build_typed(psb_ctx* c) {
     k_span_roots<<<grid_for(n), BT, 0, s>>>(n, c->parent, c->range_lo, c->range_hi, sfirst);
     k_pack_leaves<T><<<grid_for(n), BT, 0, s>>>(n, (const T*)c->x, (const T*)c->y, (const T*)c->z, (const T*)c->h,
                                                 (const T*)c->m, (const T*)c->rho, sfirst, c->leaf4, c->mrho, c->mf,
-                                                c->leafK, c->spanb, c->leafD[0], c->leafD[1], c->leafD[2],
-                                                kern_norm3(c->kern));
+                                                c->leafK, c->spanb, (float)kern_norm3(c->kern));
     if (sizeof(T) == 8 && c->ncol > 0) {
         const int rc = pack_columns(c, s);
         if (rc != PSB_OK) return rc;
@@ -574,13 +578,29 @@ static int repack_values_typed(psb_ctx* c) {
     const int64_t n = c->n;
     cudaStream_t s = c->stream;
     k_pack_values<T><<<grid_for(n), BT, 0, s>>>(n, (const T*)c->m, (const T*)c->rho, c->mrho, c->mf, c->leafK,
-                                              c->leafD[2]);
+                                              c->leafD_filled ? c->leafD[2] : nullptr);
     if (sizeof(T) == 8 && c->ncol > 0) {
         const int rc = pack_columns(c, s);
         if (rc != PSB_OK) return rc;
     }
     PSB_CUDA_TRY(c, cudaGetLastError(), "value pack kernels");
     return PSB_OK;
+}
+
+template <class T> static int double_records_typed(psb_ctx* c) {
+    const int64_t n = c->n;
+    for (double2*& d : c->leafD) PSB_CUDA_TRY(c, dgrow_t(c, &d, sizeof(double2) * n), "cudaMalloc double leaf records");
+    k_pack_double<T><<<grid_for(n), BT, 0, c->stream>>>(n, (const T*)c->x, (const T*)c->y, (const T*)c->z, (const T*)c->h,
+                                                        (const T*)c->m, (const T*)c->rho, c->leafD[0], c->leafD[1],
+                                                        c->leafD[2], kern_norm3(c->kern));
+    PSB_CUDA_TRY(c, cudaGetLastError(), "double record kernel");
+    c->leafD_filled = true;
+    return PSB_OK;
+}
+
+int double_records(psb_ctx* c) {
+    if (c->leafD_filled) return PSB_OK;
+    return c->dt == PSB_F64 ? double_records_typed<double>(c) : double_records_typed<float>(c);
 }
 
 int repack_values(psb_ctx* c) {

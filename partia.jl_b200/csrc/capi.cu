@@ -93,6 +93,7 @@ cudaError_t dgrow(psb_ctx* c, void** p, size_t bytes) { return grow_buf(c, *p, c
 void reset_tree(psb_ctx* c) {
     c->built = false;
     c->root = 0;
+    c->leafD_filled = false;
 }
 
 void release_buffers(psb_ctx* c) {

@@ -31,7 +31,7 @@ template <class T> TreeView<T> tree_view(psb_ctx* c) {
     v.ncol = c->ncol;
     v.node_lo = c->node_lo; v.node_hi = c->node_hi; v.leaf4 = c->leaf4;
     v.mrho = c->mrho; v.mf = c->mf; v.leafK = c->leafK; v.spanb = c->spanb;
-    for (int d = 0; d < 3; ++d) v.leafD[d] = c->leafD[d];
+    for (int d = 0; d < 3; ++d) v.leafD[d] = c->leafD_filled ? c->leafD[d] : nullptr;
     v.coord_err = c->coord_err;
     v.kern = (int)c->kern;
     v.Kd = kern_support(v.kern);
@@ -451,6 +451,11 @@ static int run_typed(psb_ctx* c, const SampleReq& rq, int hmode, const void* hs,
         if (rc) return rc;
     }
 
+    if (prec == PREC_FP64 && what != WHAT_DIGEST && ns > 0 && !c->leafD_filled) {
+        const int rc = double_records(c);
+        if (rc) return rc;
+        ++launches;
+    }
     A.tv = tree_view<T>(c);
     A.hmode = hmode;
     A.err = c->d_err;
@@ -757,6 +762,10 @@ static int run_points_pipelined(psb_ctx* c, const SampleReq& rq, int hmode, cons
     const bool need_h = (st != ST_SCATTER) && hmode != PSB_H_NEAREST;
     if (need_h && !hs) return fail(c, PSB_EINVAL, "hs must not be NULL for this strategy and hmode");
     const bool ph = need_h && hmode == PSB_H_PER_SAMPLE;
+    if (prec == PREC_FP64 && !c->leafD_filled) {
+        if ((rc = double_records(c))) return rc;
+        ++launches;
+    }
 
     for (auto& q : c->cstream)
         if (!q) PSB_CUDA_TRY(c, cudaStreamCreateWithFlags(&q, cudaStreamNonBlocking), "stream");

@@ -378,8 +378,15 @@ __global__ void __launch_bounds__(128) k_points(const Args<T> A) {
                 if (with_cols) {
                     st.m[lane] = __ldg(&tv.m[li]);
                     if constexpr (PREC == PREC_FP64) {
-                        const double2 s = __ldg(&tv.leafD[2][li]);
-                        st.ib[lane] = __ldg(&tv.leafD[1][li]).y; st.s3[lane] = s.x; st.mr[lane] = s.y;
+                        if (tv.leafD[0]) {
+                            const double2 s = __ldg(&tv.leafD[2][li]);
+                            st.ib[lane] = __ldg(&tv.leafD[1][li]).y; st.s3[lane] = s.x; st.mr[lane] = s.y;
+                        } else {  // no double records (a call that may not allocate): k_pack_double's arithmetic
+                            const double ih = __ddiv_rn(1.0, (double)__ldg(&tv.h[li]));
+                            st.ib[lane] = ih;
+                            st.s3[lane] = __dmul_rn(__dmul_rn(__dmul_rn(tv.sig, ih), ih), ih);
+                            st.mr[lane] = __ddiv_rn((double)__ldg(&tv.m[li]), (double)__ldg(&tv.rho[li]));
+                        }
                     } else {
                         const float4 K = __ldg(&tv.leafK[li]);
                         st.ib[lane] = K.x; st.s3[lane] = K.y; st.mr[lane] = K.w;

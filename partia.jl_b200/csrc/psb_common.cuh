@@ -114,7 +114,7 @@ template <class T> struct TreeView {
     const float* mrho;       // m / rho (float)
     const float* mf;         // m (float)
     const float4* leafK;     // (1/h, sigma/h^3, sigma/h^4, m/rho) in float
-    // FP64 pair sums: (x, y), (z, 1/h) and (sigma/h^3, m/rho) in double
+    // FP64 pair sums: (x, y), (z, 1/h) and (sigma/h^3, m/rho) in double, or null (k_points does without)
     const double2* leafD[3];
     // at the first leaf of every span: (max over the span of |leaf4.x| +
     // |leaf4.y| + |leaf4.z|, max |h|), both rounded up (float error bounds)

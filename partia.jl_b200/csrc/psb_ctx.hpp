@@ -46,6 +46,7 @@ struct psb_ctx {
     float4* leafK = nullptr;  // per leaf (1/h, sigma/h^3, sigma/h^4, m/rho), float
     // FP64 pair sums, per leaf in double: (x, y), (z, 1/h), (sigma/h^3, m/rho)
     double2* leafD[3] = {nullptr, nullptr, nullptr};
+    bool leafD_filled = false;  // for the present tree and values (double_records)
     // coordinates and h lie in the range where the float tests of the walk are
     // proven (build_typed); other sets take its form in their own arithmetic
     bool band_ok = false;
@@ -153,6 +154,8 @@ int build_lbvh(psb_ctx* c);
 // Re-derive the leaf records that depend on m, rho and the columns (after a
 // values-only update of a built LBVH); queued on the context stream.
 int repack_values(psb_ctx* c);
+// Fill the FP64 pair sums' leaf records (leafD) if the build's particles have none yet.
+int double_records(psb_ctx* c);
 // Test hook: turn every end-of-walk escape link into a link to the root.
 int loop_escapes(psb_ctx* c);
 

@@ -55,9 +55,10 @@ def test_ordinary_sets_take_little(ns, prec):
     dens = scratch_of(lambda: ctx.density(*s, strategy=L.PSB_GATHER, hmode=L.PSB_H_NEAREST, prec=prec, out=out))
     # a list of 32 entries of 20 bytes, h, counters and the sort's 24 bytes a sample,
     # an eighth of a chunk (32 * 20 + 16 + 9 bytes), at least 65536 in all; 8 MiB
-    # for the allocator's granularity
+    # for the allocator's granularity; in FP64 the particles' 48 bytes of records
     chunks = max(ns / 8, 65536)
-    assert dens <= (ns * (640 + 13 + 32) + chunks * 665) * 1.02 / MIB + 8
+    records = 48 * 200_000 if prec == L.PSB_PREC_FP64 else 0
+    assert dens <= (ns * (640 + 13 + 32) + chunks * 665 + records) * 1.02 / MIB + 8
 
 
 def dense_samples(ns, share, seed, reach=0.3):
