@@ -967,6 +967,10 @@ __global__ void __launch_bounds__(HEAVY_THREADS, 2) k_heavy(const Args<T> A) {
                     ++w;
                 }
                 if (A.stats && lane == 0) atomicAdd(&A.stats[0], (unsigned long long)n_pairs);
+                if (A.stats && tid == 0) {
+                    atomicAdd(&A.stats[3], (unsigned long long)f);
+                    atomicAdd(&A.stats[4], (unsigned long long)f);
+                }
                 if (sp.mlist && tid == 0) sp.mlist[atomicAdd(sp.mcount, 1u)] = base;
             }
         }
@@ -1284,9 +1288,9 @@ __global__ void __launch_bounds__(BODY_THREADS, 1024 / BODY_THREADS) k_density(c
     constexpr bool BAND = (PREC == PREC_FP32C) && (sizeof(T) == 8);
     const TreeView<T>& tv = A.tv;
     const ListPart Q = list_part(A.sp, nlist);
-    if (Q.n < 0) return;
     const int n = Q.n;
-    const int64_t k = sample_of(A.src, A.sp.tile0 + Q.bt, Q.lane);
+    const int64_t k = n < 0 ? -1 : sample_of(A.src, A.sp.tile0 + Q.bt, Q.lane);
+    const unsigned active = __ballot_sync(PSB_FULL, k >= 0);
     if (k < 0) return;
     T p[3], dd[3];
     sample_coords(A.src, k, p, dd);
@@ -1327,10 +1331,12 @@ __global__ void __launch_bounds__(BODY_THREADS, 1024 / BODY_THREADS) k_density(c
         nx.load(tv, A, lo + j, 0, !unit, Rs, nullptr);
         return true;
     };
+    unsigned n_bodyit = 0;
     bool has = fetch();
     while (has) {
         const PairData<T, PREC, 1> cur = nx;
         has = fetch();
+        ++n_bodyit;
         CT W, c;
         if constexpr (BAND) {
             f32c_pair_weights<ST, KF>(
@@ -1354,6 +1360,8 @@ __global__ void __launch_bounds__(BODY_THREADS, 1024 / BODY_THREADS) k_density(c
     }
     if (Q.dst >= 0) A.sp.part[(Q.chunk < 0 ? A.sp.ncap : 0) + Q.dst] = D.get();
     else A.out[0][k] = (PREC == PREC_FP64) ? (T)D.get() : (T)(CT)D.get();
+    n_bodyit = __reduce_max_sync(active, n_bodyit);
+    if (A.stats && (int)(threadIdx.x & 31) == __ffs(active) - 1) atomicAdd(&A.stats[5], (unsigned long long)n_bodyit);
 }
 
 // The samples of several list parts: the list's sums, then the chunks' in the
@@ -1476,6 +1484,7 @@ __global__ void __launch_bounds__(128) k_seq(const __grid_constant__ Args<T> A) 
         if (WHAT == WHAT_DENSITY) rb[u] = 1;
     }
     const bool two = nsum > 32;
+    unsigned long long n_bodyit = 0;
     // the tiles' lists (seq_all), then the chunks, or (FP32C of double particles) the samples of several parts
     const unsigned n1 = sp.seq_all ? (unsigned)sp.ntiles * 32u : 0u;
     const unsigned nm = min(FOLD ? *sp.top : *sp.mcount, sp.ncap);
@@ -1613,6 +1622,7 @@ __global__ void __launch_bounds__(128) k_seq(const __grid_constant__ Args<T> A) 
                     }
                 }
                 __syncwarp();
+                ++n_bodyit;
                 const int nj = min(32, np - w);
 #pragma unroll 4
                 for (int j = 0; j < nj; ++j) {
@@ -1664,6 +1674,7 @@ __global__ void __launch_bounds__(128) k_seq(const __grid_constant__ Args<T> A) 
         }
         __syncwarp();
     }
+    if (lane == 0 && A.stats && n_bodyit) atomicAdd(&A.stats[5], n_bodyit);
 }
 
 }  // namespace psb

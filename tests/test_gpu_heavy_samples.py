@@ -80,3 +80,27 @@ def test_pair_sums_by_a_warp(kc, ns, kid, prec):
         for k in range(cat.L):
             assert np.array_equal(got[k], one[k], equal_nan=True), (strategy, k)
         assert np.array_equal(dens, done)
+
+
+@pytest.mark.parametrize("prec", [L.PSB_PREC_FP64, L.PSB_PREC_FP32C])
+@pytest.mark.parametrize("ns", [50, 6000])
+@pytest.mark.parametrize("reach", [0.03, 0.3])
+def test_statistics_count_all_forms(reach, ns, prec):
+    """A loop iteration of a warp holds at most 32 pairs, a span test at most 32
+    leaves, whichever kernel takes the sample."""
+    rng = np.random.default_rng(45)
+    n = 20_000
+    x, y, z = rng.random((3, n))
+    one = np.ones(n)
+    ctx = Context(0)
+    ctx.set_particles(x, y, z, one / n, np.full(n, 0.05), one, [one])
+    ctx.build(want_perm=False)
+    s = tuple(rng.random((3, ns)))
+    hs = np.full(ns, 0.03)
+    hs[::10] = reach
+    kw = dict(strategy=L.PSB_GATHER, hmode=L.PSB_H_PER_SAMPLE, hs=hs, prec=prec)
+    for call in (lambda: ctx.interp_points(*s, CatalogC(scalars=[0], shepard=[0]), **kw), lambda: ctx.density(*s, **kw)):
+        call()
+        st = ctx.last_stats
+        assert 0 < st.pairs <= 32 * st.body_iters
+        assert st.pairs <= 32 * st.span_tests and st.spans <= st.span_tests
