@@ -578,7 +578,7 @@ static int repack_values_typed(psb_ctx* c) {
     const int64_t n = c->n;
     cudaStream_t s = c->stream;
     k_pack_values<T><<<grid_for(n), BT, 0, s>>>(n, (const T*)c->m, (const T*)c->rho, c->mrho, c->mf, c->leafK,
-                                              c->leafD_filled ? c->leafD[2] : nullptr);
+                                              c->leafD_filled ? c->leafD + 2 * n : nullptr);
     if (sizeof(T) == 8 && c->ncol > 0) {
         const int rc = pack_columns(c, s);
         if (rc != PSB_OK) return rc;
@@ -589,10 +589,10 @@ static int repack_values_typed(psb_ctx* c) {
 
 template <class T> static int double_records_typed(psb_ctx* c) {
     const int64_t n = c->n;
-    for (double2*& d : c->leafD) PSB_CUDA_TRY(c, dgrow_t(c, &d, sizeof(double2) * n), "cudaMalloc double leaf records");
+    PSB_CUDA_TRY(c, dgrow_t(c, &c->leafD, 3 * sizeof(double2) * n), "cudaMalloc double leaf records");
     k_pack_double<T><<<grid_for(n), BT, 0, c->stream>>>(n, (const T*)c->x, (const T*)c->y, (const T*)c->z, (const T*)c->h,
-                                                        (const T*)c->m, (const T*)c->rho, c->leafD[0], c->leafD[1],
-                                                        c->leafD[2], kern_norm3(c->kern));
+                                                        (const T*)c->m, (const T*)c->rho, c->leafD, c->leafD + n,
+                                                        c->leafD + 2 * n, kern_norm3(c->kern));
     PSB_CUDA_TRY(c, cudaGetLastError(), "double record kernel");
     c->leafD_filled = true;
     return PSB_OK;

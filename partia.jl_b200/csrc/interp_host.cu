@@ -31,7 +31,7 @@ template <class T> TreeView<T> tree_view(psb_ctx* c) {
     v.ncol = c->ncol;
     v.node_lo = c->node_lo; v.node_hi = c->node_hi; v.leaf4 = c->leaf4;
     v.mrho = c->mrho; v.mf = c->mf; v.leafK = c->leafK; v.spanb = c->spanb;
-    for (int d = 0; d < 3; ++d) v.leafD[d] = c->leafD_filled ? c->leafD[d] : nullptr;
+    for (int d = 0; d < 3; ++d) v.leafD[d] = c->leafD_filled ? c->leafD + d * c->n : nullptr;
     v.coord_err = c->coord_err;
     v.kern = (int)c->kern;
     v.Kd = kern_support(v.kern);

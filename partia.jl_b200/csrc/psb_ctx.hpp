@@ -45,7 +45,8 @@ struct psb_ctx {
     float* mrho = nullptr; float* mf = nullptr;
     float4* leafK = nullptr;  // per leaf (1/h, sigma/h^3, sigma/h^4, m/rho), float
     // FP64 pair sums, per leaf in double: (x, y), (z, 1/h), (sigma/h^3, m/rho)
-    double2* leafD[3] = {nullptr, nullptr, nullptr};
+    // (three arrays of n in one allocation)
+    double2* leafD = nullptr;
     bool leafD_filled = false;  // for the present tree and values (double_records)
     // coordinates and h lie in the range where the float tests of the walk are
     // proven (build_typed); other sets take its form in their own arithmetic
