@@ -565,7 +565,13 @@ static int build_typed(psb_ctx* c) {
     // (k_collect, WIDE) and lines take the general kernel.
     double ext = 0;
     for (int d = 0; d < 3; ++d) ext = std::max(ext, (double)hb[3 + d] - (double)hb[d]);
-    c->band_ok = maxabs <= 1e18 && ext >= 1e-12 && (double)hmax <= 1e18;
+    // They also leave too little out where a float's step at the coordinates is
+    // larger than the particles' spacing (a set far from the origin).  1M uniform
+    // particles, 64^3 grid, symmetric, FP64: 0.68 ms at the origin, 0.87 and 2.92
+    // at a step of 1.2 and 12 spacings, 1.04 in the particles' arithmetic; 4740
+    // particles about one point, gather, a step of 2: 0.95 and 0.66.
+    const bool near = sizeof(T) == 4 || maxabs * 1.1920928955078125e-07 * std::cbrt((double)n) <= ext;
+    c->band_ok = maxabs <= 1e18 && ext >= 1e-12 && (double)hmax <= 1e18 && near;
     c->band_lines = maxabs <= 1e15 && ext >= 1e-12 && (double)hmax <= 1e15;
     // |float(v) - v| <= 2^-24 |v|; the node tests allow twice that
     c->coord_err = (float)(maxabs * 1.1920928955078125e-07);

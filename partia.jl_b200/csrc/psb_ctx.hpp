@@ -49,7 +49,7 @@ struct psb_ctx {
     double2* leafD = nullptr;
     bool leafD_filled = false;  // for the present tree and values (double_records)
     // coordinates and h lie in the range where the float tests of the walk are
-    // proven (build_typed); other sets take its form in their own arithmetic
+    // proven and of use (build_typed); other sets take its form in their own arithmetic
     bool band_ok = false;
     bool band_lines = false;  // the same for the line kernels
     float2* spanb = nullptr;  // at a span's first leaf: (max |leaf4.xyz|_1, max |h|) over the span, rounded up

@@ -101,3 +101,25 @@ def test_particles_in_one_place(n, dtype, prec):
         ctx.extra_flags = 0
         for a, b in zip([*got, dens], [*one, done]):
             assert same(a, b, dtype), strategy
+
+
+@pytest.mark.parametrize("prec", [L.PSB_PREC_FP64, L.PSB_PREC_FP32C])
+@pytest.mark.parametrize("shift", [1e5, 3e6, 1e9])
+def test_sets_far_from_the_origin(shift, prec):
+    """A float's step at the coordinates from a fraction of the particles' spacing to
+    far above the set's extent: the oracle's pairs, in about as many span tests as
+    at the origin (where the float tests leave nothing out, every span is tested)."""
+    n, ns = 4000, 3000
+    arrs, cols = particles(n, 75, 1.0, np.float64)
+    s = np.random.default_rng(76).random((3, ns))
+    cat = CatalogC(**SPEC)
+    near = context(arrs, cols)
+    moved = [a + shift for a in arrs[:3]] + arrs[3:]
+    orc, ctx = O.Oracle(*moved, cols=cols), context(moved, cols)
+    for strategy in STRATEGIES:
+        kw = dict(strategy=strategy, prec=prec)
+        near.interp_points(*s, cat, **kw)
+        ctx.interp_points(*(s + shift), cat, **kw)
+        count, _, _ = orc.digest(tuple(s + shift), strategy=strategy)
+        assert ctx.last_stats.pairs == int(count.sum())
+        assert ctx.last_stats.span_tests <= 1.5 * near.last_stats.span_tests
