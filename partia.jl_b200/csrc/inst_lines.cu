@@ -26,6 +26,14 @@ cudaError_t launch_line_tile_d1(const Args<double>&, int, int, bool, cudaStream_
 cudaError_t launch_line_tile(const Args<double>& a, int prec, int st, int kc, bool wide, cudaStream_t s) {
     return prec == PREC_FP64 ? launch_line_tile_d0(a, st, kc, wide, s) : launch_line_tile_d1(a, st, kc, wide, s);
 }
+cudaError_t launch_line_share(const Args<double>& a, int prec, int st, const int32_t* parent, unsigned* together,
+                              cudaStream_t s) {
+    const bool d = prec == PREC_FP64;
+    auto kern = st == ST_GATHER ? k_line_share<ST_GATHER> : (st == ST_SCATTER ? k_line_share<ST_SCATTER> : k_line_share<ST_SYMMETRIC>);
+    kern<<<1, SHARE_THREADS, 0, s>>>(a, parent, d ? LINE_SHARE_FP64 : LINE_SHARE_FP32C,
+                                     d ? LINE_SHARE_TILES_FP64 : LINE_SHARE_TILES_FP32C, together);
+    return cudaGetLastError();
+}
 cudaError_t launch_line_warp(const Args<double>& a, int prec, int st, cudaStream_t s) {
     return prec == PREC_FP64 ? dispatch_line_warp<PREC_FP64>(a, st, s) : dispatch_line_warp<PREC_FP32C>(a, st, s);
 }

@@ -647,19 +647,26 @@ static int run_typed(psb_ctx* c, const SampleReq& rq, int hmode, const void* hs,
                     char* ovf = (char*)scratch(c, 19, 256 + sizeof(int32_t) * (size_t)A.src.ntiles * 8);
                     if (!ovf) return fail(c, PSB_ENOMEM, "scratch allocation failed (line tiles)");
                     PSB_CUDA_TRY(c, cudaMemsetAsync(ovf, 0, sizeof(unsigned), s), "memset line tiles");
-                    A.sp.ovf_count = (unsigned*)ovf;
+                    A.sp.ovf_count = (unsigned*)ovf;  // then whether all tiles run together
                     A.sp.ovf_tiles = (int32_t*)(ovf + 256);
+                    if constexpr (sizeof(T) == 8)
+                        PSB_CUDA_TRY(c, launch_line_share(A, prec, st, c->parent, A.sp.ovf_count + 1, s), "line share kernel launch");
                 }
                 if constexpr (sizeof(T) == 8) {
+                    if (listed) A.tile_lines = wide ? 4 : 32;
                     PSB_CUDA_TRY(c, launch_line_tile(A, prec, st, A.rec.kc, wide, s), "line kernel launch");
+                    if (listed && (wide || prec == PREC_FP32C)) {  // all tiles together: one of the two returns at once
+                        if (prec == PREC_FP64) PSB_CUDA_TRY(c, launch_line_tile(A, prec, st, A.rec.kc, false, s), "line kernel launch");
+                        else PSB_CUDA_TRY(c, launch_lines<T>(A, prec, st, A.rec.kc, what, s), "line kernel launch");
+                        ++launches;
+                    }
                     if (listed) {
                         A.tile_list = A.sp.ovf_tiles;
                         A.tile_count = A.sp.ovf_count;
-                        A.tile_lines = wide ? 4 : 32;
                         PSB_CUDA_TRY(c, launch_line_warp(A, prec, st, s), "line kernel launch");
                     }
                 }
-                launches += listed ? 2 : 1;
+                launches += listed ? 3 : 1;
                 if (costs) PSB_CUDA_TRY(c, cudaStreamWaitEvent(s, c->sev[1], 0), "stream wait");
             } else if (rq.line) {
                 PSB_CUDA_TRY(c, launch_lines<T>(A, prec, st, A.rec.kc, what, s), "line kernel launch");

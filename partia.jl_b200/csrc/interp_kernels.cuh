@@ -387,8 +387,22 @@ template <class CT, int KC> struct LStage {
     CT col[KC][SPAN];
 };
 
-// The general line kernel: float inputs, digests, and sets or frames outside
-// the float tests' range (the others take k_line_tile and k_line_warp).
+// A line that the float tests hold for: a unit direction (mm its square), an
+// origin whose squares do not overflow a float.
+__device__ __forceinline__ bool line_plain(const double o[3], double mm) {
+    return fabs(mm - 1.0) <= 1e-12 && fabs(o[0]) + fabs(o[1]) + fabs(o[2]) <= 1e15;
+}
+// A tile (G = 1), or a group of 32 / G lines, for k_line_warp, whose list has
+// entries of tile_lines lines.
+template <class T> __device__ __forceinline__ void list_lines(const Args<T>& A, int64_t group, int G) {
+    const int n = G == 1 ? 32 / A.tile_lines : 1;
+    const unsigned at = atomicAdd(A.sp.ovf_count, (unsigned)n);
+    for (int q = 0; q < n; ++q) A.sp.ovf_tiles[at + q] = (int32_t)(group * n + q);
+}
+
+// The general line kernel: float inputs, digests, sets or frames outside the
+// float tests' range, and explicit lines that take their tiles together in FP32C
+// (k_line_share; the others take k_line_tile and k_line_warp).
 // FP32C with double inputs: float tests with a double fallback, leaf spans.
 // Otherwise the reference's own arithmetic node by node, so that the pruning
 // decisions (including the rounding of the line-box lower bound) are the
@@ -434,6 +448,15 @@ __global__ void __launch_bounds__(128) k_lines(const Args<T> A) {
     if (valid) sample_coords(A.src, k, o, m);
     const float of[3] = {(float)o[0], (float)o[1], (float)o[2]};
     const float mf3[3] = {(float)m[0], (float)m[1], (float)m[2]};
+    if constexpr (BAND && WHAT == WHAT_INTERP) {
+        if (A.sp.ovf_count) {
+            if (!A.sp.ovf_count[1]) return;
+            if (!__all_sync(PSB_FULL, !valid || line_plain(o, m[0] * m[0] + m[1] * m[1] + m[2] * m[2]))) {
+                if (lane == 0) list_lines(A, tile, 1);
+                return;
+            }
+        }
+    }
     // |o|_1 and the particle coordinate scale S (coord_err = 2^-23 S)
     const float onorm = fabsf(of[0]) + fabsf(of[1]) + fabsf(of[2]);
     const float S = tv.coord_err / U1;

@@ -52,7 +52,7 @@ __global__ void __launch_bounds__(128, 8) k_line_warp(const __grid_constant__ Ar
     // the float node test needs a unit direction and floats that do not
     // overflow; other lines take the reference's arithmetic
     const double mm = md[0] * md[0] + md[1] * md[1] + md[2] * md[2];
-    const bool plain = fabs(mm - 1.0) <= 1e-12 && onorm <= 1e15f;
+    const bool plain = line_plain(od, mm);
     T ha = T(0);
     if (ST != ST_SCATTER) ha = (A.hmode == PSB_H_PER_SAMPLE) ? A.hs[k] : A.hs[0];
     const T Kt = (T)tv.Kd;
@@ -171,6 +171,76 @@ __global__ void __launch_bounds__(128, 8) k_line_warp(const __grid_constant__ Ar
 // another tile go to k_line_warp.  (Parallel beams always run together.)
 constexpr double LINE_TUBE = 1.0;
 
+// Where the lines of a tile meet much the same spans whatever their directions
+// (a small set, large supports), all tiles take their lines together: FP64 here
+// with G = 1, FP32C in k_lines.  A warp per line pays for every span its line
+// meets, a tile for the spans that any of its lines meets, and a tile lasts as
+// long as its walk whether others run beside it or not.  So the tiles are taken
+// from a share of (spans of a line) / (spans of its tile) on, of 32 tiles and 64
+// spans, and of that share times the tiles.  Lines in any direction, ms a call,
+// a warp per line and tiles:
+//                                share     FP64, 100,000 / 500,000 lines      FP32C
+//   Plummer   1000 particles, M4  0.74      3.1   1.0    14.0   3.2       3.0   0.8    13.6  2.4
+//   Plummer   5000, M6            0.57      8.8   3.6    41.6  14.1       8.7   3.0    40.8 10.3
+//   Plummer 30,000, M6            0.27     16.9  17.3    80.9  66.6      16.8  14.0    80.6 50.0
+//   Plummer 30,000, M4            0.18      9.6  13.7    45.8  51.5       9.6  12.0    45.5 41.5
+//   clumps  30,000, M6            0.19      9.9  10.0    46.9  40.8       9.7   6.6    45.6 23.2
+//   clumps  30,000, M4            0.15      6.0   8.8    27.8  35.4       5.8   5.4    26.9 18.6
+//   uniform 30,000, M6            0.12      7.9  14.0    37.4  55.8       7.8  11.7    36.9 42.2
+// and 20,000 lines through the second: 2.2 2.5 (FP64), 2.1 1.9.  (G = 8 takes 1.9
+// to 2.5 times the time of G = 1 on lines apart.)
+constexpr float LINE_SHARE_FP64 = 0.185f, LINE_SHARE_TILES_FP64 = 600.f;
+constexpr float LINE_SHARE_FP32C = 0.14f, LINE_SHARE_TILES_FP32C = 400.f;
+constexpr int SHARE_THREADS = 1024;
+template <int ST>
+__global__ void __launch_bounds__(SHARE_THREADS)
+    k_line_share(const __grid_constant__ Args<double> A, const int32_t* parent, float least, float tiles,
+                 unsigned* together) {
+    const TreeView<double>& tv = A.tv;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    __shared__ float4 lo_s[64], hi_s[64];
+    __shared__ int line_s[SHARE_THREADS / 32], tile_s[SHARE_THREADS / 32];
+    if (threadIdx.x < 64) {  // the box of a leaf's span, and its largest h
+        const int64_t b = (tv.n - 1) * threadIdx.x / 63;
+        const float x = (float)tv.x[b], y = (float)tv.y[b], z = (float)tv.z[b];
+        float4 lo = make_float4(x, y, z, (float)tv.h[b]), hi = lo;
+        for (int32_t p = parent[tv.n + b - 1]; p > 0; p = parent[p - 1]) {
+            const int4 lk = tv.links[p - 1];
+            if (lk.w - lk.z >= SPAN) break;
+            lo = tv.node_lo[p - 1];
+            hi = tv.node_hi[p - 1];
+        }
+        lo_s[threadIdx.x] = lo;
+        hi_s[threadIdx.x] = hi;
+    }
+    __syncthreads();
+    // a warp takes a tile, a line per lane
+    const int64_t k = sample_of(A.src, (A.src.ntiles - 1) * warp / (SHARE_THREADS / 32 - 1), lane);
+    double o[3] = {0.0, 0.0, 0.0}, m[3] = {0.0, 0.0, 1.0}, ha = 0.0;
+    if (k >= 0) {
+        sample_coords(A.src, k, o, m);
+        if (ST != ST_SCATTER) ha = (A.hmode == PSB_H_PER_SAMPLE) ? A.hs[k] : A.hs[0];
+    }
+    const float of[3] = {(float)o[0], (float)o[1], (float)o[2]}, mf[3] = {(float)m[0], (float)m[1], (float)m[2]};
+    const float ra = tv.Kf * (float)ha;
+    int by_line = 0, by_tile = 0;
+    for (int i = 0; i < 64; ++i) {
+        const float4 lo = lo_s[i];
+        const unsigned met = __ballot_sync(
+            PSB_FULL, k >= 0 && lb_d2_line_box(of, mf, 0.f, lo, hi_s[i]) <= hi_r2_node<ST>(ra * ra, lo.w, tv.Kf));
+        by_line += __popc(met);
+        by_tile += met != 0;
+    }
+    if (lane == 0) { line_s[warp] = by_line; tile_s[warp] = by_tile; }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        int l = 0, t = 0;
+        for (int w = 0; w < SHARE_THREADS / 32; ++w) { l += line_s[w]; t += tile_s[w]; }
+        const float share = (float)l / (32.f * (float)max(t, 1));
+        *together = share >= least && share * (float)A.src.ntiles >= tiles;
+    }
+}
+
 // Per-warp shared memory: the leaves of a span that reach the tile.
 template <class CT, int KC> struct TStage {
     float4 L[SPAN];   // offset from the span's first leaf, h
@@ -202,6 +272,7 @@ template <int PREC, int ST, int KC, int G>
 __global__ void __launch_bounds__(128, KC <= 1 ? 8 : 6) k_line_tile(const __grid_constant__ Args<double> A) {
     using CT = typename std::conditional<PREC == PREC_FP64, double, float>::type;
     using Acc = typename std::conditional<PREC == PREC_FP64, PlainD, KahanF>::type;
+    constexpr bool F32C = PREC == PREC_FP32C;
     __shared__ TStage<CT, KC> stage_all[4];
     const TreeView<double>& tv = A.tv;
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
@@ -210,6 +281,8 @@ __global__ void __launch_bounds__(128, KC <= 1 ? 8 : 6) k_line_tile(const __grid
     const int64_t wid = (int64_t)blockIdx.x * (blockDim.x >> 5) + wib;
     int64_t tile = wid / G;
     if (tile >= (A.tile_count ? min((int64_t)*A.tile_count, A.src.ntiles) : A.src.ntiles)) return;
+    // explicit lines, all tiles together: k_lines' (FP32C), or those of G = 1 where both are launched
+    if (A.sp.ovf_count && (A.sp.ovf_count[1] ? F32C || G > 1 : A.tile_lines == 4 && G == 1)) return;
     if (A.tile_list) tile = A.tile_list[tile];  // heavy first, or the heavy ones
     if (A.tile_cost && A.tile_cost[2 * tile] < 0.f) return;  // handed over
     // lane g of the G lanes of this warp's line lane / G
@@ -240,10 +313,10 @@ __global__ void __launch_bounds__(128, KC <= 1 ? 8 : 6) k_line_tile(const __grid
         }
         const double r = (sqrt(e) + A.line_extent * sqrt(e2)) * (1.0 + 1e-12);
         if (A.sp.ovf_count) {
-            const bool near = r <= A.line_tube && fabs(mm - 1.0) <= 1e-12;
+            // (a line's limits are those of the float tests, k_line_warp's `plain`)
+            const bool near = (r <= A.line_tube || A.sp.ovf_count[1]) && line_plain(o, mm);
             if (!__all_sync(PSB_FULL, !valid || near)) {
-                // (a group of 32 / G lines)
-                if (lane == 0) A.sp.ovf_tiles[atomicAdd(A.sp.ovf_count, 1u)] = G == 1 ? (int32_t)tile : (int32_t)wid;
+                if (lane == 0) list_lines(A, G == 1 ? tile : wid, G);
                 return;
             }
         }

@@ -223,5 +223,7 @@ inline cudaError_t launch_split(const Args<float>& a, int prec, int st, int kc, 
 template <class T> cudaError_t launch_lines(const Args<T>& a, int prec, int st, int kc, int what, cudaStream_t s);
 cudaError_t launch_line_tile(const Args<double>& a, int prec, int st, int kc, bool wide, cudaStream_t s);
 cudaError_t launch_line_warp(const Args<double>& a, int prec, int st, cudaStream_t s);
+cudaError_t launch_line_share(const Args<double>& a, int prec, int st, const int32_t* parent, unsigned* together,
+                              cudaStream_t s);
 
 }  // namespace psb
