@@ -397,7 +397,8 @@ __global__ void k_cost_keys(TileCost* cost, int64_t n, bool wide, uint64_t* keys
     const float t = cost[i].tile + cost[n].tile / (float)n, l = cost[i].line + cost[n].line / (float)n;
     keys[i] = 0xFFFFFFFFull - (uint64_t)__float_as_uint(t);
     vals[i] = (uint32_t)i;
-    const float share = cost[n + 1].tile * fmaxf(0.5f / 4736.f, 1.5f / (float)n);
+    const float slots = (float)n / 4736.f, mean = cost[n + 1].tile / (float)n;
+    const float share = mean * (wide ? 1.5f : fmaxf(fmaxf(2.f, 0.5f * slots), fminf(slots, 3.4f)));
     // G = 8: about 1.6 times the instructions, half the time
     const bool by_line = l < (wide ? 1.6f : 1.f) * t || ((wide ? 0.5f : 1.f) * t > share && l < 10.f * t);
     if (list && by_line) {
