@@ -304,7 +304,13 @@ static int run_split(psb_ctx* c, Args<T>& A, int prec, int st, int* launches, in
 // Line calls of fewer tiles than LINE_WARP_TILES take a warp per line
 // (k_line_warp), those of fewer than LINE_WIDE_TILES eight lanes per line
 // (k_line_tile's G): a warp per tile would not fill the GPU (4736 warps at a time).
-constexpr int64_t LINE_WARP_TILES = 512, LINE_WIDE_TILES = 4096;
+// Beams of 1M uniform particles, one lane and eight: 1250 tiles 4.1 3.4 ms, 1682
+// 3.8 4.2, 2048 3.6 4.8, 3740 3.4 7.2; of 3000, 1250 0.39 0.55, so eight lanes
+// only from LINE_WIDE_N particles on.
+constexpr int64_t LINE_WARP_TILES = 512, LINE_WIDE_TILES = 1536, LINE_WIDE_N = 10000;
+// Beams through fewer particles take the tiles in their order: the costs and
+// their sort take 0.07 ms.
+constexpr int64_t LINE_COST_N = 4096;
 
 // Tile costs of parallel beams.  A line's work is the particles whose support
 // it crosses and the spans that hold them, and the lines through dense clumps
@@ -317,14 +323,21 @@ constexpr int64_t LINE_WARP_TILES = 512, LINE_WIDE_TILES = 4096;
 // estimated in instructions from a sample of the particles projected onto the
 // frame plane (a support of more than COST_SPAN tiles either way goes to a
 // term common to all tiles).  A tile takes the cheaper form, but a warp per
-// line also if it alone would take more than half of the beam's share of a
-// warp (4736 run at a time); the tiles run heaviest first.  Only the order
-// and the kernel change, never a result.
+// line also where it would run on alone; the tiles run heaviest first.  Only
+// the order and the kernel change, never a result.
+//
+// Which tiles run on alone (k_cost_keys): a tile beside 31 others of its SM gets
+// a small part of the issue slots, and more as they finish, so it may cost up to
+// 3.4 of the means that a slot takes (4736 run at a time), or 1.2 of them and a
+// fifth of the factor that the lines apart would cost where there are fewer
+// tiles than slots.  FP32C, ms a beam; with everything over 1.5 means handed
+// over, with nothing, and so:
+//   1M uniform, 500^2 8.7 4.0 4.0;  4M Plummer, 700^2 30.4 14.7 14.3, 400^2 12.0 22.6 10.7
+//   4M clumps, 700^2 14.0 22.9 12.2, 400^2 6.9 35.2 9.7;  300,000 clumps, 700^2 4.1 3.0 3.0
 //
 // 8M clump particles, 1024^2 beam: the tile through the densest clump (72,499
 // particles tested, 9 times the mean tile's instructions) ran for 65M cycles
-// of which the others took 34M.  The beam takes 32.1 -> 18.3 ms (FP32C), 2M on
-// 512^2 13.0 -> 7.9 ms, 1M on 512^2 in FP64 30.5 -> 6.1 ms.
+// of which the others took 34M.  The beam takes 32.1 -> 17.9 ms (FP32C).
 constexpr int COST_SPAN = 8;
 constexpr int64_t COST_SAMPLE = int64_t(1) << 18;  // particles looked at, at most twice as many
 struct TileCost { float tile, line; };
@@ -388,7 +401,7 @@ __global__ void k_cost_total(TileCost* cost, int64_t n) {
     }
 }
 // The form of each tile, and keys for an ascending sort that puts the largest
-// cost first.  wide: the tile kernel is its G = 8.  list, count: the tiles
+// cost first.  wide: the tile kernel is its G = 8 (few tiles: over 1.5 means).  list, count: the tiles
 // handed to k_line_warp (null: none); their cost is marked negative.
 __global__ void k_cost_keys(TileCost* cost, int64_t n, bool wide, uint64_t* keys, uint32_t* vals, unsigned* count,
                             int32_t* list) {
@@ -398,7 +411,7 @@ __global__ void k_cost_keys(TileCost* cost, int64_t n, bool wide, uint64_t* keys
     keys[i] = 0xFFFFFFFFull - (uint64_t)__float_as_uint(t);
     vals[i] = (uint32_t)i;
     const float slots = (float)n / 4736.f, mean = cost[n + 1].tile / (float)n;
-    const float share = mean * (wide ? 1.5f : fmaxf(fmaxf(2.f, 0.5f * slots), fminf(slots, 3.4f)));
+    const float share = mean * (wide ? 1.5f : fmaxf(fmaxf(1.2f + 0.2f * l / fmaxf(t, 1.f), 0.5f * slots), fminf(slots, 3.4f)));
     // G = 8: about 1.6 times the instructions, half the time
     const bool by_line = l < (wide ? 1.6f : 1.f) * t || ((wide ? 0.5f : 1.f) * t > share && l < 10.f * t);
     if (list && by_line) {
@@ -598,8 +611,9 @@ static int run_typed(psb_ctx* c, const SampleReq& rq, int hmode, const void* hs,
             if constexpr (sizeof(T) == 8) PSB_CUDA_TRY(c, launch_line_warp(A, prec, st, s), "line kernel launch");
             ++launches;
         } else {
-            const bool wide = line_warp && A.src.ntiles < LINE_WIDE_TILES;
-            const bool costs = rq.line && what == WHAT_INTERP && A.src.kind == SRC_BEAM && (line_warp || A.src.ntiles >= 4096);
+            const bool wide = line_warp && A.src.ntiles < LINE_WIDE_TILES && c->n >= LINE_WIDE_N;
+            const bool costs = rq.line && what == WHAT_INTERP && A.src.kind == SRC_BEAM &&
+                               (line_warp ? c->n >= LINE_COST_N : A.src.ntiles >= 4096);
             if (costs) {
                 const int64_t nt = A.src.ntiles, nbx = (A.src.nx + 7) >> 3, nby = (A.src.ny + 3) >> 2;
                 TileCost* cost = (TileCost*)scratch(c, 93, sizeof(TileCost) * (nt + 2));

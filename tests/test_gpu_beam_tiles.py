@@ -1,5 +1,5 @@
 """Beams over strongly clumped particles: tiles by eight lanes a line (512 to
-4095 tiles) or one (more), those through the clumps handed to a warp per line on
+1535 tiles) or one (more), those through the clumps handed to a warp per line on
 a stream of its own.  Every line has the bits of the same line in a call that
 takes a warp for each, and the pairs are the oracle's.
 """
