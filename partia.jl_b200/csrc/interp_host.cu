@@ -292,7 +292,8 @@ static int run_split(psb_ctx* c, Args<T>& A, int prec, int st, int* launches, in
         F.tile_count = ls[k].ctr;
         F.src.ntiles = nb;  // grid of the list pass: at most nb tiles
         PSB_CUDA_TRY(c, launch_points<T>(F, prec, st, A.rec.kc, what, sk), "overflow pass launch");
-        *launches += seq && A.sp.seq_all ? 4 : 5;
+        const bool chain = seq && !A.sp.seq_all && std::min<int64_t>(nb * 32, ncap) >= (int64_t)CHAIN_SAMPLES;
+        *launches += seq && A.sp.seq_all ? 4 : (chain ? 6 : 5);
     }
     for (int k = 1; k < nsets; ++k) {  // the call's later work on s follows every stream
         PSB_CUDA_TRY(c, cudaEventRecord(c->sev[k], ss[k]), "event");

@@ -1029,6 +1029,22 @@ template <int KC> struct PairData<double, PREC_FP32C, KC> {
     }
 };
 
+// FP32C of double particles, samples of several parts: from CHAIN_SAMPLES of them
+// in a batch on, those of few parts go to k_bodies and k_density with a lane per
+// sample (CHAIN), the others stay k_seq's, whose warp takes a sample in order at
+// a third of the rate but does not wait for the longest of 32.  729,000 grid points,
+// gather, FP32C: 1000 particles of a Plummer sphere 9.0 -> 6.6 ms (M6 18.1 -> 10.9),
+// 20,000 of clumps 8.4 -> 8.4 (M6 29 -> 30); from 16,384 samples on 6.0 and 7.5, but
+// 200,000 points about 300,000 clump particles 5.4 -> 6.7.
+constexpr unsigned CHAIN_SAMPLES = 65536;
+// whether a sample (its first chunk and that chunk's owner word) has more than HEAVY_PARTS parts
+__device__ __forceinline__ bool long_chain(const SplitBufs& sp, int32_t c, uint32_t own) {
+    if (own & OWN_HEAVY) return true;
+    int parts = 1;  // the tile's list
+    for (; c >= 0 && parts <= HEAVY_PARTS; c = sp.next[c]) ++parts;
+    return parts > HEAVY_PARTS;
+}
+
 // The list part of a thread of the pair-sum kernels.  Blocks below `nlist` take
 // some tiles' lists (a warp per tile, one lane per sample), the blocks after
 // them a chunk of the pool per thread.
@@ -1084,7 +1100,30 @@ __device__ __forceinline__ ListPart list_part(const SplitBufs& sp, unsigned nlis
     return q;
 }
 
-template <class T, int PREC, int ST, int KC, int KF, bool DG>
+// The same for sums that run on through a sample's parts with a lane per sample
+// (CHAIN): a thread takes a sample of up to HEAVY_PARTS parts, from its first on.
+__device__ __forceinline__ ListPart chain_part(const SplitBufs& sp) {
+    ListPart q;
+    q.n = -1;
+    q.dst = -1;
+    q.bt = 0;
+    q.lane = threadIdx.x & 31;
+    q.chunk = -1;
+    q.e0 = 0;
+    q.step = 32;
+    const unsigned i = blockIdx.x * blockDim.x + threadIdx.x, count = min(*sp.mcount, sp.ncap);
+    if (i >= count || count < CHAIN_SAMPLES) return q;
+    const int32_t c = (int32_t)sp.mlist[i];
+    const uint32_t w = sp.own[c], o = w & OWN_IDX;
+    if (sp.cnt[o] >= CNT_HEAVY || long_chain(sp, c, w)) return q;  // k_seq's, or the single kernel's
+    q.bt = o >> 5;
+    q.lane = (int)(o & 31);
+    q.e0 = (uint32_t)q.bt * (RCAP * 32) + q.lane;
+    q.n = RCAP;
+    return q;
+}
+
+template <class T, int PREC, int ST, int KC, int KF, bool DG, bool CHAIN = false>
 __global__ void __launch_bounds__(BODY_THREADS, 128 / BODY_THREADS * ((KC <= 4 || (KC == 5 && sizeof(T) == 4)) ? 4 : (KC <= 6 ? 3 : 2)))
     k_bodies(const Args<T> A, unsigned nlist) {
     using CT = typename std::conditional<PREC == PREC_FP64, double, float>::type;
@@ -1093,9 +1132,9 @@ __global__ void __launch_bounds__(BODY_THREADS, 128 / BODY_THREADS * ((KC <= 4 |
     constexpr bool SHIFT = (PREC == PREC_FP32C);
     constexpr bool EXS = BAND && KF == 1;  // column shifts formed in double (span_shift), from k_collect
     const TreeView<T>& tv = A.tv;
-    const ListPart Q = list_part(A.sp, nlist);
+    const ListPart Q = CHAIN ? chain_part(A.sp) : list_part(A.sp, nlist);
     if (!__any_sync(PSB_FULL, Q.n >= 0)) return;
-    const int n = max(Q.n, 0);
+    int n = max(Q.n, 0);
     const int64_t bt = Q.bt;
     const int lane = Q.lane;  // the sample's lane in its tile
     const int64_t tile = A.sp.tile0 + bt;
@@ -1170,7 +1209,8 @@ __global__ void __launch_bounds__(BODY_THREADS, 128 / BODY_THREADS * ((KC <= 4 |
     const float* esh = !EXS ? nullptr
                        : Q.chunk < 0 ? A.sp.eshift + (size_t)bt * RCAP * kc * 32 + lane
                                      : A.sp.eshift + (size_t)Q.e0 * kc;
-    const int est = Q.step;
+    int est = Q.step;
+    int32_t more = CHAIN && n > 0 ? A.sp.head[bt * 32 + lane] : -1;  // CHAIN: the part after this one
     int e = 0;
     unsigned m = 0;
     int64_t lo = 0;
@@ -1181,6 +1221,16 @@ __global__ void __launch_bounds__(BODY_THREADS, 128 / BODY_THREADS * ((KC <= 4 |
     PairData<T, PREC, KC> nx;
     bool hn = false;
     auto fetch = [&]() {
+        if (CHAIN && m == 0 && e == n && more >= 0) {
+            const size_t e0 = (size_t)A.sp.ebase + (size_t)more * RCAP;
+            ent4 = A.sp.ent4 + e0;
+            emask = A.sp.emask + e0;
+            if (EXS) esh = A.sp.eshift + e0 * kc;
+            est = 1;
+            e = 0;
+            n = A.sp.ccnt[more];
+            more = A.sp.next[more];
+        }
         if (m == 0 && e < n) {
             const float4 q = ent4[e * est];
             m = emask[e * est];  // never 0: k_collect writes entries with accepted leaves only
@@ -1281,14 +1331,14 @@ __global__ void __launch_bounds__(BODY_THREADS, 128 / BODY_THREADS * ((KC <= 4 |
 // by span behind its walk with a third of its lanes busy
 // (1M clump particles, gather at the particles: 10.4 ms in k_points; now the
 // walk, k_heavy and this kernel take 3.5 ms).
-template <class T, int PREC, int ST, int KF>
+template <class T, int PREC, int ST, int KF, bool CHAIN = false>
 __global__ void __launch_bounds__(BODY_THREADS, 1024 / BODY_THREADS) k_density(const Args<T> A, unsigned nlist) {
     using CT = typename std::conditional<PREC == PREC_FP64, double, float>::type;
     using Acc = typename std::conditional<PREC == PREC_FP64, PlainD, KahanF>::type;
     constexpr bool BAND = (PREC == PREC_FP32C) && (sizeof(T) == 8);
     const TreeView<T>& tv = A.tv;
-    const ListPart Q = list_part(A.sp, nlist);
-    const int n = Q.n;
+    const ListPart Q = CHAIN ? chain_part(A.sp) : list_part(A.sp, nlist);
+    int n = Q.n;
     const int64_t k = n < 0 ? -1 : sample_of(A.src, A.sp.tile0 + Q.bt, Q.lane);
     const unsigned active = __ballot_sync(PSB_FULL, k >= 0);
     if (k < 0) return;
@@ -1311,7 +1361,8 @@ __global__ void __launch_bounds__(BODY_THREADS, 1024 / BODY_THREADS) k_density(c
     D.zero();
     const float4* ent4 = A.sp.ent4 + Q.e0;
     const uint32_t* emask = A.sp.emask + Q.e0;
-    const int est = Q.step;
+    int est = Q.step;
+    int32_t more = CHAIN ? A.sp.head[Q.bt * 32 + Q.lane] : -1;  // CHAIN: the part after this one
     PairData<T, PREC, 1> nx;
     float Rs[3] = {0.f, 0.f, 0.f};
     int e = 0;
@@ -1319,7 +1370,16 @@ __global__ void __launch_bounds__(BODY_THREADS, 1024 / BODY_THREADS) k_density(c
     int64_t lo = 0;
     auto fetch = [&]() -> bool {
         if (m == 0) {
-            if (e >= n) return false;
+            if (e >= n) {
+                if (!CHAIN || more < 0) return false;
+                const size_t e0 = (size_t)A.sp.ebase + (size_t)more * RCAP;
+                ent4 = A.sp.ent4 + e0;
+                emask = A.sp.emask + e0;
+                est = 1;
+                e = 0;
+                n = A.sp.ccnt[more];
+                more = A.sp.next[more];
+            }
             const float4 q = ent4[e * est];
             m = emask[e * est];
             ++e;
@@ -1435,7 +1495,7 @@ __global__ void __launch_bounds__(128) k_fold(const Args<T> A) {
 // have most, up to 45,000) took 82 ms a call, in windows 51; the tiles' walk
 // and single kernel that such samples took before there were parts, 53.  M6: 154, 99,
 // 92; 500,000 points about clumps (M6) 72, 40, 104.  A lane per sample through
-// all its parts: 93 and 163, 90.
+// all its parts, however many: 93 and 163, 90 (see CHAIN_SAMPLES).
 //
 // A small call is as long as its longest lane: 37 points waited 230 us for
 // k_bodies.  1M uniform particles, scatter, 12 FP64 outputs, a call of 32
@@ -1488,6 +1548,7 @@ __global__ void __launch_bounds__(128) k_seq(const __grid_constant__ Args<T> A) 
     // the tiles' lists (seq_all), then the chunks, or (FP32C of double particles) the samples of several parts
     const unsigned n1 = sp.seq_all ? (unsigned)sp.ntiles * 32u : 0u;
     const unsigned nm = min(FOLD ? *sp.top : *sp.mcount, sp.ncap);
+    const bool chained = !FOLD && !sp.seq_all && nm >= CHAIN_SAMPLES;  // those of few parts are k_bodies'
     const unsigned nw = gridDim.x * (blockDim.x >> 5);
     for (unsigned i = blockIdx.x * (blockDim.x >> 5) + wib; i < n1 + nm; i += nw) {
         const int32_t c0 = i < n1 ? -1 : (FOLD ? (int32_t)(i - n1) : (int32_t)sp.mlist[i - n1]);
@@ -1496,6 +1557,7 @@ __global__ void __launch_bounds__(128) k_seq(const __grid_constant__ Args<T> A) 
         const int cn = sp.cnt[own];
         const bool heavy = i >= n1 && (w0 & OWN_HEAVY) != 0;
         if (cn == CNT_DEAD || (cn == CNT_HEAVY) != heavy) continue;  // warp-uniform
+        if (chained && !long_chain(sp, c0, w0)) continue;
         const int32_t more = i < n1 && cn == RCAP ? sp.head[own] : -1;  // a list of several parts
         if (!FOLD && more >= 0) continue;
         const int64_t k = sample_of(A.src, sp.tile0 + (own >> 5), own & 31);

@@ -159,6 +159,34 @@ static void dispatch_seq(const Args<T>& a, int st, bool density, cudaStream_t s)
     else dispatch_seq_s<T, P, ST_SYMMETRIC>(a, density, s);
 }
 
+// the samples of a few parts with a lane each (CHAIN)
+template <class T, int P, int S, int KF, bool DG>
+static void dispatch_chain_kfd(const Args<T>& a, int kc, unsigned g, cudaStream_t s) {
+    if (kc <= 1) k_bodies<T, P, S, 1, KF, DG, true><<<g, BODY_THREADS, 0, s>>>(a, 0);
+    else if (kc <= 4) k_bodies<T, P, S, 4, KF, DG, true><<<g, BODY_THREADS, 0, s>>>(a, 0);
+    else k_bodies<T, P, S, 8, KF, DG, true><<<g, BODY_THREADS, 0, s>>>(a, 0);
+}
+template <class T, int P, int S, int KF>
+static void dispatch_chain_kf(const Args<T>& a, int kc, bool density, unsigned g, cudaStream_t s) {
+    if (density) k_density<T, P, S, KF, true><<<g, BODY_THREADS, 0, s>>>(a, 0);
+    else if (a.rec.need_dg) dispatch_chain_kfd<T, P, S, KF, true>(a, kc, g, s);
+    else dispatch_chain_kfd<T, P, S, KF, false>(a, kc, g, s);
+}
+template <class T, int P, int S>
+static void dispatch_chain_s(const Args<T>& a, int kc, bool density, unsigned g, cudaStream_t s) {
+    if (a.tv.kern == KERN_M4) dispatch_chain_kf<T, P, S, 0>(a, kc, density, g, s);
+    else dispatch_chain_kf<T, P, S, 1>(a, kc, density, g, s);
+}
+template <class T, int P>
+static void dispatch_chain(const Args<T>& a, int st, int kc, bool density, cudaStream_t s) {
+    const int64_t most = std::min<int64_t>(a.sp.ntiles * 32, a.sp.ncap);
+    if (most < (int64_t)CHAIN_SAMPLES) return;
+    const unsigned g = (unsigned)((most + BODY_THREADS - 1) / BODY_THREADS);
+    if (st == ST_GATHER) dispatch_chain_s<T, P, ST_GATHER>(a, kc, density, g, s);
+    else if (st == ST_SCATTER) dispatch_chain_s<T, P, ST_SCATTER>(a, kc, density, g, s);
+    else dispatch_chain_s<T, P, ST_SYMMETRIC>(a, kc, density, g, s);
+}
+
 template <class T, int P>
 static cudaError_t dispatch_split_p(const Args<T>& a, int st, int kc, int pass, cudaStream_t s) {
     // blocks of the tiles' lists and of the chunk pool
@@ -170,6 +198,7 @@ static cudaError_t dispatch_split_p(const Args<T>& a, int st, int kc, int pass, 
     if (pass == SPLIT_FOLD || pass == SPLIT_FOLD_DENSITY) {
         if constexpr (SEQ) {
             dispatch_seq<T, P>(a, st, pass == SPLIT_FOLD_DENSITY, s);
+            if (!a.sp.seq_all) dispatch_chain<T, P>(a, st, kc, pass == SPLIT_FOLD_DENSITY, s);
         } else {
             if (pass == SPLIT_FOLD_DENSITY) k_fold<T, P, 1, WHAT_DENSITY><<<gf, 128, 0, s>>>(a);
             else if (kc <= 1) k_fold<T, P, 1, WHAT_INTERP><<<gf, 128, 0, s>>>(a);

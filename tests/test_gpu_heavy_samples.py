@@ -104,3 +104,32 @@ def test_statistics_count_all_forms(reach, ns, prec):
         st = ctx.last_stats
         assert 0 < st.pairs <= 32 * st.body_iters
         assert st.pairs <= 32 * st.span_tests and st.spans <= st.span_tests
+
+
+@pytest.mark.parametrize("kid", [L.PSB_KERNEL_M4, L.PSB_KERNEL_M6])
+@pytest.mark.parametrize("kc", [1, 3, 6])
+def test_many_samples_of_a_few_parts(kc, kid):
+    """More samples of several parts in a batch than go to a lane each in FP32C,
+    most of them of two to four parts and some of more: the single kernel's bits."""
+    rng = np.random.default_rng(47)
+    n, ns = 4000, 300_000  # four batches of 75,000
+    x, y, z = rng.random((3, n))
+    m, rho = rng.uniform(0.5, 1.5, n) / n, rng.uniform(0.5, 2.0, n)
+    h = 1.2 * n ** (-1 / 3) * rng.uniform(0.5, 2.0, n)
+    cols = [rng.standard_normal(n) for _ in range(kc)]
+    s = rng.random((3, ns))
+    hs = rng.choice([0.12, 0.16, 0.3], ns, p=[0.5, 0.45, 0.05])
+    ctx = Context(0)
+    ctx.set_particles(x, y, z, m, h, rho, cols, kernel=kid)
+    ctx.build(want_perm=False)
+    cat = CatalogC(scalars=range(kc), shepard=[0] * kc, grads=[-1, kc - 1])
+    kw = dict(strategy=L.PSB_GATHER, hmode=L.PSB_H_PER_SAMPLE, hs=hs, prec=L.PSB_PREC_FP32C)
+    ctx.extra_flags = L.PSB_FLAG_SINGLE_KERNEL
+    one, done = ctx.interp_points(*s, cat, **kw), ctx.density(*s, **kw)
+    pairs = ctx.last_stats.pairs
+    ctx.extra_flags = 0
+    for _ in range(3):  # (the pool grows to the need)
+        got, dens = ctx.interp_points(*s, cat, **kw), ctx.density(*s, **kw)
+        assert ctx.last_stats.pairs == pairs
+        for a, b in zip([*got, dens], [*one, done]):
+            assert np.array_equal(a, b, equal_nan=True)
