@@ -659,21 +659,27 @@ static int run_typed(psb_ctx* c, const SampleReq& rq, int hmode, const void* hs,
                 // tiles of lines together; those of an explicit call that do not
                 // run together come back in a list, one warp per line
                 const bool listed = A.src.kind == SRC_ARRAYS;
+                const float share_tiles = prec == PREC_FP64 ? LINE_SHARE_TILES_FP64 : LINE_SHARE_TILES_FP32C;
+                const bool together = listed && 0.9f * (float)A.src.ntiles >= share_tiles;
                 if (listed) {
                     char* ovf = (char*)scratch(c, 19, 256 + sizeof(int32_t) * (size_t)A.src.ntiles * 8);
                     if (!ovf) return fail(c, PSB_ENOMEM, "scratch allocation failed (line tiles)");
-                    PSB_CUDA_TRY(c, cudaMemsetAsync(ovf, 0, sizeof(unsigned), s), "memset line tiles");
+                    PSB_CUDA_TRY(c, cudaMemsetAsync(ovf, 0, 2 * sizeof(unsigned), s), "memset line tiles");
                     A.sp.ovf_count = (unsigned*)ovf;  // then whether all tiles run together
                     A.sp.ovf_tiles = (int32_t*)(ovf + 256);
                     if constexpr (sizeof(T) == 8)
-                        PSB_CUDA_TRY(c, launch_line_share(A, prec, st, c->parent, A.sp.ovf_count + 1, s), "line share kernel launch");
+                        if (together)
+                            PSB_CUDA_TRY(c, launch_line_share(A, prec, st, c->parent, A.sp.ovf_count + 1, s),
+                                         "line share kernel launch");
                 }
                 if constexpr (sizeof(T) == 8) {
                     if (listed) A.tile_lines = wide ? 4 : 32;
                     PSB_CUDA_TRY(c, launch_line_tile(A, prec, st, A.rec.kc, wide, s), "line kernel launch");
-                    if (listed && (wide || prec == PREC_FP32C)) {  // all tiles together: one of the two returns at once
-                        if (prec == PREC_FP64) PSB_CUDA_TRY(c, launch_line_tile(A, prec, st, A.rec.kc, false, s), "line kernel launch");
-                        else PSB_CUDA_TRY(c, launch_lines<T>(A, prec, st, A.rec.kc, what, s), "line kernel launch");
+                    if (together && (wide || prec == PREC_FP32C)) {  // all tiles together: one of the two returns at once
+                        if (prec == PREC_FP64)
+                            PSB_CUDA_TRY(c, launch_line_tile(A, prec, st, A.rec.kc, false, s), "line kernel launch");
+                        else
+                            PSB_CUDA_TRY(c, launch_lines<T>(A, prec, st, A.rec.kc, what, s), "line kernel launch");
                         ++launches;
                     }
                     if (listed) {
@@ -682,7 +688,7 @@ static int run_typed(psb_ctx* c, const SampleReq& rq, int hmode, const void* hs,
                         PSB_CUDA_TRY(c, launch_line_warp(A, prec, st, s), "line kernel launch");
                     }
                 }
-                launches += listed ? 3 : 1;
+                launches += listed ? (together ? 3 : 2) : 1;
                 if (costs) PSB_CUDA_TRY(c, cudaStreamWaitEvent(s, c->sev[1], 0), "stream wait");
             } else if (rq.line) {
                 PSB_CUDA_TRY(c, launch_lines<T>(A, prec, st, A.rec.kc, what, s), "line kernel launch");

@@ -176,8 +176,9 @@ constexpr double LINE_TUBE = 1.0;
 // with G = 1, FP32C in k_lines.  A warp per line pays for every span its line
 // meets, a tile for the spans that any of its lines meets, and a tile lasts as
 // long as its walk whether others run beside it or not.  So the tiles are taken
-// from a share of (spans of a line) / (spans of its tile) on, of 32 tiles and 64
-// spans, and of that share times the tiles.  Lines in any direction, ms a call,
+// from a share of (spans of a line) / (spans of its tile) on, of 16 tiles and 64
+// spans, and of that share times the tiles (calls of so few tiles that no share
+// below 0.9 is enough are not asked about).  Lines in any direction, ms a call,
 // a warp per line and tiles:
 //                                share     FP64, 100,000 / 500,000 lines      FP32C
 //   Plummer   1000 particles, M4  0.74      3.1   1.0    14.0   3.2       3.0   0.8    13.6  2.4
@@ -191,7 +192,7 @@ constexpr double LINE_TUBE = 1.0;
 // to 2.5 times the time of G = 1 on lines apart.)
 constexpr float LINE_SHARE_FP64 = 0.185f, LINE_SHARE_TILES_FP64 = 600.f;
 constexpr float LINE_SHARE_FP32C = 0.14f, LINE_SHARE_TILES_FP32C = 400.f;
-constexpr int SHARE_THREADS = 1024;
+constexpr int SHARE_THREADS = 512;
 template <int ST>
 __global__ void __launch_bounds__(SHARE_THREADS)
     k_line_share(const __grid_constant__ Args<double> A, const int32_t* parent, float least, float tiles,
