@@ -118,7 +118,7 @@ template <class T> struct Args {
     const int32_t* tile_list;
     const unsigned* tile_count;
     // line calls: the particles' box (centre, largest extent) and the distance
-    // within which a tile's lines run together (k_lines)
+    // within which a tile's lines run together (k_line_tile)
     double line_centre[3];
     double line_extent;
     double line_tube;

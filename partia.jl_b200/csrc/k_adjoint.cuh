@@ -1,6 +1,7 @@
 // k_adjoint.cuh -- adjoint (vector-Jacobian product) kernels for every kernel
-// family: M4's Hessian is written out below (m4_whess), the others take f'/q
-// and its q-derivative from kern_g12; the support K enters every radius rule.
+// family: M4's f'/q and its q-derivative are written out below (m4_wce), the
+// others' come from kern_g12; the Hessian is used in products with vectors only
+// and never formed.  The support K enters every radius rule.
 //
 // For a loss L = sum_s sum_k gout_k(s) out_k(s) the forward pass in FP64 first
 // writes, per sample, the cotangents lambda of its sums (S1, G, Dm, Dg, Sw_c,

@@ -1,9 +1,10 @@
 // k_line_warp.cuh -- line integrals of double particles: one warp per line, and
 // tiles of 32 lines that run together.
 //
-// k_line_warp: lines that do not run together (sight lines in any direction), and calls of
-// too few tiles to fill the GPU, where the tile kernel's union walk visits far
-// more than any one line needs, or leaves most SMs idle.  The warp walks the
+// k_line_warp: lines that do not run together (sight lines in any direction, but
+// see k_line_share), and calls of too few tiles to fill the GPU, where the tile
+// kernel's union walk visits far more than any one line needs, or leaves most
+// SMs idle.  The warp walks the
 // tree for its line 32 nodes at a time (window_walk) and takes a span's leaves
 // one per lane, with the exact inclusion test; each sum then runs through the
 // accepted leaves in leaf order in a lane of its own, so a line's bits are
@@ -18,7 +19,7 @@ namespace psb {
 
 // Bound by issue: about 60 instructions per 32 nodes, 100 per span and 8 per
 // pair.  20,011 sight lines through 300k clump particles (M5, FP64, two
-// scalars): 74 ms in tiles of 32, 3.1 ms here.
+// scalars): 79 ms in tiles of 32, a call takes 3.5 ms with this.
 template <int PREC, int ST>
 __global__ void __launch_bounds__(128, 8) k_line_warp(const __grid_constant__ Args<double> A) {
     using T = double;
@@ -267,8 +268,7 @@ template <class CT, int KC> struct TStage {
 // G = 1: a warp takes a tile, one line per lane.  G = 8: a warp takes four of
 // a tile's lines, eight lanes each (every eighth leaf, every eighth pair, the
 // sums in order in every lane): about 1.5 times the instructions, at an eighth
-// of the time for the longest line.  It serves heavy tiles (k_beam_tile_cost)
-// and calls of few tiles.
+// of the time for the longest line.  It serves calls of few tiles.
 template <int PREC, int ST, int KC, int G>
 __global__ void __launch_bounds__(128, KC <= 1 ? 8 : 6) k_line_tile(const __grid_constant__ Args<double> A) {
     using CT = typename std::conditional<PREC == PREC_FP64, double, float>::type;

@@ -1,9 +1,10 @@
 // k_split.cuh -- the point path over pair lists: walk, then sums.
 //
-// k_collect walks the LBVH for a tile of 32 samples (one warp, the same walk,
-// spans and inclusion decisions as k_points) and records, per sample, the
-// accepted leaves as one entry per span (first leaf, 32-bit mask, the sample's
-// offset from the first leaf) plus the sample's smoothing length.  It keeps no accumulators, so it runs with few registers.
+// k_collect walks the LBVH for a tile of 32 samples (one warp, 32 nodes a step,
+// with the spans and inclusion decisions of k_points) and records, per sample,
+// the accepted leaves as one entry per span (first leaf, 32-bit mask, the
+// sample's offset from the first leaf) plus the sample's smoothing length.  It
+// keeps no accumulators, so it runs with few registers.
 // k_bodies then evaluates the kernel weights and sums of every recorded pair:
 // each lane runs through a list part (a sample's list in its tile, or one of
 // its chunks) in one flattened loop, so a warp iteration does 32 pair bodies

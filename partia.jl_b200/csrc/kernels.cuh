@@ -4,7 +4,7 @@
 // (KernelFunctionValid), the 3D norm (KernelFunctionnorm(K, Val(3), T)) and
 // f, f' of the dimensionless kernel (and f'/q with its q-derivative for the
 // adjoint).  Ids follow psb_kernel.  M4 keeps its own functions (m4_fdf,
-// m4_fdf_edge in interp.cuh, m4_whess in k_adjoint.cuh).
+// m4_fdf_edge in interp.cuh, m4_wce in k_adjoint.cuh).
 #pragma once
 
 namespace psb {
