@@ -1,7 +1,9 @@
-"""The FP64 pair sums' leaf records: filled by the first FP64 call after a build.
+"""The FP64 pair sums' leaf records: filled by the first FP64 call after a build,
+of sets of up to 2^20 particles by the build.
 
-Contexts that only run FP32C hold none; results do not depend on when they were
-filled, nor on whether a call found them (the call that may not allocate).
+Contexts of larger sets that only run FP32C hold none; results do not depend on
+when they were filled, nor on whether a call found them (the call that may not
+allocate).
 """
 import ctypes as C
 
@@ -48,9 +50,10 @@ def test_only_fp64_calls_hold_them():
 
 
 @pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("n", [20_000, 1_100_000])
 @pytest.mark.parametrize("kid", [L.PSB_KERNEL_M4, L.PSB_KERNEL_C2])
-def test_results_do_not_depend_on_when_they_were_filled(kid, dtype):
-    n, ns = 20_000, 3000
+def test_results_do_not_depend_on_when_they_were_filled(n, kid, dtype):
+    ns = 3000
     arrs, cols = arrays(n, 83, dtype)
     rng = np.random.default_rng(84)
     s = [torch.tensor(a.astype(dtype), device="cuda") for a in rng.random((3, ns))]
@@ -75,7 +78,7 @@ def test_results_do_not_depend_on_when_they_were_filled(kid, dtype):
     ctx = Context(0)
     ctx.set_particles(*arrs, cols=cols, kernel=kid)
     perm, *_ = ctx.build()
-    bare = without(ctx)  # no records yet
+    bare = without(ctx)  # no records yet, of the larger sets
     first = fields(ctx)
     held = without(ctx)  # with them
     assert equal(bare, held)
